@@ -146,6 +146,27 @@ def load() -> C.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (_host.so, csrc/lf_host.cpp), bound to the loaded kernel library."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(
+                "loopfuse_b200/_host.so is missing or does not fit this PyTorch: build it with "
+                f"`python -m loopfuse_b200.build`. There is no fallback implementation. ({e})"
+            ) from e
+        module.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in EXPORTS},
+                    check)
+        _host = module
+    return _host
+
+
 class LfError(RuntimeError):
     pass
 

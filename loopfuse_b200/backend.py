@@ -21,13 +21,13 @@ from __future__ import annotations
 
 import dataclasses
 import os
-from functools import partial
 from typing import Any, Callable, Optional
 
 import torch
 from torch._functorch.aot_autograd import aot_module_simplified
+from torch._subclasses import FakeTensor
 
-from . import functional as F
+from . import _native, functional as F
 from .capture import analyse_graph, evaluate_scalar
 from .spec import (AttentionSpec, MASK_CAUSAL, MASK_CAUSAL_WINDOW, MASK_NONE, MOD_MUL, ScalarExpr,
                    ScoreMod, TILE_K, TILE_Q, skip_table)
@@ -89,7 +89,6 @@ class CompiledAttention:
         self.debug = _flag("DEBUG")
         self.check_status = self.debug or _flag("LF_CHECK_STATUS")
         self._plans: dict = {}
-        self._prepared: dict = {}
         self._status: dict = {}
 
     # -- binding -------------------------------------------------------------------------
@@ -172,6 +171,12 @@ class CompiledAttention:
                              spec.mask_kind)
 
     # -- launch --------------------------------------------------------------------------
+    def dispatcher(self):
+        """The native callable of the graph: finds the bound call for the arguments' sizes (the
+        first time through ``bind``) and launches it. ``__call__`` is the same in Python, for the
+        runs that print or check something around the launch."""
+        return _native.host().Dispatcher(self.bind)
+
     def _status_for(self, device) -> Optional[torch.Tensor]:
         if not self.check_status:
             return None
@@ -180,20 +185,17 @@ class CompiledAttention:
             st = self._status[device] = F.new_status(device)
         return st
 
-    def _prepared_prefill(self, plan: AttentionPlan, q, k, v, status) -> "F.PreparedPrefill":
-        """Prefill launches bound to (buffers, plan): a loop that calls the compiled function on
-        the same buffers pays the argument marshalling once."""
-        key = (q.data_ptr(), k.data_ptr(), v.data_ptr(), q.shape, k.shape, q.stride(),
-               k.stride(), v.stride(), id(plan))
-        prep = self._prepared.get(key)
-        if prep is None:
-            if len(self._prepared) >= 16:
-                self._prepared.clear()
-            prep = F.PreparedPrefill(q, k, v, scale=plan.scale, mods=plan.mods,
-                                     mask_kind=plan.mask_kind, window=plan.window,
-                                     status=status)
-            self._prepared[key] = prep
-        return prep
+    def bind(self, *args: Any):
+        """A native call for the sizes of ``args`` (what the dispatcher keeps per set of sizes)."""
+        plan, spec = self.plan(list(args)), self.spec
+        kind = {"decode": 1, "paged_decode": 2}.get(plan.kernel, 0)
+        at = (spec.q, spec.k.placeholder, spec.v.placeholder, spec.k.block_table,
+              spec.v.block_table, spec.q_bias, spec.score_bias, spec.out_bias, spec.q_pe,
+              spec.k_pe)
+        bias_pos = self._bias_pos(plan) if spec.score_bias is not None else -1
+        return _native.host().Call(kind, tuple(-1 if i is None else i for i in at), plan.scale,
+                                   plan.mods, plan.mask_kind, plan.window, bias_pos,
+                                   self.workspace)
 
     def __call__(self, *flat_args: Any):
         args = list(flat_args)
@@ -265,9 +267,9 @@ class CompiledAttention:
             if spec.out_bias is not None:
                 F.add_bf16(out, args[spec.out_bias], out=out)
         else:
-            k, v = args[spec.k.placeholder], args[spec.v.placeholder]
-            out = torch.empty((plan.B, plan.Hq, plan.Sq, plan.D), dtype=q.dtype, device=q.device)
-            self._prepared_prefill(plan, q, k, v, status).run(out)
+            out = F.prefill_attention(
+                q, args[spec.k.placeholder], args[spec.v.placeholder], scale=plan.scale,
+                mods=plan.mods, mask_kind=plan.mask_kind, window=plan.window, status=status)
         self._check(status, plan)
         return (out,)
 
@@ -294,5 +296,34 @@ def loopfuse_backend(gm, sample_inputs, mode="max-autotune", **kwargs):
 
     ``mode`` is accepted for compatibility; the kernels are hand-tuned, nothing is autotuned.
     """
-    compiler = partial(loopfuse_compiler, mode=mode, **kwargs)
-    return aot_module_simplified(gm, sample_inputs, fw_compiler=compiler)
+    made = []
+
+    def compiler(graph, inputs):
+        made.append(loopfuse_compiler(graph, inputs, mode=mode, **kwargs))
+        return made[-1]
+
+    compiled = aot_module_simplified(gm, sample_inputs, fw_compiler=compiler)
+    if len(made) == 1 and _is_plain(gm, sample_inputs, made[0]):
+        return made[0].dispatcher()
+    return compiled
+
+
+_PLAIN_TENSORS = (torch.Tensor, torch.nn.Parameter, FakeTensor)
+
+
+def _is_plain(gm, sample_inputs, attention: CompiledAttention) -> bool:
+    """Whether the AOT wrapper around ``attention`` does nothing per call, so that the graph's
+    callable can be the native dispatcher itself (the wrapper costs a small call as much as its
+    launch): an inference graph of plain tensors and scalars that takes no parameters of its own
+    and returns one fresh tensor."""
+    if attention.analysis_only or attention.check_status:
+        return False
+    if list(gm.parameters()) or list(gm.buffers()):
+        return False
+    for t in sample_inputs:
+        if isinstance(t, torch.Tensor) and (t.requires_grad or type(t) not in _PLAIN_TENSORS):
+            return False
+    outputs = [n for n in gm.graph.nodes if n.op == "output"][0].args[0]
+    return (len(outputs) == 1 and outputs[0].op != "placeholder"
+            and len(attention.placeholders) == len(sample_inputs)
+            and sum(n.op == "placeholder" for n in gm.graph.nodes) == len(sample_inputs))

@@ -1,4 +1,5 @@
-"""Build liblf_sm100.so (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Build liblf_sm100.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and _host.so
+(the native host path of the tensor-level entry points) with the host compiler.
 
 Usage: ``python -m loopfuse_b200.build [--force] [--verbose] [--debug-bounds]``. The build needs
 only nvcc; it cross-compiles on hosts without a GPU. The library is written next to this file so
@@ -35,6 +36,11 @@ def fingerprint_files() -> list[Path]:
     public header. A change to any of them forces a rebuild."""
     files = set(CSRC.glob("*.cu")) | set(CSRC.glob("*.cuh")) | set(CSRC.glob("*.h"))
     return sorted(files) + [PUBLIC_HEADER]
+
+
+HOST_SOURCE = CSRC / "lf_host.cpp"
+HOST_PATH = PKG_DIR / "_host.so"
+HOST_STAMP_PATH = CSRC / ".build_stamp_host"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -98,7 +104,38 @@ def build_native(force: bool = False, verbose: bool = False,
     return lib_path
 
 
+def build_host(force: bool = False) -> Path:
+    """Compile lf_host.cpp against the installed PyTorch's headers; skip when unchanged."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    h = hashlib.sha256(torch.__version__.encode())
+    for path in (HOST_SOURCE, PUBLIC_HEADER):
+        h.update(path.read_bytes())
+    if (not force and HOST_PATH.exists() and HOST_STAMP_PATH.exists()
+            and HOST_STAMP_PATH.read_text() == h.hexdigest()):
+        return HOST_PATH
+    cuda = Path(_nvcc()).resolve().parents[1] / "include"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + sysconfig.get_paths()["include"], "-isystem", str(cuda)]
+    for inc in include_paths():
+        cmd += ["-isystem", inc]
+    cmd += [str(HOST_SOURCE), "-o", str(HOST_PATH)]
+    for lib in library_paths():
+        cmd += ["-L" + lib, "-Wl,-rpath," + lib]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    out = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if out.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SOURCE.name}:\n{out.stdout}")
+    HOST_STAMP_PATH.write_text(h.hexdigest())
+    return HOST_PATH
+
+
 if __name__ == "__main__":
     path = build_native(force="--force" in sys.argv, verbose="--verbose" in sys.argv,
                         debug_bounds="--debug-bounds" in sys.argv)
     print(path)
+    print(build_host(force="--force" in sys.argv))
