@@ -1,0 +1,28 @@
+"""The running-max prefill kernel takes exp2 against the reference a row already has and looks for
+a block's maximum only when a row sum leaves its range: rows whose later keys score far above (and
+far below) everything before, at sizes around the tile edges and on both sides of the rule that
+gives a CTA one query tile or two."""
+import pytest
+import torch
+
+from loopfuse_b200 import functional as F, spec as S
+from oracle import attention_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-2
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("gain", [0.0, 3.0, 40.0])
+@pytest.mark.parametrize("B,H,S_", [(1, 2, 127), (1, 3, 449), (4, 20, 257)])
+def test_rows_whose_later_keys_score_far_above_the_first(B, H, S_, D, gain):
+    g = torch.Generator().manual_seed(3)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    q, k, v = mk(B, H, S_, D), mk(B, H, S_, D), mk(B, H, S_, D)
+    k[:, :, S_ // 2:] *= gain      # 40: logits of +-300 in the log2 domain after blocks of +-6
+    st = F.new_status("cuda")
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
+                              mask_kind=S.MASK_CAUSAL, status=st)
+    F.check_status(st)
+    want = O.attention_ref(q, k, v, mask="causal", batch_chunk=B)
+    assert (out.float().cpu() - want).abs().max().item() <= TOL
