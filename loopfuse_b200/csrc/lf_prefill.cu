@@ -1088,7 +1088,11 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   static thread_local int sm_count = 0;
   if (sm_count == 0) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   PrefillParams pp = p;
-  pp.single = (p.n_qtiles > 1 && static_cast<int64_t>(pairs) * p.Hq * B < sm_count) ? 1 : 0;
+  // One query tile per CTA only where all the tiles are resident at once, one per SM. (With more
+  // tiles than SMs the second wave cost more than pairs do: 7 tiles x 32 heads, 4096 keys, D = 128:
+  // 102 us as 224 single tiles, 71 us as 128 pairs.)
+  pp.single =
+      (p.n_qtiles > 1 && static_cast<int64_t>(p.n_qtiles) * p.Hq * B <= sm_count) ? 1 : 0;
   dim3 grid(pp.single ? p.n_qtiles : pairs, p.Hq, B);
   // (without a second score product the two extra maps are never read)
   prefill_kernel<D, MODE, PE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mqpe ? *mqpe : mq,
