@@ -62,6 +62,14 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
   return r;
 }
 
+// 32 bytes (a whole sector) per thread, read once.
+__device__ __forceinline__ void ldg_stream_32(const void* p, uint32_t* r) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "l"(p));
+}
+
 // 16-byte asynchronous copy global -> shared (bypasses L1), grouped per thread.
 __device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* gmem_src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gmem_src)

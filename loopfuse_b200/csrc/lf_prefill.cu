@@ -76,6 +76,9 @@ constexpr int kModeGeneric = 2;  // logit2 = mods(raw * a) * c2
 // row sum.
 constexpr int kModeBounded = 3;
 constexpr float kBoundedMaxC2 = 80.f;
+// logit2 = (raw * a + bias) * c2: the usual biased attention, a scale and an additive score bias with
+// nothing behind it. (Any other chain around a bias is generic.)
+constexpr int kModeBias = 4;
 
 // Division by a divisor fixed at launch time: q = (mulhi(n, mul) + n) >> shift (Granlund &
 // Montgomery's round-up method; exact for every 0 <= n < 2^31). The item decode of the
@@ -116,6 +119,7 @@ struct PrefillParams {
   const __nv_bfloat16* bias;  // additive score bias [B, Hq, Sq, Skv] (generic mode only) or null
   int64_t bias_stride[3];
   int32_t bias_pos;           // the bias is added after this many ops of `mods`
+  int32_t bias_sectors;       // bias rows are 32-byte aligned
   int32_t* status;
   int32_t* dbg_ranges;
   // Persistent (bounded-mode) kernel only: the work queue.
@@ -584,6 +588,32 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       float l_run = 0.f;
       bool ok = true;
       const int nblk = hi_t[t] - lo_t[t];
+      // Bias mode: this row's 64 bias values of a block (128 contiguous bytes) are requested a block
+      // ahead, so that their latency lies under the exp2 pass and the hand-shake; read when the
+      // scores were there, they cost a round trip to HBM per block. (Rows past Sq read the last
+      // row; both are clipped later. A block that crosses Skv is read value by value on the spot.)
+      [[maybe_unused]] uint32_t bq[32];
+      [[maybe_unused]] const __nv_bfloat16* brow =
+          MODE == kModeBias ? p.bias + b * p.bias_stride[0] + h * p.bias_stride[1] +
+                                  static_cast<int64_t>(min(grow, p.Sq - 1)) * p.bias_stride[2]
+                            : nullptr;
+      auto request_bias = [&](int k) {
+        const int col = (lo_t[t] + k) * kTileK;
+        if (k >= nblk || col + kTileK > p.Skv ||
+            !LF_BOUNDS(col >= 0 && b < static_cast<int>(gridDim.z) && h < p.Hq, p.status, 61))
+          return;
+        if (p.bias_sectors) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) ldg_stream_32(brow + col + i * 16, &bq[i * 8]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 v4 = *reinterpret_cast<const uint4*>(brow + col + i * 8);
+            bq[4 * i] = v4.x; bq[4 * i + 1] = v4.y; bq[4 * i + 2] = v4.z; bq[4 * i + 3] = v4.w;
+          }
+        }
+      };
+      if constexpr (MODE == kModeBias) request_bias(0);
       for (int k = 0; k < nblk; ++k) {
         const int c0 = (lo_t[t] + k) * kTileK;
         const int buf = k & 1;
@@ -604,6 +634,30 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         const int rel_hi = c_hi - c0;  // [rel_lo, rel_hi]
         const bool masked = rel_lo > 0 || rel_hi < kTileK - 1;
 
+        if constexpr (MODE == kModeBias) {
+          if (c0 + kTileK > p.Skv) {
+            const int whole = (p.Skv - c0) >> 3;  // 8-column groups; the next one crosses Skv
+            uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (c0 + whole * 8 + e < p.Skv)
+                w[e >> 1] |= static_cast<uint32_t>(__bfloat16_as_ushort(brow[c0 + whole * 8 + e]))
+                             << ((e & 1) * 16);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              uint4 v4 = make_uint4(w[0], w[1], w[2], w[3]);  // (columns past Skv are masked)
+              if (i < whole) v4 = *reinterpret_cast<const uint4*>(brow + c0 + i * 8);
+              bq[4 * i] = v4.x; bq[4 * i + 1] = v4.y; bq[4 * i + 2] = v4.z; bq[4 * i + 3] = v4.w;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            uint32_t& s0 = sr[i >> 4][(2 * i) & 31];
+            uint32_t& s1 = sr[i >> 4][(2 * i + 1) & 31];
+            s0 = __float_as_uint(fmaf(__uint_as_float(s0), p.a, bf16lo_to_f32(bq[i])));
+            s1 = __float_as_uint(fmaf(__uint_as_float(s1), p.a, bf16hi_to_f32(bq[i])));
+          }
+        }
         if constexpr (MODE == kModeGeneric) {
           // The chain is interpreted op by op over the row's 64 scores in registers: one
           // (warp-uniform) dispatch per op and block, not one per score - the reference compiles
@@ -683,7 +737,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // of the exp2 (causal B=1 Hq=32 Hkv=8 S=8192 D=128 559 -> 528 us, B=2 Hq=32 S=4096 D=64
         // 294 -> 267 us). The row sum is taken over the bf16-rounded values that the PV product sees, so that numerator and
         // denominator carry the same rounding.
-        if constexpr (MODE == kModeNone) {
+        if constexpr (MODE == kModeNone || MODE == kModeBias) {
           if (!__any_sync(0xffffffffu, masked || m_used == -INFINITY)) {
             float fs[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t pk[32];
@@ -701,6 +755,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             const float sum = (fs[0] + fs[1]) + (fs[2] + fs[3]);
             if (!__any_sync(0xffffffffu, !(sum <= kFastRowSum))) {
               l_run += sum;
+              if constexpr (MODE == kModeBias) request_bias(k + 1);
               tmem_st_32x32b_x32(s_addr, pk);
               tmem_wait_st();
               tc_fence_before();
@@ -873,6 +928,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         }
         const float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
         l_run = l_run * alpha + psum;
+        if constexpr (MODE == kModeBias) request_bias(k + 1);
         tmem_st_32x32b_x32(s_addr, pk);
         tmem_wait_st();
         tc_fence_before();
@@ -1303,6 +1359,9 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   }
   p.bias = static_cast<const __nv_bfloat16*>(a->score_bias);
   p.bias_pos = a->bias_pos;
+  p.bias_sectors = reinterpret_cast<uintptr_t>(a->score_bias) % 32 == 0 &&
+                   a->bias_stride[0] % 16 == 0 && a->bias_stride[1] % 16 == 0 &&
+                   a->bias_stride[2] % 16 == 0;
   for (int i = 0; i < 3; ++i) p.bias_stride[i] = a->bias_stride[i];
   if (p.bias) {
     if (p.paged) return LF_ERR_UNSUPPORTED;
@@ -1354,6 +1413,20 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
       }
     }
   }
+  if (p.bias && a->bias_pos == a->n_mod) {
+    bool plain = true;  // a bias behind multipliers only
+    float pre = a->scale;
+    for (int i = 0; i < a->n_mod; ++i) {
+      if (a->mod_op[i] == LF_MOD_MUL) pre *= a->mod_arg[i];
+      else if (a->mod_op[i] == LF_MOD_DIV) pre /= a->mod_arg[i];
+      else plain = false;
+    }
+    if (plain) {
+      mode = kModeBias;
+      p.a = pre;
+      p.c2 = kLog2eF;
+    }
+  }
   {
     if (mode == kModeGeneric) {
       p.a = a->scale;
@@ -1368,7 +1441,7 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
 
   if (has_pe) {
     // The two-product form runs in the plain running-max mode only (scale, then mask).
-    if (mode == kModeBounded || mode == kModeSoftcap || mode == kModeGeneric)
+    if (mode != kModeNone)
       return LF_ERR_UNSUPPORTED;
   }
   const int kv_tile = choose_kv_tile(a, mode);
@@ -1423,6 +1496,7 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
              : pack == 4       ? launch_prefill_bounded<128, 4>(mq, mk, mv, mo, p, a->B, st)
              : pack == 2       ? launch_prefill_bounded<128, 2>(mq, mk, mv, mo, p, a->B, st)
                                : launch_prefill_bounded<128>(mq, mk, mv, mo, p, a->B, st);
+    if (mode == kModeBias) return launch_prefill<128, kModeBias>(mq, mk, mv, p, a->B, st);
     return launch_prefill<128, kModeGeneric>(mq, mk, mv, p, a->B, st);
   }
   if (mode == kModeNone) return launch_prefill<64, kModeNone>(mq, mk, mv, p, a->B, st);
@@ -1432,6 +1506,7 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
            : pack == 4       ? launch_prefill_bounded<64, 4>(mq, mk, mv, mo, p, a->B, st)
            : pack == 2       ? launch_prefill_bounded<64, 2>(mq, mk, mv, mo, p, a->B, st)
                              : launch_prefill_bounded<64>(mq, mk, mv, mo, p, a->B, st);
+  if (mode == kModeBias) return launch_prefill<64, kModeBias>(mq, mk, mv, p, a->B, st);
   return launch_prefill<64, kModeGeneric>(mq, mk, mv, p, a->B, st);
 }
 

@@ -26,3 +26,21 @@ def test_rows_whose_later_keys_score_far_above_the_first(B, H, S_, D, gain):
     F.check_status(st)
     want = O.attention_ref(q, k, v, mask="causal", batch_chunk=B)
     assert (out.float().cpu() - want).abs().max().item() <= TOL
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Skv,pad,shift", [(130, 193, 7, 0), (65, 64, 16, 8), (257, 1001, 15, 0)])
+def test_score_bias_behind_multipliers(Sq, Skv, pad, shift, D):
+    """Bias rows of 32- and of only 16-byte alignment (`shift`), blocks that cross Skv in the middle
+    of an 8-column group, rows past the last tile."""
+    g = torch.Generator().manual_seed(4)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    q, k, v = mk(2, 3, Sq, D), mk(2, 3, Skv, D), mk(2, 3, Skv, D)
+    wide = mk(2, 3, Sq, (Skv + pad + shift + 7) // 8 * 8)
+    bias = wide[..., shift:shift + Skv]
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
+                              mods=[S.ScoreMod(S.MOD_MUL, 3.0), S.ScoreMod(S.MOD_DIV, 1.5)],
+                              score_bias=wide.cuda()[..., shift:shift + Skv])
+    s = q.float() @ k.float().transpose(-2, -1) * D ** -0.5 * 2.0 + bias.float()
+    want = torch.softmax(s, dim=-1) @ v.float()
+    assert (out.float().cpu() - want).abs().max().item() <= TOL
