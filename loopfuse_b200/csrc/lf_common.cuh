@@ -292,6 +292,18 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, ui
       : "memory");
 }
 
+// Four rows of a 2-D tensor (any row numbers; rows past the end arrive as zeros), 64 bf16 columns each,
+// through a map whose box is one row high.
+__device__ __forceinline__ void tma_gather4(uint32_t smem_dst, const void* tmap, uint64_t* bar, int x,
+                                            int r0, int r1, int r2, int r3) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      :
+      : "r"(smem_dst), "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+      : "memory");
+}
+
 // 4-D tiled store shared -> global (bulk async group of the issuing thread). Rows of the box
 // that lie outside the tensor are dropped by the hardware.
 __device__ __forceinline__ void tma_store_4d(const void* tmap, const void* smem_src, int c0,

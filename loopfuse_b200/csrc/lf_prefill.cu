@@ -9,13 +9,14 @@
 //
 // prefill_kernel: one CTA owns two consecutive 128-row query tiles of one (batch, q head) and
 // walks the 64-key KV tiles that the skip range leaves (fully masked tiles are never loaded or
-// multiplied). 352 threads:
+// multiplied). 384 threads:
 //   warps 0-3   softmax for query tile 0 (one thread per score row)
 //   warps 4-7   softmax for query tile 1
 //   warp  8     TMA producer: Q tiles once, then pairs of K/V tiles into a ring, in the order
 //               the MMA warps consume them: {K(lo), K(lo+1)}, {V(lo), K(lo+2)}, {V(lo+1), ...
 //   warp  9/10  MMA issuers (one thread each, one per query tile): S_t[buf] = Q_t K^T,
 //               O_t += P_t V
+//   warp  11    second producer of paged operands (idle otherwise)
 //
 // Tensor memory (512 columns x 128 lanes of 32 bit):
 //   tile t, buffer b: S at column t*128 + b*64 (64 fp32 columns); P (bf16, two per column)
@@ -47,7 +48,7 @@ namespace lf {
 constexpr int kTileQ = LF_PREFILL_TILE_Q;
 constexpr int kTileK = LF_PREFILL_TILE_K;
 static_assert(kTileQ == 128 && kTileK == 64, "the kernel is written for 128 x 64 tiles");
-constexpr int kPrefillThreads = 11 * 32;  // 8 softmax warps, 1 producer warp, 2 MMA-issuer warps
+constexpr int kPrefillThreads = 12 * 32;  // 8 softmax, 1 producer, 2 MMA-issuer, 1 gather warp
 constexpr int kMaxStages = 16;
 constexpr uint32_t kStageBytesTotal = 8 * 2048;
 // K/V ring depth in stages of two 64-key tiles: 4 x 32 KB at D=128, 8 x 16 KB at D=64 (which
@@ -141,6 +142,7 @@ struct PrefillParams {
   int64_t kp_stride[3], vp_stride[3];  // (page, slot, kv head)
   int64_t bt_stride;
   int32_t page_size, page_shift, n_pages;
+  int32_t gather;  // paged operands come by TMA row gather: tmap_k / tmap_v are 2-D maps of the pools
   int32_t pe_steps;  // PE variant: 16-column steps of the second score product (D_pe / 16, rounded up)
 };
 
@@ -194,6 +196,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   constexpr int kSoftmaxWarps = 8;
   constexpr int kProducerWarp = kSoftmaxWarps;
   constexpr int kMmaWarp0 = kSoftmaxWarps + 1;
+  constexpr int kGatherWarp = kSoftmaxWarps + 3;
 
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -240,7 +243,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     mbar_init(&bars->q_full[0], 1);
     mbar_init(&bars->q_full[1], 1);
     for (int s = 0; s < kStages; ++s) {
-      // (paged operands: one arrival for the TMA part, one for the warp's own copies)
+      // (paged operands: one arrival of either gather warp, or one for the TMA part and one for the
+      // warp's own copies)
       mbar_init(&bars->kv_full[s], p.paged ? 2 : 1);
       mbar_init(&bars->kv_empty[s], 2);
     }
@@ -268,7 +272,127 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
-  if (warp == kProducerWarp && p.paged) {
+  if ((warp == kProducerWarp || warp == kGatherWarp) && p.gather) {
+    // ---------------- producer with a paged K and / or V, by TMA row gather ----------------
+    // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table entries,
+    // then gather the rows) as tile::gather4 loads of four rows x 64 columns, straight into the
+    // 128-byte-swizzled tile; the pool is seen as a 2-D tensor of token rows, and tokens past Skv ask
+    // for a row past its end (zeros). A stage holds two tiles: the lower half of the warp looks up the
+    // first one's tokens, four per lane, the upper half the second one's, one stage ahead; the row
+    // numbers go through shared memory to the elected lane, which issues all gathers. (Issued by the
+    // lanes that hold the numbers, one diverged lane after the other, a gather took ~200 clocks.)
+    // Two warps share the gathers of every tile: eight each.
+    // Nothing waits for the rows here, so the whole ring is in flight; the cp.async form below has
+    // two stages in flight and a look-up in front of each.
+    const bool elected = elect_one_sync();
+    const int part = warp == kProducerWarp ? 0 : 1;
+    if (elected && part == 0) {
+      for (int t = 0; t < 2; ++t) {
+        if (!has_work[t]) continue;
+        mbar_arrive_expect_tx(&bars->q_full[t], kQTileBytes);
+#pragma unroll
+        for (int kb = 0; kb < kBlocksD; ++kb)
+          tma_load_4d(sQ + t * kQTileBytes + kb * kQBlockBytes, &tmap_q, &bars->q_full[t], kb * 64,
+                      (iq0 + t) * kTileQ, h, b);
+      }
+    }
+    __syncwarp();
+    const int n_rows = p.n_pages * p.page_size;
+    int4* row_ids = reinterpret_cast<int4*>(smem + 512) + part * 16;  // [tile of the stage][8]
+    static_assert(sizeof(PrefillBarriers) <= 512, "row numbers behind the barriers");
+    auto page_of = [&](int t) { return p.page_shift >= 0 ? (t >> p.page_shift) : (t / p.page_size); };
+    const int quad = (part * 8 + (lane & 7)) * 4;  // first of this lane's four tokens in its tile
+    // A stage is tile ja of K (or V, `first_is_v`) and tile jb of K (< 0: none). This lane's tile:
+    auto my_tile = [&](int ja, int jb) { return lane < 16 ? ja : jb; };
+    auto my_paged = [&](bool first_is_v) { return (p.paged >> (lane < 16 && first_is_v ? 1 : 0)) & 1; };
+    // Table entries of this lane's tokens, loaded but not looked at.
+    auto look_up = [&](bool first_is_v, int ja, int jb) -> int4 {
+      const int j = my_tile(ja, jb);
+      int id[4] = {0, 0, 0, 0};
+      if (j >= 0 && !(lane & 8) && my_paged(first_is_v)) {
+        const int32_t* table = (lane < 16 && first_is_v ? p.v_table : p.k_table) +
+                               static_cast<int64_t>(b) * p.bt_stride;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = j * kTileK + quad + e;
+          if (t < p.Skv) id[e] = table[page_of(t)];
+        }
+      }
+      return make_int4(id[0], id[1], id[2], id[3]);
+    };
+    int n = 0;
+    bool ok = true;
+    auto load_pair = [&](bool first_is_v, int ja, int jb, const int4& id) {
+      if (!ok) return;
+      {  // rows of this lane's tokens, checked
+        const int j = my_tile(ja, jb);
+        auto row_of = [&](int t, int32_t pg) -> int {
+          if (j < 0 || t >= p.Skv) return n_rows;
+          if (pg < 0 || pg >= p.n_pages) {
+            if (p.status && my_paged(first_is_v)) atomicExch(p.status, LF_DEV_BAD_PAGE);
+            pg = 0;
+          }
+          return pg * p.page_size + (t - page_of(t) * p.page_size);
+        };
+        const int t = j * kTileK + quad;
+        const int4 r = make_int4(row_of(t, id.x), row_of(t + 1, id.y), row_of(t + 2, id.z),
+                                 row_of(t + 3, id.w));
+        __syncwarp();  // (the elected lane has read the last stage's)
+        if (!(lane & 8)) row_ids[(lane >> 4) * 8 + (lane & 7)] = r;
+        __syncwarp();
+      }
+      const int stage = n % kStages;
+      const uint32_t parity = ((n / kStages) & 1) ^ 1;
+      ++n;
+      if (!mbar_wait(&bars->kv_empty[stage], parity)) {
+        report_timeout(p.status, 1);
+        ok = false;
+        return;
+      }
+      if (elected) {
+        auto bytes_of = [&](bool is_v) -> uint32_t {
+          return ((p.paged >> (is_v ? 1 : 0)) & 1) ? kKVTileBytes / 2 : part == 0 ? kKVTileBytes : 0u;
+        };
+        const uint32_t tx = bytes_of(first_is_v) + (jb >= 0 ? bytes_of(false) : 0u);
+        if (tx) mbar_arrive_expect_tx(&bars->kv_full[stage], tx);
+        else mbar_arrive(&bars->kv_full[stage]);
+        auto load = [&](bool is_v, int j, const int4* ids, unsigned char* dst) {
+          const CUtensorMap* tma = is_v ? &tmap_v : &tmap_k;
+          if ((p.paged >> (is_v ? 1 : 0)) & 1) {
+            const int x = hkv * static_cast<int>(is_v ? p.vp_stride[2] : p.kp_stride[2]);
+            const uint32_t d = smem_u32(dst);
+#pragma unroll 8
+            for (int i = 0; i < 8; ++i) {
+              const int4 r = ids[i];
+#pragma unroll
+              for (int kb = 0; kb < kBlocksD; ++kb)
+                tma_gather4(d + kb * kKVBlockBytes + (part * 8 + i) * 512, tma, &bars->kv_full[stage],
+                            x + kb * 64, r.x, r.y, r.z, r.w);
+            }
+          } else if (part == 0) {
+#pragma unroll
+            for (int kb = 0; kb < kBlocksD; ++kb)
+              tma_load_4d(dst + kb * kKVBlockBytes, tma, &bars->kv_full[stage], kb * 64, j * kTileK,
+                          hkv, b);
+          }
+        };
+        unsigned char* dst = sKV + stage * (2 * kKVTileBytes);
+        load(first_is_v, ja, row_ids, dst);
+        if (jb >= 0) load(false, jb, row_ids + 8, dst + kKVTileBytes);
+      }
+    };
+    if (hi > lo) {
+      auto second = [&](int j) { return j < hi ? j : -1; };
+      int4 id = look_up(false, lo, second(lo + 1));
+      int4 next = look_up(true, lo, second(lo + 2));
+      load_pair(false, lo, second(lo + 1), id);
+      for (int j = lo; j < hi; ++j) {
+        id = next;
+        if (j + 1 < hi) next = look_up(true, j + 1, second(j + 3));
+        load_pair(true, j, second(j + 2), id);
+      }
+    }
+  } else if (warp == kProducerWarp && p.paged) {
     // ---------------- producer with a paged K and / or V ----------------
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table
     // entries, then gather the rows) fused into the tile load: a dense operand still arrives by
@@ -561,7 +685,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         __syncwarp();
       }
     }
-  } else {
+  } else if (warp < kSoftmaxWarps) {
     // ---------------- softmax warps ----------------
     const int t = warp >> 2;                 // query tile of this warp group
     const int row = (warp & 3) * 32 + lane;  // row inside the tile == tensor-memory lane
@@ -1063,6 +1187,35 @@ static int encode_tile_map(CUtensorMap* map, const void* base, int B, int H, int
   return LF_OK;
 }
 
+// Tensor map over the token rows of a paged pool, for row gathers: `rows` rows of `cols` elements, box of
+// one row x 64 columns (box_rows == 1 tells these from the maps above).
+static int encode_gather_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols,
+                             int64_t row_stride) {
+  auto fn = get_encode_fn();
+  if (!fn) return LF_ERR_CUDA;
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_stride) * 2};
+  cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled(gather)");
+    return LF_ERR_CUDA;
+  }
+  return LF_OK;
+}
+
+// Elements between the token rows of a pool [n_pages, page_size, Hkv, D] with strides (page, slot,
+// kv head) when the pool is one 2-D tensor of rows that hold all heads; 0 when it is not.
+static int64_t gather_row_stride(const int64_t* st, int n_pages, int page_size, int Hkv, int D) {
+  const int64_t row = page_size == 1 ? st[0] : st[1];
+  if (page_size > 1 && n_pages > 1 && st[0] != page_size * st[1]) return 0;
+  if (row <= 0 || row % 8 || st[2] < 0 || (Hkv - 1) * st[2] + D > row) return 0;
+  if (static_cast<int64_t>(n_pages) * page_size > 0x7fffff00ll || row > (1 << 30)) return 0;
+  return row;
+}
+
 // Encoded tensor maps are kept in a small cache: a map depends only on (address, shape,
 // strides, box), and serving loops call with the same buffers again and again. Direct-mapped,
 // one mutex; a miss just encodes again, so the cache never changes a result. A CUtensorMap holds
@@ -1106,7 +1259,8 @@ static int make_tile_map(CUtensorMap* map, const void* base, int B, int H, int S
       return LF_OK;
     }
   }
-  const int rc = encode_tile_map(map, base, B, H, S, D, stride, box_rows, box_cols);
+  const int rc = box_rows == 1 ? encode_gather_map(map, base, S, D, stride[2])
+                               : encode_tile_map(map, base, B, H, S, D, stride, box_rows, box_cols);
   if (rc != LF_OK) return rc;
   g_tile_map_misses.fetch_add(1, std::memory_order_relaxed);
   std::lock_guard<std::mutex> lock(g_tile_map_mutex);
@@ -1333,6 +1487,7 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   p.page_size = a->page_size;
   p.page_shift = -1;
   p.n_pages = a->n_pages;
+  p.gather = 0;
   if (p.paged) {
     if (a->page_size <= 0 || a->n_pages <= 0) return LF_ERR_INVALID_ARG;
     if (a->bt_stride < (a->Skv + a->page_size - 1) / a->page_size) return LF_ERR_INVALID_ARG;
@@ -1456,14 +1611,24 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   CUtensorMap mq, mk, mv;
   int rc = make_tile_map(&mq, a->q, a->B, a->Hq, a->Sq, a->D, a->q_stride, kTileQ / pack);
   if (rc != LF_OK) return rc;
+  auto pool_map = [&](CUtensorMap* m, const void* pool, int64_t row_stride, int64_t head_stride) {
+    const int64_t st[3] = {0, 0, row_stride};
+    return make_tile_map(m, pool, 0, 0, a->n_pages * a->page_size,
+                         static_cast<int>((a->Hkv - 1) * head_stride + a->D), st, 1);
+  };
+  const int64_t k_row = p.paged & 1 ? gather_row_stride(a->k_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
+  const int64_t v_row = p.paged & 2 ? gather_row_stride(a->v_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
+  p.gather = p.paged && k_row && v_row;
   if (p.paged & 1) {
-    mk = mq;  // never used: the producer warp gathers K itself
+    mk = mq;  // (not used when the producer warp copies the rows of K itself)
+    if (p.gather && (rc = pool_map(&mk, a->k, k_row, a->k_stride[2])) != LF_OK) return rc;
   } else {
     rc = make_tile_map(&mk, a->k, a->B, a->Hkv, a->Skv, a->D, a->k_stride, kv_tile);
     if (rc != LF_OK) return rc;
   }
   if (p.paged & 2) {
     mv = mq;
+    if (p.gather && (rc = pool_map(&mv, a->v, v_row, a->v_stride[2])) != LF_OK) return rc;
   } else {
     rc = make_tile_map(&mv, a->v, a->B, a->Hkv, a->Skv, a->D, a->v_stride, kv_tile);
     if (rc != LF_OK) return rc;

@@ -44,3 +44,30 @@ def test_score_bias_behind_multipliers(Sq, Skv, pad, shift, D):
     s = q.float() @ k.float().transpose(-2, -1) * D ** -0.5 * 2.0 + bias.float()
     want = torch.softmax(s, dim=-1) @ v.float()
     assert (out.float().cpu() - want).abs().max().item() <= TOL
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("P,Skv,heads_first", [(1, 67, False), (3, 130, False), (16, 577, False),
+                                               (16, 577, True)])
+def test_paged_prefill_pool_layouts(P, Skv, heads_first, D):
+    """Pages of one token, of no power of two, and a pool whose heads lie outside its slots (no single
+    tensor of token rows: the rows are then copied by the producer warp); keys that end inside a
+    tile; K and V through tables of their own."""
+    g = torch.Generator().manual_seed(5)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    B, Hkv, G = 2, 2, 2
+    blocks = -(-Skv // P)
+    pages = B * blocks + 3
+    q = mk(B, Hkv * G, 150, D)
+    pool = lambda: (mk(pages, Hkv, P, D).transpose(1, 2) if heads_first else mk(pages, P, Hkv, D))
+    kp, vp = pool(), pool()
+    table = lambda: torch.randperm(pages, generator=g)[:B * blocks].view(B, blocks).int()
+    kt, vt = table(), table()
+    dev = lambda t: t.cuda() if t.is_contiguous() else t.transpose(1, 2).cuda().transpose(1, 2)
+    st = F.new_status("cuda")
+    out = F.prefill_attention(q.cuda(), dev(kp), dev(vp), scale=D ** -0.5, k_block_table=kt.cuda(),
+                              v_block_table=vt.cuda(), seq_len=Skv, status=st)
+    F.check_status(st)
+    want = O.attention_ref(q, O.paged_kv_ref(kp, kt)[:, :, :Skv], O.paged_kv_ref(vp, vt)[:, :, :Skv],
+                           batch_chunk=B)
+    assert (out.float().cpu() - want).abs().max().item() <= TOL
