@@ -276,7 +276,10 @@ class Runner:
                                                            workspace=ws)
             page = w.page_size
         splits = _native.load().lf_decode_auto_splits(w.B, w.Hkv, w.group, w.S, w.D, page)
-        self.launches_per_call = 2 if splits > 1 else 1
+        # Splits merge in their cluster; in a grid of many waves a second kernel merges them.
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        merged = splits <= 16 and splits * w.Hkv * w.B <= 8 * sms
+        self.launches_per_call = 1 if splits == 1 or merged else 2
 
 
 def events():

@@ -1,31 +1,29 @@
 // Decode attention for sm_100a: one query row per head, KV streamed once from HBM.
 //
-// Bandwidth-bound, so the work is laid out to keep many 16-byte loads in flight:
-//   * a CTA owns one (batch, kv head, KV split); its 4 warps interleave over the tokens of
-//     the split, each thread issuing UNROLL K-row and UNROLL V-row 16-byte streaming loads
-//     before any arithmetic;
-//   * a K/V row of D bf16 is covered by D/8 lanes, so a warp reads 32/(D/8) whole rows per
-//     load instruction (fully used 32-byte sectors);
-//   * the G query heads that share the kv head are kept in registers and reuse every loaded
-//     row (GQA), scores are reduced with shuffles, softmax is online in the log2 domain;
-//   * with splits > 1 each CTA writes an un-normalised partial (acc, max, sum) to the
-//     workspace and lf_combine merges them (log-sum-exp combine);
+// Bandwidth-bound, so the work is laid out to keep many bytes in flight:
+//   * a CTA owns one (batch, kv head, KV split); its warps take alternate 16-token groups of the
+//     split, each group's K and V rows travelling global -> shared with 16-byte cp.async into a ring
+//     private to the warp, so the bytes in flight do not cost registers;
+//   * the G query heads that share the kv head are the M dimension of tensor-core products (see
+//     decode_mma_kernel), softmax is online in the log2 domain;
+//   * with splits > 1 the CTAs of a (batch, kv head) form a thread-block cluster and merge their
+//     un-normalised partials (acc, max, sum) through distributed shared memory (log-sum-exp
+//     combine); where they cannot (more splits than a cluster holds, or grids of many waves), each
+//     CTA writes its partial to the workspace and lf_combine merges them;
 //   * the paged variant stages its slice of the block table through shared memory, checks
 //     every page id against the pool size (status word, clamped, never a trap) and turns
 //     (page, slot) into row pointers.
 #include "lf_common.cuh"
 
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 
 namespace lf {
 
-constexpr int kDecodeWarps = 4;
-constexpr int kDecodeThreads = kDecodeWarps * 32;
-constexpr int kDecodeUnroll = 4;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kMmaStages = 3;  // cp.async ring depth of the tensor-core decode kernel
 
 struct DecodeParams {
   const __nv_bfloat16* q;
@@ -42,272 +40,62 @@ struct DecodeParams {
   int32_t B, Hkv, Skv, splits, chunk;  // chunk = tokens per split
   int32_t page_size, page_shift, n_pages;  // page_shift >= 0 when page_size is 2^shift
   float scale;
+  float cap;        // kModsSoftcap: logit2 = tanh(scale * dot) * cap (log2(e) included)
+  int32_t cluster;  // the splits of a unit are one cluster and merge among themselves
+  int32_t part_off; // ... through partials at this byte of shared memory (the same in all of them)
   ModChain mods;
 };
 
-template <int D, int G, bool PAGED, bool HAS_MOD>
-__global__ void __launch_bounds__(kDecodeThreads)
-    decode_split_kernel(const DecodeParams p) {
-  constexpr int LPR = D / 8;        // lanes per K/V row
-  constexpr int RPW = 32 / LPR;     // rows per warp-wide load
-  constexpr int U = kDecodeUnroll;  // rows in flight per thread and tensor
-  constexpr int TOK_PER_WARP_IT = U * RPW;
-  constexpr int TOK_PER_CTA_IT = TOK_PER_WARP_IT * kDecodeWarps;
+// Score function of a decode kernel. Softcap has a form of its own: the interpreted chain is a
+// switch per score and op, mostly instruction-cache misses in a launch of a few microseconds.
+constexpr int kModsNone = 0, kModsSoftcap = 1, kModsGeneric = 2;
 
-  const int split = blockIdx.x;
-  const int kvh = blockIdx.y;
-  const int b = blockIdx.z;
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int rg = lane / LPR;   // row group inside the warp
-  const int col = lane % LPR;  // which 8-element slice of the row
+// Dot product (scaled by log2(e) * scale already when MODS == kModsNone) -> logit in the log2 domain.
+template <int MODS>
+__device__ __forceinline__ float decode_logit2(const DecodeParams& p, float d) {
+  if constexpr (MODS == kModsSoftcap) return tanh_approx(d) * p.cap;
+  else if constexpr (MODS == kModsGeneric) return apply_mods(p.mods, d) * kLog2e;
+  else return d;
+}
 
-  const int t0 = split * p.chunk;
-  const int t1 = min(p.Skv, t0 + p.chunk);
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // Layout: [page ids of this split] (paged only), then the cross-warp merge area.
-  int32_t* s_pages_k = reinterpret_cast<int32_t*>(smem_raw);
-  int32_t* s_pages_v = s_pages_k;
-  int n_pages_local = 0;
-  int first_page = 0;
-  size_t merge_off = 0;
-  if constexpr (PAGED) {
-    auto page_of = [&](int t) { return p.page_shift >= 0 ? (t >> p.page_shift) : (t / p.page_size); };
-    if (t1 > t0) {
-      first_page = page_of(t0);
-      n_pages_local = page_of(t1 - 1) - first_page + 1;
-    }
-    const bool two_tables = p.block_table_v != p.block_table;
-    const int pages_pad = (n_pages_local + 3) & ~3;
-    if (two_tables) s_pages_v = s_pages_k + pages_pad;
-    merge_off = static_cast<size_t>(pages_pad) * 4 * (two_tables ? 2 : 1);
-    for (int which = 0; which < (two_tables ? 2 : 1); ++which) {
-      const int32_t* bt = (which == 0 ? p.block_table : p.block_table_v) +
-                          static_cast<int64_t>(b) * p.bt_stride + first_page;
-      int32_t* dst = which == 0 ? s_pages_k : s_pages_v;
-      for (int i = threadIdx.x; i < n_pages_local; i += kDecodeThreads) {
-        int32_t pg = bt[i];
-        if (pg < 0 || pg >= p.n_pages) {
-          if (p.status) atomicExch(p.status, LF_DEV_BAD_PAGE);
-          pg = 0;
-        }
-        dst[i] = pg;
-      }
-    }
-    __syncthreads();
-  }
-  float* s_merge = reinterpret_cast<float*>(smem_raw + merge_off);
-
-  // Query rows for the G grouped heads, this lane's 8-element slice, as fp32. Without a
-  // score-mod chain the softmax scale and log2(e) are folded into q.
-  float qf[G][8];
-  {
-    const float qmul = HAS_MOD ? p.scale : p.scale * kLog2e;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const __nv_bfloat16* qp =
-          p.q + b * p.q_stride[0] + kvh * p.q_stride[1] + g * p.q_stride[2] + col * 8;
-      const uint4 raw = *reinterpret_cast<const uint4*>(qp);
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        qf[g][2 * i] = bf16lo_to_f32(w[i]) * qmul;
-        qf[g][2 * i + 1] = bf16hi_to_f32(w[i]) * qmul;
-      }
-    }
-  }
-
-  float m_run[G], l_run[G], acc[G][8];
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m_run[g] = -INFINITY;
-    l_run[g] = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[g][e] = 0.f;
-  }
-
-  const __nv_bfloat16* kbase;
-  const __nv_bfloat16* vbase;
-  if constexpr (PAGED) {
-    kbase = p.k + kvh * p.k_stride[2] + col * 8;
-    vbase = p.v + kvh * p.v_stride[2] + col * 8;
-  } else {
-    kbase = p.k + b * p.k_stride[0] + kvh * p.k_stride[1] + col * 8;
-    vbase = p.v + b * p.v_stride[0] + kvh * p.v_stride[1] + col * 8;
-  }
-
-  for (int base = t0 + warp * TOK_PER_WARP_IT; base < t1; base += TOK_PER_CTA_IT) {
-    uint4 kr[U], vr[U];
-    bool valid[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int t = base + u * RPW + rg;
-      valid[u] = t < t1;
-      int tc = valid[u] ? t : (t1 - 1);  // clamp: the row is loaded but scored -inf
-      if (!LF_BOUNDS(tc >= t0 && tc < p.Skv, p.status, 40)) tc = t0;
-      int64_t koff, voff;
-      if constexpr (PAGED) {
-        const int pg_abs = p.page_shift >= 0 ? (tc >> p.page_shift) : (tc / p.page_size);
-        const int slot = tc - pg_abs * p.page_size;
-        int pl = pg_abs - first_page;
-        if (!LF_BOUNDS(pl >= 0 && pl < n_pages_local && slot >= 0 && slot < p.page_size,
-                       p.status, 41))
-          pl = 0;
-        const int64_t pgk = s_pages_k[pl];
-        const int64_t pgv = s_pages_v[pl];
-        koff = pgk * p.k_stride[0] + slot * p.k_stride[1];
-        voff = pgv * p.v_stride[0] + slot * p.v_stride[1];
-      } else {
-        koff = tc * p.k_stride[2];
-        voff = tc * p.v_stride[2];
-      }
-      kr[u] = ldg_stream_16(kbase + koff);
-      vr[u] = ldg_stream_16(vbase + voff);
-    }
-
-    // Scores: partial dot over this lane's 8 elements, then all-reduce over the row's lanes.
-    float s[G][U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t w[4] = {kr[u].x, kr[u].y, kr[u].z, kr[u].w};
-      float kf[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        kf[2 * i] = bf16lo_to_f32(w[i]);
-        kf[2 * i + 1] = bf16hi_to_f32(w[i]);
-      }
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float d = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) d = fmaf(qf[g][e], kf[e], d);
-        s[g][u] = d;
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        float d = s[g][u];
-#pragma unroll
-        for (int off = LPR / 2; off >= 1; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-        if constexpr (HAS_MOD) d = apply_mods(p.mods, d) * kLog2e;
-        s[g][u] = valid[u] ? d : -INFINITY;
-      }
-    }
-
-    // Online softmax update (log2 domain) and PV accumulation.
-    float pw[G][U];
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float m_new = m_run[g];
-#pragma unroll
-      for (int u = 0; u < U; ++u) m_new = fmaxf(m_new, s[g][u]);
-      const float m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = ex2_approx(m_run[g] - m_safe);
-      float psum = 0.f;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        pw[g][u] = ex2_approx(s[g][u] - m_safe);
-        psum += pw[g][u];
-      }
-      l_run[g] = l_run[g] * alpha + psum;
-      m_run[g] = m_new;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[g][e] *= alpha;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t w[4] = {vr[u].x, vr[u].y, vr[u].z, vr[u].w};
-      float vf[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        vf[2 * i] = bf16lo_to_f32(w[i]);
-        vf[2 * i + 1] = bf16hi_to_f32(w[i]);
-      }
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pw[g][u], vf[e], acc[g][e]);
-      }
-    }
-  }
-
-  // Merge the row groups of a warp (they hold disjoint token subsets of the same columns).
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-#pragma unroll
-    for (int off = LPR; off < 32; off <<= 1) {
-      const float m_o = __shfl_xor_sync(0xffffffffu, m_run[g], off);
-      const float l_o = __shfl_xor_sync(0xffffffffu, l_run[g], off);
-      const float m_new = fmaxf(m_run[g], m_o);
-      const float m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-      const float a_s = ex2_approx(m_run[g] - m_safe);
-      const float a_o = ex2_approx(m_o - m_safe);
-      l_run[g] = l_run[g] * a_s + l_o * a_o;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float acc_o = __shfl_xor_sync(0xffffffffu, acc[g][e], off);
-        acc[g][e] = acc[g][e] * a_s + acc_o * a_o;
-      }
-      m_run[g] = m_new;
-    }
-  }
-
-  // Merge the warps through shared memory: s_merge[warp][g][0..D) acc, then m, l.
+// Merge the partials of a unit's splits within their cluster. `mine` (shared memory of every CTA of
+// the cluster, at the same offset): [G][D + 2] un-normalised output, max, sum. Each CTA finishes a
+// slice of the G * D outputs. A launch less than the combine kernel, and no round trip of the
+// partials through global memory (one sequence, 8 kv heads x 4, 8190 keys: 4.7 us for the combine).
+template <int D>
+__device__ __forceinline__ void merge_in_cluster(const DecodeParams& p, float* mine, int G, int b,
+                                                 int kvh, int threads) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const int rank = static_cast<int>(cluster.block_rank());
   constexpr int kStride = D + 2;
-  if (rg == 0) {
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float* dst = s_merge + (warp * G + g) * kStride;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dst[col * 8 + e] = acc[g][e];
-      if (col == 0) {
-        dst[D] = m_run[g];
-        dst[D + 1] = l_run[g];
-      }
-    }
-  }
-  __syncthreads();
-
-  // One thread per (g, column) finishes the merge and writes the result.
-  for (int idx = threadIdx.x; idx < G * D; idx += kDecodeThreads) {
-    const int g = idx / D;
-    const int c = idx - g * D;
+  for (int idx = rank * threads + threadIdx.x; idx < G * D; idx += p.splits * threads) {
+    const int g = idx / D, c = idx - g * D;
     float m_all = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kDecodeWarps; ++w)
-      m_all = fmaxf(m_all, s_merge[(w * G + g) * kStride + D]);
+    for (int r = 0; r < p.splits; ++r)
+      m_all = fmaxf(m_all, cluster.map_shared_rank(mine, r)[g * kStride + D]);
     const float m_safe = (m_all == -INFINITY) ? 0.f : m_all;
     float l_all = 0.f, o = 0.f;
-#pragma unroll
-    for (int w = 0; w < kDecodeWarps; ++w) {
-      const float* src = s_merge + (w * G + g) * kStride;
+#pragma unroll 4
+    for (int r = 0; r < p.splits; ++r) {
+      const float* src = cluster.map_shared_rank(mine, r) + g * kStride;
       const float a = ex2_approx(src[D] - m_safe);
       l_all += src[D + 1] * a;
       o += src[c] * a;
     }
-    const int64_t unit = (static_cast<int64_t>(b) * p.Hkv + kvh) * G + g;
-    if (p.splits == 1) {
-      __nv_bfloat16* op = p.out + b * p.o_stride[0] + kvh * p.o_stride[1] + g * p.o_stride[2];
-      op[c] = __float2bfloat16_rn(o / l_all);
-    } else {
-      p.part_o[(unit * p.splits + split) * D + c] = o;
-      if (c == 0) {
-        p.part_ml[(unit * p.splits + split) * 2] = m_all;
-        p.part_ml[(unit * p.splits + split) * 2 + 1] = l_all;
-      }
-    }
+    __nv_bfloat16* op = p.out + b * p.o_stride[0] + kvh * p.o_stride[1] + g * p.o_stride[2];
+    op[c] = __float2bfloat16_rn(o / l_all);
   }
+  cluster.sync();  // (nobody leaves while its shared memory is being read)
 }
 
 // ---------------------------------------------------------------------------------------
-// Grouped / paged decode on tensor cores (mma.sync m16n8k16, bf16 -> fp32).
+// Decode on tensor cores (mma.sync m16n8k16, bf16 -> fp32).
 //
-// For G > 2 query rows per kv head (and for every paged cache) the FMA + shuffle form above
-// becomes instruction-bound long before HBM is saturated; here the G rows are the (zero-padded)
-// M dimension of 16x8x16 MMAs and the fragments come straight from 16-byte global loads:
+// The G query rows of a kv head are rows 0..7 (zero-padded) of the 16-row M dimension of 16x8x16
+// MMAs; rows 8..15 are padding unless WIDE_P. The fragments come straight
+// from the 16-byte pieces that were copied:
 //
 //   QK^T  8 tokens at a time. Lane (n = lane/4, c = lane%4) loads the 16-byte pieces
 //         d = 32i + 8c .. +8 of token n's K row (i < D/32); the four 32-bit words of a piece
@@ -319,9 +107,14 @@ __global__ void __launch_bounds__(kDecodeThreads)
 //         wants; output column n of MMA (h, e) stands for d = 64h + 8n + e.
 //   The fp32 score fragment of the QK MMAs has the layout of the bf16 A fragment of the PV
 //   MMA, so P never leaves registers.
+//   WIDE_P (dense calls with G <= 2, which have rows to spare): P enters the PV product as the sum of
+//   three bf16, i.e. with fp32's 24 bits and at no extra MMA: rows g take its rounding, rows 8 + g
+//   the rounding of the rest, rows 2 + g (whose Q rows repeat rows g) what that leaves.
 // A CTA is one (batch, kv head, KV split); its WARPS warps (4, or 2 when smaller CTAs let the
 // whole grid be resident at once) take alternate 16-token groups (one page when page_size is
-// 16) and are merged through shared memory like above.
+// 16) and are merged through shared memory. Against the FMA + shuffle form that dense calls with G <=
+// 2 used (B200, D = 128): B=64 Hkv=32 2048 keys 318 -> 307 us, B=1 Hkv=32 4096 keys 20.3 -> 16.8 us,
+// B=1 Hkv=4 G=2 16000 keys 27.9 -> 16.4 us, B=16 Hkv=32 1000 keys 45.0 -> 46.3 us.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_16816_rows0to7(float& d0, float& d1, uint32_t a0, uint32_t a2,
                                                    uint32_t b0, uint32_t b1) {
@@ -332,8 +125,18 @@ __device__ __forceinline__ void mma_16816_rows0to7(float& d0, float& d1, uint32_
       : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.f), "f"(0.f));
 }
 
-template <int D, bool PAGED, bool HAS_MOD, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
+// The same with all sixteen rows.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+      "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// STAGES: depth of a warp's ring in 16-token groups; STAGES - 1 are in flight.
+template <int D, bool PAGED, int MODS, int WARPS, int STAGES, bool WIDE_P>
+__global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     decode_mma_kernel(const DecodeParams p, const int G) {
   constexpr int KI = D / 32;  // 16-byte pieces of a K row per lane
   constexpr int VH = D / 64;  // 64-wide halves of a V row
@@ -350,7 +153,7 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
   const int t0 = split * p.chunk;
   const int t1 = min(p.Skv, t0 + p.chunk);
 
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   int32_t* s_pages_k = reinterpret_cast<int32_t*>(smem_raw);
   int32_t* s_pages_v = s_pages_k;
   int first_page = 0;
@@ -363,7 +166,9 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
       n_pages_local = page_of(t1 - 1) - first_page + 1;
     }
     const bool two_tables = p.block_table_v != p.block_table;
-    const int pages_pad = (n_pages_local + 3) & ~3;
+    // The rings start on a 128-byte line: 16 bytes off it, a row's copy writes three lines instead of
+    // two (192 units of 1200 keys 34.4 -> 25 us).
+    const int pages_pad = (n_pages_local + 31) & ~31;
     if (two_tables) s_pages_v = s_pages_k + pages_pad;
     merge_off = static_cast<size_t>(pages_pad) * 4 * (two_tables ? 2 : 1);
     for (int which = 0; which < (two_tables ? 2 : 1); ++which) {
@@ -424,65 +229,69 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
     }
   };
 
-  // Q fragments (rows g >= G are zero padding).
+  // Q fragments (rows g >= G are zero padding; WIDE_P: rows 2 and 3 are rows 0 and 1 once more).
+  const int q_row = WIDE_P && g < 4 ? (g & 1) : g;
+  auto chunk_of = [&](int i) { return 4 * i + c; };  // 16-byte piece of a row
   uint4 qr[KI];
 #pragma unroll
   for (int i = 0; i < KI; ++i) {
     qr[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (g < G)
+    if (q_row < G)
       qr[i] = *reinterpret_cast<const uint4*>(p.q + b * p.q_stride[0] + kvh * p.q_stride[1] +
-                                              g * p.q_stride[2] + 32 * i + 8 * c);
+                                              q_row * p.q_stride[2] + 8 * chunk_of(i));
   }
-  const float smul = HAS_MOD ? p.scale : p.scale * kLog2e;
+  const float smul = MODS != kModsNone ? p.scale : p.scale * kLog2e;
 
   float m_run = -INFINITY, l_run = 0.f;
-  float o[NT][2];
+  constexpr int kOut = WIDE_P ? 4 : 2;
+  float o[NT][kOut];
 #pragma unroll
-  for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = 0.f;
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < kOut; ++e) o[j][e] = 0.f;
 
   // K/V rows travel global -> shared with 16-byte cp.async into a ring private to the warp
-  // (kMmaStages groups of 16 tokens; kMmaStages-1 groups are in flight while one is consumed),
-  // so the bytes in flight do not cost registers. A 16-byte chunk j of row r sits at chunk
-  // position j ^ (r & 7): fragment reads of eight different rows then hit distinct banks.
-  constexpr int CPR = D / 8;               // 16-byte chunks per row
+  // (STAGES groups of 16 tokens; STAGES-1 groups are in flight while one is consumed),
+  // so the bytes in flight do not cost registers. The 16-byte piece j of row r sits at piece j ^ (r & 7):
+  // fragment reads of eight different rows then hit distinct banks. (One 256-byte bulk copy per row is
+  // an instruction per lane and group, but the SM takes them at 11 ns each: 64 units of 8190 keys 101
+  // -> 190 us.)
+  constexpr int CPR = D / 8;         // 16-byte pieces per row
+  constexpr int RPI = 32 / CPR;      // rows that one instruction of the warp copies
   constexpr int kRowBytes = D * 2;
   constexpr int kStageBytes = 2 * 16 * kRowBytes;  // 16 K rows then 16 V rows
   const int t_last = t1 - 1;
-  unsigned char* ring = smem_raw + merge_off + warp * (kMmaStages * kStageBytes);
-  const uint32_t ring_u32 = smem_u32(ring);
+  unsigned char* ring = smem_raw + merge_off + warp * (STAGES * kStageBytes);
+  const int r0 = lane / CPR, j0 = lane % CPR;
+  const uint32_t ring_u32 = smem_u32(ring) + r0 * kRowBytes;
+  const int64_t ks = PAGED ? p.k_stride[1] : p.k_stride[2];
+  const int64_t vs = PAGED ? p.v_stride[1] : p.v_stride[2];
   auto copy_group = [&](int tg, int stage) {
     if (tg < t1) {
-      const uint32_t dst0 = ring_u32 + stage * kStageBytes;
-      const int j = lane % CPR;
-      const int r_max = t_last - tg;  // rows past the end of the split re-read the last token
-      // A group that lies inside one page (always true for dense caches) has affine row
+      const uint32_t dst = ring_u32 + stage * kStageBytes;
+      // A whole group that lies inside one page (always true for dense caches) has affine row
       // addresses: one table lookup per group instead of one per row.
-      bool one_page = true;
-      if constexpr (PAGED) one_page = page_of(tg) == page_of(min(tg + 15, t_last));
-      if (one_page) {
-        const __nv_bfloat16* kp = k_row(tg) + 8 * j;
-        const __nv_bfloat16* vp = v_row(tg) + 8 * j;
-        const int64_t ks = PAGED ? p.k_stride[1] : p.k_stride[2];
-        const int64_t vs = PAGED ? p.v_stride[1] : p.v_stride[2];
+      bool affine = tg + 15 <= t_last;
+      if constexpr (PAGED) affine = affine && page_of(tg) == page_of(tg + 15);
+      if (!LF_BOUNDS(stage >= 0 && stage < STAGES, p.status, 46)) {
+      } else if (affine) {
+        const __nv_bfloat16* kp = k_row(tg) + r0 * ks + 8 * j0;
+        const __nv_bfloat16* vp = v_row(tg) + r0 * vs + 8 * j0;
 #pragma unroll
-        for (int q = 0; q < 16 * CPR / 32; ++q) {
-          const int r = lane / CPR + q * (32 / CPR);
-          const int rc = min(r, r_max);
-          const uint32_t off = r * kRowBytes + ((j ^ (r & 7)) << 4);
-          if (!LF_BOUNDS(off + 16 <= 16u * kRowBytes && stage >= 0 && stage < kMmaStages,
-                         p.status, 46))
-            continue;
-          cp_async_16(dst0 + off, kp + rc * ks);
-          cp_async_16(dst0 + 16 * kRowBytes + off, vp + rc * vs);
+        for (int q = 0; q < 16 / RPI; ++q) {
+          const uint32_t to = dst + q * RPI * kRowBytes + ((j0 ^ ((r0 + q * RPI) & 7)) << 4);
+          cp_async_16(to, kp);
+          cp_async_16(to + 16 * kRowBytes, vp);
+          kp += RPI * ks;
+          vp += RPI * vs;
         }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 16 * CPR / 32; ++q) {
-          const int r = lane / CPR + q * (32 / CPR);
-          const int tok = tg + min(r, r_max);
-          const uint32_t off = r * kRowBytes + ((j ^ (r & 7)) << 4);
-          cp_async_16(dst0 + off, k_row(tok) + 8 * j);
-          cp_async_16(dst0 + 16 * kRowBytes + off, v_row(tok) + 8 * j);
+      } else {  // (rows past the end of the split re-read its last token)
+#pragma unroll 4
+        for (int q = 0; q < 16 / RPI; ++q) {
+          const int tok = min(tg + r0 + q * RPI, t_last);
+          const uint32_t to = dst + q * RPI * kRowBytes + ((j0 ^ ((r0 + q * RPI) & 7)) << 4);
+          cp_async_16(to, k_row(tok) + 8 * j0);
+          cp_async_16(to + 16 * kRowBytes, v_row(tok) + 8 * j0);
         }
       }
     }
@@ -490,41 +299,39 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
   };
   const int tg0 = t0 + warp * 16;
 #pragma unroll
-  for (int st = 0; st < kMmaStages - 1; ++st) copy_group(tg0 + st * 16 * WARPS, st);
+  for (int st = 0; st < STAGES - 1; ++st) copy_group(tg0 + st * 16 * WARPS, st);
 
   int it = 0;
   for (int tg = tg0; tg < t1; tg += 16 * WARPS, ++it) {
-    copy_group(tg + (kMmaStages - 1) * 16 * WARPS, (it + kMmaStages - 1) % kMmaStages);
-    cp_async_wait<kMmaStages - 1>();
+    copy_group(tg + (STAGES - 1) * 16 * WARPS, (it + STAGES - 1) % STAGES);
+    cp_async_wait<STAGES - 1>();
     __syncwarp();
-    const unsigned char* stage = ring + (it % kMmaStages) * kStageBytes;
+    const unsigned char* stage = ring + (it % STAGES) * kStageBytes;
     // K: token n = g of each 8-token half; V: rows 2c, 2c+1, 2c+8, 2c+9 of the 16-token group.
     uint4 kr[2][KI];
 #pragma unroll
-    for (int s8 = 0; s8 < 2; ++s8) {
-      const int r = 8 * s8 + g;
+    for (int s8 = 0; s8 < 2; ++s8)
 #pragma unroll
       for (int i = 0; i < KI; ++i)
-        kr[s8][i] = *reinterpret_cast<const uint4*>(stage + r * kRowBytes +
-                                                    (((4 * i + c) ^ (r & 7)) << 4));
-    }
+        kr[s8][i] =
+            *reinterpret_cast<const uint4*>(stage + (8 * s8 + g) * kRowBytes + ((chunk_of(i) ^ g) << 4));
 
     // Scores of the two 8-token halves: this lane ends up with tokens 2c, 2c+1 of each.
-    float sc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    // (two accumulators each: half the chain of dependent MMAs)
+    float sc[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, sc_b[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll
     for (int s8 = 0; s8 < 2; ++s8)
 #pragma unroll
       for (int i = 0; i < KI; ++i) {
         mma_16816_rows0to7(sc[s8][0], sc[s8][1], qr[i].x, qr[i].y, kr[s8][i].x, kr[s8][i].y);
-        mma_16816_rows0to7(sc[s8][0], sc[s8][1], qr[i].z, qr[i].w, kr[s8][i].z, kr[s8][i].w);
+        mma_16816_rows0to7(sc_b[s8][0], sc_b[s8][1], qr[i].z, qr[i].w, kr[s8][i].z, kr[s8][i].w);
       }
     float mx = -INFINITY;
 #pragma unroll
     for (int s8 = 0; s8 < 2; ++s8)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        float v = sc[s8][e] * smul;
-        if constexpr (HAS_MOD) v = apply_mods(p.mods, v) * kLog2e;
+        float v = decode_logit2<MODS>(p, (sc[s8][e] + sc_b[s8][e]) * smul);
         if (tg + 8 * s8 + 2 * c + e >= t1) v = -INFINITY;
         sc[s8][e] = v;
         mx = fmaxf(mx, v);
@@ -533,8 +340,15 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float m_new = fmaxf(m_run, mx);
     const float m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-    const float alpha = ex2_approx(m_run - m_safe);
-    m_run = m_new;
+    if (__any_sync(0xffffffffu, m_new > m_run)) {  // (a new maximum becomes rare after a few groups)
+      const float alpha = ex2_approx(m_run - m_safe);
+      m_run = m_new;
+      l_run *= alpha;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < kOut; ++e) o[j][e] *= alpha;
+    }
     float pr[2][2];
     float psum = 0.f;
 #pragma unroll
@@ -544,13 +358,20 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
         pr[s8][e] = ex2_approx(sc[s8][e] - m_safe);
         psum += pr[s8][e];
       }
-    l_run = l_run * alpha + psum;  // this lane's share; the quad is summed after the loop
-    const uint32_t pa0 = pack_bf16x2(pr[0][0], pr[0][1]);
-    const uint32_t pa2 = pack_bf16x2(pr[1][0], pr[1][1]);
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      o[j][0] *= alpha;
-      o[j][1] *= alpha;
+    l_run += psum;  // this lane's share; the quad is summed after the loop
+    uint32_t pa0 = pack_bf16x2(pr[0][0], pr[0][1]);
+    uint32_t pa2 = pack_bf16x2(pr[1][0], pr[1][1]);
+    [[maybe_unused]] uint32_t pa1 = 0u, pa3 = 0u;
+    if constexpr (WIDE_P) {
+      const float r0 = pr[0][0] - bf16lo_to_f32(pa0), r1 = pr[0][1] - bf16hi_to_f32(pa0);
+      const float r2 = pr[1][0] - bf16lo_to_f32(pa2), r3 = pr[1][1] - bf16hi_to_f32(pa2);
+      pa1 = pack_bf16x2(r0, r1);
+      pa3 = pack_bf16x2(r2, r3);
+      if (g >= 2) {
+        pa0 = pack_bf16x2(r0 - bf16lo_to_f32(pa1), r1 - bf16hi_to_f32(pa1));
+        pa2 = pack_bf16x2(r2 - bf16lo_to_f32(pa3), r3 - bf16hi_to_f32(pa3));
+        pa1 = pa3 = 0u;
+      }
     }
 #pragma unroll
     for (int h = 0; h < VH; ++h) {
@@ -570,13 +391,21 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
         const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;  // high or low halves of two words
         const uint32_t b0 = __byte_perm(w0[e >> 1], w1[e >> 1], sel);
         const uint32_t b1 = __byte_perm(w2[e >> 1], w3[e >> 1], sel);
-        mma_16816_rows0to7(o[h * 8 + e][0], o[h * 8 + e][1], pa0, pa2, b0, b1);
+        if constexpr (WIDE_P) mma_16816(o[h * 8 + e], pa0, pa1, pa2, pa3, b0, b1);
+        else mma_16816_rows0to7(o[h * 8 + e][0], o[h * 8 + e][1], pa0, pa2, b0, b1);
       }
     }
     __syncwarp();  // every lane is done with this stage before it is refilled
   }
   cp_async_wait<0>();
 
+  if constexpr (WIDE_P) {  // rows 8 + g (same lane) and 2 + g hold the finer parts of row g
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        o[j][e] += o[j][2 + e] + __shfl_down_sync(0xffffffffu, o[j][e], 8);
+  }
   // Row sum over the quad (the four lanes of a row hold disjoint tokens).
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
@@ -620,7 +449,14 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
     const int64_t unit = (static_cast<int64_t>(b) * p.Hkv + kvh) * G + gg;
     if (!LF_BOUNDS(gg < G && cc < D && b < p.B && kvh < p.Hkv && split < p.splits, p.status, 47))
       continue;
-    if (p.splits == 1) {
+    if (p.cluster) {
+      float* mine = reinterpret_cast<float*>(smem_raw + p.part_off) + gg * kStride;
+      mine[cc] = acc;
+      if (cc == 0) {
+        mine[D] = m_all;
+        mine[D + 1] = l_all;
+      }
+    } else if (p.splits == 1) {
       __nv_bfloat16* op = p.out + b * p.o_stride[0] + kvh * p.o_stride[1] + gg * p.o_stride[2];
       op[cc] = __float2bfloat16_rn(acc / l_all);
     } else {
@@ -631,6 +467,8 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
       }
     }
   }
+  if (p.cluster)
+    merge_in_cluster<D>(p, reinterpret_cast<float*>(smem_raw + p.part_off), G, b, kvh, WARPS * 32);
 }
 
 // Log-sum-exp combine of split-KV partials: one warp per (batch, kv head, g) output row.
@@ -743,122 +581,147 @@ static int device_sm_count() {
 
 static int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
-static bool uses_mma_kernel(int G, bool paged) { return paged || G > 2; }
-
 // Shared memory the tensor-core kernel may spend on block-table slices (both tables), so that
 // two CTAs (K/V rings of 96 KB each at D = 128) still fit on one SM.
 constexpr size_t kMaxTableBytes = 16 * 1024;
 
 static size_t table_smem_bytes(int chunk, int page_size) {
-  // Room for the K table and a separate V table, each padded to 16 bytes.
-  return 2 * (((static_cast<size_t>(chunk / page_size) + 2 + 3) & ~size_t(3)) * 4);
+  // Room for the K table and a separate V table, each padded to 128 bytes.
+  return 2 * (((static_cast<size_t>(chunk / page_size) + 2 + 31) & ~size_t(31)) * 4);
 }
 
 // Largest token chunk of one split whose block-table slice fits (paged caches only).
 static int max_chunk_for_table(int page_size) {
-  const int entries = static_cast<int>(kMaxTableBytes / 8) - 4;  // per table, minus padding
+  const int entries = static_cast<int>(kMaxTableBytes / 8) - 34;  // per table, minus padding
   const int64_t tokens = static_cast<int64_t>(entries) * page_size;
   return static_cast<int>(tokens > (1 << 30) ? (1 << 30) : tokens / 64 * 64);
 }
 
-// Split count for splits == 0. page_size: 0 for a dense cache, else the tokens per page.
+constexpr int kMaxCluster = 16;  // (more than 8 CTAs: a non-portable cluster size)
+
+// Split count for splits == 0. page_size: 0 for a dense cache, else the tokens per page. Powers of
+// two only: clusters of other sizes are placed badly (16 x 8 units of 1001 keys took 18.5 us in twos,
+// 22 in threes, 20 in fours, 33 in sixes; 8 x 4 units of 4000 keys 20.4 us in eights, 29 in nines).
 static int choose_splits(int B, int Hkv, int G, int Skv, int D, int page_size) {
+  (void)G;
   (void)D;
-  const bool paged = page_size > 0;
-  const int units = B * Hkv;
+  const int64_t units = static_cast<int64_t>(B) * Hkv;
   const int sms = device_sm_count();
-  int max_by_len = Skv / 256;  // keep >= 256 tokens per split
-  if (max_by_len < 1) max_by_len = 1;
-  if (max_by_len > 32) max_by_len = 32;
-  int s;
-  if (uses_mma_kernel(G, paged)) {
-    // Two CTAs of the tensor-core kernel are resident per SM and each keeps ~16 KB in flight
-    // per warp, so one wave already saturates HBM: split only to fill the machine (splitting
-    // costs the partial round trip and a short, badly pipelined loop per CTA; splitting four
-    // ways to even out the waves of 512 units measured 20 % slower than not splitting).
-    const int resident = sms * 2;
-    s = units >= resident ? 1 : (resident + units - 1) / units;
-  } else {
-    // The FMA kernel has ~8 small CTAs per SM: aim for >= 6 waves so the tail wave is cheap.
-    s = (sms * 8 * 6 + units - 1) / units;
-  }
-  if (s > max_by_len) s = max_by_len;
-  if (s < 1) s = 1;
-  if (paged) {
+  constexpr int kMinTokens = 120;  // per split: below, its start-up costs what the split saves
+  // As many CTAs as one wave of one per SM takes. (Two per SM gain nothing over that: 64 units of 8190
+  // keys 47 us in twos, 49 in fours, 49 in eights.) Sixteen-CTA clusters only where one fits in every
+  // GPC: 16 units of 8190 keys 22.6 us in eights, 28.6 in sixteens.
+  int s = 1;
+  while (s < kMaxCluster && units * s * 2 <= sms && Skv / (s * 2) >= kMinTokens) s *= 2;
+  // If that leaves 40 % of the SMs without work, four times as many smaller ones: 40 units of 8190
+  // keys 39 us in twos, 37 in eights; of 3001 keys 24 and 20.
+  if (units * s * 5 < 3ll * sms && s <= 4 && Skv / (s * 4) >= kMinTokens &&
+      units * s * 4 >= 2ll * sms)
+    s = s == 4 ? 8 : s * 4;
+  // A grid of many waves gains from halves where the caches are long: its last wave is shorter (640
+  // units of 3001 keys 188 -> 166 us, 2048 units of 2048 keys 315 -> 307 us).
+  if (units >= 4ll * sms && Skv >= 2000) s = 2;
+  if (page_size > 0) {
     // The block-table slice of a split must fit in shared memory (one-token pages at long
     // context): split further until it does.
     const int max_chunk = max_chunk_for_table(page_size);
-    while (s < 32 && round_up((Skv + s - 1) / s, 64) > max_chunk) ++s;
+    while (s < 32 && round_up((Skv + s - 1) / s, 16) > max_chunk) s = s < 16 ? s * 2 : s + 1;
   }
   return s;
 }
 
-template <int D, int G, bool PAGED>
-static int launch_decode_g(const DecodeParams& p, cudaStream_t st, size_t smem) {
-  dim3 grid(p.splits, p.Hkv, p.B);
-  if (p.mods.n > 0)
-    decode_split_kernel<D, G, PAGED, true><<<grid, kDecodeThreads, smem, st>>>(p);
-  else
-    decode_split_kernel<D, G, PAGED, false><<<grid, kDecodeThreads, smem, st>>>(p);
-  return check_launch("decode_split_kernel");
+// Launch with the splits of a unit as a cluster, when p.cluster says so.
+template <class Kernel, class... Args>
+static cudaError_t launch_splits(Kernel kernel, const DecodeParams& p, int threads, size_t smem,
+                                 cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.splits, p.Hkv, p.B);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  if (p.cluster) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Warps per CTA of the tensor-core kernel. Four warps (two CTAs resident per SM, K/V rings of
-// 96 KB each at D = 128) by default. When the grid is more than one wave of such CTAs but fits
-// in one wave of half-sized ones (four resident per SM, same bytes in flight per SM), two warps:
-// 512 CTAs on 148 SMs are 1.73 waves of the large shape, whose second wave leaves a quarter of
-// the machine idle, but a single resident grid of the small one.
-static int mma_warps_per_cta(int64_t ctas) {
-  const int sms = device_sm_count();
-  return (ctas > 2ll * sms && ctas <= 4ll * sms) ? 2 : 4;
-}
-
-template <int D, bool PAGED, bool HAS_MOD, int WARPS>
-static int launch_decode_mma_w(const DecodeParams& p, int G, cudaStream_t st, size_t table_bytes) {
-  dim3 grid(p.splits, p.Hkv, p.B);
-  // page ids + the per-warp K/V rings (the warp-merge area reuses the rings)
-  const size_t ring = static_cast<size_t>(WARPS) * kMmaStages * 2 * 16 * D * 2;
-  const size_t merge = static_cast<size_t>(WARPS) * G * (D + 2) * sizeof(float);
-  const size_t smem = table_bytes + (ring > merge ? ring : merge);
-  static thread_local int configured_dev = -1;
+// Per kernel, thread and device: shared memory beyond 48 KB and clusters beyond 8 CTAs are opted in to.
+template <class Kernel>
+static int configure_decode(Kernel kernel, int smem, int& configured_dev) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (configured_dev != dev) {
-    cudaError_t e = cudaFuncSetAttribute(decode_mma_kernel<D, PAGED, HAS_MOD, WARPS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    if (e != cudaSuccess) {
-      set_cuda_error(e, "cudaFuncSetAttribute(decode_mma_kernel)");
-      return LF_ERR_CUDA;
-    }
-    configured_dev = dev;
+  if (configured_dev == dev) return LF_OK;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) {
+    set_cuda_error(e, "cudaFuncSetAttribute(decode kernel)");
+    return LF_ERR_CUDA;
   }
-  decode_mma_kernel<D, PAGED, HAS_MOD, WARPS><<<grid, WARPS * 32, smem, st>>>(p, G);
-  return check_launch("decode_mma_kernel");
+  configured_dev = dev;
+  return LF_OK;
+}
+
+static int launched(cudaError_t e, const char* where) {
+  if (e == cudaSuccess) return check_launch(where);
+  cudaGetLastError();
+  set_cuda_error(e, where);
+  return LF_ERR_CUDA;
+}
+
+template <int D, bool PAGED, int MODS, bool WIDE_P, int WARPS, int STAGES>
+static int launch_decode_w(DecodeParams p, int G, cudaStream_t st, size_t table_bytes) {
+  // page ids + the per-warp K/V rings (the warp-merge area and the partial reuse the rings)
+  const size_t ring = static_cast<size_t>(WARPS) * STAGES * 2 * 16 * D * 2;
+  const size_t merge = static_cast<size_t>(WARPS + 1) * G * (D + 2) * sizeof(float);
+  const size_t smem = table_bytes + (ring > merge ? ring : merge);
+  p.part_off = static_cast<int32_t>(table_bytes + WARPS * static_cast<size_t>(G) * (D + 2) * 4);
+  static thread_local int configured_dev = -1;
+  const auto kernel = decode_mma_kernel<D, PAGED, MODS, WARPS, STAGES, WIDE_P>;
+  const int rc = configure_decode(kernel, 224 * 1024, configured_dev);
+  if (rc != LF_OK) return rc;
+  return launched(launch_splits(kernel, p, WARPS * 32, smem, st, p, G), "decode_mma_kernel");
+}
+
+template <int D, bool PAGED, int MODS, bool WIDE_P>
+static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, size_t table_bytes) {
+  const int64_t ctas = static_cast<int64_t>(p.splits) * p.Hkv * p.B;
+  const int sms = device_sm_count();
+  // Warps and ring depth, by how full the machine is (times: B200, D = 128, G = 4 paged):
+  //   one CTA per SM at most: eight warps, since four do not keep up with HBM on their own (128 units
+  //     of 8190 keys 96 -> 83 us), except that eights and sixteens of such CTAs find no place for their
+  //     clusters (16 units of 8190 keys 23 us in eights of four warps, 29 of eight);
+  //   otherwise four, two CTAs resident per SM (K/V rings of 96 KB each);
+  //   up to three CTAs per SM: two-stage rings, so that they are all resident (320 units of 1001 keys
+  //     35 -> 32 us);
+  //   up to four: half-sized CTAs, for the same reason.
+  if (ctas * 10 <= 9ll * sms && p.splits <= 4)
+    return launch_decode_w<D, PAGED, MODS, WIDE_P, 8, 3>(p, G, st, table_bytes);
+  if (ctas <= 2ll * sms || ctas > 4ll * sms)
+    return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 3>(p, G, st, table_bytes);
+  if (ctas <= 3ll * sms)
+    return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 2>(p, G, st, table_bytes);
+  return launch_decode_w<D, PAGED, MODS, WIDE_P, 2, 3>(p, G, st, table_bytes);
 }
 
 template <int D, bool PAGED>
-static int launch_decode_mma(const DecodeParams& p, int G, cudaStream_t st, size_t smem) {
-  // `smem` arrives as warp-merge area (sized for four warps) + block-table slices.
-  const size_t table_bytes = smem - static_cast<size_t>(kDecodeWarps) * G * (D + 2) * sizeof(float);
-  const int warps = mma_warps_per_cta(static_cast<int64_t>(p.splits) * p.Hkv * p.B);
-  if (p.mods.n > 0) {
-    return warps == 2 ? launch_decode_mma_w<D, PAGED, true, 2>(p, G, st, table_bytes)
-                      : launch_decode_mma_w<D, PAGED, true, 4>(p, G, st, table_bytes);
-  }
-  return warps == 2 ? launch_decode_mma_w<D, PAGED, false, 2>(p, G, st, table_bytes)
-                    : launch_decode_mma_w<D, PAGED, false, 4>(p, G, st, table_bytes);
-}
-
-// Dense caches with one or two query rows per kv head stay on the FMA kernel (it already
-// streams at HBM speed there); everything else runs on the tensor-core kernel.
-template <int D, bool PAGED>
-static int launch_decode(const DecodeParams& p, int G, cudaStream_t st, size_t smem) {
-  if (uses_mma_kernel(G, PAGED)) return launch_decode_mma<D, PAGED>(p, G, st, smem);
-  switch (G) {
-    case 1: return launch_decode_g<D, 1, PAGED>(p, st, smem);
-    case 2: return launch_decode_g<D, 2, PAGED>(p, st, smem);
-    default: return LF_ERR_UNSUPPORTED;
-  }
+static int launch_decode(const DecodeParams& p, int G, int mods, cudaStream_t st,
+                         size_t table_bytes) {
+  auto with_mods = [&](auto m) {
+    constexpr int kMods = decltype(m)::value;
+    if constexpr (!PAGED)
+      if (G <= 2) return launch_decode_shape<D, PAGED, kMods, true>(p, G, st, table_bytes);
+    return launch_decode_shape<D, PAGED, kMods, false>(p, G, st, table_bytes);
+  };
+  if (mods == kModsNone) return with_mods(std::integral_constant<int, kModsNone>{});
+  if (mods == kModsSoftcap) return with_mods(std::integral_constant<int, kModsSoftcap>{});
+  return with_mods(std::integral_constant<int, kModsGeneric>{});
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -885,10 +748,10 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
   if (splits > 32) return LF_ERR_TOO_LARGE;
   if (splits == 0)
     splits = choose_splits(a->B, a->Hkv, a->G, a->Skv, a->D, paged ? a->page_size : 0);
-  // Token chunk per split: a multiple of 64 (and of the page size when that is a power of
-  // two up to 64), so a split never starts in the middle of a warp's token batch.
-  int chunk = round_up((a->Skv + splits - 1) / splits, 64);
-  splits = (a->Skv + chunk - 1) / chunk;
+  // Token chunk per split: a multiple of 16, so a split never starts in the middle of a warp's token
+  // batch. Where the rounding leaves the last splits empty the count stays as it is (a power of two
+  // makes the better cluster); their partials have weight zero.
+  const int chunk = round_up((a->Skv + splits - 1) / splits, 16);
   if (splits > 1) {
     const size_t need = lf_decode_workspace_bytes(a->B, a->Hkv, a->G, a->D, splits);
     if (!a->workspace || a->workspace_bytes < need) return LF_ERR_WORKSPACE;
@@ -930,28 +793,52 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
     p.mods.arg[i] = i < a->n_mod ? a->mod_arg[i] : 0.f;
   }
 
+  // A softcap chain, (MUL|DIV)* TANH (MUL|DIV)*, folds into two multipliers.
+  int mods = a->n_mod > 0 ? kModsGeneric : kModsNone;
+  p.cap = 0.f;
+  p.part_off = 0;
+  {
+    int i = 0;
+    float pre = a->scale, post = kLog2e;
+    auto fold = [&](float& x) {
+      for (; i < a->n_mod && (a->mod_op[i] == LF_MOD_MUL || a->mod_op[i] == LF_MOD_DIV); ++i)
+        x = a->mod_op[i] == LF_MOD_MUL ? x * a->mod_arg[i] : x / a->mod_arg[i];
+    };
+    fold(pre);
+    if (i < a->n_mod && a->mod_op[i] == LF_MOD_TANH) {
+      ++i;
+      fold(post);
+      if (i == a->n_mod) {
+        mods = kModsSoftcap;
+        p.scale = pre;
+        p.cap = post;
+      }
+    }
+  }
+  // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
+  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups.
+  p.cluster = splits > 1 && splits <= kMaxCluster &&
+              static_cast<int64_t>(splits) * a->Hkv * a->B <= 8ll * device_sm_count();
+
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  size_t smem = static_cast<size_t>(kDecodeWarps) * a->G * (a->D + 2) * sizeof(float);
+  size_t table_bytes = 0;
   if (paged) {
     // A split's block-table slice lives in shared memory next to the K/V rings. The automatic
     // split count already keeps it small enough; an explicit count that does not is refused
     // (pass a larger `splits`, or 0).
-    const size_t table_bytes = table_smem_bytes(chunk, p.page_size);
+    table_bytes = table_smem_bytes(chunk, p.page_size);
     if (table_bytes > kMaxTableBytes) return LF_ERR_TOO_LARGE;
-    smem += table_bytes;
-  } else if (smem > 48 * 1024) {
-    return LF_ERR_TOO_LARGE;
   }
 
   int rc;
   if (a->D == 128)
-    rc = paged ? launch_decode<128, true>(p, a->G, st, smem)
-               : launch_decode<128, false>(p, a->G, st, smem);
+    rc = paged ? launch_decode<128, true>(p, a->G, mods, st, table_bytes)
+               : launch_decode<128, false>(p, a->G, mods, st, table_bytes);
   else
-    rc = paged ? launch_decode<64, true>(p, a->G, st, smem)
-               : launch_decode<64, false>(p, a->G, st, smem);
+    rc = paged ? launch_decode<64, true>(p, a->G, mods, st, table_bytes)
+               : launch_decode<64, false>(p, a->G, mods, st, table_bytes);
   if (rc != LF_OK) return rc;
-  if (splits > 1)
+  if (splits > 1 && !p.cluster)
     rc = lf_combine_f32(p.part_o, p.part_ml, a->out, a->B, a->Hkv, a->G, a->D, splits,
                         a->o_stride, stream);
   return rc;

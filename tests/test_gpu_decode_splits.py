@@ -1,0 +1,72 @@
+"""Decode where its splits, CTA shapes and score functions change: clusters of 2 to 16 that merge in
+shared memory (the last splits ragged or empty, block-table slices of different padding), the combine
+kernel beyond 16, eight, four and two warps per CTA, the folded softcap beside the interpreted chain,
+and P at full precision where one or two query rows share a kv head."""
+import pytest
+import torch
+
+from loopfuse_b200 import functional as F, spec as S
+from oracle import attention_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+MODS = {
+    "none": [],
+    "softcap": [S.ScoreMod(S.MOD_DIV, 30.0), S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_MUL, 30.0)],
+    "chain": [S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_ADD, 0.5), S.ScoreMod(S.MOD_MUL, 3.0)],
+}
+
+
+def want_of(q, k, v, mods):
+    s = (q.double() @ k.double().transpose(-1, -2)) * q.shape[-1] ** -0.5
+    if mods == "softcap":
+        s = torch.tanh(s / 30.0) * 30.0
+    elif mods == "chain":
+        s = (torch.tanh(s) + 0.5) * 3.0
+    return torch.softmax(s, -1) @ v.double()
+
+
+def check(out, want, v, mods, wide_p):
+    """Half an ulp of the bf16 result, 2^-8 |o|; P in bf16, 2^-9 of weights that sum to one, times
+    max |v|; tanh.approx, 2^-11 of its range, moves a logit by 30 * 2^-11 (3 * 2^-11 for the chain)
+    and with it every weight by that fraction, twice (its own and the sum's)."""
+    vmax = v.abs().max().item()
+    tanh = {"none": 0.0, "softcap": 30.0, "chain": 3.0}[mods] * 2.0 ** -11 * 2.0
+    bound = 2.0 ** -8 * want.abs() + vmax * ((2.0 ** -15 if wide_p else 2.0 ** -9) + tanh)
+    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("mods", ["none", "softcap", "chain"])
+@pytest.mark.parametrize("B,Hkv,G,Skv,splits", [
+    (1, 1, 1, 1, 0), (1, 2, 2, 3, 2), (2, 3, 1, 257, 2), (2, 3, 8, 515, 4), (1, 3, 2, 2100, 16),
+    (1, 2, 4, 2100, 8), (2, 5, 4, 700, 20), (40, 8, 1, 65, 1), (56, 8, 2, 33, 1), (17, 16, 4, 130, 2),
+])
+def test_dense_splits(B, Hkv, G, Skv, splits, mods, D):
+    g = torch.Generator().manual_seed(5)
+    q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, mods=MODS[mods],
+                             splits=splits)
+    check(out, want_of(q, k, v, mods), v, mods, wide_p=G <= 2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("P,Skv,splits", [(16, 1, 0), (16, 1000, 2), (16, 2111, 16), (1, 517, 4),
+                                          (24, 700, 8), (64, 1217, 8), (16, 1203, 20)])
+def test_paged_splits(P, Skv, splits, D):
+    B, Hkv, G = 2, 3, 4
+    g = torch.Generator().manual_seed(6)
+    blocks = -(-Skv // P)
+    q = torch.randn(B, Hkv, G, D, generator=g).bfloat16()
+    kp, vp = [torch.randn(B * blocks + 3, P, Hkv, D, generator=g).bfloat16() for _ in range(2)]
+    kt, vt = [torch.randperm(B * blocks + 3, generator=g)[:B * blocks].view(B, blocks).int()
+              for _ in range(2)]
+    for table_v in (None, vt):
+        st = F.new_status("cuda")
+        out = F.paged_decode_attention(q.cuda(), kp.cuda(), vp.cuda(), kt.cuda(), seq_len=Skv,
+                                       block_table_v=None if table_v is None else table_v.cuda(),
+                                       scale=D ** -0.5, splits=splits, status=st)
+        F.check_status(st)
+        k = O.paged_kv_ref(kp, kt)[:, :, :Skv]
+        v = O.paged_kv_ref(vp, kt if table_v is None else table_v)[:, :, :Skv]
+        check(out, want_of(q, k, v, "none"), v, "none", wide_p=False)
