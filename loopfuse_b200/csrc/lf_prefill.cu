@@ -277,11 +277,12 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table entries,
     // then gather the rows) as tile::gather4 loads of four rows x 64 columns, straight into the
     // 128-byte-swizzled tile; the pool is seen as a 2-D tensor of token rows, and tokens past Skv ask
-    // for a row past its end (zeros). A stage holds two tiles: the lower half of the warp looks up the
-    // first one's tokens, four per lane, the upper half the second one's, one stage ahead; the row
-    // numbers go through shared memory to the elected lane, which issues all gathers. (Issued by the
-    // lanes that hold the numbers, one diverged lane after the other, a gather took ~200 clocks.)
-    // Two warps share the gathers of every tile: eight each.
+    // for a row past its end (zeros). Two warps share the gathers of every tile: eight each, issued by
+    // the elected lane. (Issued by the lanes that hold the row numbers, one diverged lane after the
+    // other, a gather took ~200 clocks.) Next to the softmax warps these two get few issue slots, so
+    // the look-up is done for eight tiles at a time: a token per lane and tile, its table entry
+    // requested a window ahead, its checked row number left in shared memory. (Tile by tile the
+    // look-up took 1500 clocks of a stage, as much as the gathers and more than the softmax.)
     // Nothing waits for the rows here, so the whole ring is in flight; the cp.async form below has
     // two stages in flight and a look-up in front of each.
     const bool elected = elect_one_sync();
@@ -298,49 +299,52 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     }
     __syncwarp();
     const int n_rows = p.n_pages * p.page_size;
-    int4* row_ids = reinterpret_cast<int4*>(smem + 512) + part * 16;  // [tile of the stage][8]
-    static_assert(sizeof(PrefillBarriers) <= 512, "row numbers behind the barriers");
+    constexpr int kWindow = 8;  // tiles
+    // [K or V][tile of the window][32 tokens] of this warp, in the output staging of warps 4..7: their
+    // tile is the last to finish, after the last gather.
+    int* const row_ids = reinterpret_cast<int*>(sStage + 4 * 2048) + part * (2 * kWindow * 32);
+    static_assert(2 * 2 * kWindow * 32 * 4 <= 4 * 2048, "row numbers in the staging of four warps");
     auto page_of = [&](int t) { return p.page_shift >= 0 ? (t >> p.page_shift) : (t / p.page_size); };
-    const int quad = (part * 8 + (lane & 7)) * 4;  // first of this lane's four tokens in its tile
-    // A stage is tile ja of K (or V, `first_is_v`) and tile jb of K (< 0: none). This lane's tile:
-    auto my_tile = [&](int ja, int jb) { return lane < 16 ? ja : jb; };
-    auto my_paged = [&](bool first_is_v) { return (p.paged >> (lane < 16 && first_is_v ? 1 : 0)) & 1; };
-    // Table entries of this lane's tokens, loaded but not looked at.
-    auto look_up = [&](bool first_is_v, int ja, int jb) -> int4 {
-      const int j = my_tile(ja, jb);
-      int id[4] = {0, 0, 0, 0};
-      if (j >= 0 && !(lane & 8) && my_paged(first_is_v)) {
-        const int32_t* table = (lane < 16 && first_is_v ? p.v_table : p.k_table) +
-                               static_cast<int64_t>(b) * p.bt_stride;
+    auto is_paged = [&](bool is_v) { return ((p.paged >> (is_v ? 1 : 0)) & 1) != 0; };
+    const int t_end = min(p.Skv, hi * kTileK);
+    // Token of this lane in tile j (each warp has half of the 64).
+    auto token = [&](int j) { return j * kTileK + part * 32 + lane; };
+    int entry_k[kWindow], entry_v[kWindow];  // table entries of the next window, not looked at
+    auto request = [&](bool is_v, int w, int (&entry)[kWindow]) {
+      const int32_t* table = (is_v ? p.v_table : p.k_table) + static_cast<int64_t>(b) * p.bt_stride;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = j * kTileK + quad + e;
-          if (t < p.Skv) id[e] = table[page_of(t)];
-        }
+      for (int e = 0; e < kWindow; ++e) {
+        const int t = token(lo + w * kWindow + e);
+        entry[e] = t < t_end ? table[page_of(t)] : 0;
       }
-      return make_int4(id[0], id[1], id[2], id[3]);
+    };
+    // Row numbers of window w from its entries, then the next window's request.
+    auto look_up = [&](bool is_v, int w, int (&entry)[kWindow]) {
+      __syncwarp();  // (the elected lane has read the last window's)
+#pragma unroll
+      for (int e = 0; e < kWindow; ++e) {
+        const int t = token(lo + w * kWindow + e);
+        int pg = entry[e];
+        if (pg < 0 || pg >= p.n_pages) {
+          if (p.status) atomicExch(p.status, LF_DEV_BAD_PAGE);
+          pg = 0;
+        }
+        const int row = pg * p.page_size + (t - page_of(t) * p.page_size);
+        row_ids[(is_v ? kWindow * 32 : 0) + e * 32 + lane] = t < t_end ? row : n_rows;
+      }
+      __syncwarp();
+      request(is_v, w + 1, entry);
     };
     int n = 0;
     bool ok = true;
-    auto load_pair = [&](bool first_is_v, int ja, int jb, const int4& id) {
+    // A stage is tile ja of K (or V, `first_is_v`) and tile jb of K (< 0: none).
+    auto load_pair = [&](bool first_is_v, int ja, int jb) {
       if (!ok) return;
-      {  // rows of this lane's tokens, checked
-        const int j = my_tile(ja, jb);
-        auto row_of = [&](int t, int32_t pg) -> int {
-          if (j < 0 || t >= p.Skv) return n_rows;
-          if (pg < 0 || pg >= p.n_pages) {
-            if (p.status && my_paged(first_is_v)) atomicExch(p.status, LF_DEV_BAD_PAGE);
-            pg = 0;
-          }
-          return pg * p.page_size + (t - page_of(t) * p.page_size);
-        };
-        const int t = j * kTileK + quad;
-        const int4 r = make_int4(row_of(t, id.x), row_of(t + 1, id.y), row_of(t + 2, id.z),
-                                 row_of(t + 3, id.w));
-        __syncwarp();  // (the elected lane has read the last stage's)
-        if (!(lane & 8)) row_ids[(lane >> 4) * 8 + (lane & 7)] = r;
-        __syncwarp();
-      }
+      if (first_is_v && is_paged(true) && (ja - lo) % kWindow == 0)
+        look_up(true, (ja - lo) / kWindow, entry_v);
+      if (!first_is_v && is_paged(false)) look_up(false, 0, entry_k);
+      if (first_is_v && is_paged(false) && jb >= 0 && (jb - lo) % kWindow == 0)
+        look_up(false, (jb - lo) / kWindow, entry_k);
       const int stage = n % kStages;
       const uint32_t parity = ((n / kStages) & 1) ^ 1;
       ++n;
@@ -351,14 +355,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       }
       if (elected) {
         auto bytes_of = [&](bool is_v) -> uint32_t {
-          return ((p.paged >> (is_v ? 1 : 0)) & 1) ? kKVTileBytes / 2 : part == 0 ? kKVTileBytes : 0u;
+          return is_paged(is_v) ? kKVTileBytes / 2 : part == 0 ? kKVTileBytes : 0u;
         };
         const uint32_t tx = bytes_of(first_is_v) + (jb >= 0 ? bytes_of(false) : 0u);
         if (tx) mbar_arrive_expect_tx(&bars->kv_full[stage], tx);
         else mbar_arrive(&bars->kv_full[stage]);
-        auto load = [&](bool is_v, int j, const int4* ids, unsigned char* dst) {
+        auto load = [&](bool is_v, int j, unsigned char* dst) {
           const CUtensorMap* tma = is_v ? &tmap_v : &tmap_k;
-          if ((p.paged >> (is_v ? 1 : 0)) & 1) {
+          if (is_paged(is_v)) {
+            const int4* ids = reinterpret_cast<const int4*>(
+                row_ids + (is_v ? kWindow * 32 : 0) + ((j - lo) % kWindow) * 32);
             const int x = hkv * static_cast<int>(is_v ? p.vp_stride[2] : p.kp_stride[2]);
             const uint32_t d = smem_u32(dst);
 #pragma unroll 8
@@ -377,20 +383,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           }
         };
         unsigned char* dst = sKV + stage * (2 * kKVTileBytes);
-        load(first_is_v, ja, row_ids, dst);
-        if (jb >= 0) load(false, jb, row_ids + 8, dst + kKVTileBytes);
+        load(first_is_v, ja, dst);
+        if (jb >= 0) load(false, jb, dst + kKVTileBytes);
       }
     };
     if (hi > lo) {
       auto second = [&](int j) { return j < hi ? j : -1; };
-      int4 id = look_up(false, lo, second(lo + 1));
-      int4 next = look_up(true, lo, second(lo + 2));
-      load_pair(false, lo, second(lo + 1), id);
-      for (int j = lo; j < hi; ++j) {
-        id = next;
-        if (j + 1 < hi) next = look_up(true, j + 1, second(j + 3));
-        load_pair(true, j, second(j + 2), id);
-      }
+      if (is_paged(false)) request(false, 0, entry_k);
+      if (is_paged(true)) request(true, 0, entry_v);
+      load_pair(false, lo, second(lo + 1));
+      for (int j = lo; j < hi; ++j) load_pair(true, j, second(j + 2));
     }
   } else if (warp == kProducerWarp && p.paged) {
     // ---------------- producer with a paged K and / or V ----------------
