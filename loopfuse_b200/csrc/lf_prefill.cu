@@ -225,17 +225,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     h = hb - b * p.Hq;
   }
   const int hkv = static_cast<int>(p.div_group.div(h));
-  // (`single`: one query tile per CTA; the second tile slot stays empty. Chosen by the host for
-  // problems whose tiles are all resident at once, one per SM: each has the tensor pipe and the
-  // issue slots of an SM to itself, and the time of the launch is that of its longest tile.)
-  const int iq0 = p.single ? pair : pair * 2;
+  // (`single`: one query tile per CTA. Its key blocks alternate between the two slots, which have a
+  // softmax warp group, S buffers and an O each and are merged at the end; chosen by the host.)
+  const bool split = p.single;
+  const int iq0 = split ? pair : pair * 2;
 
   int lo_t[2], hi_t[2];
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0, &lo_t[0],
              &hi_t[0]);
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0 + 1,
              &lo_t[1], &hi_t[1]);
-  const bool tile_valid[2] = {iq0 * kTileQ < p.Sq, !p.single && (iq0 + 1) * kTileQ < p.Sq};
+  const bool tile_valid[2] = {iq0 * kTileQ < p.Sq, !split && (iq0 + 1) * kTileQ < p.Sq};
   const bool has_work[2] = {tile_valid[0] && hi_t[0] > lo_t[0], tile_valid[1] && hi_t[1] > lo_t[1]};
   int lo = 0, hi = 0;
   if (has_work[0] && has_work[1]) {
@@ -597,9 +597,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     // issues MMAs and commits.
     if (hi > lo) {
       const int t = warp - kMmaWarp0;
+      const int tq = split ? 0 : t;  // query tile of this slot
       const bool elected = elect_one_sync();
       bool ok = true;
-      if (has_work[t] && !mbar_wait(&bars->q_full[t], 0)) {
+      if (has_work[tq] && !mbar_wait(&bars->q_full[tq], 0)) {
         report_timeout(p.status, 2);
         ok = false;
       }
@@ -607,14 +608,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       // units, no carry out of the 14-bit field since shared memory ends below 256 KB).
       constexpr uint32_t kStageUnits = (2 * kKVTileBytes) >> 4;  // a stage is a pair of tiles
       constexpr uint32_t kHalfUnits = kKVTileBytes >> 4;
-      const uint64_t qdesc = make_smem_desc_sw128(smem_u32(sQ) + t * kQTileBytes, 16, 1024);
+      const uint64_t qdesc = make_smem_desc_sw128(smem_u32(sQ) + tq * kQTileBytes, 16, 1024);
       const uint64_t kdesc0 = make_smem_desc_sw128(smem_u32(sKV), 16, 1024);
       const uint64_t vdesc0 = make_smem_desc_sw128(smem_u32(sKV), kKVBlockBytes, 1024);
       const uint32_t s_col = tmem_base + t * 128;
       const uint32_t o_col = tmem_base + kColO + t * 128;
       int n = 0;  // ring position, walks the same sequence as the producer
 
-      auto active = [&](int j) { return has_work[t] && j >= lo_t[t] && j < hi_t[t]; };
+      auto active = [&](int j) {
+        return split ? ((j - lo) & 1) == t : has_work[t] && j >= lo_t[t] && j < hi_t[t];
+      };
+      auto block_of = [&](int j) { return split ? (j - lo) >> 1 : j - lo_t[t]; };  // of this slot
       auto wait_stage = [&](int where) -> int {  // next ring stage, waited full; -1 on time-out
         const int stage = n % kStages;
         const uint32_t parity = (n / kStages) & 1;
@@ -628,7 +632,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       };
       // `half` selects the first or second tile of the stage.
       auto issue_qk = [&](int stage, int half, int j) {
-        const int buf = (j - lo_t[t]) & 1;
+        const int buf = block_of(j) & 1;
         const uint64_t kd = kdesc0 + static_cast<uint64_t>(stage * kStageUnits + half * kHalfUnits);
         const uint32_t d = s_col + buf * 64;
         if (elected) {
@@ -672,13 +676,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           __syncwarp();
         }
       }
-      const int nblk_t = has_work[t] ? hi_t[t] - lo_t[t] : 0;
+      const int nblk_t = split ? (hi - lo + 1 - t) >> 1 : has_work[t] ? hi_t[t] - lo_t[t] : 0;
       for (int j = lo; j < hi && ok; ++j) {
         const int st = wait_stage(4);  // {V(j), K(j+2)}
         if (st < 0) break;
         tc_fence_after();
+        // (Split: K(j+2) is this slot's next block, not the one after it; its scores are made
+        // while the softmax of block j runs. Its buffer was read by the slot's last PV.)
+        if (split && j + 2 < hi && active(j)) issue_qk(st, 1, j + 2);
         if (active(j)) {
-          const int kt = j - lo_t[t];
+          const int kt = block_of(j);
           if (!mbar_wait(&bars->p_full[t][kt & 1], (kt >> 1) & 1)) {
             report_timeout(p.status, 6 + t);
             ok = false;
@@ -693,16 +700,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             if (kt == nblk_t - 1) tc_commit(&bars->o_final[t]);
           }
         }
-        if (j + 2 < hi && active(j + 2)) issue_qk(st, 1, j + 2);
+        if (!split && j + 2 < hi && active(j + 2)) issue_qk(st, 1, j + 2);
         if (elected) tc_commit(&bars->kv_empty[st]);
         __syncwarp();
       }
     }
   } else if (warp < kSoftmaxWarps) {
     // ---------------- softmax warps ----------------
-    const int t = warp >> 2;                 // query tile of this warp group
+    const int t = warp >> 2;                 // slot of this warp group
+    const int tq = split ? 0 : t;            // and its query tile
     const int row = (warp & 3) * 32 + lane;  // row inside the tile == tensor-memory lane
-    const int grow = (iq0 + t) * kTileQ + row;
+    const int grow = (iq0 + tq) * kTileQ + row;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t s_base = tmem_base + lane_addr + t * 128;
     const uint32_t o_addr = tmem_base + lane_addr + kColO + t * 128;
@@ -713,7 +721,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       p.dbg_ranges[idx + 1] = hi_t[t];
     }
 
-    if (has_work[t]) {
+    if (has_work[tq]) {
       // Visible column interval of this row: [c_lo, c_hi].
       int c_hi = p.Skv - 1;
       int c_lo = 0;
@@ -724,7 +732,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       float m_used = -INFINITY;  // max the stored P and O are scaled by (log2 domain)
       float l_run = 0.f;
       bool ok = true;
-      const int nblk = hi_t[t] - lo_t[t];
+      // Block k of this slot is block first + k * step of the tile.
+      const int first = lo_t[tq] + (split ? t : 0), step = split ? 2 : 1;
+      const int nblk = split ? (hi - lo + 1 - t) >> 1 : hi_t[t] - lo_t[t];
       // Bias mode: this row's 64 bias values of a block (128 contiguous bytes) are requested a block
       // ahead, so that their latency lies under the exp2 pass and the hand-shake; read when the
       // scores were there, they cost a round trip to HBM per block. (Rows past Sq read the last
@@ -735,7 +745,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
                                   static_cast<int64_t>(min(grow, p.Sq - 1)) * p.bias_stride[2]
                             : nullptr;
       auto request_bias = [&](int k) {
-        const int col = (lo_t[t] + k) * kTileK;
+        const int col = (first + k * step) * kTileK;
         if (k >= nblk || col + kTileK > p.Skv ||
             !LF_BOUNDS(col >= 0 && b * p.Hq + h < p.n_heads, p.status, 61))
           return;
@@ -752,7 +762,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       };
       if constexpr (MODE == kModeBias) request_bias(0);
       for (int k = 0; k < nblk; ++k) {
-        const int c0 = (lo_t[t] + k) * kTileK;
+        const int c0 = (first + k * step) * kTileK;
         const int buf = k & 1;
         const uint32_t s_addr = s_base + buf * 64;
         if (!mbar_wait(&bars->s_full[t][buf], (k >> 1) & 1)) {
@@ -1073,37 +1083,81 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       }
 
       // Epilogue: O_t / l -> bf16 -> global (one row per thread).
-      if (ok) {
+      if (ok && nblk > 0) {
         if (!mbar_wait(&bars->o_final[t], 0)) {
           report_timeout(p.status, 10 + t);
           ok = false;
         }
       }
+      // Split: the slots tell each other their reference and sum, and each finishes half of the
+      // columns from both accumulators (the same tensor-memory lanes, so a warp reads the other
+      // slot's directly). A slot without a block has sum 0 and an accumulator nobody wrote.
+      float inv, w_own = 1.f, w_other = 0.f;
+      bool two = false;  // the other slot has something to add
+      if (split) {
+        float2* ml = reinterpret_cast<float2*>(sStage);  // [slot][row]
+        ml[t * 128 + row] = make_float2(m_used, l_run);
+        tc_fence_before();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const float2 other = ml[(t ^ 1) * 128 + row];
+        asm volatile("bar.sync 1, 256;" ::: "memory");  // (the staging buffers start there)
+        two = hi - lo > 1;
+        const float m_all = fmaxf(m_used, other.x);
+        const float m_safe = m_all == -INFINITY ? 0.f : m_all;
+        w_own = ex2_approx(m_used - m_safe);
+        w_other = ex2_approx(other.x - m_safe);
+        inv = 1.f / (l_run * w_own + other.y * w_other);
+        w_own *= inv;
+        w_other *= inv;
+      } else {
+        inv = 1.f / l_run;
+      }
+      const float out_scale = split ? 1.f : inv;
       if (ok) {
         tc_fence_after();
-        const float inv = 1.f / l_run;
         // Each warp owns 32 rows. A 32-column chunk (64 bytes per row) goes through a swizzled
         // 2 KB buffer of the warp so that one store instruction writes eight 64-byte row
         // segments instead of thirty-two 16-byte pieces.
         unsigned char* stage = sStage + warp * 2048;
         __nv_bfloat16* obase = p.out + b * p.o_stride[0] + h * p.o_stride[1];
-        const int row0 = (iq0 + t) * kTileQ + (warp & 3) * 32;  // first global row of the warp
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
+        const int row0 = (iq0 + tq) * kTileQ + (warp & 3) * 32;  // first global row of the warp
+        const int c_first = split ? t * (D / 64) : 0, c_end = split ? (t + 1) * (D / 64) : D / 32;
+#pragma unroll 1
+        for (int c = c_first; c < c_end; ++c) {
           uint32_t orr[32];
-          tmem_ld_32x32b_x32(o_addr + c * 32, orr);
-          tmem_wait_ld();
+          if (!split) {
+            tmem_ld_32x32b_x32(o_addr + c * 32, orr);
+            tmem_wait_ld();
+          } else {
+            const uint32_t other_addr = o_addr + (t ? -128 : 128);
+            if (two) {
+              uint32_t oth[32];
+              tmem_ld_32x32b_x32(o_addr + c * 32, orr);
+              tmem_ld_32x32b_x32(other_addr + c * 32, oth);
+              tmem_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                orr[i] = __float_as_uint(__uint_as_float(orr[i]) * w_own +
+                                         __uint_as_float(oth[i]) * w_other);
+            } else {
+              tmem_ld_32x32b_x32(tmem_base + lane_addr + kColO + c * 32, orr);  // slot 0 has it all
+              tmem_wait_ld();
+              const float w = t == 0 ? w_own : w_other;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * w);
+            }
+          }
 #pragma unroll
           for (int q = 0; q < 4; ++q) {  // piece q of row r sits at position q ^ ((r >> 1) & 3)
             uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(orr[8 * q]) * inv,
-                              __uint_as_float(orr[8 * q + 1]) * inv);
-            w.y = pack_bf16x2(__uint_as_float(orr[8 * q + 2]) * inv,
-                              __uint_as_float(orr[8 * q + 3]) * inv);
-            w.z = pack_bf16x2(__uint_as_float(orr[8 * q + 4]) * inv,
-                              __uint_as_float(orr[8 * q + 5]) * inv);
-            w.w = pack_bf16x2(__uint_as_float(orr[8 * q + 6]) * inv,
-                              __uint_as_float(orr[8 * q + 7]) * inv);
+            w.x = pack_bf16x2(__uint_as_float(orr[8 * q]) * out_scale,
+                              __uint_as_float(orr[8 * q + 1]) * out_scale);
+            w.y = pack_bf16x2(__uint_as_float(orr[8 * q + 2]) * out_scale,
+                              __uint_as_float(orr[8 * q + 3]) * out_scale);
+            w.z = pack_bf16x2(__uint_as_float(orr[8 * q + 4]) * out_scale,
+                              __uint_as_float(orr[8 * q + 5]) * out_scale);
+            w.w = pack_bf16x2(__uint_as_float(orr[8 * q + 6]) * out_scale,
+                              __uint_as_float(orr[8 * q + 7]) * out_scale);
             *reinterpret_cast<uint4*>(stage + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = w;
           }
           __syncwarp();
@@ -1311,11 +1365,30 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   static thread_local int sm_count = 0;
   if (sm_count == 0) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   PrefillParams pp = p;
-  // One query tile per CTA only where all the tiles are resident at once, one per SM. (With more
-  // tiles than SMs the second wave cost more than pairs do: 7 tiles x 32 heads, 4096 keys, D = 128:
-  // 102 us as 224 single tiles, 71 us as 128 pairs.)
-  pp.single =
-      (p.n_qtiles > 1 && static_cast<int64_t>(p.n_qtiles) * p.Hq * B <= sm_count) ? 1 : 0;
+  // One query tile per CTA, its key blocks split over the two slots:
+  //   - where all the tiles are resident at once, one per SM: half the steps of the longest tile (8
+  //     heads, 1024 queries, 8192 keys, D = 64: 111 -> 59 us);
+  //   - where one tile is all a head has;
+  //   - up to two tiles per SM, where pairs would leave the short ones' SMs idle while the longest
+  //     pair runs: a pair of tiles takes as many steps as its longer tile has blocks; single tiles,
+  //     longest first, the mean load, half of the shortest tile, and about five steps for the start
+  //     and end of the second CTA of an SM (causal, 16 heads, 2048 keys, D = 64: 34.9 -> 25.4 us;
+  //     7 tiles x 32 heads that see 3.4 to 4.1 thousand keys each: pairs 71 us, singles 75). With a
+  //     paged operand a step of singles gathers twice the rows: 1.4 steps.
+  // Above that pairs are the better: a K/V tile in shared memory serves two query tiles.
+  const int64_t n_tiles = static_cast<int64_t>(p.n_qtiles) * p.Hq * B;
+  pp.single = p.n_qtiles == 1 || n_tiles <= sm_count;
+  if (!pp.single && n_tiles <= 2ll * sm_count) {
+    int lo, hi;
+    skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, 0, &lo, &hi);
+    const int shortest = hi - lo;
+    skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1,
+               &lo, &hi);
+    const int longest = hi - lo;
+    const double singles = 0.25 * (shortest + longest) * static_cast<double>(n_tiles) / sm_count +
+                           0.5 * shortest;
+    pp.single = singles * (p.paged ? 1.4 : 1.0) + 5.0 < longest;
+  }
   // Order of the CTAs: the heaviest tiles of a group of heads, then the next lighter ones, ..., then
   // the next group. With a head's tiles next to each other the last head's longest tile started
   // when the rest was nearly done (causal B=1 Hq=32 Hkv=8 S=8192 D=128 535 -> 475

@@ -71,3 +71,30 @@ def test_paged_prefill_pool_layouts(P, Skv, heads_first, D):
     want = O.attention_ref(q, O.paged_kv_ref(kp, kt)[:, :, :Skv], O.paged_kv_ref(vp, vt)[:, :, :Skv],
                            batch_chunk=B)
     assert (out.float().cpu() - want).abs().max().item() <= TOL
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,offset", [
+    (1, 1, 1, 5, 5, 0),           # one block: the second slot has none
+    (1, 2, 1, 33, 150, 117),      # three blocks, two and one
+    (1, 3, 3, 257, 257, 0),       # tiles of two and four blocks and one row
+    (1, 2, 2, 384, 256, -200),    # rows and a tile that see nothing
+    (2, 160, 4, 70, 200, 130),    # more heads than SMs, one tile each
+    (3, 10, 5, 1100, 1100, 0),    # 270 tiles, singles although they are not all resident
+    (5, 10, 5, 1300, 1300, 0),    # pairs, two heads' worth of tiles per SM and more
+])
+def test_one_tile_split_over_both_slots(B, Hq, Hkv, Sq, Skv, offset, D):
+    """Each slot's rows grow past the other's reference (the second half of the keys scores far above
+    the first), so that the merge weighs them very differently."""
+    g = torch.Generator().manual_seed(8)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    q, k, v = mk(B, Hq, Sq, D), mk(B, Hkv, Skv, D), mk(B, Hkv, Skv, D)
+    k[:, :, Skv // 2::3] *= 6.0
+    st = F.new_status("cuda")
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
+                              mask_kind=S.MASK_CAUSAL, causal_offset=offset, status=st)
+    F.check_status(st)
+    want = O.attention_ref(q, k, v, mask="causal", offset=offset, batch_chunk=B)
+    got = out.float().cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert (got - want).nan_to_num().abs().max().item() <= TOL
