@@ -285,13 +285,20 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
           kp += RPI * ks;
           vp += RPI * vs;
         }
-      } else {  // (rows past the end of the split re-read its last token)
-#pragma unroll 4
+      } else {
+        // Rows that pages scatter: lane r < 16 finds K row r of the group, lane 16 + r V row r, and the
+        // lanes that copy a row get its place by shuffle. (With every lane looking up every row it
+        // copies: 416 units of 6443 one-token pages 300 us, now
+        // 217.) Rows past the end of the split re-read its
+        // last token.
+        const int tok = min(tg + (lane & 15), t_last);
+        const int64_t off = lane < 16 ? k_row(tok) - kbase : v_row(tok) - vbase;
+#pragma unroll
         for (int q = 0; q < 16 / RPI; ++q) {
-          const int tok = min(tg + r0 + q * RPI, t_last);
-          const uint32_t to = dst + q * RPI * kRowBytes + ((j0 ^ ((r0 + q * RPI) & 7)) << 4);
-          cp_async_16(to, k_row(tok) + 8 * j0);
-          cp_async_16(to + 16 * kRowBytes, v_row(tok) + 8 * j0);
+          const int r = r0 + q * RPI;
+          const uint32_t to = dst + q * RPI * kRowBytes + ((j0 ^ (r & 7)) << 4);
+          cp_async_16(to, kbase + __shfl_sync(0xffffffffu, off, r) + 8 * j0);
+          cp_async_16(to + 16 * kRowBytes, vbase + __shfl_sync(0xffffffffu, off, 16 + r) + 8 * j0);
         }
       }
     }
@@ -618,9 +625,9 @@ static int choose_splits(int B, int Hkv, int G, int Skv, int D, int page_size) {
   if (units * s * 5 < 3ll * sms && s <= 4 && Skv / (s * 4) >= kMinTokens &&
       units * s * 4 >= 2ll * sms)
     s = s == 4 ? 8 : s * 4;
-  // A grid of many waves gains from halves where the caches are long: its last wave is shorter (640
-  // units of 3001 keys 188 -> 166 us, 2048 units of 2048 keys 315 -> 307 us).
-  if (units >= 4ll * sms && Skv >= 2000) s = 2;
+  // A dense grid of many waves gains from halves where the caches are long: its last wave is shorter
+  // (2048 units of 2048 keys 308 -> 304 us; paged 314 -> 322, 800 units 120 -> 126).
+  if (page_size == 0 && units >= 6ll * sms + sms / 2 && Skv >= 2000) s = 2;
   if (page_size > 0) {
     // The block-table slice of a split must fit in shared memory (one-token pages at long
     // context): split further until it does.
@@ -700,14 +707,15 @@ static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, si
   //   otherwise four, two CTAs resident per SM (K/V rings of 96 KB each);
   //   up to three CTAs per SM: two-stage rings, so that they are all resident (320 units of 1001 keys
   //     35 -> 32 us);
-  //   up to four: half-sized CTAs, for the same reason.
+  //   up to five: half-sized CTAs as well, six resident (512 units of 2048 keys 87 -> 85 us, 640 of
+  //     3001 keys 171 -> 150); at D = 64, where the rings are half as large, three stages of up to four.
   if (ctas * 10 <= 9ll * sms && p.splits <= 4)
     return launch_decode_w<D, PAGED, MODS, WIDE_P, 8, 3>(p, G, st, table_bytes);
-  if (ctas <= 2ll * sms || ctas > 4ll * sms)
+  if (ctas <= 2ll * sms || ctas > (D == 128 ? 5ll : 4ll) * sms)
     return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 3>(p, G, st, table_bytes);
   if (ctas <= 3ll * sms)
     return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 2>(p, G, st, table_bytes);
-  return launch_decode_w<D, PAGED, MODS, WIDE_P, 2, 3>(p, G, st, table_bytes);
+  return launch_decode_w<D, PAGED, MODS, WIDE_P, 2, D == 128 ? 2 : 3>(p, G, st, table_bytes);
 }
 
 template <int D, bool PAGED>
