@@ -26,6 +26,8 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t x, uint32_t y) {
 
 // One thread adds one 16-byte piece; consecutive threads take consecutive pieces of a row.
 __global__ void __launch_bounds__(256) add_bf16_kernel(const AddParams p) {
+  pdl_trigger();
+  pdl_wait();
   for (int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; gid < p.total;
        gid += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>(gid % p.cpr);
@@ -77,6 +79,7 @@ extern "C" int lf_add_bf16(const void* a, const void* b, void* out, int32_t B, i
   int64_t blocks = (p.total + 255) / 256;
   const int64_t cap = static_cast<int64_t>(sms) * 32;  // a multiple of the SM count
   if (blocks > cap) blocks = cap;
-  add_bf16_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_pdl(add_bf16_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0,
+             static_cast<cudaStream_t>(stream), p);
   return check_launch("add_bf16_kernel");
 }

@@ -138,6 +138,7 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 template <int D, bool PAGED, int MODS, int WARPS, int STAGES, bool WIDE_P>
 __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     decode_mma_kernel(const DecodeParams p, const int G) {
+  pdl_wait();
   constexpr int KI = D / 32;  // 16-byte pieces of a K row per lane
   constexpr int VH = D / 64;  // 64-wide halves of a V row
   constexpr int NT = D / 8;   // output n-tiles (8 columns each)
@@ -405,6 +406,9 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     __syncwarp();  // every lane is done with this stage before it is refilled
   }
   cp_async_wait<0>();
+  // (Not earlier: the next launch's CTAs would take the places that this one's leave as they come,
+  // and crowd on some SMs. 512 units of 2048 keys 87 -> 94 us with the trigger at the top.)
+  pdl_trigger();
 
   if constexpr (WIDE_P) {  // rows 8 + g (same lane) and 2 + g hold the finer parts of row g
 #pragma unroll
@@ -484,6 +488,8 @@ __global__ void __launch_bounds__(128)
     combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                    __nv_bfloat16* __restrict__ out, int64_t units, int32_t Hkv, int32_t G,
                    int32_t splits, int64_t os0, int64_t os1, int64_t os2) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int EPL = D / 32;  // elements per lane
   const int64_t unit = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -646,14 +652,21 @@ static cudaError_t launch_splits(Kernel kernel, const DecodeParams& p, int threa
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
   if (p.cluster) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = p.splits;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  // Large grids wait for the kernel before them to leave the SMs: their CTAs are then dealt out
+  // evenly (512 units of 2048 keys 88 us, 90 when they start between another launch's last ones).
+  if (static_cast<int64_t>(p.splits) * p.Hkv * p.B <= 2ll * device_sm_count()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
   }
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
@@ -888,15 +901,13 @@ int lf_combine_f32(const float* part_o, const float* part_ml, void* out, int32_t
   const unsigned blocks = static_cast<unsigned>((units + 3) / 4);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (D == 128)
-    lf::combine_kernel<128><<<blocks, 128, 0, st>>>(part_o, part_ml,
-                                                    static_cast<__nv_bfloat16*>(out), units, Hkv,
-                                                    G, splits, o_stride[0], o_stride[1],
-                                                    o_stride[2]);
+    lf::launch_pdl(lf::combine_kernel<128>, dim3(blocks), 128, 0, st, part_o, part_ml,
+                   static_cast<__nv_bfloat16*>(out), units, Hkv, G, splits, o_stride[0],
+                   o_stride[1], o_stride[2]);
   else
-    lf::combine_kernel<64><<<blocks, 128, 0, st>>>(part_o, part_ml,
-                                                   static_cast<__nv_bfloat16*>(out), units, Hkv,
-                                                   G, splits, o_stride[0], o_stride[1],
-                                                   o_stride[2]);
+    lf::launch_pdl(lf::combine_kernel<64>, dim3(blocks), 128, 0, st, part_o, part_ml,
+                   static_cast<__nv_bfloat16*>(out), units, Hkv, G, splits, o_stride[0],
+                   o_stride[1], o_stride[2]);
   return lf::check_launch("combine_kernel");
 }
 

@@ -32,6 +32,8 @@ struct KvAppendParams {
 // whole 256-byte (D = 128) rows.
 template <int D>
 __global__ void __launch_bounds__(256) kv_append_kernel(const KvAppendParams p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int CPR = D / 8;  // 16-byte pieces per row
   const int64_t total = static_cast<int64_t>(p.B) * p.Hkv * p.T * CPR;
   for (int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; gid < total;
@@ -127,8 +129,8 @@ extern "C" int lf_kv_append_bf16(const LfKvAppendArgs* a, void* stream) {
   if (blocks > cap) blocks = cap;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (a->D == 128)
-    kv_append_kernel<128><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
+    launch_pdl(kv_append_kernel<128>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p);
   else
-    kv_append_kernel<64><<<static_cast<unsigned>(blocks), 256, 0, st>>>(p);
+    launch_pdl(kv_append_kernel<64>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p);
   return check_launch("kv_append_kernel");
 }

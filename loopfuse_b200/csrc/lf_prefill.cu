@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   constexpr int kMmaWarp0 = kSoftmaxWarps + 1;
   constexpr int kGatherWarp = kSoftmaxWarps + 3;
 
+  pdl_trigger();
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  pdl_wait();  // (the set-up above touches no global memory)
 
   if ((warp == kProducerWarp || warp == kGatherWarp) && p.gather) {
     // ---------------- producer with a paged K and / or V, by TMA row gather ----------------
@@ -1408,8 +1410,8 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   pp.div_group = FastDiv::make(p.group);
   const unsigned grid = static_cast<unsigned>(per_group * groups * tiles);
   // (without a second score product the two extra maps are never read)
-  prefill_kernel<D, MODE, PE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mqpe ? *mqpe : mq,
-                                                                   mkpe ? *mkpe : mk, pp);
+  launch_pdl(prefill_kernel<D, MODE, PE>, dim3(grid), kPrefillThreads, smem, st, mq, mk, mv,
+             mqpe ? *mqpe : mq, mkpe ? *mkpe : mk, pp);
   return check_launch("prefill_kernel");
 }
 
