@@ -112,8 +112,10 @@ class CompiledAttention:
         return self.spec.bias_pos - (len(self.spec.mods) - len(plan.mods))
 
     def plan(self, flat_args: list) -> AttentionPlan:
-        """The plan for this call's sizes; cached per (shapes, integer arguments)."""
-        key = tuple(a.shape if isinstance(a, torch.Tensor) else a for a in flat_args)
+        """The plan for this call's sizes; cached per (shapes, scalar arguments). A float argument
+        or closure variable reaches the graph as a 0-dim tensor: its value counts, not its shape."""
+        key = tuple(a if not isinstance(a, torch.Tensor) else a.shape if a.dim() else a.item()
+                    for a in flat_args)
         plan = self._plans.get(key)
         if plan is None:
             plan = self._make_plan(flat_args)

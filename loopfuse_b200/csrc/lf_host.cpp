@@ -87,16 +87,19 @@ void check_rc(int rc, const char* what) {
   throw PyErrorSet{};
 }
 
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // Runs `f(stream)` with the tensors' device current, without the GIL (a launch may block when the
 // queue of the stream is full).
 template <class F>
 int launch(const c10::Device& dev, F f) {
   const c10::cuda::CUDAGuard guard(dev);
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-  PyThreadState* ts = PyEval_SaveThread();
-  const int rc = f(stream);
-  PyEval_RestoreThread(ts);
-  return rc;
+  const NoGil no_gil;
+  return f(stream);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -847,7 +850,8 @@ Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
 
 PyTypeObject call_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// What a call's plan depends on: the sizes of the tensors and the values of everything else.
+// What a call's plan depends on: the sizes of the tensors and the values of everything else, 0-dim
+// tensors among them (a float argument or closure variable reaches the graph as one).
 struct Seen {
   std::vector<int64_t> key;
   Call* call;
@@ -862,6 +866,14 @@ struct Dispatcher {
 
 constexpr size_t kMaxSeen = 64;
 
+// Value of a 0-dim tensor. One that lives on the GPU is waited for: the launch takes it as a number.
+double scalar_value(const Tensor& t) {
+  if (t.is_cpu() && t.scalar_type() == at::kDouble) return *t.const_data_ptr<double>();
+  if (t.is_cpu() && t.scalar_type() == at::kFloat) return *t.const_data_ptr<float>();
+  const NoGil no_gil;
+  return t.item().toDouble();
+}
+
 // Key of the arguments into `key` (at most `cap` words); -1: not representable. Each argument is
 // preceded by a word that tells tensors from scalars, so keys of different kinds never match.
 int make_key(PyObject* const* args, Py_ssize_t n, int64_t* key, int cap) {
@@ -871,9 +883,13 @@ int make_key(PyObject* const* args, Py_ssize_t n, int64_t* key, int cap) {
     if (THPVariable_Check(o)) {
       const Tensor& t = THPVariable_Unpack(o);
       const auto s = t.sizes();
-      if (w + 1 + static_cast<int>(s.size()) > cap) return -1;
+      if (w + 2 + static_cast<int>(s.size()) > cap) return -1;
       key[w++] = -1 - static_cast<int64_t>(s.size());
       for (int64_t x : s) key[w++] = x;
+      if (s.empty()) {
+        const double d = scalar_value(t);
+        std::memcpy(&key[w++], &d, 8);
+      }
     } else if (PyLong_CheckExact(o)) {
       int over = 0;
       const long long v = PyLong_AsLongLongAndOverflow(o, &over);

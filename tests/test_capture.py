@@ -224,3 +224,35 @@ def test_unsupported_graphs_raise(case):
         args = (q, q.clone(), q.clone())
     with pytest.raises(BackendCompilerFailed):
         compile_plan(fn, args)
+
+
+def test_scalar_argument_changes_between_calls():
+    """A float argument reaches the graph as a 0-dim tensor: the plan goes by its value."""
+    def fn(q, k, v, cap):
+        s = torch.tanh(q @ k.transpose(-2, -1) / cap) * cap
+        return torch.softmax(torch.ops.loopfuse.causal_mask(s), dim=-1) @ v
+
+    q = torch.zeros(1, 2, 64, 64).bfloat16()
+    compiled = torch.compile(fn, backend=loopfuse_backend, dynamic=True)
+    for cap in (50.0, 30.0, 50.0):
+        for scalar in (cap, torch.tensor(cap)):
+            assert mod_names(compiled(q, q, q, scalar)) == [("div", cap), ("tanh", 0.0),
+                                                            ("mul", cap)]
+
+
+def test_native_dispatcher_tells_scalar_tensors_apart(native_lib):
+    """The dispatcher binds a call per set of sizes and scalar values, 0-dim tensors among them."""
+    from loopfuse_b200 import _native
+    bound = []
+
+    def bind(*args):
+        bound.append(args[1].item())
+        return _native.host().Call(0, (0, 0, 0) + (-1,) * 7, 1.0, (), 0, 0, -1, None)
+
+    call = _native.host().Dispatcher(bind)
+    q = torch.zeros(1, 1, 4, 64)
+    for x in (50.0, 30.0, 50.0, 30.0):
+        for dtype in (torch.float64, torch.float32, torch.int64):
+            with pytest.raises(RuntimeError, match="CUDA"):     # (found or bound, then refused)
+                call(q, torch.tensor(x, dtype=dtype))
+    assert bound == [50.0, 30.0]

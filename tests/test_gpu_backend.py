@@ -220,3 +220,20 @@ def test_cpu_tensors_fail_loudly():
     fn = torch.compile(w.fn(), backend=loopfuse_backend, dynamic=True)
     with pytest.raises(Exception, match="CUDA"):
         fn(*inputs)
+
+
+def test_scalar_argument_changes_between_calls():
+    """A float argument reaches the graph as a 0-dim tensor: each call uses its own value."""
+    def fn(q, k, v, cap):
+        s = torch.tanh(q @ k.transpose(-2, -1) * (q.shape[-1] ** -0.5) / cap) * cap
+        return torch.softmax(torch.ops.loopfuse.causal_mask(s), dim=-1) @ v
+
+    g = torch.Generator().manual_seed(12)
+    q, k, v = [(2.0 * torch.randn(1, 2, 200, 64, generator=g)).bfloat16() for _ in range(3)]
+    torch._dynamo.reset()
+    compiled = torch.compile(fn, backend=loopfuse_backend, dynamic=True)
+    for cap in (50.0, 1.0, 50.0, 4.0):
+        want = fn(q.float(), k.float(), v.float(), cap)
+        for scalar in (cap, torch.tensor(cap), torch.tensor(cap, device="cuda")):
+            out = compiled(q.cuda(), k.cuda(), v.cuda(), scalar)
+            assert (out.float().cpu() - want).abs().max().item() <= TOL
