@@ -414,8 +414,11 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        o[j][e] += o[j][2 + e] + __shfl_down_sync(0xffffffffu, o[j][e], 8);
+      for (int e = 0; e < 2; ++e) {
+        const float fine = o[j][2 + e] + __shfl_down_sync(0xffffffffu, o[j][e], 8);
+        // (a value row with an infinity: the parts of its weight have either sign or are zero)
+        if (fabsf(o[j][e]) != INFINITY) o[j][e] += fine;
+      }
   }
   // Row sum over the quad (the four lanes of a row hold disjoint tokens).
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);

@@ -70,3 +70,20 @@ def test_paged_splits(P, Skv, splits, D):
         k = O.paged_kv_ref(kp, kt)[:, :, :Skv]
         v = O.paged_kv_ref(vp, kt if table_v is None else table_v)[:, :, :Skv]
         check(out, want_of(q, k, v, "none"), v, "none", wide_p=False)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hkv,G,Skv,splits", [(1, 2, 1, 40, 1), (1, 2, 2, 700, 4), (1, 2, 4, 40, 1)])
+def test_infinite_values_stay_infinite(B, Hkv, G, Skv, splits, D):
+    """A value row with an infinity: its weight is positive, so that column is that infinity (the
+    finer parts of P must not turn it into inf - inf); a NaN stays in its column; the others are
+    untouched."""
+    g = torch.Generator().manual_seed(9)
+    q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    v[:, :, 5, 3], v[:, :, 17, 9], v[:, :, 21, 40] = float("inf"), float("-inf"), float("nan")
+    out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits).cpu()
+    assert bool((out[..., 3] == float("inf")).all()) and bool((out[..., 9] == float("-inf")).all())
+    assert bool(out[..., 40].isnan().all())
+    v[:, :, [5, 17, 21], [3, 9, 40]] = 0.0
+    keep = [c for c in range(D) if c not in (3, 9, 40)]
+    check(out[..., keep], want_of(q, k, v, "none")[..., keep], v, "none", wide_p=G <= 2)
