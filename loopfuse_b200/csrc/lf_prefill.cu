@@ -60,7 +60,9 @@ struct StagesFor {
 };
 constexpr float kLog2eF = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
-constexpr float kFastRowSum = 1099511627776.f;  // 2^40
+// Largest row sum of a block that the fast pass accepts: 64 keys at the lazy rescale's 2^8, so that O
+// stays as far inside fp32 as with it (at 2^40, values of 1e27 could overflow to infinity).
+constexpr float kFastRowSum = 16384.f;  // 2^14
 // tanh(x) by odd polynomial: x*(1 - x^2/3) up to |x| <= 0.125 (abs. error < 4.1e-6), degree 7
 // up to |x| <= 0.4 (abs. error < 6e-6); MUFU tanh beyond.
 constexpr float kTanhPoly1Limit = 0.125f;

@@ -98,3 +98,26 @@ def test_one_tile_split_over_both_slots(B, Hq, Hkv, Sq, Skv, offset, D):
     got = out.float().cpu()
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     assert (got - want).nan_to_num().abs().max().item() <= TOL
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("biased", [False, True])
+@pytest.mark.parametrize("B,H,Sq", [(1, 2, 100), (4, 40, 256)])
+def test_large_values_behind_a_low_reference_do_not_overflow(B, H, Sq, D, biased):
+    """Later keys score 2^30 above the first ones and the values are of the order of 1e30: P against
+    the first keys' reference, times V, would leave fp32 although the result is of V's order. 2^-8 of
+    the largest value: P and the output are bf16."""
+    g = torch.Generator().manual_seed(11)
+    Skv = 1024
+    q = torch.ones(B, H, Sq, D).bfloat16()
+    k = torch.zeros(B, H, Skv, D).bfloat16()
+    v = (torch.randn(B, H, Skv, D, generator=g) * 1e30).bfloat16()
+    bias = None
+    if biased:
+        bias = torch.zeros(B, H, Sq, Skv, dtype=torch.bfloat16, device="cuda")
+        bias[..., Skv // 2:] = 20.75
+    else:
+        k[:, :, Skv // 2:] = 20.75 / D
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), score_bias=bias)
+    want = v[:, :, Skv // 2:].double().mean(2, keepdim=True).expand(B, H, Sq, D)
+    assert (out.double().cpu() - want).abs().max().item() <= 2.0 ** -8 * want.abs().max().item()
