@@ -249,14 +249,18 @@ void lf_skip_range(int32_t mask_kind, int32_t window, int32_t causal_offset, int
 /* Decode attention (Sq == 1 per head, G grouped heads per kv head), split over KV. */
 int lf_decode_bf16(const LfDecodeArgs* args, void* stream);
 int lf_decode_paged_bf16(const LfDecodeArgs* args, void* stream);
-/* Split count the library picks for splits == 0, and the workspace it then needs. `page_size`
- * is 0 for a dense cache, else the tokens per page of the paged cache (a split's slice of the
- * block table is staged in shared memory; with small pages and a long context the library splits
- * further until the slice fits, and an explicit split count that leaves it too large is refused
- * with LF_ERR_TOO_LARGE). */
+/* Split count the library picks for splits == 0, and the workspace that a split count needs (a call
+ * with as much is never refused for its workspace). `page_size` is 0 for a dense cache, else the
+ * tokens per page of the paged cache (a split's slice of the block table is staged in shared memory;
+ * with small pages and a long context the library splits further until the slice fits, and an
+ * explicit split count that leaves it too large is refused with LF_ERR_TOO_LARGE). */
 int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t G, int32_t Skv, int32_t D,
                           int32_t page_size);
 size_t lf_decode_workspace_bytes(int32_t B, int32_t Hkv, int32_t G, int32_t D, int32_t splits);
+/* Kernels that lf_decode_bf16 (`paged` != 0: lf_decode_paged_bf16) launches for these arguments: 1, or
+ * 2 when the splits' partials go through the workspace; or the negative LfStatus that it refuses
+ * them with. Launches nothing. */
+int lf_decode_launches(const LfDecodeArgs* args, int32_t paged);
 
 /* Decode for callers that cannot allocate. No counterpart in the reference (it has neither
  * split-KV nor a workspace). Same arguments and result as lf_decode_bf16, except that

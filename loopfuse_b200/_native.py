@@ -16,7 +16,7 @@ LF_MAX_MODS = 8
 EXPORTS = [
     "lf_query", "lf_strerror", "lf_last_cuda_error", "lf_prefill_bf16", "lf_skip_range",
     "lf_decode_bf16", "lf_decode_paged_bf16", "lf_decode_auto_splits",
-    "lf_decode_workspace_bytes", "lf_combine_f32", "lf_paged_gather_bf16",
+    "lf_decode_workspace_bytes", "lf_decode_launches", "lf_combine_f32", "lf_paged_gather_bf16",
     "lf_decode_bf16_static", "lf_prefill_kv_tile", "lf_prefill_q_tile", "lf_tile_map_cache_stats",
     "lf_kv_append_bf16", "lf_selftest_wait_timeout", "lf_add_bf16", "lf_debug_bounds",
 ]
@@ -133,6 +133,8 @@ def load() -> C.CDLL:
     lib.lf_decode_auto_splits.restype = C.c_int
     lib.lf_decode_workspace_bytes.argtypes = [C.c_int32] * 5
     lib.lf_decode_workspace_bytes.restype = C.c_size_t
+    lib.lf_decode_launches.argtypes = [C.POINTER(LfDecodeArgs), C.c_int32]
+    lib.lf_decode_launches.restype = C.c_int
     lib.lf_combine_f32.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32,
                                    C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int64),
                                    C.c_void_p]

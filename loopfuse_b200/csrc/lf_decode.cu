@@ -618,9 +618,7 @@ constexpr int kMaxCluster = 16;  // (more than 8 CTAs: a non-portable cluster si
 // Split count for splits == 0. page_size: 0 for a dense cache, else the tokens per page. Powers of
 // two only: clusters of other sizes are placed badly (16 x 8 units of 1001 keys took 18.5 us in twos,
 // 22 in threes, 20 in fours, 33 in sixes; 8 x 4 units of 4000 keys 20.4 us in eights, 29 in nines).
-static int choose_splits(int B, int Hkv, int G, int Skv, int D, int page_size) {
-  (void)G;
-  (void)D;
+static int choose_splits(int B, int Hkv, int Skv, int page_size) {
   const int64_t units = static_cast<int64_t>(B) * Hkv;
   const int sms = device_sm_count();
   constexpr int kMinTokens = 120;  // per split: below, its start-up costs what the split saves
@@ -644,6 +642,14 @@ static int choose_splits(int B, int Hkv, int G, int Skv, int D, int page_size) {
     while (s < 32 && round_up((Skv + s - 1) / s, 16) > max_chunk) s = s < 16 ? s * 2 : s + 1;
   }
   return s;
+}
+
+// Splits whose partials go through the workspace when `splits` are asked for: chunks of 64 tokens, and
+// none that is empty. Never more than were asked for, and what a workspace has to hold.
+static int partial_chunk(int Skv, int splits) { return round_up((Skv + splits - 1) / splits, 64); }
+static int partial_splits(int Skv, int splits) {
+  const int chunk = partial_chunk(Skv, splits);
+  return (Skv + chunk - 1) / chunk;
 }
 
 // Launch with the splits of a unit as a cluster, when p.cluster says so.
@@ -750,7 +756,8 @@ static int launch_decode(const DecodeParams& p, int G, int mods, cudaStream_t st
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
+// `stream` == nullptr: only tell how many kernels the call launches.
+static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
   if (!a || !a->q || !a->k || !a->v || !a->out) return LF_ERR_INVALID_ARG;
   if (a->B <= 0 || a->Hkv <= 0 || a->G <= 0 || a->Skv <= 0) return LF_ERR_INVALID_ARG;
   if (a->D != 64 && a->D != 128) return LF_ERR_UNSUPPORTED;
@@ -770,14 +777,21 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
   int splits = a->splits;
   if (splits < 0) return LF_ERR_INVALID_ARG;
   if (splits > 32) return LF_ERR_TOO_LARGE;
-  if (splits == 0)
-    splits = choose_splits(a->B, a->Hkv, a->G, a->Skv, a->D, paged ? a->page_size : 0);
+  if (splits == 0) splits = choose_splits(a->B, a->Hkv, a->Skv, paged ? a->page_size : 0);
+  // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
+  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups.
   // Token chunk per split: a multiple of 16, so a split never starts in the middle of a warp's token
-  // batch. Where the rounding leaves the last splits empty the count stays as it is (a power of two
-  // makes the better cluster); their partials have weight zero.
-  const int chunk = round_up((a->Skv + splits - 1) / splits, 16);
-  if (splits > 1) {
-    const size_t need = lf_decode_workspace_bytes(a->B, a->Hkv, a->G, a->D, splits);
+  // batch. Where the rounding leaves a cluster's last splits empty the count stays as it is; their
+  // partials have weight zero. (Powers of two make the better clusters: over 70 sizes whose count the
+  // rounding to 64 would trim, to 3, 6, 7 or 11..15, 6 % less time warm and 3 % cold.)
+  const bool cluster = splits > 1 && splits <= kMaxCluster &&
+                       static_cast<int64_t>(splits) * a->Hkv * a->B <= 8ll * device_sm_count();
+  if (!cluster) splits = partial_splits(a->Skv, splits);
+  const int chunk = cluster ? round_up((a->Skv + splits - 1) / splits, 16)
+                            : partial_chunk(a->Skv, splits);
+  const int partials = partial_splits(a->Skv, splits);
+  if (partials > 1) {
+    const size_t need = lf_decode_workspace_bytes(a->B, a->Hkv, a->G, a->D, partials);
     if (!a->workspace || a->workspace_bytes < need) return LF_ERR_WORKSPACE;
     if (!aligned16(a->workspace)) return LF_ERR_ALIGNMENT;
   }
@@ -839,12 +853,8 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
       }
     }
   }
-  // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
-  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups.
-  p.cluster = splits > 1 && splits <= kMaxCluster &&
-              static_cast<int64_t>(splits) * a->Hkv * a->B <= 8ll * device_sm_count();
+  p.cluster = cluster;
 
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   size_t table_bytes = 0;
   if (paged) {
     // A split's block-table slice lives in shared memory next to the K/V rings. The automatic
@@ -853,7 +863,10 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
     table_bytes = table_smem_bytes(chunk, p.page_size);
     if (table_bytes > kMaxTableBytes) return LF_ERR_TOO_LARGE;
   }
+  const bool combine = splits > 1 && !cluster;
+  if (stream == nullptr) return combine ? 2 : 1;
 
+  cudaStream_t st = static_cast<cudaStream_t>(*stream);
   int rc;
   if (a->D == 128)
     rc = paged ? launch_decode<128, true>(p, a->G, mods, st, table_bytes)
@@ -862,9 +875,9 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
     rc = paged ? launch_decode<64, true>(p, a->G, mods, st, table_bytes)
                : launch_decode<64, false>(p, a->G, mods, st, table_bytes);
   if (rc != LF_OK) return rc;
-  if (splits > 1 && !p.cluster)
+  if (combine)
     rc = lf_combine_f32(p.part_o, p.part_ml, a->out, a->B, a->Hkv, a->G, a->D, splits,
-                        a->o_stride, stream);
+                        a->o_stride, *stream);
   return rc;
 }
 
@@ -872,12 +885,10 @@ static int decode_impl(const LfDecodeArgs* a, void* stream, bool paged) {
 
 extern "C" {
 
-int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t G, int32_t Skv, int32_t D,
-                          int32_t paged) {
+int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t /*G*/, int32_t Skv, int32_t /*D*/,
+                          int32_t page_size) {
   if (B <= 0 || Hkv <= 0 || Skv <= 0) return 1;
-  int splits = lf::choose_splits(B, Hkv, G, Skv, D, paged > 0 ? paged : 0);
-  const int chunk = lf::round_up((Skv + splits - 1) / splits, 64);
-  return (Skv + chunk - 1) / chunk;
+  return lf::choose_splits(B, Hkv, Skv, page_size > 0 ? page_size : 0);
 }
 
 size_t lf_decode_workspace_bytes(int32_t B, int32_t Hkv, int32_t G, int32_t D, int32_t splits) {
@@ -887,11 +898,15 @@ size_t lf_decode_workspace_bytes(int32_t B, int32_t Hkv, int32_t G, int32_t D, i
 }
 
 int lf_decode_bf16(const LfDecodeArgs* args, void* stream) {
-  return lf::decode_impl(args, stream, false);
+  return lf::decode_impl(args, &stream, false);
 }
 
 int lf_decode_paged_bf16(const LfDecodeArgs* args, void* stream) {
-  return lf::decode_impl(args, stream, true);
+  return lf::decode_impl(args, &stream, true);
+}
+
+int lf_decode_launches(const LfDecodeArgs* args, int32_t paged) {
+  return lf::decode_impl(args, nullptr, paged != 0);
 }
 
 int lf_combine_f32(const float* part_o, const float* part_ml, void* out, int32_t B, int32_t Hkv,
@@ -993,14 +1008,12 @@ extern "C" int lf_decode_bf16_static(const LfDecodeArgs* args, void* stream) {
   if (!args) return LF_ERR_INVALID_ARG;
   if (args->B <= 0 || args->Hkv <= 0 || args->G <= 0 || args->Skv <= 0)
     return LF_ERR_INVALID_ARG;
-  // Resolve the split count exactly as lf_decode_bf16 will, then size the partials.
   int splits = args->splits;
   if (splits < 0) return LF_ERR_INVALID_ARG;
-  if (splits == 0)
-    splits = lf::choose_splits(args->B, args->Hkv, args->G, args->Skv, args->D, 0);
-  const int chunk = lf::round_up((args->Skv + splits - 1) / splits, 64);
-  splits = (args->Skv + chunk - 1) / chunk;
-  const size_t need = lf_decode_workspace_bytes(args->B, args->Hkv, args->G, args->D, splits);
+  if (splits > 32) splits = lf::partial_splits(args->Skv, splits);
+  if (splits == 0) splits = lf::choose_splits(args->B, args->Hkv, args->Skv, 0);
+  const size_t need = lf_decode_workspace_bytes(args->B, args->Hkv, args->G, args->D,
+                                                lf::partial_splits(args->Skv, splits));
   if (need > static_cast<size_t>(LF_STATIC_SCRATCH_BYTES)) return LF_ERR_TOO_LARGE;
   void* scratch = nullptr;
   const int rc = lf::static_scratch_address(&scratch);
@@ -1009,5 +1022,5 @@ extern "C" int lf_decode_bf16_static(const LfDecodeArgs* args, void* stream) {
   local.splits = splits;
   local.workspace = scratch;
   local.workspace_bytes = static_cast<size_t>(LF_STATIC_SCRATCH_BYTES);
-  return lf::decode_impl(&local, stream, false);
+  return lf::decode_impl(&local, &stream, false);
 }

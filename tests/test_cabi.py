@@ -1,6 +1,7 @@
 """The C-ABI library without a GPU: it builds, loads, exports every declared symbol, and
 rejects bad arguments with error codes before any CUDA work."""
 import ctypes as C
+import random
 import re
 from pathlib import Path
 
@@ -92,3 +93,40 @@ def test_build_fingerprint_covers_every_included_file():
             assert target in covered, f"{target} is not in the build fingerprint"
             todo.append(target)
     assert any(p.name == "lf_prefill_wide.cuh" for p in seen)
+
+
+def decode_call(B, Hkv, G, Skv, D, page, splits, workspace_bytes):
+    """The arguments of a decode call on made-up addresses, for what only looks at them."""
+    a = _native.LfDecodeArgs()
+    a.q = a.k = a.v = a.out = a.block_table = 0x1000
+    a.B, a.Hkv, a.G, a.Skv, a.D, a.splits = B, Hkv, G, Skv, D, splits
+    a.page_size, a.n_pages = page, 1 if page else 0
+    a.workspace, a.workspace_bytes = (0x1000 if workspace_bytes else None), workspace_bytes
+    return a
+
+
+def test_announced_splits_and_workspace_are_what_a_call_takes(native_lib):
+    """lf_decode_auto_splits, lf_decode_workspace_bytes, then a call with splits = 0 or that count:
+    accepted; and the count is a power of two unless small pages ask for more than 16."""
+    rng = random.Random(1)
+    cases = [(2, 8, 4, 1100, 128, 0), (3, 1, 1, 2055, 128, 0), (2, 4, 4, 7369, 128, 0)]
+    for _ in range(4000):
+        length = int(2 ** rng.uniform(0, 16))
+        cases.append((int(2 ** rng.uniform(0, 8)), rng.choice((1, 2, 3, 8, 32)),
+                      rng.choice((1, 2, 4, 8)), length, rng.choice((64, 128)),
+                      rng.choice((0, 0, 1, 3, 16, 24, 64))))
+    for B, Hkv, G, Skv, D, page in cases:
+        auto = native_lib.lf_decode_auto_splits(B, Hkv, G, Skv, D, page)
+        assert auto in (1, 2, 4, 8, 16) or (page and 16 < auto <= 32), (B, Hkv, Skv, page, auto)
+        need = native_lib.lf_decode_workspace_bytes(B, Hkv, G, D, auto)
+        launches = [native_lib.lf_decode_launches(
+            C.byref(decode_call(B, Hkv, G, Skv, D, page, n, need)), page > 0) for n in (0, auto)]
+        assert launches[0] == launches[1] and launches[0] in (1, 2), (B, Hkv, G, Skv, D, page)
+        n = rng.randint(2, 32)
+        need = native_lib.lf_decode_workspace_bytes(B, Hkv, G, D, n)
+        rc = native_lib.lf_decode_launches(C.byref(decode_call(B, Hkv, G, Skv, D, page, n, need)),
+                                           page > 0)
+        assert rc in (1, 2) or (page and rc == -7), (B, Hkv, G, Skv, D, page, n)
+        if Skv > 64:            # (more than one split has tokens: its partials need room)
+            a = decode_call(B, Hkv, G, Skv, D, page, n, 0)
+            assert native_lib.lf_decode_launches(C.byref(a), page > 0) == -4

@@ -2,10 +2,12 @@
 shared memory (the last splits ragged or empty, block-table slices of different padding), the combine
 kernel beyond 16, eight, four and two warps per CTA, the folded softcap beside the interpreted chain,
 and P at full precision where one or two query rows share a kv head."""
+import ctypes as C
+
 import pytest
 import torch
 
-from loopfuse_b200 import functional as F, spec as S
+from loopfuse_b200 import _native, functional as F, spec as S
 from oracle import attention_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -87,3 +89,17 @@ def test_infinite_values_stay_infinite(B, Hkv, G, Skv, splits, D):
     v[:, :, [5, 17, 21], [3, 9, 40]] = 0.0
     keep = [c for c in range(D) if c not in (3, 9, 40)]
     check(out[..., keep], want_of(q, k, v, "none")[..., keep], v, "none", wide_p=G <= 2)
+
+
+@pytest.mark.parametrize("B,Hkv,G,Skv", [(2, 8, 4, 1100), (3, 1, 1, 2055), (2, 4, 4, 7369)])
+def test_library_chosen_splits_of_ragged_lengths(B, Hkv, G, Skv):
+    """Lengths that a chunk of 64 would cut into 6, 11 and 15 splits: eights and sixteens, the last of
+    them with few tokens or none."""
+    g = torch.Generator().manual_seed(10)
+    q, k, v = [torch.randn(B, Hkv, n, 128, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    auto = _native.load().lf_decode_auto_splits(B, Hkv, G, Skv, 128, 0)
+    assert auto in (8, 16)
+    out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=128 ** -0.5)
+    check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
+    again = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=128 ** -0.5, splits=auto)
+    assert torch.equal(out, again)
