@@ -270,8 +270,9 @@ int lf_decode_launches(const LfDecodeArgs* args, int32_t paged);
  * time - a serving loop with a frozen memory pool, a plugin called from inside another
  * runtime - and only own their input and output buffers.
  *   - Nothing is allocated or freed, by this call or by anything it calls.
- *   - A problem whose partials (lf_decode_workspace_bytes for the resolved split count) exceed
- *     LF_STATIC_SCRATCH_BYTES is refused with LF_ERR_TOO_LARGE; pass a smaller `splits`.
+ *   - An explicit split count whose partials (lf_decode_workspace_bytes) exceed
+ *     LF_STATIC_SCRATCH_BYTES is refused with LF_ERR_TOO_LARGE; pass a smaller `splits`, or 0 (the
+ *     library then splits only as far as the partials fit).
  *   - The first call on each device looks up the array's device address (with that device
  *     current); make that first call before starting any stream capture.
  *   - All calls on a device share the one array. Its old contents never matter (every partial

@@ -1014,7 +1014,10 @@ extern "C" int lf_decode_bf16_static(const LfDecodeArgs* args, void* stream) {
   if (splits == 0) splits = lf::choose_splits(args->B, args->Hkv, args->Skv, 0);
   const size_t need = lf_decode_workspace_bytes(args->B, args->Hkv, args->G, args->D,
                                                 lf::partial_splits(args->Skv, splits));
-  if (need > static_cast<size_t>(LF_STATIC_SCRATCH_BYTES)) return LF_ERR_TOO_LARGE;
+  if (need > static_cast<size_t>(LF_STATIC_SCRATCH_BYTES)) {
+    if (args->splits != 0) return LF_ERR_TOO_LARGE;
+    splits = 1;  // (the library's own count: without a split there are no partials)
+  }
   void* scratch = nullptr;
   const int rc = lf::static_scratch_address(&scratch);
   if (rc != LF_OK) return rc;

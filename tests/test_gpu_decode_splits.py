@@ -103,3 +103,24 @@ def test_library_chosen_splits_of_ragged_lengths(B, Hkv, G, Skv):
     check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
     again = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=128 ** -0.5, splits=auto)
     assert torch.equal(out, again)
+
+
+def test_static_scratch_splits_only_as_far_as_its_partials_fit():
+    """A grid of many waves that the library would split in two, with partials of 17 MB: unsplit."""
+    lib = _native.load()
+    q = torch.randn(64, 32, 8, 128, device="cuda").bfloat16()
+    k, v = [torch.randn(64, 1, 2000, 128, device="cuda").bfloat16().expand(64, 32, 2000, 128)
+            for _ in range(2)]
+    assert lib.lf_decode_auto_splits(64, 32, 8, 2000, 128, 0) == 2
+    want = F.decode_attention(q, k, v, scale=128 ** -0.5, splits=1)
+    out = torch.empty_like(q)
+    a = _native.LfDecodeArgs()
+    a.q, a.k, a.v, a.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
+    a.B, a.Hkv, a.G, a.Skv, a.D, a.scale = 64, 32, 8, 2000, 128, 128 ** -0.5
+    for i in range(3):
+        a.q_stride[i], a.o_stride[i] = q.stride(i), out.stride(i)
+        a.k_stride[i], a.v_stride[i] = k.stride(i), v.stride(i)
+    assert lib.lf_decode_bf16_static(C.byref(a), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out, want)
+    a.splits = 2
+    assert lib.lf_decode_bf16_static(C.byref(a), torch.cuda.current_stream().cuda_stream) == -7
