@@ -257,9 +257,9 @@ int lf_decode_paged_bf16(const LfDecodeArgs* args, void* stream);
 int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t G, int32_t Skv, int32_t D,
                           int32_t page_size);
 size_t lf_decode_workspace_bytes(int32_t B, int32_t Hkv, int32_t G, int32_t D, int32_t splits);
-/* Kernels that lf_decode_bf16 (`paged` != 0: lf_decode_paged_bf16) launches for these arguments: 1, or
- * 2 when the splits' partials go through the workspace; or the negative LfStatus that it refuses
- * them with. Launches nothing. */
+/* Kernels that lf_decode_bf16 (`paged` != 0: lf_decode_paged_bf16) launches for these arguments on the
+ * current device: 2 when the splits' partials go through the workspace, else 1 (the workspace is then
+ * checked, but not touched); or the negative LfStatus that it refuses them with. Launches nothing. */
 int lf_decode_launches(const LfDecodeArgs* args, int32_t paged);
 
 /* Decode for callers that cannot allocate. No counterpart in the reference (it has neither

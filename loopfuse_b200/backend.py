@@ -84,7 +84,6 @@ class CompiledAttention:
         self.spec = spec
         self.mode = mode
         self.placeholders = [n for n in gm.graph.nodes if n.op == "placeholder"]
-        self.workspace = F.DecodeWorkspace()
         self.analysis_only = _flag("CODEGEN_ONLY")
         self.debug = _flag("DEBUG")
         self.check_status = self.debug or _flag("LF_CHECK_STATUS")
@@ -196,8 +195,7 @@ class CompiledAttention:
               spec.k_pe)
         bias_pos = self._bias_pos(plan) if spec.score_bias is not None else -1
         return _native.host().Call(kind, tuple(-1 if i is None else i for i in at), plan.scale,
-                                   plan.mods, plan.mask_kind, plan.window, bias_pos,
-                                   self.workspace)
+                                   plan.mods, plan.mask_kind, plan.window, bias_pos)
 
     def __call__(self, *flat_args: Any):
         args = list(flat_args)
@@ -226,15 +224,13 @@ class CompiledAttention:
                 o4 = out
             if plan.kernel == "decode":
                 F.decode_attention(q4, args[spec.k.placeholder], args[spec.v.placeholder],
-                                   scale=plan.scale, mods=plan.mods, out=o4,
-                                   workspace=self.workspace, status=status)
+                                   scale=plan.scale, mods=plan.mods, out=o4, status=status)
             else:
                 kt, vt = args[spec.k.block_table], args[spec.v.block_table]
                 F.paged_decode_attention(
                     q4, args[spec.k.placeholder], args[spec.v.placeholder], kt,
                     block_table_v=None if spec.v.block_table == spec.k.block_table else vt,
-                    scale=plan.scale, mods=plan.mods, out=o4, workspace=self.workspace,
-                    status=status)
+                    scale=plan.scale, mods=plan.mods, out=o4, status=status)
             self._check(status, plan)
             return (out,)
         # Prefill. K and V may be paged independently, as in the reference's own paged-attention

@@ -17,6 +17,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -73,6 +74,7 @@ struct Lib {
   int (*decode_paged)(const LfDecodeArgs*, void*) = nullptr;
   int (*auto_splits)(int32_t, int32_t, int32_t, int32_t, int32_t, int32_t) = nullptr;
   size_t (*workspace_bytes)(int32_t, int32_t, int32_t, int32_t, int32_t) = nullptr;
+  int (*launches)(const LfDecodeArgs*, int32_t) = nullptr;
   int (*kv_append)(const LfKvAppendArgs*, void*) = nullptr;
   int (*add)(const void*, const void*, void*, int32_t, int32_t, int32_t, int32_t, const int64_t*,
              const int64_t*, const int64_t*, void*) = nullptr;
@@ -490,20 +492,23 @@ struct DecodeOptions {
   int splits = 0;
 };
 
-// Scratch of `nbytes` from a DecodeWorkspace (its buffer is reused while it is large enough).
-void* workspace_ptr(PyObject* ws, size_t nbytes, const Tensor& like) {
+// Scratch of `nbytes` from a DecodeWorkspace (its buffer is reused while it is large enough, on the
+// stream that it was made on). The caller holds the tensor until the launch is queued: the object may
+// let go of it meanwhile.
+Tensor workspace_tensor(PyObject* ws, size_t nbytes, const Tensor& like, const void* stream) {
   static PyObject* s_buf = PyUnicode_InternFromString("_buf");
+  static PyObject* s_stream = PyUnicode_InternFromString("_stream");
   PyObject* buf = PyObject_GetAttr(ws, s_buf);
-  if (!buf) throw PyErrorSet{};
-  if (THPVariable_Check(buf)) {
-    const Tensor& t = THPVariable_Unpack(buf);
-    if (static_cast<size_t>(t.numel()) >= nbytes && t.device() == like.device()) {
-      void* p = t.data_ptr();
-      Py_DECREF(buf);
-      return p;
-    }
+  PyObject* on = buf ? PyObject_GetAttr(ws, s_stream) : nullptr;
+  Tensor t;
+  if (on && THPVariable_Check(buf) && PyLong_Check(on) && PyLong_AsVoidPtr(on) == stream) {
+    t = THPVariable_Unpack(buf);
+    if (static_cast<size_t>(t.numel()) < nbytes || t.device() != like.device()) t = Tensor();
   }
-  Py_DECREF(buf);
+  Py_XDECREF(buf);
+  Py_XDECREF(on);
+  PyErr_Clear();  // (an object with a get() of its own need not have these)
+  if (t.defined()) return t;
   PyObject* like_obj = THPVariable_Wrap(like);
   PyObject* dev = like_obj ? PyObject_GetAttrString(like_obj, "device") : nullptr;
   Py_XDECREF(like_obj);
@@ -511,9 +516,10 @@ void* workspace_ptr(PyObject* ws, size_t nbytes, const Tensor& like) {
   PyObject* got = PyObject_CallMethod(ws, "get", "nO", static_cast<Py_ssize_t>(nbytes), dev);
   Py_DECREF(dev);
   if (!got) throw PyErrorSet{};
-  void* p = THPVariable_Check(got) ? THPVariable_Unpack(got).data_ptr() : nullptr;
-  Py_DECREF(got);  // (the workspace object holds it)
-  return p;
+  if (THPVariable_Check(got)) t = THPVariable_Unpack(got);
+  Py_DECREF(got);
+  if (!t.defined()) type_error("workspace.get() must return a tensor");
+  return t;
 }
 
 // Dense (`paged` null) or paged decode of query `dq`; `out` has the strides `ostride` in the
@@ -569,7 +575,25 @@ void run_decode(const Tensor& q, const DecodeQuery& dq, const Tensor& k_in, cons
   const c10::cuda::CUDAGuard guard(dev);
   a.splits = o.splits ? o.splits : lib.auto_splits(a.B, a.Hkv, a.G, a.Skv, a.D, a.page_size);
   a.workspace_bytes = lib.workspace_bytes(a.B, a.Hkv, a.G, a.D, a.splits);
-  if (a.workspace_bytes) a.workspace = workspace_ptr(workspace, a.workspace_bytes, q);
+  // Splits that merge in their cluster leave the workspace alone: the library wants one, any address
+  // will do. Otherwise, without a workspace of the caller's, the partials are an allocation of this
+  // call on its stream. (Into one that calls shared, a call on another stream or thread could write
+  // between the two kernels of this one, and a captured graph after it has been replaced.)
+  Tensor held;
+  c10::DataPtr own;
+  if (a.workspace_bytes) {
+    a.workspace = out.data_ptr();
+    if (lib.launches(&a, paged != nullptr) == 2) {
+      if (workspace == Py_None) {
+        own = c10::cuda::CUDACachingAllocator::get()->allocate(a.workspace_bytes);
+        a.workspace = own.get();
+      } else {
+        held = workspace_tensor(workspace, a.workspace_bytes, q,
+                                c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+        a.workspace = held.data_ptr();
+      }
+    }
+  }
   check_rc(launch(dev,
                   [&](void* st) {
                     return paged ? lib.decode_paged(&a, st) : lib.decode(&a, st);
@@ -746,23 +770,18 @@ struct Call {
   int at[kOperands];
   PrefillOptions prefill;
   DecodeOptions decode;
-  PyObject* workspace;
 };
 
-void call_dealloc(PyObject* self) {
-  Py_XDECREF(reinterpret_cast<Call*>(self)->workspace);
-  Py_TYPE(self)->tp_free(self);
-}
+void call_dealloc(PyObject* self) { Py_TYPE(self)->tp_free(self); }
 
-// kind, operand positions (a tuple of kOperands ints), scale, mods, mask_kind, window, bias_pos,
-// workspace
+// kind, operand positions (a tuple of kOperands ints), scale, mods, mask_kind, window, bias_pos
 PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
   return guarded([&]() -> PyObject* {
     int kind, mask_kind, window, bias_pos;
     double scale;
-    PyObject *at, *mods, *workspace;
-    if (!PyArg_ParseTuple(args, "iO!dOiiiO", &kind, &PyTuple_Type, &at, &scale, &mods, &mask_kind,
-                          &window, &bias_pos, &workspace))
+    PyObject *at, *mods;
+    if (!PyArg_ParseTuple(args, "iO!dOiii", &kind, &PyTuple_Type, &at, &scale, &mods, &mask_kind,
+                          &window, &bias_pos))
       throw PyErrorSet{};
     if (PyTuple_GET_SIZE(at) != kOperands) type_error("operand positions: wrong count");
     int pos[kOperands];
@@ -782,8 +801,6 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     c->decode = DecodeOptions();
     c->decode.scale = scale;
     c->decode.mods = m;
-    Py_INCREF(workspace);
-    c->workspace = workspace;
     return reinterpret_cast<PyObject*>(c);
   });
 }
@@ -844,7 +861,7 @@ Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
   }
   const bool two = paged && c.at[kVTable] != c.at[kKTable];
   Paged pg{t[kKTable], two ? t[kVTable] : nullptr, -1};
-  run_decode(q, dq, k, v, paged ? &pg : nullptr, c.decode, c.workspace, nullptr, out, os);
+  run_decode(q, dq, k, v, paged ? &pg : nullptr, c.decode, Py_None, nullptr, out, os);
   return out;
 }
 
@@ -994,6 +1011,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     get("lf_decode_paged_bf16", lib.decode_paged);
     get("lf_decode_auto_splits", lib.auto_splits);
     get("lf_decode_workspace_bytes", lib.workspace_bytes);
+    get("lf_decode_launches", lib.launches);
     get("lf_kv_append_bf16", lib.kv_append);
     get("lf_add_bf16", lib.add);
     Py_INCREF(a[1]);

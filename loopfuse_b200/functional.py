@@ -176,20 +176,24 @@ def _prefill_record(q, k, v, scale, mods, mask_kind, window, causal_offset, out,
 
 
 class DecodeWorkspace:
-    """Caller-owned scratch for split-KV partials, grown on demand and reused across calls."""
+    """Caller-owned scratch for split-KV partials, grown on demand and reused by the calls that it is
+    passed to. It belongs to one thread at a time. A call on another stream than the last one's
+    gets a new buffer, so work in flight keeps the old one. (A call without a workspace allocates its
+    partials from PyTorch's caching allocator.)"""
 
     def __init__(self) -> None:
         self._buf: Optional[torch.Tensor] = None
+        self._stream: Optional[int] = None
 
     def get(self, nbytes: int, device) -> Optional[torch.Tensor]:
         if nbytes == 0:
             return None
-        if self._buf is None or self._buf.numel() < nbytes or self._buf.device != device:
+        stream = torch.cuda.current_stream(device).cuda_stream
+        if (self._buf is None or self._buf.numel() < nbytes or self._buf.device != device
+                or self._stream != stream):
             self._buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            self._stream = stream
         return self._buf
-
-
-_default_ws = DecodeWorkspace()
 
 
 def decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: float = 1.0,
@@ -198,8 +202,7 @@ def decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale
                      workspace: Optional[DecodeWorkspace] = None,
                      status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Unmasked attention of G query rows per kv head: q [B,Hkv,G,D], k/v [B,Hkv,Skv,D]."""
-    return _native.host().decode(q, k, v, out, workspace or _default_ws, status, scale, mods,
-                                 splits)
+    return _native.host().decode(q, k, v, out, workspace, status, scale, mods, splits)
 
 
 def _pool_view(pool: torch.Tensor, name: str) -> torch.Tensor:
@@ -232,8 +235,7 @@ def paged_decode_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
     (or [pages, Hkv, D] for one-token pages); block_table int32 [B, blocks]. Token t of sequence
     b lives at pool[block_table[b, t // page_size], t % page_size]."""
     return _native.host().paged_decode(q, k_pool, v_pool, block_table, block_table_v, out,
-                                       workspace or _default_ws, status, seq_len, scale, mods,
-                                       splits)
+                                       workspace, status, seq_len, scale, mods, splits)
 
 
 def paged_gather(pool: torch.Tensor, block_table: torch.Tensor, *, seq_len: Optional[int] = None,

@@ -247,7 +247,7 @@ def test_native_dispatcher_tells_scalar_tensors_apart(native_lib):
 
     def bind(*args):
         bound.append(args[1].item())
-        return _native.host().Call(0, (0, 0, 0) + (-1,) * 7, 1.0, (), 0, 0, -1, None)
+        return _native.host().Call(0, (0, 0, 0) + (-1,) * 7, 1.0, (), 0, 0, -1)
 
     call = _native.host().Dispatcher(bind)
     q = torch.zeros(1, 1, 4, 64)

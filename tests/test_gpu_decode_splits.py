@@ -3,6 +3,7 @@ shared memory (the last splits ragged or empty, block-table slices of different 
 kernel beyond 16, eight, four and two warps per CTA, the folded softcap beside the interpreted chain,
 and P at full precision where one or two query rows share a kv head."""
 import ctypes as C
+import threading
 
 import pytest
 import torch
@@ -124,3 +125,48 @@ def test_static_scratch_splits_only_as_far_as_its_partials_fit():
     assert torch.equal(out, want)
     a.splits = 2
     assert lib.lf_decode_bf16_static(C.byref(a), torch.cuda.current_stream().cuda_stream) == -7
+
+
+def many_splits(seed):
+    """20 splits, whose partials go through a workspace; the values tell the seeds apart."""
+    g = torch.Generator().manual_seed(seed)
+    q, k, v = [torch.randn(2, 4, n, 128, generator=g).bfloat16().cuda() for n in (4, 1700, 1700)]
+    return lambda **kw: F.decode_attention(q, k, v + seed, scale=128 ** -0.5, splits=20, **kw)
+
+
+def test_two_streams_and_two_threads_do_not_share_partials():
+    calls = [many_splits(1), many_splits(2)]
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    got = [[], []]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    ws = F.DecodeWorkspace()
+    for kw in ({}, {"workspace": ws}):
+        for _ in range(100):
+            for i in range(2):
+                with torch.cuda.stream(streams[i]):
+                    got[i].append(calls[i](**kw))
+
+    def loop(i):
+        for _ in range(200):
+            got[i].append(calls[i]())
+
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert len(got[i]) == 400 and all(torch.equal(o, want[i]) for o in got[i])
+
+
+def test_a_workspace_keeps_its_buffer_on_its_stream_only():
+    ws, call = F.DecodeWorkspace(), many_splits(3)
+    want = call(workspace=ws)
+    first = ws._buf
+    assert torch.equal(call(workspace=ws), want) and ws._buf is first
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+        assert torch.equal(call(workspace=ws), want) and ws._buf is not first
+    torch.cuda.synchronize()
