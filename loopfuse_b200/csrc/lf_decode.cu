@@ -618,7 +618,7 @@ constexpr int kMaxCluster = 16;  // (more than 8 CTAs: a non-portable cluster si
 // Split count for splits == 0. page_size: 0 for a dense cache, else the tokens per page. Powers of
 // two only: clusters of other sizes are placed badly (16 x 8 units of 1001 keys took 18.5 us in twos,
 // 22 in threes, 20 in fours, 33 in sixes; 8 x 4 units of 4000 keys 20.4 us in eights, 29 in nines).
-static int choose_splits(int B, int Hkv, int Skv, int page_size) {
+static int choose_splits(int B, int Hkv, int Skv, int D, int page_size) {
   const int64_t units = static_cast<int64_t>(B) * Hkv;
   const int sms = device_sm_count();
   constexpr int kMinTokens = 120;  // per split: below, its start-up costs what the split saves
@@ -632,9 +632,10 @@ static int choose_splits(int B, int Hkv, int Skv, int page_size) {
   if (units * s * 5 < 3ll * sms && s <= 4 && Skv / (s * 4) >= kMinTokens &&
       units * s * 4 >= 2ll * sms)
     s = s == 4 ? 8 : s * 4;
-  // A dense grid of many waves gains from halves where the caches are long: its last wave is shorter
-  // (2048 units of 2048 keys 308 -> 304 us; paged 314 -> 322, 800 units 120 -> 126).
-  if (page_size == 0 && units >= 6ll * sms + sms / 2 && Skv >= 2000) s = 2;
+  // A dense grid of many waves gains from halves where the caches are long and rows are 256 bytes: its
+  // last wave is shorter (D = 128, 2048 units of 2048 keys 309 -> 304 us, of 3000 445 -> 438, 1024 of 4000
+  // 303 -> 300; of 1000 keys 170 -> 173 us; D = 64, 2048 of 2048 156 -> 161; paged 314 -> 322).
+  if (page_size == 0 && D == 128 && units >= 6ll * sms + sms / 2 && Skv >= 2000) s = 2;
   if (page_size > 0) {
     // The block-table slice of a split must fit in shared memory (one-token pages at long
     // context): split further until it does.
@@ -777,9 +778,10 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
   int splits = a->splits;
   if (splits < 0) return LF_ERR_INVALID_ARG;
   if (splits > 32) return LF_ERR_TOO_LARGE;
-  if (splits == 0) splits = choose_splits(a->B, a->Hkv, a->Skv, paged ? a->page_size : 0);
+  if (splits == 0) splits = choose_splits(a->B, a->Hkv, a->Skv, a->D, paged ? a->page_size : 0);
   // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
-  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups.
+  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups. (In pairs:
+  // 2048 units of 2048 keys, each call on other buffers, 313 -> 324 us; 3000 one-token pages 475 -> 510.)
   // Token chunk per split: a multiple of 16, so a split never starts in the middle of a warp's token
   // batch. Where the rounding leaves a cluster's last splits empty the count stays as it is; their
   // partials have weight zero. (Powers of two make the better clusters: over 70 sizes whose count the
@@ -885,10 +887,10 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
 
 extern "C" {
 
-int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t /*G*/, int32_t Skv, int32_t /*D*/,
+int lf_decode_auto_splits(int32_t B, int32_t Hkv, int32_t /*G*/, int32_t Skv, int32_t D,
                           int32_t page_size) {
   if (B <= 0 || Hkv <= 0 || Skv <= 0) return 1;
-  return lf::choose_splits(B, Hkv, Skv, page_size > 0 ? page_size : 0);
+  return lf::choose_splits(B, Hkv, Skv, D, page_size > 0 ? page_size : 0);
 }
 
 size_t lf_decode_workspace_bytes(int32_t B, int32_t Hkv, int32_t G, int32_t D, int32_t splits) {
@@ -1011,7 +1013,7 @@ extern "C" int lf_decode_bf16_static(const LfDecodeArgs* args, void* stream) {
   int splits = args->splits;
   if (splits < 0) return LF_ERR_INVALID_ARG;
   if (splits > 32) splits = lf::partial_splits(args->Skv, splits);
-  if (splits == 0) splits = lf::choose_splits(args->B, args->Hkv, args->Skv, 0);
+  if (splits == 0) splits = lf::choose_splits(args->B, args->Hkv, args->Skv, args->D, 0);
   const size_t need = lf_decode_workspace_bytes(args->B, args->Hkv, args->G, args->D,
                                                 lf::partial_splits(args->Skv, splits));
   if (need > static_cast<size_t>(LF_STATIC_SCRATCH_BYTES)) {

@@ -130,3 +130,11 @@ def test_announced_splits_and_workspace_are_what_a_call_takes(native_lib):
         if Skv > 64:            # (more than one split has tokens: its partials need room)
             a = decode_call(B, Hkv, G, Skv, D, page, n, 0)
             assert native_lib.lf_decode_launches(C.byref(a), page > 0) == -4
+
+
+def test_many_waves_are_halved_only_where_it_pays(native_lib):
+    auto = native_lib.lf_decode_auto_splits
+    assert auto(64, 32, 1, 2048, 128, 0) == 2       # 256-byte rows, long caches
+    assert auto(64, 32, 1, 2048, 64, 0) == 1
+    assert auto(64, 32, 1, 1000, 128, 0) == 1
+    assert auto(64, 32, 1, 2048, 128, 16) == 1

@@ -170,3 +170,15 @@ def test_a_workspace_keeps_its_buffer_on_its_stream_only():
         torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
         assert torch.equal(call(workspace=ws), want) and ws._buf is not first
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("G,Skv,splits", [(1, 130, 2), (4, 17, 2), (1, 300, 4), (2, 200, 16)])
+def test_splits_of_grids_of_many_waves(G, Skv, splits, D):
+    """More than eight CTAs per SM: the partials go through the workspace (and counts are trimmed to
+    chunks of 64 tokens)."""
+    B, Hkv = 40, 32
+    g = torch.Generator().manual_seed(14)
+    q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
+    check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
