@@ -13,6 +13,7 @@
 //
 // The kernels' entry points come in as addresses (bind()), so that the module serves the normal
 // and the range-checking build of the library alike.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/core/Tensor.h>
@@ -56,10 +57,8 @@ PyObject* guarded(F f) {
   } catch (const Raise& e) {
     PyErr_SetString(e.type, e.text.c_str());
   } catch (const PyErrorSet&) {
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {  // (out of memory, an index out of range, ... as the types that torch raises)
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }

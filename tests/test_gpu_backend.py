@@ -237,3 +237,13 @@ def test_scalar_argument_changes_between_calls():
         for scalar in (cap, torch.tensor(cap), torch.tensor(cap, device="cuda")):
             out = compiled(q.cuda(), k.cuda(), v.cuda(), scalar)
             assert (out.float().cpu() - want).abs().max().item() <= TOL
+
+
+def test_errors_of_the_allocator_and_of_shapes_keep_their_type():
+    from loopfuse_b200 import functional as F
+    q = torch.zeros(1, 1, 1, 64, dtype=torch.bfloat16, device="cuda")
+    huge = q.expand(4096, 4096, 1024, 64)                     # an output of 2 TB
+    with pytest.raises(torch.OutOfMemoryError):
+        F.prefill_attention(huge, q.expand(4096, 4096, 1, 64), q.expand(4096, 4096, 1, 64))
+    with pytest.raises(IndexError):
+        F.decode_attention(q, q, q, out=torch.empty(1, 64, dtype=torch.bfloat16, device="cuda"))
