@@ -126,6 +126,9 @@ long long int_arg(PyObject* o) {
   }
   return v;
 }
+int splits_arg(PyObject* o) {  // (None: the library chooses, like 0)
+  return o == Py_None ? 0 : static_cast<int>(int_arg(o));
+}
 double float_arg(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw PyErrorSet{};
@@ -694,7 +697,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     DecodeOptions o;
     o.scale = float_arg(a[6]);
     o.mods = mods_arg(a[7]);
-    o.splits = static_cast<int>(int_arg(a[8]));
+    o.splits = splits_arg(a[8]);
     const DecodeQuery dq = query_of(q);
     if (!out.defined()) out = new_bf16(q.sizes(), dev);
     int64_t os[3];
@@ -725,7 +728,7 @@ PyObject* py_paged_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     DecodeOptions o;
     o.scale = float_arg(a[9]);
     o.mods = mods_arg(a[10]);
-    o.splits = static_cast<int>(int_arg(a[11]));
+    o.splits = splits_arg(a[11]);
     const DecodeQuery dq = query_of(q);
     if (!out.defined()) out = new_bf16(q.sizes(), dev);
     int64_t os[3];

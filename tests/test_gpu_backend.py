@@ -247,3 +247,10 @@ def test_errors_of_the_allocator_and_of_shapes_keep_their_type():
         F.prefill_attention(huge, q.expand(4096, 4096, 1, 64), q.expand(4096, 4096, 1, 64))
     with pytest.raises(IndexError):
         F.decode_attention(q, q, q, out=torch.empty(1, 64, dtype=torch.bfloat16, device="cuda"))
+
+
+def test_no_split_count_means_the_library_chooses():
+    from loopfuse_b200 import functional as F
+    g = torch.Generator().manual_seed(13)
+    q, k, v = [torch.randn(1, 2, n, 64, generator=g).bfloat16().cuda() for n in (1, 600, 600)]
+    assert torch.equal(F.decode_attention(q, k, v, splits=None), F.decode_attention(q, k, v))
