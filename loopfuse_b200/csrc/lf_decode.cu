@@ -94,8 +94,8 @@ __device__ __forceinline__ void merge_in_cluster(const DecodeParams& p, float* m
 // Decode on tensor cores (mma.sync m16n8k16, bf16 -> fp32).
 //
 // The G query rows of a kv head are rows 0..7 (zero-padded) of the 16-row M dimension of 16x8x16
-// MMAs; rows 8..15 are padding unless WIDE_P. The fragments come straight
-// from the 16-byte pieces that were copied:
+// MMAs; rows 8..15 are padding in QK^T. The fragments come straight from the 16-byte pieces that were
+// copied:
 //
 //   QK^T  8 tokens at a time. Lane (n = lane/4, c = lane%4) loads the 16-byte pieces
 //         d = 32i + 8c .. +8 of token n's K row (i < D/32); the four 32-bit words of a piece
@@ -107,14 +107,18 @@ __device__ __forceinline__ void merge_in_cluster(const DecodeParams& p, float* m
 //         wants; output column n of MMA (h, e) stands for d = 64h + 8n + e.
 //   The fp32 score fragment of the QK MMAs has the layout of the bf16 A fragment of the PV
 //   MMA, so P never leaves registers.
-//   WIDE_P (dense calls with G <= 2, which have rows to spare): P enters the PV product as the sum of
-//   three bf16, i.e. with fp32's 24 bits and at no extra MMA: rows g take its rounding, rows 8 + g
-//   the rounding of the rest, rows 2 + g (whose Q rows repeat rows g) what that leaves.
-// A CTA is one (batch, kv head, KV split); its WARPS warps (4, or 2 when smaller CTAs let the
-// whole grid be resident at once) take alternate 16-token groups (one page when page_size is
-// 16) and are merged through shared memory. Against the FMA + shuffle form that dense calls with G <=
-// 2 used (B200, D = 128): B=64 Hkv=32 2048 keys 318 -> 307 us, B=1 Hkv=32 4096 keys 20.3 -> 16.8 us,
-// B=1 Hkv=4 G=2 16000 keys 27.9 -> 16.4 us, B=16 Hkv=32 1000 keys 45.0 -> 46.3 us.
+//   P enters the PV product as the sum of P_TERMS bf16, in rows that would be padding and at no extra
+//   MMA: rows g take its rounding, rows 8 + g the rounding of the rest; with three (dense calls with
+//   G <= 2, whose former FMA kernel had P in fp32) rows 2 + g, whose Q rows repeat rows g, what that
+//   leaves. With one, P's rounding error is a fifth of the result's and depends on how the keys are
+//   dealt out to warps and splits (the largest P of each is exactly 1); with two the result's error is
+//   that of its own rounding. Against fp64, 1 x 8 x 4 heads, 8190 keys, softcap: 2.05e-3 in 31 splits,
+//   2.08e-3 in 16, now 1.66e-3; 64 x 8 x 4, 2048 keys, paged: 2.22e-3 -> 1.66e-3 at 87.0 -> 86.7 us.
+// A CTA is one (batch, kv head, KV split); its WARPS warps (launch_decode_shape says how many) take
+// alternate 16-token groups (one page when page_size is 16) and are merged through shared memory.
+// Against the FMA + shuffle form that dense calls with G <= 2 used (B200, D = 128): B=64 Hkv=32 2048 keys
+// 318 -> 307 us, B=1 Hkv=32 4096 keys 20.3 -> 16.8 us, B=1 Hkv=4 G=2 16000 keys 27.9 -> 16.4 us, B=16
+// Hkv=32 1000 keys 45.0 -> 46.3 us.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_16816_rows0to7(float& d0, float& d1, uint32_t a0, uint32_t a2,
                                                    uint32_t b0, uint32_t b1) {
@@ -135,7 +139,7 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 }
 
 // STAGES: depth of a warp's ring in 16-token groups; STAGES - 1 are in flight.
-template <int D, bool PAGED, int MODS, int WARPS, int STAGES, bool WIDE_P>
+template <int D, bool PAGED, int MODS, int WARPS, int STAGES, int P_TERMS>
 __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     decode_mma_kernel(const DecodeParams p, const int G) {
   pdl_wait();
@@ -230,8 +234,8 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     }
   };
 
-  // Q fragments (rows g >= G are zero padding; WIDE_P: rows 2 and 3 are rows 0 and 1 once more).
-  const int q_row = WIDE_P && g < 4 ? (g & 1) : g;
+  // Q fragments (rows g >= G are zero padding; three parts of P: rows 2 and 3 are rows 0 and 1 again).
+  const int q_row = P_TERMS == 3 && g < 4 ? (g & 1) : g;
   auto chunk_of = [&](int i) { return 4 * i + c; };  // 16-byte piece of a row
   uint4 qr[KI];
 #pragma unroll
@@ -244,12 +248,11 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
   const float smul = MODS != kModsNone ? p.scale : p.scale * kLog2e;
 
   float m_run = -INFINITY, l_run = 0.f;
-  constexpr int kOut = WIDE_P ? 4 : 2;
-  float o[NT][kOut];
+  float o[NT][4];  // rows g, then rows 8 + g
 #pragma unroll
   for (int j = 0; j < NT; ++j)
 #pragma unroll
-    for (int e = 0; e < kOut; ++e) o[j][e] = 0.f;
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
 
   // K/V rows travel global -> shared with 16-byte cp.async into a ring private to the warp
   // (STAGES groups of 16 tokens; STAGES-1 groups are in flight while one is consumed),
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int e = 0; e < kOut; ++e) o[j][e] *= alpha;
+        for (int e = 0; e < 4; ++e) o[j][e] *= alpha;
     }
     float pr[2][2];
     float psum = 0.f;
@@ -369,12 +372,11 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
     l_run += psum;  // this lane's share; the quad is summed after the loop
     uint32_t pa0 = pack_bf16x2(pr[0][0], pr[0][1]);
     uint32_t pa2 = pack_bf16x2(pr[1][0], pr[1][1]);
-    [[maybe_unused]] uint32_t pa1 = 0u, pa3 = 0u;
-    if constexpr (WIDE_P) {
-      const float r0 = pr[0][0] - bf16lo_to_f32(pa0), r1 = pr[0][1] - bf16hi_to_f32(pa0);
-      const float r2 = pr[1][0] - bf16lo_to_f32(pa2), r3 = pr[1][1] - bf16hi_to_f32(pa2);
-      pa1 = pack_bf16x2(r0, r1);
-      pa3 = pack_bf16x2(r2, r3);
+    const float r0 = pr[0][0] - bf16lo_to_f32(pa0), r1 = pr[0][1] - bf16hi_to_f32(pa0);
+    const float r2 = pr[1][0] - bf16lo_to_f32(pa2), r3 = pr[1][1] - bf16hi_to_f32(pa2);
+    uint32_t pa1 = pack_bf16x2(r0, r1);
+    uint32_t pa3 = pack_bf16x2(r2, r3);
+    if constexpr (P_TERMS == 3) {
       if (g >= 2) {
         pa0 = pack_bf16x2(r0 - bf16lo_to_f32(pa1), r1 - bf16hi_to_f32(pa1));
         pa2 = pack_bf16x2(r2 - bf16lo_to_f32(pa3), r3 - bf16hi_to_f32(pa3));
@@ -399,8 +401,7 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
         const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;  // high or low halves of two words
         const uint32_t b0 = __byte_perm(w0[e >> 1], w1[e >> 1], sel);
         const uint32_t b1 = __byte_perm(w2[e >> 1], w3[e >> 1], sel);
-        if constexpr (WIDE_P) mma_16816(o[h * 8 + e], pa0, pa1, pa2, pa3, b0, b1);
-        else mma_16816_rows0to7(o[h * 8 + e][0], o[h * 8 + e][1], pa0, pa2, b0, b1);
+        mma_16816(o[h * 8 + e], pa0, pa1, pa2, pa3, b0, b1);
       }
     }
     __syncwarp();  // every lane is done with this stage before it is refilled
@@ -410,16 +411,16 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
   // and crowd on some SMs. 512 units of 2048 keys 87 -> 94 us with the trigger at the top.)
   pdl_trigger();
 
-  if constexpr (WIDE_P) {  // rows 8 + g (same lane) and 2 + g hold the finer parts of row g
+  // Rows 8 + g (same lane), and with three parts rows 2 + g, hold the finer parts of row g.
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
+  for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float fine = o[j][2 + e] + __shfl_down_sync(0xffffffffu, o[j][e], 8);
-        // (a value row with an infinity: the parts of its weight have either sign or are zero)
-        if (fabsf(o[j][e]) != INFINITY) o[j][e] += fine;
-      }
-  }
+    for (int e = 0; e < 2; ++e) {
+      float fine = o[j][2 + e];
+      if constexpr (P_TERMS == 3) fine += __shfl_down_sync(0xffffffffu, o[j][e], 8);
+      // (a value row with an infinity: the parts of its weight have either sign or are zero)
+      if (fabsf(o[j][e]) != INFINITY) o[j][e] += fine;
+    }
   // Row sum over the quad (the four lanes of a row hold disjoint tokens).
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
@@ -705,7 +706,7 @@ static int launched(cudaError_t e, const char* where) {
   return LF_ERR_CUDA;
 }
 
-template <int D, bool PAGED, int MODS, bool WIDE_P, int WARPS, int STAGES>
+template <int D, bool PAGED, int MODS, int P_TERMS, int WARPS, int STAGES>
 static int launch_decode_w(DecodeParams p, int G, cudaStream_t st, size_t table_bytes) {
   // page ids + the per-warp K/V rings (the warp-merge area and the partial reuse the rings)
   const size_t ring = static_cast<size_t>(WARPS) * STAGES * 2 * 16 * D * 2;
@@ -713,13 +714,13 @@ static int launch_decode_w(DecodeParams p, int G, cudaStream_t st, size_t table_
   const size_t smem = table_bytes + (ring > merge ? ring : merge);
   p.part_off = static_cast<int32_t>(table_bytes + WARPS * static_cast<size_t>(G) * (D + 2) * 4);
   static thread_local int configured_dev = -1;
-  const auto kernel = decode_mma_kernel<D, PAGED, MODS, WARPS, STAGES, WIDE_P>;
+  const auto kernel = decode_mma_kernel<D, PAGED, MODS, WARPS, STAGES, P_TERMS>;
   const int rc = configure_decode(kernel, 224 * 1024, configured_dev);
   if (rc != LF_OK) return rc;
   return launched(launch_splits(kernel, p, WARPS * 32, smem, st, p, G), "decode_mma_kernel");
 }
 
-template <int D, bool PAGED, int MODS, bool WIDE_P>
+template <int D, bool PAGED, int MODS, int P_TERMS>
 static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, size_t table_bytes) {
   const int64_t ctas = static_cast<int64_t>(p.splits) * p.Hkv * p.B;
   const int sms = device_sm_count();
@@ -733,12 +734,12 @@ static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, si
   //   up to five: half-sized CTAs as well, six resident (512 units of 2048 keys 87 -> 85 us, 640 of
   //     3001 keys 171 -> 150); at D = 64, where the rings are half as large, three stages of up to four.
   if (ctas * 10 <= 9ll * sms && p.splits <= 4)
-    return launch_decode_w<D, PAGED, MODS, WIDE_P, 8, 3>(p, G, st, table_bytes);
+    return launch_decode_w<D, PAGED, MODS, P_TERMS, 8, 3>(p, G, st, table_bytes);
   if (ctas <= 2ll * sms || ctas > (D == 128 ? 5ll : 4ll) * sms)
-    return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 3>(p, G, st, table_bytes);
+    return launch_decode_w<D, PAGED, MODS, P_TERMS, 4, 3>(p, G, st, table_bytes);
   if (ctas <= 3ll * sms)
-    return launch_decode_w<D, PAGED, MODS, WIDE_P, 4, 2>(p, G, st, table_bytes);
-  return launch_decode_w<D, PAGED, MODS, WIDE_P, 2, D == 128 ? 2 : 3>(p, G, st, table_bytes);
+    return launch_decode_w<D, PAGED, MODS, P_TERMS, 4, 2>(p, G, st, table_bytes);
+  return launch_decode_w<D, PAGED, MODS, P_TERMS, 2, D == 128 ? 2 : 3>(p, G, st, table_bytes);
 }
 
 template <int D, bool PAGED>
@@ -747,8 +748,8 @@ static int launch_decode(const DecodeParams& p, int G, int mods, cudaStream_t st
   auto with_mods = [&](auto m) {
     constexpr int kMods = decltype(m)::value;
     if constexpr (!PAGED)
-      if (G <= 2) return launch_decode_shape<D, PAGED, kMods, true>(p, G, st, table_bytes);
-    return launch_decode_shape<D, PAGED, kMods, false>(p, G, st, table_bytes);
+      if (G <= 2) return launch_decode_shape<D, PAGED, kMods, 3>(p, G, st, table_bytes);
+    return launch_decode_shape<D, PAGED, kMods, 2>(p, G, st, table_bytes);
   };
   if (mods == kModsNone) return with_mods(std::integral_constant<int, kModsNone>{});
   if (mods == kModsSoftcap) return with_mods(std::integral_constant<int, kModsSoftcap>{});

@@ -182,3 +182,32 @@ def test_splits_of_grids_of_many_waves(G, Skv, splits, D):
     q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
     out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
     check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hkv,G,Skv,splits,page", [
+    (1, 2, 4, 700, 1, 0), (1, 2, 8, 2100, 16, 0), (2, 3, 4, 515, 0, 0), (40, 8, 8, 65, 1, 0),
+    (2, 3, 1, 517, 4, 1), (2, 2, 8, 1000, 2, 16), (70, 8, 4, 130, 1, 16), (2, 2, 2, 1203, 20, 24),
+])
+def test_probabilities_keep_two_bf16_parts(B, Hkv, G, Skv, splits, page, D):
+    """However the keys are dealt out to warps and splits, P's rounding does not show. The result is
+    rounded by up to 2^-8 of itself, each weight by 2^-18; scores, exp2 and sums in fp32 add about
+    2^-19 each: 2^-16 of the weighted |v| in all (with P in one bf16, 2^-9 of each weight)."""
+    g = torch.Generator().manual_seed(15)
+    q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    if not page:
+        out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
+    else:
+        blocks = -(-Skv // page)
+        table = torch.randperm(B * blocks, generator=g).view(B, blocks).int()
+        pools = []
+        for x in (k, v):
+            pool = torch.zeros(B * blocks, page, Hkv, D).bfloat16()
+            rows = torch.nn.functional.pad(x, (0, 0, 0, blocks * page - Skv)).transpose(1, 2)
+            pool[table.long()] = rows.reshape(B, blocks, page, Hkv, D)
+            pools.append(pool.cuda())
+        out = F.paged_decode_attention(q.cuda(), *pools, table.cuda(), seq_len=Skv,
+                                       scale=D ** -0.5, splits=splits)
+    want = want_of(q, k, v, "none")
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -16 * want_of(q, k, v.abs(), "none")
+    assert bool(((out.double().cpu() - want).abs() <= bound).all())
