@@ -699,6 +699,45 @@ static int configure_decode(Kernel kernel, int smem, int& configured_dev) {
   return LF_OK;
 }
 
+// What launch_decode returns when the device cannot hold a cluster of a call's splits.
+constexpr int kNoCluster = 1;
+
+// Whether a cluster of `splits` CTAs can be resident at all. Sixteens of this size can on a whole B200,
+// but not on every part of one (fewer SMs per GPC); the combine kernel serves the others. Asked
+// once per kernel, thread and device for each cluster size, with the most shared memory it uses.
+struct ClusterFit {
+  int dev = -1;
+  uint32_t known = 0, fits = 0;  // bit s: clusters of s
+};
+template <class Kernel>
+static bool cluster_fits(Kernel kernel, int splits, int threads, size_t smem, ClusterFit& cache) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (cache.dev != dev) cache = ClusterFit{dev, 0, 0};
+  const uint32_t bit = 1u << splits;
+  if (!(cache.known & bit)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    cache.known |= bit;
+    if (n > 0) cache.fits |= bit;
+  }
+  return (cache.fits & bit) != 0;
+}
+
 static int launched(cudaError_t e, const char* where) {
   if (e == cudaSuccess) return check_launch(where);
   cudaGetLastError();
@@ -706,22 +745,30 @@ static int launched(cudaError_t e, const char* where) {
   return LF_ERR_CUDA;
 }
 
+// (`st` null: nothing is launched, only a cluster that cannot be is told.)
 template <int D, bool PAGED, int MODS, int P_TERMS, int WARPS, int STAGES>
-static int launch_decode_w(DecodeParams p, int G, cudaStream_t st, size_t table_bytes) {
+static int launch_decode_w(DecodeParams p, int G, const cudaStream_t* st, size_t table_bytes) {
   // page ids + the per-warp K/V rings (the warp-merge area and the partial reuse the rings)
-  const size_t ring = static_cast<size_t>(WARPS) * STAGES * 2 * 16 * D * 2;
-  const size_t merge = static_cast<size_t>(WARPS + 1) * G * (D + 2) * sizeof(float);
-  const size_t smem = table_bytes + (ring > merge ? ring : merge);
+  constexpr size_t ring = static_cast<size_t>(WARPS) * STAGES * 2 * 16 * D * 2;
+  constexpr size_t max_merge = static_cast<size_t>(WARPS + 1) * 8 * (D + 2) * sizeof(float);
+  static_assert(max_merge <= ring, "the warps' merge area lies in the rings");
+  const size_t smem = table_bytes + ring;
   p.part_off = static_cast<int32_t>(table_bytes + WARPS * static_cast<size_t>(G) * (D + 2) * 4);
   static thread_local int configured_dev = -1;
+  static thread_local ClusterFit fit;
   const auto kernel = decode_mma_kernel<D, PAGED, MODS, WARPS, STAGES, P_TERMS>;
   const int rc = configure_decode(kernel, 224 * 1024, configured_dev);
-  if (rc != LF_OK) return rc;
-  return launched(launch_splits(kernel, p, WARPS * 32, smem, st, p, G), "decode_mma_kernel");
+  if (rc != LF_OK) return st ? rc : kNoCluster;
+  if (p.cluster && !cluster_fits(kernel, p.splits, WARPS * 32,
+                                 ring + (PAGED ? kMaxTableBytes : 0), fit))
+    return kNoCluster;
+  if (!st) return LF_OK;
+  return launched(launch_splits(kernel, p, WARPS * 32, smem, *st, p, G), "decode_mma_kernel");
 }
 
 template <int D, bool PAGED, int MODS, int P_TERMS>
-static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, size_t table_bytes) {
+static int launch_decode_shape(const DecodeParams& p, int G, const cudaStream_t* st,
+                               size_t table_bytes) {
   const int64_t ctas = static_cast<int64_t>(p.splits) * p.Hkv * p.B;
   const int sms = device_sm_count();
   // Warps and ring depth, by how full the machine is (times: B200, D = 128, G = 4 paged):
@@ -743,7 +790,7 @@ static int launch_decode_shape(const DecodeParams& p, int G, cudaStream_t st, si
 }
 
 template <int D, bool PAGED>
-static int launch_decode(const DecodeParams& p, int G, int mods, cudaStream_t st,
+static int launch_decode(const DecodeParams& p, int G, int mods, const cudaStream_t* st,
                          size_t table_bytes) {
   auto with_mods = [&](auto m) {
     constexpr int kMods = decltype(m)::value;
@@ -780,18 +827,6 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
   if (splits < 0) return LF_ERR_INVALID_ARG;
   if (splits > 32) return LF_ERR_TOO_LARGE;
   if (splits == 0) splits = choose_splits(a->B, a->Hkv, a->Skv, a->D, paged ? a->page_size : 0);
-  // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
-  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups. (In pairs:
-  // 2048 units of 2048 keys, each call on other buffers, 313 -> 324 us; 3000 one-token pages 475 -> 510.)
-  // Token chunk per split: a multiple of 16, so a split never starts in the middle of a warp's token
-  // batch. Where the rounding leaves a cluster's last splits empty the count stays as it is; their
-  // partials have weight zero. (Powers of two make the better clusters: over 70 sizes whose count the
-  // rounding to 64 would trim, to 3, 6, 7 or 11..15, 6 % less time warm and 3 % cold.)
-  const bool cluster = splits > 1 && splits <= kMaxCluster &&
-                       static_cast<int64_t>(splits) * a->Hkv * a->B <= 8ll * device_sm_count();
-  if (!cluster) splits = partial_splits(a->Skv, splits);
-  const int chunk = cluster ? round_up((a->Skv + splits - 1) / splits, 16)
-                            : partial_chunk(a->Skv, splits);
   const int partials = partial_splits(a->Skv, splits);
   if (partials > 1) {
     const size_t need = lf_decode_workspace_bytes(a->B, a->Hkv, a->G, a->D, partials);
@@ -806,7 +841,7 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
   p.out = static_cast<__nv_bfloat16*>(a->out);
   const int64_t units = static_cast<int64_t>(a->B) * a->Hkv * a->G;
   p.part_o = static_cast<float*>(a->workspace);
-  p.part_ml = p.part_o ? p.part_o + units * splits * a->D : nullptr;
+  p.part_ml = p.part_o ? p.part_o + units * partials * a->D : nullptr;
   p.block_table = a->block_table;
   p.block_table_v = a->block_table_v ? a->block_table_v : a->block_table;
   p.status = a->status;
@@ -820,8 +855,6 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
   p.B = a->B;
   p.Hkv = a->Hkv;
   p.Skv = a->Skv;
-  p.splits = splits;
-  p.chunk = chunk;
   p.page_size = paged ? a->page_size : 1;
   p.page_shift = -1;
   for (int sh = 0; sh < 31; ++sh)
@@ -856,30 +889,45 @@ static int decode_impl(const LfDecodeArgs* a, void* const* stream, bool paged) {
       }
     }
   }
-  p.cluster = cluster;
 
-  size_t table_bytes = 0;
-  if (paged) {
-    // A split's block-table slice lives in shared memory next to the K/V rings. The automatic
-    // split count already keeps it small enough; an explicit count that does not is refused
-    // (pass a larger `splits`, or 0).
-    table_bytes = table_smem_bytes(chunk, p.page_size);
-    if (table_bytes > kMaxTableBytes) return LF_ERR_TOO_LARGE;
-  }
-  const bool combine = splits > 1 && !cluster;
-  if (stream == nullptr) return combine ? 2 : 1;
-
-  cudaStream_t st = static_cast<cudaStream_t>(*stream);
-  int rc;
-  if (a->D == 128)
-    rc = paged ? launch_decode<128, true>(p, a->G, mods, st, table_bytes)
-               : launch_decode<128, false>(p, a->G, mods, st, table_bytes);
-  else
-    rc = paged ? launch_decode<64, true>(p, a->G, mods, st, table_bytes)
-               : launch_decode<64, false>(p, a->G, mods, st, table_bytes);
+  const cudaStream_t st = stream ? static_cast<cudaStream_t>(*stream) : nullptr;
+  auto attempt = [&](bool cluster) -> int {
+    // Tokens per split: a multiple of 16, so a split never starts in the middle of a warp's token batch.
+    // Where the rounding leaves a cluster's last splits empty the count stays as it is; their partials
+    // have weight zero. (Powers of two make the better clusters: over 70 sizes whose count a rounding to
+    // 64 would trim, to 3, 6, 7 or 11..15, 6 % less time warm and 3 % cold.)
+    p.cluster = cluster;
+    p.splits = cluster ? splits : partials;
+    p.chunk = cluster ? round_up((a->Skv + splits - 1) / splits, 16) : partial_chunk(a->Skv, splits);
+    size_t table_bytes = 0;
+    if (paged) {
+      // A split's block-table slice lives in shared memory next to the K/V rings. The automatic
+      // split count already keeps it small enough; an explicit count that does not is refused
+      // (pass a larger `splits`, or 0).
+      table_bytes = table_smem_bytes(p.chunk, p.page_size);
+      if (table_bytes > kMaxTableBytes) return LF_ERR_TOO_LARGE;
+    }
+    if (!stream && !cluster) return LF_OK;
+    const cudaStream_t* to = stream ? &st : nullptr;
+    if (a->D == 128)
+      return paged ? launch_decode<128, true>(p, a->G, mods, to, table_bytes)
+                   : launch_decode<128, false>(p, a->G, mods, to, table_bytes);
+    return paged ? launch_decode<64, true>(p, a->G, mods, to, table_bytes)
+                 : launch_decode<64, false>(p, a->G, mods, to, table_bytes);
+  };
+  // The splits merge in their cluster where one holds them and the grid is about one wave; a grid
+  // of many waves hides the combine kernel's time, and its CTAs need not be placed in groups. (In pairs:
+  // 2048 units of 2048 keys, each call on other buffers, 313 -> 324 us; 3000 one-token pages 475 -> 510.)
+  int rc = kNoCluster;
+  if (splits > 1 && splits <= kMaxCluster &&
+      static_cast<int64_t>(splits) * a->Hkv * a->B <= 8ll * device_sm_count())
+    rc = attempt(true);
+  if (rc == kNoCluster) rc = attempt(false);
   if (rc != LF_OK) return rc;
+  const bool combine = p.splits > 1 && !p.cluster;
+  if (!stream) return combine ? 2 : 1;
   if (combine)
-    rc = lf_combine_f32(p.part_o, p.part_ml, a->out, a->B, a->Hkv, a->G, a->D, splits,
+    rc = lf_combine_f32(p.part_o, p.part_ml, a->out, a->B, a->Hkv, a->G, a->D, p.splits,
                         a->o_stride, *stream);
   return rc;
 }

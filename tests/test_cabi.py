@@ -5,6 +5,9 @@ import random
 import re
 from pathlib import Path
 
+import pytest
+import torch
+
 from loopfuse_b200 import _native
 
 HEADER = Path(__file__).resolve().parents[1] / "include" / "lf_sm100.h"
@@ -138,3 +141,16 @@ def test_many_waves_are_halved_only_where_it_pays(native_lib):
     assert auto(64, 32, 1, 2048, 64, 0) == 1
     assert auto(64, 32, 1, 1000, 128, 0) == 1
     assert auto(64, 32, 1, 2048, 128, 16) == 1
+
+
+def test_splits_go_through_the_workspace_where_no_cluster_can_hold_them(native_lib):
+    """Where the device does not say that it can hold a cluster of the splits, the combine kernel
+    merges them (here: there is no device to say so)."""
+    if torch.cuda.is_available():
+        pytest.skip("a device is there")
+    need = native_lib.lf_decode_workspace_bytes(1, 8, 4, 128, 16)
+    for page in (0, 16):
+        a = decode_call(1, 8, 4, 8190, 128, page, 16, need)
+        assert native_lib.lf_decode_launches(C.byref(a), page > 0) == 2
+        a.splits = 1
+        assert native_lib.lf_decode_launches(C.byref(a), page > 0) == 1

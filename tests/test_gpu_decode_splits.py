@@ -211,3 +211,18 @@ def test_probabilities_keep_two_bf16_parts(B, Hkv, G, Skv, splits, page, D):
     want = want_of(q, k, v, "none")
     bound = 2.0 ** -8 * want.abs() + 2.0 ** -16 * want_of(q, k, v.abs(), "none")
     assert bool(((out.double().cpu() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("splits", range(2, 21))
+def test_every_split_count_merges(splits):
+    """Clusters of up to 16, which a whole B200 can hold, and the combine kernel beyond."""
+    B, Hkv, G, Skv, D = 1, 3, 4, 1003, 128
+    g = torch.Generator().manual_seed(16)
+    q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
+    check(out, want_of(q, k, v, "none"), v, "none", wide_p=True)
+    a = _native.LfDecodeArgs()
+    a.q = a.k = a.v = a.out = a.workspace = q.data_ptr()     # (only looked at)
+    a.workspace_bytes = 1 << 30
+    a.B, a.Hkv, a.G, a.Skv, a.D, a.splits = B, Hkv, G, Skv, D, splits
+    assert _native.load().lf_decode_launches(C.byref(a), 0) == (1 if splits <= 16 else 2)
