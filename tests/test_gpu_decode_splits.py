@@ -1,7 +1,7 @@
 """Decode where its splits, CTA shapes and score functions change: clusters of 2 to 16 that merge in
 shared memory (the last splits ragged or empty, block-table slices of different padding), the combine
 kernel beyond 16, eight, four and two warps per CTA, the folded softcap beside the interpreted chain,
-and P at full precision where one or two query rows share a kv head."""
+and P at more than one bf16's precision."""
 import ctypes as C
 import threading
 
@@ -21,22 +21,26 @@ MODS = {
 
 
 def want_of(q, k, v, mods):
+    """(result, allowed error) in fp64. The result is rounded to bf16, up to 2^-8 of itself. P has two
+    bf16 parts at least, 2^-18 of each weight; scores, exp2 and sums in fp32 add about 2^-19 each: 2^-16
+    of the weighted |v|. tanh.approx (which fast-math tanhf is too) is 2^-11 off its value at most: a
+    logit l that comes from it moves its weight, and by it the sum, by 2^-11 |l|."""
     s = (q.double() @ k.double().transpose(-1, -2)) * q.shape[-1] ** -0.5
+    from_tanh = torch.zeros_like(s)
     if mods == "softcap":
-        s = torch.tanh(s / 30.0) * 30.0
+        s = from_tanh = torch.tanh(s / 30.0) * 30.0
     elif mods == "chain":
-        s = (torch.tanh(s) + 0.5) * 3.0
-    return torch.softmax(s, -1) @ v.double()
+        from_tanh = torch.tanh(s) * 3.0
+        s = from_tanh + 1.5
+    p, v = torch.softmax(s, -1), v.double()
+    want, moved = p @ v, p * from_tanh.abs()
+    return want, (2.0 ** -8 * want.abs() + 2.0 ** -16 * (p @ v.abs())
+                  + 2.0 ** -11 * (moved @ v.abs() + moved.sum(-1, keepdim=True) * want.abs()))
 
 
-def check(out, want, v, mods, wide_p):
-    """Half an ulp of the bf16 result, 2^-8 |o|; P in bf16, 2^-9 of weights that sum to one, times
-    max |v|; tanh.approx, 2^-11 of its range, moves a logit by 30 * 2^-11 (3 * 2^-11 for the chain)
-    and with it every weight by that fraction, twice (its own and the sum's)."""
-    vmax = v.abs().max().item()
-    tanh = {"none": 0.0, "softcap": 30.0, "chain": 3.0}[mods] * 2.0 ** -11 * 2.0
-    bound = 2.0 ** -8 * want.abs() + vmax * ((2.0 ** -15 if wide_p else 2.0 ** -9) + tanh)
-    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+def check(out, q, k, v, mods="none"):
+    want, allowed = want_of(q, k, v, mods)
+    assert bool(((out.double().cpu() - want).abs() <= allowed).all())
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -50,7 +54,24 @@ def test_dense_splits(B, Hkv, G, Skv, splits, mods, D):
     q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
     out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, mods=MODS[mods],
                              splits=splits)
-    check(out, want_of(q, k, v, mods), v, mods, wide_p=G <= 2)
+    check(out, q, k, v, mods)
+
+
+@pytest.mark.parametrize("mods", ["none", "softcap", "chain"])
+@pytest.mark.parametrize("B,Hkv,G,Skv,splits", [(2, 3, 1, 257, 2), (1, 3, 2, 2100, 16),
+                                                (1, 2, 4, 2100, 8), (2, 5, 4, 700, 20)])
+def test_the_allowed_error_sees_a_missing_split(B, Hkv, G, Skv, splits, mods):
+    """Zeros, and results that lack the first or the last split, are outside of it (in the oracle)."""
+    g = torch.Generator().manual_seed(5)
+    q, k, v = [torch.randn(B, Hkv, n, 64, generator=g).bfloat16() for n in (G, Skv, Skv)]
+    chunk = -(-Skv // splits)
+    with pytest.raises(AssertionError):
+        check(torch.zeros(B, Hkv, G, 64), q, k, v, mods)
+    for lacking in (slice(chunk, None), slice(0, (splits - 1) * chunk)):
+        out = want_of(q, k[:, :, lacking], v[:, :, lacking], mods)[0]
+        with pytest.raises(AssertionError):
+            check(out, q, k, v, mods)
+    check(want_of(q, k, v, mods)[0].bfloat16(), q, k, v, mods)
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -72,7 +93,7 @@ def test_paged_splits(P, Skv, splits, D):
         F.check_status(st)
         k = O.paged_kv_ref(kp, kt)[:, :, :Skv]
         v = O.paged_kv_ref(vp, kt if table_v is None else table_v)[:, :, :Skv]
-        check(out, want_of(q, k, v, "none"), v, "none", wide_p=False)
+        check(out, q, k, v)
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -89,7 +110,7 @@ def test_infinite_values_stay_infinite(B, Hkv, G, Skv, splits, D):
     assert bool(out[..., 40].isnan().all())
     v[:, :, [5, 17, 21], [3, 9, 40]] = 0.0
     keep = [c for c in range(D) if c not in (3, 9, 40)]
-    check(out[..., keep], want_of(q, k, v, "none")[..., keep], v, "none", wide_p=G <= 2)
+    check(out[..., keep], q, k, v[..., keep])
 
 
 @pytest.mark.parametrize("B,Hkv,G,Skv", [(2, 8, 4, 1100), (3, 1, 1, 2055), (2, 4, 4, 7369)])
@@ -101,7 +122,7 @@ def test_library_chosen_splits_of_ragged_lengths(B, Hkv, G, Skv):
     auto = _native.load().lf_decode_auto_splits(B, Hkv, G, Skv, 128, 0)
     assert auto in (8, 16)
     out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=128 ** -0.5)
-    check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
+    check(out, q, k, v)
     again = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=128 ** -0.5, splits=auto)
     assert torch.equal(out, again)
 
@@ -181,7 +202,7 @@ def test_splits_of_grids_of_many_waves(G, Skv, splits, D):
     g = torch.Generator().manual_seed(14)
     q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
     out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
-    check(out, want_of(q, k, v, "none"), v, "none", wide_p=G <= 2)
+    check(out, q, k, v)
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -190,9 +211,8 @@ def test_splits_of_grids_of_many_waves(G, Skv, splits, D):
     (2, 3, 1, 517, 4, 1), (2, 2, 8, 1000, 2, 16), (70, 8, 4, 130, 1, 16), (2, 2, 2, 1203, 20, 24),
 ])
 def test_probabilities_keep_two_bf16_parts(B, Hkv, G, Skv, splits, page, D):
-    """However the keys are dealt out to warps and splits, P's rounding does not show. The result is
-    rounded by up to 2^-8 of itself, each weight by 2^-18; scores, exp2 and sums in fp32 add about
-    2^-19 each: 2^-16 of the weighted |v| in all (with P in one bf16, 2^-9 of each weight)."""
+    """However the keys are dealt out to warps and splits, P's rounding does not show (with P in one
+    bf16, 2^-9 of each weight, it does)."""
     g = torch.Generator().manual_seed(15)
     q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
     if not page:
@@ -208,9 +228,7 @@ def test_probabilities_keep_two_bf16_parts(B, Hkv, G, Skv, splits, page, D):
             pools.append(pool.cuda())
         out = F.paged_decode_attention(q.cuda(), *pools, table.cuda(), seq_len=Skv,
                                        scale=D ** -0.5, splits=splits)
-    want = want_of(q, k, v, "none")
-    bound = 2.0 ** -8 * want.abs() + 2.0 ** -16 * want_of(q, k, v.abs(), "none")
-    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+    check(out, q, k, v)
 
 
 @pytest.mark.parametrize("splits", range(2, 21))
@@ -220,7 +238,7 @@ def test_every_split_count_merges(splits):
     g = torch.Generator().manual_seed(16)
     q, k, v = [torch.randn(B, Hkv, n, D, generator=g).bfloat16() for n in (G, Skv, Skv)]
     out = F.decode_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5, splits=splits)
-    check(out, want_of(q, k, v, "none"), v, "none", wide_p=True)
+    check(out, q, k, v)
     a = _native.LfDecodeArgs()
     a.q = a.k = a.v = a.out = a.workspace = q.data_ptr()     # (only looked at)
     a.workspace_bytes = 1 << 30
