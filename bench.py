@@ -32,6 +32,7 @@ One JSON line is printed by rank 0. Besides the contract keys it carries
 from __future__ import annotations
 
 import argparse
+import ctypes
 import dataclasses
 import json
 import os
@@ -54,8 +55,8 @@ METRIC = "prefill TFLOP/s (causal-adjusted FLOPs) per job; decode HBM GB/s under
 NCU_TRAFFIC_BYTES = {
     "causal_softcap": 4 * (108.67e6 + 14.64e6),
     "window_gqa_softcap": 2 * (100.74e6 + 30.84e6),
-    "decode": 8 * (268.51e6 + 4.03e6),
-    "paged_decode_gqa": 2 * (268.79e6 + 5.29e6),
+    "decode": 8 * (268.56e6 + 3.22e6),
+    "paged_decode_gqa": 2 * (268.78e6 + 4.01e6),
 }
 FULL_BATCH: dict = {}   # workload name -> batch of the benchmark configuration
 
@@ -275,11 +276,14 @@ class Runner:
             self.launch = lambda: F.paged_decode_attention(q, kp, vp, table, scale=scale, out=out,
                                                            workspace=ws)
             page = w.page_size
-        splits = _native.load().lf_decode_auto_splits(w.B, w.Hkv, w.group, w.S, w.D, page)
-        # Splits merge in their cluster; in a grid of many waves a second kernel merges them.
-        sms = torch.cuda.get_device_properties(0).multi_processor_count
-        merged = splits <= 16 and splits * w.Hkv * w.B <= 8 * sms
-        self.launches_per_call = 1 if splits == 1 or merged else 2
+        # Kernels per call, as the library says: the addresses are only looked at.
+        a = _native.LfDecodeArgs()
+        a.q = a.k = a.v = a.out = a.workspace = a.block_table = out.data_ptr()
+        a.workspace_bytes = 1 << 40
+        a.B, a.Hkv, a.G, a.Skv, a.D = w.B, w.Hkv, w.group, w.S, w.D
+        a.page_size = a.n_pages = page
+        self.launches_per_call = _native.load().lf_decode_launches(ctypes.byref(a), page > 0)
+        _native.check(min(self.launches_per_call, 0), "lf_decode_launches")
 
 
 def events():

@@ -8,8 +8,9 @@
 //     decode_mma_kernel), softmax is online in the log2 domain;
 //   * with splits > 1 the CTAs of a (batch, kv head) form a thread-block cluster and merge their
 //     un-normalised partials (acc, max, sum) through distributed shared memory (log-sum-exp
-//     combine); where they cannot (more splits than a cluster holds, or grids of many waves), each
-//     CTA writes its partial to the workspace and lf_combine merges them;
+//     combine); where they cannot (more splits than a cluster holds, grids of many waves, or a device
+//     that cannot hold the cluster), each CTA writes its partial to the workspace and lf_combine
+//     merges them;
 //   * the paged variant stages its slice of the block table through shared memory, checks
 //     every page id against the pool size (status word, clamped, never a trap) and turns
 //     (page, slot) into row pointers.
@@ -291,10 +292,9 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
         }
       } else {
         // Rows that pages scatter: lane r < 16 finds K row r of the group, lane 16 + r V row r, and the
-        // lanes that copy a row get its place by shuffle. (With every lane looking up every row it
-        // copies: 416 units of 6443 one-token pages 300 us, now
-        // 217.) Rows past the end of the split re-read its
-        // last token.
+        // lanes that copy a row get its place by shuffle (416 units of 6443 one-token pages 300 -> 217 us
+        // against every lane looking up every row that it copies). Rows past the end of the split
+        // re-read its last token.
         const int tok = min(tg + (lane & 15), t_last);
         const int64_t off = lane < 16 ? k_row(tok) - kbase : v_row(tok) - vbase;
 #pragma unroll
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(WARPS * 32, (STAGES == 3 ? 8 : 12) / WARPS)
   }
   cp_async_wait<0>();
   // (Not earlier: the next launch's CTAs would take the places that this one's leave as they come,
-  // and crowd on some SMs. 512 units of 2048 keys 87 -> 94 us with the trigger at the top.)
+  // and crowd on some SMs: 512 units of 2048 keys take 8 % longer with the trigger at the top.)
   pdl_trigger();
 
   // Rows 8 + g (same lane), and with three parts rows 2 + g, hold the finer parts of row g.
@@ -673,7 +673,7 @@ static cudaError_t launch_splits(Kernel kernel, const DecodeParams& p, int threa
     ++cfg.numAttrs;
   }
   // Large grids wait for the kernel before them to leave the SMs: their CTAs are then dealt out
-  // evenly (512 units of 2048 keys 88 us, 90 when they start between another launch's last ones).
+  // evenly (512 units of 2048 keys take 2 % longer when they start between another launch's last ones).
   if (static_cast<int64_t>(p.splits) * p.Hkv * p.B <= 2ll * device_sm_count()) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
@@ -778,8 +778,8 @@ static int launch_decode_shape(const DecodeParams& p, int G, const cudaStream_t*
   //   otherwise four, two CTAs resident per SM (K/V rings of 96 KB each);
   //   up to three CTAs per SM: two-stage rings, so that they are all resident (320 units of 1001 keys
   //     35 -> 32 us);
-  //   up to five: half-sized CTAs as well, six resident (512 units of 2048 keys 87 -> 85 us, 640 of
-  //     3001 keys 171 -> 150); at D = 64, where the rings are half as large, three stages of up to four.
+  //   up to five: half-sized CTAs as well, six resident (640 units of 3001 keys 171 -> 150 us; 512 of
+  //     2048 the same 87); at D = 64, where the rings are half as large, three stages of up to four.
   if (ctas * 10 <= 9ll * sms && p.splits <= 4)
     return launch_decode_w<D, PAGED, MODS, P_TERMS, 8, 3>(p, G, st, table_bytes);
   if (ctas <= 2ll * sms || ctas > (D == 128 ? 5ll : 4ll) * sms)

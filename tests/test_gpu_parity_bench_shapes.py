@@ -196,7 +196,7 @@ def test_generic_score_mods_prefill_and_decode(name):
     F.check_status(st)
     want = O.attention_ref(q, k, v, scale=D ** -0.5, mods=ref_mods, mask="causal")
     assert max_err(out, want) <= TOL
-    for G in (1, 4):                                   # FMA kernel / tensor-core kernel
+    for G in (1, 4):                                   # three / two bf16 parts of P
         qd = randn_bf16(2, 2, G, D, seed=4)
         kd = randn_bf16(2, 2, 500, D, seed=5)
         vd = randn_bf16(2, 2, 500, D, seed=6)
