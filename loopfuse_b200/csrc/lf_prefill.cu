@@ -233,49 +233,88 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   const bool split = p.single;
   const int iq0 = split ? pair : pair * 2;
 
-  int lo_t[2], hi_t[2];
-  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0, &lo_t[0],
-             &hi_t[0]);
-  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0 + 1,
-             &lo_t[1], &hi_t[1]);
-  const bool tile_valid[2] = {iq0 * kTileQ < p.Sq, !split && (iq0 + 1) * kTileQ < p.Sq};
-  const bool has_work[2] = {tile_valid[0] && hi_t[0] > lo_t[0], tile_valid[1] && hi_t[1] > lo_t[1]};
+  // (Scalars and selects: an array indexed with the warp's slot lies in local memory, and with nearly all of
+  // the SM's memory taken as shared memory such a read goes to L2.)
+  int lo0, hi0, lo1, hi1;
+  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0, &lo0, &hi0);
+  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0 + 1, &lo1,
+             &hi1);
+  const bool valid0 = iq0 * kTileQ < p.Sq, valid1 = !split && (iq0 + 1) * kTileQ < p.Sq;
+  const bool work0 = valid0 && hi0 > lo0, work1 = valid1 && hi1 > lo1;
+  auto lo_t = [&](int t) { return t ? lo1 : lo0; };
+  auto hi_t = [&](int t) { return t ? hi1 : hi0; };
+  auto tile_valid = [&](int t) { return t ? valid1 : valid0; };
+  auto has_work = [&](int t) { return t ? work1 : work0; };
   int lo = 0, hi = 0;
-  if (has_work[0] && has_work[1]) {
-    lo = min(lo_t[0], lo_t[1]);
-    hi = max(hi_t[0], hi_t[1]);
-  } else if (has_work[0]) {
-    lo = lo_t[0];
-    hi = hi_t[0];
-  } else if (has_work[1]) {
-    lo = lo_t[1];
-    hi = hi_t[1];
+  if (work0 && work1) {
+    lo = min(lo0, lo1);
+    hi = max(hi0, hi1);
+  } else if (work0) {
+    lo = lo0;
+    hi = hi0;
+  } else if (work1) {
+    lo = lo1;
+    hi = hi1;
   }
 
   // ---------------- setup ----------------
-  if (warp == kMmaWarp0 && lane == 0) {
-    mbar_init(&bars->q_full[0], 1);
-    mbar_init(&bars->q_full[1], 1);
-    for (int s = 0; s < kStages; ++s) {
-      // (paged operands: one arrival of either gather warp, or one for the TMA part and one for the
-      // warp's own copies)
-      mbar_init(&bars->kv_full[s], p.paged ? 2 : 1);
-      mbar_init(&bars->kv_empty[s], 2);
-    }
-    for (int t = 0; t < 2; ++t) {
-      for (int bf = 0; bf < 2; ++bf) {
-        mbar_init(&bars->s_full[t][bf], 1);
-        mbar_init(&bars->p_full[t][bf], 128);
+  // The producer warp sets the barriers up and requests Q and the first K tiles (of dense operands) before
+  // the CTA meets: their latency then lies under the allocation of tensor memory (about 1000 clocks of
+  // the 4700 from a CTA's start to its first scores).
+  if (warp == kProducerWarp) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_q);
+      tma_prefetch_desc(&tmap_k);
+      tma_prefetch_desc(&tmap_v);
+      mbar_init(&bars->q_full[0], 1);
+      mbar_init(&bars->q_full[1], 1);
+      for (int s = 0; s < kStages; ++s) {
+        // (paged operands: one arrival of either gather warp, or one for the TMA part and one for the
+        // warp's own copies)
+        mbar_init(&bars->kv_full[s], p.paged ? 2 : 1);
+        mbar_init(&bars->kv_empty[s], 2);
       }
-      mbar_init(&bars->pv_done[t], 1);
-      mbar_init(&bars->o_final[t], 1);
+      for (int t = 0; t < 2; ++t) {
+        for (int bf = 0; bf < 2; ++bf) {
+          mbar_init(&bars->s_full[t][bf], 1);
+          mbar_init(&bars->p_full[t][bf], 4);
+        }
+        mbar_init(&bars->pv_done[t], 1);
+        mbar_init(&bars->o_final[t], 1);
+      }
+      mbar_fence_init();
     }
-    mbar_fence_init();
-  }
-  if (warp == kProducerWarp && lane == 0) {
-    tma_prefetch_desc(&tmap_q);
-    tma_prefetch_desc(&tmap_k);
-    tma_prefetch_desc(&tmap_v);
+    __syncwarp();
+    pdl_wait();
+    if (elect_one_sync()) {
+#pragma unroll 1
+      for (int t = 0; t < 2; ++t) {
+        if (!has_work(t)) continue;
+        mbar_arrive_expect_tx(&bars->q_full[t], kQTileBytes);
+#pragma unroll
+        for (int kb = 0; kb < kBlocksD; ++kb)
+          tma_load_4d(sQ + t * kQTileBytes + kb * kQBlockBytes, &tmap_q, &bars->q_full[t], kb * 64,
+                      (iq0 + t) * kTileQ, h, b);
+        if constexpr (PE)
+          tma_load_4d(sQ + t * kQTileBytes + kBlocksD * kQBlockBytes, &tmap_qpe, &bars->q_full[t], 0,
+                      (iq0 + t) * kTileQ, h, b);
+      }
+      if (!p.paged && hi > lo) {
+        const int n_k = lo + 1 < hi ? 2 : 1;
+        mbar_arrive_expect_tx(&bars->kv_full[0], n_k * kKTileBytes);
+#pragma unroll 1
+        for (int i = 0; i < n_k; ++i) {
+#pragma unroll
+          for (int kb = 0; kb < kBlocksD; ++kb)
+            tma_load_4d(sKV + i * kKVTileBytes + kb * kKVBlockBytes, &tmap_k, &bars->kv_full[0], kb * 64,
+                        (lo + i) * kTileK, hkv, b);
+          if constexpr (PE)
+            tma_load_4d(sKV + i * kKVTileBytes + kBlocksD * kKVBlockBytes, &tmap_kpe, &bars->kv_full[0],
+                        0, (lo + i) * kTileK, hkv, b);
+        }
+      }
+    }
+    __syncwarp();
   }
   if (warp == 0) {
     tmem_alloc(&bars->tmem_base, 512);
@@ -302,17 +341,6 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     // two stages in flight and a look-up in front of each.
     const bool elected = elect_one_sync();
     const int part = warp == kProducerWarp ? 0 : 1;
-    if (elected && part == 0) {
-      for (int t = 0; t < 2; ++t) {
-        if (!has_work[t]) continue;
-        mbar_arrive_expect_tx(&bars->q_full[t], kQTileBytes);
-#pragma unroll
-        for (int kb = 0; kb < kBlocksD; ++kb)
-          tma_load_4d(sQ + t * kQTileBytes + kb * kQBlockBytes, &tmap_q, &bars->q_full[t], kb * 64,
-                      (iq0 + t) * kTileQ, h, b);
-      }
-    }
-    __syncwarp();
     const int n_rows = p.n_pages * p.page_size;
     constexpr int kWindow = 8;  // tiles
     // [K or V][tile of the window][32 tokens] of this warp, in the output staging of warps 4..7: their
@@ -423,17 +451,6 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     constexpr int kChunks = D / 8;            // 16-byte pieces per row
     constexpr int kRowsPerPass = 32 / kChunks;  // rows one pass of the warp covers
     const bool elected = elect_one_sync();
-    if (elected) {
-      for (int t = 0; t < 2; ++t) {
-        if (!has_work[t]) continue;
-        mbar_arrive_expect_tx(&bars->q_full[t], kQTileBytes);
-#pragma unroll
-        for (int kb = 0; kb < kBlocksD; ++kb)
-          tma_load_4d(sQ + t * kQTileBytes + kb * kQBlockBytes, &tmap_q, &bars->q_full[t],
-                      kb * 64, (iq0 + t) * kTileQ, h, b);
-      }
-    }
-    __syncwarp();
     int n = 0;
     int published = 0;  // stages whose copies have been published
     bool ok = true;
@@ -534,26 +551,12 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     // has diverged into a single-lane branch gets few issue slots next to the softmax warps).
     {
       const bool elected = elect_one_sync();
-      for (int t = 0; t < 2; ++t) {
-        if (!has_work[t]) continue;
-        if (elected) {
-          mbar_arrive_expect_tx(&bars->q_full[t], kQTileBytes);
-#pragma unroll
-          for (int kb = 0; kb < kBlocksD; ++kb)
-            tma_load_4d(sQ + t * kQTileBytes + kb * kQBlockBytes, &tmap_q, &bars->q_full[t],
-                        kb * 64, (iq0 + t) * kTileQ, h, b);
-          if constexpr (PE)
-            tma_load_4d(sQ + t * kQTileBytes + kBlocksD * kQBlockBytes, &tmap_qpe,
-                        &bars->q_full[t], 0, (iq0 + t) * kTileQ, h, b);
-        }
-        __syncwarp();
-      }
-      int n = 0;
+      int n = 1;  // (stage 0 was requested above)
       bool ok = true;
       // A ring stage holds two 64-key tiles that the MMA warps need at the same time:
       // {K(lo), K(lo+1)} first, then {V(j), K(j+2)} for every j; one full / one empty barrier
       // per stage. `jb < 0` means the second half is not loaded (past the end of the range).
-      auto load_pair = [&](const CUtensorMap* tma, int ja, int jb) {
+      auto load_pair = [&](int ja, int jb) {
         if (!ok) return;
         const int stage = n % kStages;
         const uint32_t parity = ((n / kStages) & 1) ^ 1;
@@ -564,16 +567,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           return;
         }
         if (elected) {
-          const bool a_is_k = tma == &tmap_k;
-          mbar_arrive_expect_tx(&bars->kv_full[stage], (a_is_k ? kKTileBytes : kVTileBytes) +
-                                                           (jb >= 0 ? kKTileBytes : 0u));
+          mbar_arrive_expect_tx(&bars->kv_full[stage], kVTileBytes + (jb >= 0 ? kKTileBytes : 0u));
           unsigned char* dst = sKV + stage * (2 * kKVTileBytes);
 #pragma unroll
           for (int kb = 0; kb < kBlocksD; ++kb)
-            tma_load_4d(dst + kb * kKVBlockBytes, tma, &bars->kv_full[stage], kb * 64,
-                        ja * kTileK, hkv, b);
-          if (PE && a_is_k)
-            tma_load_4d(dst + kBlocksD * kKVBlockBytes, &tmap_kpe, &bars->kv_full[stage], 0,
+            tma_load_4d(dst + kb * kKVBlockBytes, &tmap_v, &bars->kv_full[stage], kb * 64,
                         ja * kTileK, hkv, b);
           if (jb >= 0) {
 #pragma unroll
@@ -587,10 +585,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         }
         __syncwarp();
       };
-      if (hi > lo) {
-        load_pair(&tmap_k, lo, lo + 1 < hi ? lo + 1 : -1);
-        for (int j = lo; j < hi; ++j) load_pair(&tmap_v, j, j + 2 < hi ? j + 2 : -1);
-      }
+      for (int j = lo; j < hi; ++j) load_pair(j, j + 2 < hi ? j + 2 : -1);
     }
   } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
     // ---------------- MMA issuers: one warp per query tile ----------
@@ -604,7 +599,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       const int tq = split ? 0 : t;  // query tile of this slot
       const bool elected = elect_one_sync();
       bool ok = true;
-      if (has_work[tq] && !mbar_wait(&bars->q_full[tq], 0)) {
+      if (has_work(tq) && !mbar_wait(&bars->q_full[tq], 0)) {
         report_timeout(p.status, 2);
         ok = false;
       }
@@ -620,9 +615,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       int n = 0;  // ring position, walks the same sequence as the producer
 
       auto active = [&](int j) {
-        return split ? ((j - lo) & 1) == t : has_work[t] && j >= lo_t[t] && j < hi_t[t];
+        return split ? ((j - lo) & 1) == t : has_work(t) && j >= lo_t(t) && j < hi_t(t);
       };
-      auto block_of = [&](int j) { return split ? (j - lo) >> 1 : j - lo_t[t]; };  // of this slot
+      auto block_of = [&](int j) { return split ? (j - lo) >> 1 : j - lo_t(t); };  // of this slot
       auto wait_stage = [&](int where) -> int {  // next ring stage, waited full; -1 on time-out
         const int stage = n % kStages;
         const uint32_t parity = (n / kStages) & 1;
@@ -639,34 +634,30 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         const int buf = block_of(j) & 1;
         const uint64_t kd = kdesc0 + static_cast<uint64_t>(stage * kStageUnits + half * kHalfUnits);
         const uint32_t d = s_col + buf * 64;
-        if (elected) {
 #pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks) {
-            mma_ss(d, qdesc + static_cast<uint64_t>((ks / 4) * (kQBlockBytes >> 4) + (ks % 4) * 2),
-                   kd + static_cast<uint64_t>((ks / 4) * (kKVBlockBytes >> 4) + (ks % 4) * 2),
-                   kIdescQK, ks > 0 ? 1u : 0u);
-          }
-          if constexpr (PE) {  // + Q_pe K_pe^T: the extra block of both tiles, same accumulator
-            for (int ks = 0; ks < p.pe_steps; ++ks)
-              mma_ss(d, qdesc + static_cast<uint64_t>(kBlocksD * (kQBlockBytes >> 4) + ks * 2),
-                     kd + static_cast<uint64_t>(kBlocksD * (kKVBlockBytes >> 4) + ks * 2),
-                     kIdescQK, 1u);
-          }
-          tc_commit(&bars->s_full[t][buf]);
+        for (int ks = 0; ks < D / 16; ++ks) {
+          mma_ss_if(elected, d,
+                    qdesc + static_cast<uint64_t>((ks / 4) * (kQBlockBytes >> 4) + (ks % 4) * 2),
+                    kd + static_cast<uint64_t>((ks / 4) * (kKVBlockBytes >> 4) + (ks % 4) * 2),
+                    kIdescQK, ks > 0 ? 1u : 0u);
         }
-        __syncwarp();
+        if constexpr (PE) {  // + Q_pe K_pe^T: the extra block of both tiles, same accumulator
+          for (int ks = 0; ks < p.pe_steps; ++ks)
+            mma_ss_if(elected, d,
+                      qdesc + static_cast<uint64_t>(kBlocksD * (kQBlockBytes >> 4) + ks * 2),
+                      kd + static_cast<uint64_t>(kBlocksD * (kKVBlockBytes >> 4) + ks * 2), kIdescQK,
+                      1u);
+        }
+        tc_commit_if(elected, &bars->s_full[t][buf]);
       };
       auto issue_pv = [&](int stage, int kt) {
         const uint64_t vd = vdesc0 + static_cast<uint64_t>(stage * kStageUnits);
         const uint32_t a = s_col + (kt & 1) * 64;
-        if (elected) {
 #pragma unroll
-          for (int ks = 0; ks < kTileK / 16; ++ks) {
-            mma_ts(o_col, a + ks * 8, vd + static_cast<uint64_t>(ks * (2048 >> 4)), kIdescPV,
-                   (kt > 0 || ks > 0) ? 1u : 0u);
-          }
+        for (int ks = 0; ks < kTileK / 16; ++ks) {
+          mma_ts_if(elected, o_col, a + ks * 8, vd + static_cast<uint64_t>(ks * (2048 >> 4)), kIdescPV,
+                    (kt > 0 || ks > 0) ? 1u : 0u);
         }
-        __syncwarp();
       };
 
       // Prologue: scores of the first two KV tiles (one stage).
@@ -676,11 +667,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           tc_fence_after();
           if (active(lo)) issue_qk(stage, 0, lo);
           if (lo + 1 < hi && active(lo + 1)) issue_qk(stage, 1, lo + 1);
-          if (elected) tc_commit(&bars->kv_empty[stage]);
-          __syncwarp();
+          tc_commit_if(elected, &bars->kv_empty[stage]);
         }
       }
-      const int nblk_t = split ? (hi - lo + 1 - t) >> 1 : has_work[t] ? hi_t[t] - lo_t[t] : 0;
+      const int nblk_t = split ? (hi - lo + 1 - t) >> 1 : has_work(t) ? hi_t(t) - lo_t(t) : 0;
       for (int j = lo; j < hi && ok; ++j) {
         const int st = wait_stage(4);  // {V(j), K(j+2)}
         if (st < 0) break;
@@ -699,14 +689,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           issue_pv(st, kt);
           // Completion points the softmax warps may wait on: the second-to-last PV (for a
           // rescale in the last block) and the last PV (for the epilogue).
-          if (elected) {
-            if (kt == nblk_t - 2) tc_commit(&bars->pv_done[t]);
-            if (kt == nblk_t - 1) tc_commit(&bars->o_final[t]);
-          }
+          tc_commit_if(elected && kt == nblk_t - 2, &bars->pv_done[t]);
+          tc_commit_if(elected && kt == nblk_t - 1, &bars->o_final[t]);
         }
         if (!split && j + 2 < hi && active(j + 2)) issue_qk(st, 1, j + 2);
-        if (elected) tc_commit(&bars->kv_empty[st]);
-        __syncwarp();
+        tc_commit_if(elected, &bars->kv_empty[st]);
       }
     }
   } else if (warp < kSoftmaxWarps) {
@@ -719,13 +706,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const uint32_t s_base = tmem_base + lane_addr + t * 128;
     const uint32_t o_addr = tmem_base + lane_addr + kColO + t * 128;
 
-    if (p.dbg_ranges && tile_valid[t] && row == 0) {
+    if (p.dbg_ranges && tile_valid(t) && row == 0) {
       const int64_t idx = ((static_cast<int64_t>(b) * p.Hq + h) * p.n_qtiles + (iq0 + t)) * 2;
-      p.dbg_ranges[idx] = lo_t[t];
-      p.dbg_ranges[idx + 1] = hi_t[t];
+      p.dbg_ranges[idx] = lo_t(t);
+      p.dbg_ranges[idx + 1] = hi_t(t);
     }
 
-    if (has_work[tq]) {
+    if (has_work(tq)) {
       // Visible column interval of this row: [c_lo, c_hi].
       int c_hi = p.Skv - 1;
       int c_lo = 0;
@@ -737,8 +724,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       float l_run = 0.f;
       bool ok = true;
       // Block k of this slot is block first + k * step of the tile.
-      const int first = lo_t[tq] + (split ? t : 0), step = split ? 2 : 1;
-      const int nblk = split ? (hi - lo + 1 - t) >> 1 : hi_t[t] - lo_t[t];
+      const int first = lo_t(tq) + (split ? t : 0), step = split ? 2 : 1;
+      const int nblk = split ? (hi - lo + 1 - t) >> 1 : hi_t(t) - lo_t(t);
       // Bias mode: this row's 64 bias values of a block (128 contiguous bytes) are requested a block
       // ahead, so that their latency lies under the exp2 pass and the hand-shake; read when the
       // scores were there, they cost a round trip to HBM per block. (Rows past Sq read the last
@@ -763,6 +750,33 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
             bq[4 * i] = v4.x; bq[4 * i + 1] = v4.y; bq[4 * i + 2] = v4.z; bq[4 * i + 3] = v4.w;
           }
         }
+      };
+      // O_t must hold every PV up to k-1 and none may be in flight. QK(k+1) is issued after PV(k-1), so
+      // "S(k+1) is ready" implies it; in the last block there is no S(k+1) and the MMA warp commits
+      // pv_done after the second-to-last PV instead.
+      auto pvs_before_complete = [&](int k) {
+        const bool last = k + 1 == nblk;
+        uint64_t* bar = last ? &bars->pv_done[t] : &bars->s_full[t][(k + 1) & 1];
+        if (!mbar_wait(bar, last ? 0u : (((k + 1) >> 1) & 1))) {
+          report_timeout(p.status, 12 + t);
+          return false;
+        }
+        tc_fence_after();
+        return true;
+      };
+      auto rescale_o = [&](int c, float alpha) {
+        uint32_t orr[32];
+        tmem_ld_32x32b_x32(o_addr + c * 32, orr);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
+        tmem_st_32x32b_x32(o_addr + c * 32, orr);
+      };
+      auto publish_p = [&](int buf) {  // (one arrival per warp: those of all lanes queue up behind each other)
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->p_full[t][buf]);
       };
       if constexpr (MODE == kModeBias) request_bias(0);
       for (int k = 0; k < nblk; ++k) {
@@ -880,43 +894,82 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           }
         }
 
-        // Fast pass, when every row of the warp has a reference and sees the whole block: P against
-        // the reference that the row has, without looking for the block's maximum first. P may then
-        // exceed 1, which bf16 and fp32 hold as exactly as any other magnitude; only when a row sum
-        // passes kFastRowSum is the block done again below, with its own maximum. Looking for the
-        // maximum was a sixth of the pass's instructions, and the vote on the rescale stood in front
-        // of the exp2 (causal B=1 Hq=32 Hkv=8 S=8192 D=128 559 -> 528 us, B=2 Hq=32 S=4096 D=64
-        // 294 -> 267 us). The row sum of such a block is taken over the bf16-rounded values that the PV
-        // product sees, so that numerator and denominator carry the same rounding; the other blocks
-        // (masked ones, a row's first, those done again) add fp32 P to it. Against fp64 that is no worse
-        // than fp32 P throughout: 1.98e-3 against 2.02e-3 (causal 2 x 4 x 512), 2.131e-3 against 2.136e-3
-        // (B=1 Hq=32 Hkv=8 S=8192).
+        // Plain and biased scores. P is taken against the reference that the row has, without looking for
+        // the block's maximum first: P may then exceed 1, which bf16 and fp32 hold as exactly as any other
+        // magnitude. Only when a row has no reference yet, or a row sum passes kFastRowSum, the block's own
+        // maximum is found and the reference moves. Looking for the maximum was a sixth of the pass's
+        // instructions, and the vote on the rescale stood in front of the exp2 (causal B=1 Hq=32 Hkv=8
+        // S=8192 D=128 559 -> 528 us, B=2 Hq=32 S=4096 D=64 294 -> 267 us). The row sum is taken over the
+        // bf16-rounded values that the PV product sees, so that numerator and denominator carry the same
+        // rounding; against fp64 that is no worse than fp32 P: 1.98e-3 against 2.02e-3 (causal 2 x 4 x 512).
+        // One copy of each part, and masks in a pass of their own: what the warps of an SM run over and
+        // over has to fit its instruction caches.
         if constexpr (MODE == kModeNone || MODE == kModeBias) {
-          if (!__any_sync(0xffffffffu, masked || m_used == -INFINITY)) {
+          if (__any_sync(0xffffffffu, masked)) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (c * 32 + i < rel_lo || c * 32 + i > rel_hi) sr[c][i] = 0xff800000u;  // -inf
+          }
+          uint32_t pk[32];
+          float sum;
+          bool move = __any_sync(0xffffffffu, m_used == -INFINITY), moved = false;
+#pragma unroll 1
+          for (;;) {
+            if (move) {
+              float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+              for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                  mx[2 * c] = max3(mx[2 * c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
+                  mx[2 * c + 1] = max3(mx[2 * c + 1], __uint_as_float(sr[c][i + 2]),
+                                       __uint_as_float(sr[c][i + 3]));
+                }
+              const float m_new =
+                  fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.c2);
+              // Lazy rescale: move the reference only when it grew by more than 2^8.
+              float alpha = 1.f;
+              if (m_new > -INFINITY && (m_used == -INFINITY || m_new - m_used > kRescaleThreshold)) {
+                alpha = ex2_approx(m_used - m_new);  // 0 when m_used is -inf
+                m_used = m_new;
+              }
+              if (k > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+                if (!pvs_before_complete(k)) {
+                  ok = false;
+                  break;
+                }
+#pragma unroll 1
+                for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
+              }
+              l_run *= alpha;
+              moved = true;
+            }
+            const float neg_m = m_used == -INFINITY ? 0.f : -m_used;
             float fs[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t pk[32];
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
-                const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c][i]), p.c2, -m_used));
-                const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c][i + 1]), p.c2, -m_used));
+                const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c][i]), p.c2, neg_m));
+                const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c][i + 1]), p.c2, neg_m));
                 const uint32_t pkv = pack_bf16x2(p0, p1);
                 pk[c * 16 + (i >> 1)] = pkv;
                 if ((i >> 1) & 1) add_bf16x2_to_f32(fs[2], fs[3], pkv);
                 else add_bf16x2_to_f32(fs[0], fs[1], pkv);
               }
-            const float sum = (fs[0] + fs[1]) + (fs[2] + fs[3]);
-            if (!__any_sync(0xffffffffu, !(sum <= kFastRowSum))) {
-              l_run += sum;
-              if constexpr (MODE == kModeBias) request_bias(k + 1);
-              tmem_st_32x32b_x32(s_addr, pk);
-              tmem_wait_st();
-              tc_fence_before();
-              mbar_arrive(&bars->p_full[t][buf]);
-              continue;
-            }
+            sum = (fs[0] + fs[1]) + (fs[2] + fs[3]);
+            if (moved) break;
+            move = __any_sync(0xffffffffu, !(sum <= kFastRowSum));
+            if (!move) break;
           }
+          if (!ok) break;
+          l_run += sum;
+          if constexpr (MODE == kModeBias) request_bias(k + 1);
+          tmem_st_32x32b_x32(s_addr, pk);
+          publish_p(buf);
+          continue;
         }
 
         // Pass 1: row max (and min, for the softcap range check), independent chains.
@@ -978,27 +1031,12 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // 0: x*(1 - x^2/3), 1: degree-7 polynomial, 2: MUFU tanh
         const int tanh_path = (flags & 2u) ? 2 : ((flags & 1u) ? 1 : 0);
         if (k > 0 && (flags & 4u)) {
-          // O_t must hold every PV up to k-1 and none may be in flight. QK(k+1) is issued after
-          // PV(k-1), so "S(k+1) is ready" implies it; in the last block there is no S(k+1) and
-          // the MMA warp commits pv_done after the second-to-last PV instead.
-          const bool last = k + 1 == nblk;
-          uint64_t* bar = last ? &bars->pv_done[t] : &bars->s_full[t][(k + 1) & 1];
-          if (!mbar_wait(bar, last ? 0u : (((k + 1) >> 1) & 1))) {
-            report_timeout(p.status, 12 + t);
+          if (!pvs_before_complete(k)) {
             ok = false;
             break;
           }
-          tc_fence_after();
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t orr[32];
-            tmem_ld_32x32b_x32(o_addr + c * 32, orr);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
-            tmem_st_32x32b_x32(o_addr + c * 32, orr);
-          }
+          for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
         }
         const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
 
@@ -1082,11 +1120,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         }
         const float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
         l_run = l_run * alpha + psum;
-        if constexpr (MODE == kModeBias) request_bias(k + 1);
         tmem_st_32x32b_x32(s_addr, pk);
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(&bars->p_full[t][buf]);
+        publish_p(buf);
       }
 
       // Epilogue: O_t / l -> bf16 -> global (one row per thread).
@@ -1181,7 +1216,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           __syncwarp();
         }
       }
-    } else if (tile_valid[t] && grow < p.Sq) {
+    } else if (tile_valid(t) && grow < p.Sq) {
       // No visible key at all for this tile: softmax of an all -inf row is NaN in the
       // eager computation, so the rows are written as NaN.
       __nv_bfloat16* orow = p.out + b * p.o_stride[0] + h * p.o_stride[1] +
