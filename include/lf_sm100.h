@@ -144,6 +144,16 @@ typedef struct {
   int32_t D_pe;
 } LfPrefillArgs;
 
+/* Row biases of a biased attention, bf16 [B, Hq, Sq, D], innermost stride 1, 16-byte aligned rows
+ * (element strides of b, h, row; 0 repeats): q_bias is added to q before the scores, out_bias to the
+ * output, each with one rounding to bf16 (the bits of lf_add_bf16). Either may be NULL. */
+typedef struct {
+  const void* q_bias;
+  const void* out_bias;
+  int64_t q_bias_stride[3];
+  int64_t out_bias_stride[3];
+} LfRowBias;
+
 typedef struct {
   const void* q;        /* bf16 [B, Hkv, G, D]: the G query heads that share a kv head */
   const void* k;        /* dense: bf16 [B, Hkv, Skv, D]. paged: pool [n_pages, page_size, Hkv, D] */
@@ -226,6 +236,12 @@ const char* lf_last_cuda_error(void);
  * score-function mode) on a host thread sets kernel attributes and looks up symbol addresses:
  * make it outside stream capture, from the thread that will capture. */
 int lf_prefill_bf16(const LfPrefillArgs* args, void* stream);
+/* lf_prefill_bf16 with row biases, in the same launch. Only where a score bias with nothing but
+ * multipliers in front of it goes through the biased kernel; LF_ERR_UNSUPPORTED otherwise, and
+ * LF_ERR_ALIGNMENT where a row bias is not 16-byte aligned (nothing is launched: add them with
+ * lf_add_bf16). */
+int lf_prefill_row_bias_bf16(const LfPrefillArgs* args, const LfRowBias* rows, void* stream);
+
 /* KV tile size (64 or 128 keys) of the kernel lf_prefill_bf16 would run for these arguments, or
  * a negative LfStatus; launches nothing. Skip ranges and `dbg_ranges` are in units of it.
  * Replaces the tile sizes the reference autotunes per kernel (loopfuse/codegen.py:360-393). */

@@ -19,6 +19,7 @@ EXPORTS = [
     "lf_decode_workspace_bytes", "lf_decode_launches", "lf_combine_f32", "lf_paged_gather_bf16",
     "lf_decode_bf16_static", "lf_prefill_kv_tile", "lf_prefill_q_tile", "lf_tile_map_cache_stats",
     "lf_kv_append_bf16", "lf_selftest_wait_timeout", "lf_add_bf16", "lf_debug_bounds",
+    "lf_prefill_row_bias_bf16",
 ]
 
 LF_STATIC_SCRATCH_BYTES = 8 << 20

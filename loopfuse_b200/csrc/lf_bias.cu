@@ -1,10 +1,9 @@
 // Elementwise bf16 add on [B, H, S, D] tensors: the query bias (Q + q_bias, before the attention
 // kernel) and the output bias (scores @ V + out_bias, after it) of the reference's modified
 // attention (tests/test_accuracy.py:176-194; the reference fuses both into its generated kernel,
-// loopfuse/codegen.py:454-998). Each is one rounding to bf16, exactly what the eager graph does,
-// so a separate pass gives the same bits as a fused one would; both are HBM-bound and small next
-// to the attention itself (the additive *score* bias, which is as large as the score matrix, is
-// read inside the attention kernel instead).
+// loopfuse/codegen.py:454-998). Each is one rounding to bf16, exactly what the eager graph does.
+// Where a score bias takes the attention through the biased kernel, both adds happen inside it
+// (lf_prefill_row_bias_bf16, the same bits); this pass serves the other graphs.
 #include "lf_common.cuh"
 
 namespace lf {
@@ -17,12 +16,6 @@ struct AddParams {
   int64_t total;      // pieces in all
   int64_t as[3], bs[3], os[3];
 };
-
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t x, uint32_t y) {
-  const float lo = __uint_as_float(x << 16) + __uint_as_float(y << 16);
-  const float hi = __uint_as_float(x & 0xffff0000u) + __uint_as_float(y & 0xffff0000u);
-  return pack_bf16x2(lo, hi);
-}
 
 // One thread adds one 16-byte piece; consecutive threads take consecutive pieces of a row.
 __global__ void __launch_bounds__(256) add_bf16_kernel(const AddParams p) {
@@ -38,12 +31,8 @@ __global__ void __launch_bounds__(256) add_bf16_kernel(const AddParams p) {
     const int64_t b = row / p.H;
     const uint4 x = *reinterpret_cast<const uint4*>(p.a + b * p.as[0] + h * p.as[1] + s * p.as[2] + c * 8);
     const uint4 y = ldg_stream_16(p.b + b * p.bs[0] + h * p.bs[1] + s * p.bs[2] + c * 8);
-    uint4 r;
-    r.x = add_bf16x2(x.x, y.x);
-    r.y = add_bf16x2(x.y, y.y);
-    r.z = add_bf16x2(x.z, y.z);
-    r.w = add_bf16x2(x.w, y.w);
-    *reinterpret_cast<uint4*>(p.out + b * p.os[0] + h * p.os[1] + s * p.os[2] + c * 8) = r;
+    *reinterpret_cast<uint4*>(p.out + b * p.os[0] + h * p.os[1] + s * p.os[2] + c * 8) =
+        add_bf16x8(x, y);
   }
 }
 

@@ -85,6 +85,15 @@ __device__ __forceinline__ float bf16hi_to_f32(uint32_t u) {
   return __uint_as_float(u & 0xffff0000u);
 }
 
+// a + b of two bf16 pairs, each rounded once.
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t x, uint32_t y) {
+  return pack_bf16x2(bf16lo_to_f32(x) + bf16lo_to_f32(y), bf16hi_to_f32(x) + bf16hi_to_f32(y));
+}
+__device__ __forceinline__ uint4 add_bf16x8(const uint4& x, const uint4& y) {
+  return make_uint4(add_bf16x2(x.x, y.x), add_bf16x2(x.y, y.y), add_bf16x2(x.z, y.z),
+                    add_bf16x2(x.w, y.w));
+}
+
 // 16-byte read-only global load that does not allocate in L1 (streamed once).
 __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
   uint4 r;

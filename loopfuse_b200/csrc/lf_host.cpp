@@ -68,6 +68,7 @@ PyObject* guarded(F f) {
 // ---------------------------------------------------------------------------------------
 struct Lib {
   int (*prefill)(const LfPrefillArgs*, void*) = nullptr;
+  int (*prefill_row_bias)(const LfPrefillArgs*, const LfRowBias*, void*) = nullptr;
   int (*q_tile)(const LfPrefillArgs*) = nullptr;
   int (*decode)(const LfDecodeArgs*, void*) = nullptr;
   int (*decode_paged)(const LfDecodeArgs*, void*) = nullptr;
@@ -389,15 +390,19 @@ Tensor run_prefill(const PrefillTensors& t, const PrefillOptions& o, Tensor out)
 // ---------------------------------------------------------------------------------------
 // Elementwise add, cache append
 // ---------------------------------------------------------------------------------------
-Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
-  const c10::Device dev = x.device();
-  require_cuda(x, dev);
-  require_cuda(y, dev);
+void check_add(const Tensor& x, at::IntArrayRef x_sizes, const Tensor& y) {
+  require_cuda(x, x.device());
+  require_cuda(y, x.device());
   check_bf16(x, "a");
   check_bf16(y, "b");
-  if (x.dim() != 4 || x.sizes() != y.sizes())
-    value_error("add_bf16 takes two 4-D tensors of one shape, got " + shape_text(x.sizes()) +
+  if (x_sizes.size() != 4 || x_sizes != y.sizes())
+    value_error("add_bf16 takes two 4-D tensors of one shape, got " + shape_text(x_sizes) +
                 " and " + shape_text(y.sizes()));
+}
+
+Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
+  const c10::Device dev = x.device();
+  check_add(x, x.sizes(), y);
   if (!out.defined()) {
     out = new_bf16(x.sizes(), dev);
   } else {
@@ -807,6 +812,36 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
   });
 }
 
+// A prefill with a query and / or output bias. In one launch where the library can (a score bias in front
+// of the mask); otherwise the query bias is added first and the output bias in place, by kernels of their
+// own. The same bits: each is one bf16 rounding, as in the eager graph.
+Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o, const Tensor* q_bias,
+                      const Tensor* out_bias) {
+  if (q_bias) check_add(*p.q, p.q->sizes(), *q_bias);
+  if (out_bias) check_add(*p.q, p.q->sizes(), *out_bias);
+  if (p.score_bias) {
+    LfPrefillArgs a;
+    LfRowBias rows;
+    Tensor out;
+    std::vector<Tensor> keep;
+    fill_prefill(a, p, o, out, keep);
+    std::memset(&rows, 0, sizeof(rows));
+    if (q_bias) rows.q_bias = q_bias->data_ptr(), strides3(rows.q_bias_stride, *q_bias);
+    if (out_bias) rows.out_bias = out_bias->data_ptr(), strides3(rows.out_bias_stride, *out_bias);
+    const int rc =
+        launch(p.q->device(), [&](void* st) { return lib.prefill_row_bias(&a, &rows, st); });
+    if (rc != LF_ERR_UNSUPPORTED && rc != LF_ERR_ALIGNMENT) {
+      check_rc(rc, "lf_prefill_row_bias_bf16");
+      return out;
+    }
+  }
+  const Tensor biased = q_bias ? run_add(*p.q, *q_bias, Tensor()) : Tensor();
+  if (q_bias) p.q = &biased;
+  Tensor out = run_prefill(p, o, Tensor());
+  if (out_bias) run_add(out, *out_bias, out);
+  return out;
+}
+
 // One pass of the graph on its arguments; returns the output tensor.
 Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
   const Tensor* t[kOperands];
@@ -816,10 +851,7 @@ Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
   }
   if (c.kind == kCallPrefill) {
     PrefillTensors p;
-    // The query bias is added first (one bf16 rounding, as in the eager graph), the score bias is
-    // read inside the attention kernel, the output bias is added in place.
-    const Tensor biased = t[kQBias] ? run_add(*t[kQ], *t[kQBias], Tensor()) : Tensor();
-    p.q = t[kQBias] ? &biased : t[kQ];
+    p.q = t[kQ];
     p.k = t[kK];
     p.v = t[kV];
     p.k_table = t[kKTable];
@@ -827,9 +859,9 @@ Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
     p.score_bias = t[kScoreBias];
     p.q_pe = t[kQPe];
     p.k_pe = t[kKPe];
-    Tensor out = run_prefill(p, c.prefill, Tensor());
-    if (t[kOutBias]) run_add(out, *t[kOutBias], out);
-    return out;
+    if (t[kQBias] || t[kOutBias])
+      return run_row_biased(p, c.prefill, t[kQBias], t[kOutBias]);
+    return run_prefill(p, c.prefill, Tensor());
   }
   const Tensor &q = *t[kQ], &k = *t[kK], &v = *t[kV];
   const bool paged = c.kind == kCallPagedDecode;
@@ -1008,6 +1040,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
       std::memcpy(&fn, &p, sizeof(p));
     };
     get("lf_prefill_bf16", lib.prefill);
+    get("lf_prefill_row_bias_bf16", lib.prefill_row_bias);
     get("lf_prefill_q_tile", lib.q_tile);
     get("lf_decode_bf16", lib.decode);
     get("lf_decode_paged_bf16", lib.decode_paged);

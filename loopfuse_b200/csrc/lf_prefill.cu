@@ -123,6 +123,10 @@ struct PrefillParams {
   int64_t bias_stride[3];
   int32_t bias_pos;           // the bias is added after this many ops of `mods`
   int32_t bias_sectors;       // bias rows are 32-byte aligned
+  // Bias mode: bf16 [B, Hq, Sq, D] tensors added to Q and to the output, or null.
+  const __nv_bfloat16* q_bias;
+  const __nv_bfloat16* out_bias;
+  int64_t qb_stride[3], ob_stride[3];
   int32_t* status;
   int32_t* dbg_ranges;
   // Persistent (bounded-mode) kernel only: the work queue.
@@ -153,6 +157,7 @@ struct PrefillParams {
 // Barrier block at the start of shared memory.
 struct __align__(8) PrefillBarriers {
   uint64_t q_full[2];
+  uint64_t q_ready[2];     // query bias: it has been added to Q (one arrival per warp)
   uint64_t kv_full[kMaxStages];
   uint64_t kv_empty[kMaxStages];
   uint64_t s_full[2][2];   // [tile][buffer]  MMA -> softmax
@@ -268,6 +273,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       tma_prefetch_desc(&tmap_v);
       mbar_init(&bars->q_full[0], 1);
       mbar_init(&bars->q_full[1], 1);
+      mbar_init(&bars->q_ready[0], split ? 8 : 4);
+      mbar_init(&bars->q_ready[1], 4);
       for (int s = 0; s < kStages; ++s) {
         // (paged operands: one arrival of either gather warp, or one for the TMA part and one for the
         // warp's own copies)
@@ -599,7 +606,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       const int tq = split ? 0 : t;  // query tile of this slot
       const bool elected = elect_one_sync();
       bool ok = true;
-      if (has_work(tq) && !mbar_wait(&bars->q_full[tq], 0)) {
+      const bool own_q = MODE == kModeBias && p.q_bias != nullptr;
+      if (has_work(tq) && !mbar_wait(own_q ? &bars->q_ready[tq] : &bars->q_full[tq], 0)) {
         report_timeout(p.status, 2);
         ok = false;
       }
@@ -778,8 +786,39 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[t][buf]);
       };
-      if constexpr (MODE == kModeBias) request_bias(0);
-      for (int k = 0; k < nblk; ++k) {
+      if constexpr (MODE == kModeBias) {
+        request_bias(0);
+        // The query bias: each thread adds its row (or half of it, when the slots share a tile) to the tile
+        // in shared memory, one bf16 rounding as in the eager graph. A pass of its own over Q in front of
+        // the kernel, and one over the output behind it, took 7 of 36 us at 4 x 8 x 1024, D = 64.
+        if (p.q_bias) {
+          constexpr int kPieces = D / 8;
+          const __nv_bfloat16* qb = p.q_bias + b * p.qb_stride[0] + h * p.qb_stride[1] +
+                                    static_cast<int64_t>(min(grow, p.Sq - 1)) * p.qb_stride[2];
+          const int first_piece = split ? t * (kPieces / 2) : 0;
+          const int n_pieces = split ? kPieces / 2 : kPieces;
+          uint4 add[kPieces];
+#pragma unroll
+          for (int i = 0; i < kPieces; ++i)
+            if (i < n_pieces) add[i] = ldg_stream_16(qb + (first_piece + i) * 8);
+          if (!mbar_wait(&bars->q_full[tq], 0)) {
+            report_timeout(p.status, 16 + t);
+            ok = false;
+          }
+#pragma unroll
+          for (int i = 0; i < kPieces; ++i)
+            if (i < n_pieces) {
+              const int c = first_piece + i;
+              uint4* piece = reinterpret_cast<uint4*>(sQ + tq * kQTileBytes + (c >> 3) * kQBlockBytes +
+                                                      row * 128 + (((c & 7) ^ (row & 7)) << 4));
+              *piece = add_bf16x8(*piece, add[i]);
+            }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->q_ready[tq]);
+        }
+      }
+      for (int k = 0; k < nblk && ok; ++k) {
         const int c0 = (first + k * step) * kTileK;
         const int buf = k & 1;
         const uint32_t s_addr = s_base + buf * 64;
@@ -1164,9 +1203,24 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         __nv_bfloat16* obase = p.out + b * p.o_stride[0] + h * p.o_stride[1];
         const int row0 = (iq0 + tq) * kTileQ + (warp & 3) * 32;  // first global row of the warp
         const int c_first = split ? t * (D / 64) : 0, c_end = split ? (t + 1) * (D / 64) : D / 32;
+        [[maybe_unused]] const __nv_bfloat16* ob =
+            MODE == kModeBias && p.out_bias
+                ? p.out_bias + b * p.ob_stride[0] + h * p.ob_stride[1] + (lane & 3) * 8
+                : nullptr;
 #pragma unroll 1
         for (int c = c_first; c < c_end; ++c) {
           uint32_t orr[32];
+          // (The output bias of the four pieces that this thread stores, requested before they are made.)
+          [[maybe_unused]] uint4 bias4[4];
+          if constexpr (MODE == kModeBias) {
+            if (ob) {
+#pragma unroll
+              for (int rr = 0; rr < 4; ++rr)
+                bias4[rr] = ldg_stream_16(
+                    ob + static_cast<int64_t>(min(row0 + rr * 8 + (lane >> 2), p.Sq - 1)) *
+                             p.ob_stride[2] + c * 32);
+            }
+          }
           if (!split) {
             tmem_ld_32x32b_x32(o_addr + c * 32, orr);
             tmem_wait_ld();
@@ -1207,8 +1261,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           for (int rr = 0; rr < 4; ++rr) {
             const int r = rr * 8 + (lane >> 2);
             const int q = lane & 3;
-            const uint4 w =
-                *reinterpret_cast<const uint4*>(stage + r * 64 + ((q ^ ((r >> 1) & 3)) << 4));
+            uint4 w = *reinterpret_cast<const uint4*>(stage + r * 64 + ((q ^ ((r >> 1) & 3)) << 4));
+            if constexpr (MODE == kModeBias) {
+              if (ob) w = add_bf16x8(w, bias4[rr]);
+            }
             if (row0 + r < p.Sq)
               *reinterpret_cast<uint4*>(obase + static_cast<int64_t>(row0 + r) * p.o_stride[2] +
                                         c * 32 + q * 8) = w;
@@ -1576,7 +1632,8 @@ static int choose_kv_tile(const LfPrefillArgs* a, int mode) {
 }
 
 // `launch` == nullptr: only resolve the kernel choice and return its KV tile size.
-static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile = nullptr) {
+static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile = nullptr,
+                        const LfRowBias* rows = nullptr) {
   if (!a || !a->q || !a->k || !a->v || !a->out) return LF_ERR_INVALID_ARG;
   if (a->B <= 0 || a->Hq <= 0 || a->Hkv <= 0 || a->Sq <= 0 || a->Skv <= 0)
     return LF_ERR_INVALID_ARG;
@@ -1671,6 +1728,20 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
       if (a->bias_stride[i] % 8) return LF_ERR_ALIGNMENT;
   }
 
+  p.q_bias = p.out_bias = nullptr;
+  for (int i = 0; i < 3; ++i) p.qb_stride[i] = p.ob_stride[i] = 0;
+  if (rows) {
+    p.q_bias = static_cast<const __nv_bfloat16*>(rows->q_bias);
+    p.out_bias = static_cast<const __nv_bfloat16*>(rows->out_bias);
+    if ((reinterpret_cast<uintptr_t>(rows->q_bias) | reinterpret_cast<uintptr_t>(rows->out_bias)) & 15u)
+      return LF_ERR_ALIGNMENT;
+    for (int i = 0; i < 3; ++i) {
+      p.qb_stride[i] = rows->q_bias ? rows->q_bias_stride[i] : 0;
+      p.ob_stride[i] = rows->out_bias ? rows->out_bias_stride[i] : 0;
+      if (p.qb_stride[i] % 8 || p.ob_stride[i] % 8) return LF_ERR_ALIGNMENT;
+    }
+  }
+
   // Pick the score-function mode. Leading and trailing constant multipliers are folded into
   // `a` (before) and `c2` (after); c2 must stay positive for the max-before-scale shortcut.
   int mode = kModeGeneric;
@@ -1744,6 +1815,7 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
     if (mode != kModeNone)
       return LF_ERR_UNSUPPORTED;
   }
+  if (rows && mode != kModeBias) return LF_ERR_UNSUPPORTED;
   const int kv_tile = choose_kv_tile(a, mode);
   if (kv_tile < 0) return kv_tile;
   // Two or four query heads per kv head under a window mask: the packed layout of the
@@ -1826,6 +1898,11 @@ extern "C" {
 
 int lf_prefill_bf16(const LfPrefillArgs* args, void* stream) {
   return lf::prefill_impl(args, &stream);
+}
+
+int lf_prefill_row_bias_bf16(const LfPrefillArgs* args, const LfRowBias* rows, void* stream) {
+  if (!rows || (!rows->q_bias && !rows->out_bias)) return LF_ERR_INVALID_ARG;
+  return lf::prefill_impl(args, &stream, nullptr, rows);
 }
 
 int lf_prefill_kv_tile(const LfPrefillArgs* args) { return lf::prefill_impl(args, nullptr); }

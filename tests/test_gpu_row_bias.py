@@ -1,0 +1,41 @@
+"""Query and output biases inside the biased prefill kernel: the same bits as adding them with passes of
+their own in front of and behind it. One query tile, a ragged last tile, both ways of giving a CTA its
+tiles (up to 148 tiles share one CTA each between its two slots, hundreds come in pairs), biases that
+repeat along a dimension, and operands that the fused form cannot take."""
+import pytest
+import torch
+
+from loopfuse_b200 import functional as F, loopfuse_backend, spec as S
+import loopfuse_b200.ops  # noqa: F401  (registers loopfuse::causal_mask)
+
+pytestmark = pytest.mark.gpu
+
+
+def _biased(q, k, v, q_bias, score_bias, out_bias):
+    s = (q + q_bias) @ k.transpose(-2, -1) * (q.shape[-1] ** -0.5)
+    s = s * 3.5 + score_bias
+    return torch.softmax(torch.ops.loopfuse.causal_mask(s), dim=-1) @ v + out_bias
+
+
+def _separate(q, k, v, q_bias, score_bias, out_bias):
+    out = F.prefill_attention(F.add_bf16(q, q_bias), k, v, scale=q.shape[-1] ** -0.5,
+                              mods=[S.ScoreMod(S.MOD_MUL, 3.5)], mask_kind=S.MASK_CAUSAL,
+                              score_bias=score_bias)
+    return F.add_bf16(out, out_bias)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,n", [(1, 2, 8), (1, 3, 136), (2, 3, 776), (5, 16, 264)])
+def test_same_bits_as_separate_adds(B, H, n, D):
+    g = torch.Generator(device="cuda").manual_seed(n + D)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    q, k, v = mk(B, H, n, D), mk(B, H, n, D), mk(B, H, n, D)
+    args = (q, k, v, mk(B, H, n, D), mk(B, H, n, n), mk(B, H, n, D))
+    fn = torch.compile(_biased, backend=loopfuse_backend, dynamic=True)
+    assert torch.equal(fn(*args), _separate(*args))
+    one_row = mk(1, H, 1, D).expand(B, H, n, D)                       # strides of 0
+    args = (q, k, v, one_row, args[4], one_row)
+    assert torch.equal(fn(*args), _separate(*args))
+    odd = mk(B, H, n, D + 4)[..., :D]                                 # rows that are not 16-byte aligned
+    with pytest.raises(Exception):
+        fn(q, k, v, odd, args[4], one_row)
