@@ -815,8 +815,9 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
 // A prefill with a query and / or output bias. In one launch where the library can (a score bias in front
 // of the mask); otherwise the query bias is added first and the output bias in place, by kernels of their
 // own. The same bits: each is one bf16 rounding, as in the eager graph.
-Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o, const Tensor* q_bias,
-                      const Tensor* out_bias) {
+// (Out of line: its argument records would be part of every call's frame.)
+[[gnu::noinline]] Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o,
+                                        const Tensor* q_bias, const Tensor* out_bias) {
   if (q_bias) check_add(*p.q, p.q->sizes(), *q_bias);
   if (out_bias) check_add(*p.q, p.q->sizes(), *out_bias);
   if (p.score_bias) {

@@ -789,8 +789,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       if constexpr (MODE == kModeBias) {
         request_bias(0);
         // The query bias: each thread adds its row (or half of it, when the slots share a tile) to the tile
-        // in shared memory, one bf16 rounding as in the eager graph. A pass of its own over Q in front of
-        // the kernel, and one over the output behind it, took 7 of 36 us at 4 x 8 x 1024, D = 64.
+        // in shared memory, one bf16 rounding as in the eager graph. (With passes of their own over Q in
+        // front of the kernel and over the output behind it 4 x 8 x 1024, D = 64 takes 29.9 us on the
+        // device instead of 28.9, and two more launches and allocations on the host.)
         if (p.q_bias) {
           constexpr int kPieces = D / 8;
           const __nv_bfloat16* qb = p.q_bias + b * p.qb_stride[0] + h * p.qb_stride[1] +
@@ -1008,159 +1009,158 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           if constexpr (MODE == kModeBias) request_bias(k + 1);
           tmem_st_32x32b_x32(s_addr, pk);
           publish_p(buf);
-          continue;
-        }
-
-        // Pass 1: row max (and min, for the softcap range check), independent chains.
-        float mxa[4], mna[4];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          mxa[2 * c] = mxa[2 * c + 1] = -INFINITY;
-          mna[2 * c] = mna[2 * c + 1] = INFINITY;
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float v0 = __uint_as_float(sr[c][i]), v1 = __uint_as_float(sr[c][i + 1]);
-            const float v2 = __uint_as_float(sr[c][i + 2]), v3 = __uint_as_float(sr[c][i + 3]);
-            mxa[2 * c] = max3(mxa[2 * c], v0, v1);
-            mxa[2 * c + 1] = max3(mxa[2 * c + 1], v2, v3);
-            if constexpr (MODE == kModeSoftcap) {
-              mna[2 * c] = min3(mna[2 * c], v0, v1);
-              mna[2 * c + 1] = min3(mna[2 * c + 1], v2, v3);
-            }
-          }
-        }
-        const float mx_all = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
-        float mx_keep = mx_all;
-        if (masked) {  // max over the visible columns only
+        } else {
+          // Pass 1: row max (and min, for the softcap range check), independent chains.
+          float mxa[4], mna[4];
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            mxa[c] = -INFINITY;
+            mxa[2 * c] = mxa[2 * c + 1] = -INFINITY;
+            mna[2 * c] = mna[2 * c + 1] = INFINITY;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const int cc = c * 32 + i;
-              const float v = (cc >= rel_lo && cc <= rel_hi) ? __uint_as_float(sr[c][i]) : -INFINITY;
-              mxa[c] = fmaxf(mxa[c], v);
+            for (int i = 0; i < 32; i += 4) {
+              const float v0 = __uint_as_float(sr[c][i]), v1 = __uint_as_float(sr[c][i + 1]);
+              const float v2 = __uint_as_float(sr[c][i + 2]), v3 = __uint_as_float(sr[c][i + 3]);
+              mxa[2 * c] = max3(mxa[2 * c], v0, v1);
+              mxa[2 * c + 1] = max3(mxa[2 * c + 1], v2, v3);
+              if constexpr (MODE == kModeSoftcap) {
+                mna[2 * c] = min3(mna[2 * c], v0, v1);
+                mna[2 * c + 1] = min3(mna[2 * c + 1], v2, v3);
+              }
             }
           }
-          mx_keep = fmaxf(mxa[0], mxa[1]);
-        }
-
-        // The score function is monotonic for the plain and softcap modes, so the max of the
-        // scores is the score of the max.
-        float tmax = mx_keep;
-        unsigned flags = 0;  // bit 0: |x| > poly-1 limit, bit 1: |x| > poly-3 limit, bit 2: rescale
-        if constexpr (MODE == kModeSoftcap) {
-          tmax = (mx_keep == -INFINITY) ? -INFINITY : tanh_approx(mx_keep * p.a);
-          // Every |x| of the warp's rows decides (masked columns included: their raw scores
-          // are ordinary finite numbers).
-          const float mn_all = fminf(fminf(mna[0], mna[1]), fminf(mna[2], mna[3]));
-          const float bound = fabsf(p.a) * fmaxf(fabsf(mx_all), fabsf(mn_all));
-          flags = (bound > kTanhPoly1Limit ? 1u : 0u) | (bound > kTanhPoly3Limit ? 2u : 0u);
-        }
-        const float m_new = fmaxf(m_used, tmax * p.c2);
-
-        // Lazy rescale: move the reference max only when it grew by more than 2^8.
-        float alpha = 1.f;
-        if (m_new > -INFINITY && (m_used == -INFINITY || m_new - m_used > kRescaleThreshold)) {
-          flags |= 4u;
-          alpha = ex2_approx(m_used - m_new);  // 0 when m_used is -inf
-          m_used = m_new;
-        }
-        flags = __reduce_or_sync(0xffffffffu, flags);  // one vote for all warp-level decisions
-        // 0: x*(1 - x^2/3), 1: degree-7 polynomial, 2: MUFU tanh
-        const int tanh_path = (flags & 2u) ? 2 : ((flags & 1u) ? 1 : 0);
-        if (k > 0 && (flags & 4u)) {
-          if (!pvs_before_complete(k)) {
-            ok = false;
-            break;
-          }
+          const float mx_all = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
+          float mx_keep = mx_all;
+          if (masked) {  // max over the visible columns only
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
-        }
-        const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
-
-        // Pass 2: p = exp2(score * c2 - m). Plain fp32 instructions and every exp2 on MUFU: the
-        // loop is bound by instruction issue, and the packed f32x2 forms (fewer instructions,
-        // but slower in their pipe) and an FMA-pipe emulation of part of the exp2 both measured
-        // slower than this in the fixed-reference kernel, which runs the same arithmetic.
-        const float neg_m = -m_safe;
-        float ps[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t pk[32];
-        auto finish_pair = [&](float z0, float z1, int c, int i, bool apply_mask) {
-          if (apply_mask) {
-            const int cc = c * 32 + i;
-            if (cc < rel_lo || cc > rel_hi) z0 = -INFINITY;
-            if (cc + 1 < rel_lo || cc + 1 > rel_hi) z1 = -INFINITY;
+            for (int c = 0; c < 2; ++c) {
+              mxa[c] = -INFINITY;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const int cc = c * 32 + i;
+                const float v = (cc >= rel_lo && cc <= rel_hi) ? __uint_as_float(sr[c][i]) : -INFINITY;
+                mxa[c] = fmaxf(mxa[c], v);
+              }
+            }
+            mx_keep = fmaxf(mxa[0], mxa[1]);
           }
-          const float p0 = ex2_approx(z0), p1 = ex2_approx(z1);
-          ps[(c * 2 + (i >> 1)) & 3] += p0;
-          ps[(c * 2 + (i >> 1) + 2) & 3] += p1;
-          pk[c * 16 + (i >> 1)] = pack_bf16x2(p0, p1);
-        };
-        if (MODE == kModeSoftcap && tanh_path < 2) {
-          // tanh(x) = x*(1 + y*(-1/3 + y*(2/15 + y*(-17/315)))), y = x^2, x = a*raw; the powers
-          // of a are folded into the coefficients so that the polynomial runs on raw^2.
-          const float a2 = p.a * p.a;
-          const float b1 = -a2 / 3.f;
-          const float ac = p.a * p.c2;
-          if (tanh_path == 0) {
+
+          // The score function is monotonic for the plain and softcap modes, so the max of the
+          // scores is the score of the max.
+          float tmax = mx_keep;
+          unsigned flags = 0;  // bit 0: |x| > poly-1 limit, bit 1: |x| > poly-3 limit, bit 2: rescale
+          if constexpr (MODE == kModeSoftcap) {
+            tmax = (mx_keep == -INFINITY) ? -INFINITY : tanh_approx(mx_keep * p.a);
+            // Every |x| of the warp's rows decides (masked columns included: their raw scores
+            // are ordinary finite numbers).
+            const float mn_all = fminf(fminf(mna[0], mna[1]), fminf(mna[2], mna[3]));
+            const float bound = fabsf(p.a) * fmaxf(fabsf(mx_all), fabsf(mn_all));
+            flags = (bound > kTanhPoly1Limit ? 1u : 0u) | (bound > kTanhPoly3Limit ? 2u : 0u);
+          }
+          const float m_new = fmaxf(m_used, tmax * p.c2);
+
+          // Lazy rescale: move the reference max only when it grew by more than 2^8.
+          float alpha = 1.f;
+          if (m_new > -INFINITY && (m_used == -INFINITY || m_new - m_used > kRescaleThreshold)) {
+            flags |= 4u;
+            alpha = ex2_approx(m_used - m_new);  // 0 when m_used is -inf
+            m_used = m_new;
+          }
+          flags = __reduce_or_sync(0xffffffffu, flags);  // one vote for all warp-level decisions
+          // 0: x*(1 - x^2/3), 1: degree-7 polynomial, 2: MUFU tanh
+          const int tanh_path = (flags & 2u) ? 2 : ((flags & 1u) ? 1 : 0);
+          if (k > 0 && (flags & 4u)) {
+            if (!pvs_before_complete(k)) {
+              ok = false;
+              break;
+            }
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
+          }
+          const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
+
+          // Pass 2: p = exp2(score * c2 - m). Plain fp32 instructions and every exp2 on MUFU: the
+          // loop is bound by instruction issue, and the packed f32x2 forms (fewer instructions,
+          // but slower in their pipe) and an FMA-pipe emulation of part of the exp2 both measured
+          // slower than this in the fixed-reference kernel, which runs the same arithmetic.
+          const float neg_m = -m_safe;
+          float ps[4] = {0.f, 0.f, 0.f, 0.f};
+          uint32_t pk[32];
+          auto finish_pair = [&](float z0, float z1, int c, int i, bool apply_mask) {
+            if (apply_mask) {
+              const int cc = c * 32 + i;
+              if (cc < rel_lo || cc > rel_hi) z0 = -INFINITY;
+              if (cc + 1 < rel_lo || cc + 1 > rel_hi) z1 = -INFINITY;
+            }
+            const float p0 = ex2_approx(z0), p1 = ex2_approx(z1);
+            ps[(c * 2 + (i >> 1)) & 3] += p0;
+            ps[(c * 2 + (i >> 1) + 2) & 3] += p1;
+            pk[c * 16 + (i >> 1)] = pack_bf16x2(p0, p1);
+          };
+          if (MODE == kModeSoftcap && tanh_path < 2) {
+            // tanh(x) = x*(1 + y*(-1/3 + y*(2/15 + y*(-17/315)))), y = x^2, x = a*raw; the powers
+            // of a are folded into the coefficients so that the polynomial runs on raw^2.
+            const float a2 = p.a * p.a;
+            const float b1 = -a2 / 3.f;
+            const float ac = p.a * p.c2;
+            if (tanh_path == 0) {
+              auto body = [&](bool apply_mask) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                  for (int i = 0; i < 32; i += 2) {
+                    const float r0 = __uint_as_float(sr[c][i]), r1 = __uint_as_float(sr[c][i + 1]);
+                    const float q0 = fmaf(r0 * r0, b1, 1.f), q1 = fmaf(r1 * r1, b1, 1.f);
+                    finish_pair(fmaf(r0 * ac, q0, neg_m), fmaf(r1 * ac, q1, neg_m), c, i,
+                                apply_mask);
+                  }
+              };
+              if (masked) body(true); else body(false);
+            } else {
+              const float b2 = a2 * a2 * (2.f / 15.f);
+              const float b3 = a2 * a2 * a2 * (-17.f / 315.f);
+              auto body = [&](bool apply_mask) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                  for (int i = 0; i < 32; i += 2) {
+                    const float r0 = __uint_as_float(sr[c][i]), r1 = __uint_as_float(sr[c][i + 1]);
+                    const float y0 = r0 * r0, y1 = r1 * r1;
+                    const float q0 = fmaf(fmaf(fmaf(y0, b3, b2), y0, b1), y0, 1.f);
+                    const float q1 = fmaf(fmaf(fmaf(y1, b3, b2), y1, b1), y1, 1.f);
+                    finish_pair(fmaf(r0 * ac, q0, neg_m), fmaf(r1 * ac, q1, neg_m), c, i,
+                                apply_mask);
+                  }
+              };
+              if (masked) body(true); else body(false);
+            }
+          } else if constexpr (MODE == kModeSoftcap) {
             auto body = [&](bool apply_mask) {
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
-                  const float r0 = __uint_as_float(sr[c][i]), r1 = __uint_as_float(sr[c][i + 1]);
-                  const float q0 = fmaf(r0 * r0, b1, 1.f), q1 = fmaf(r1 * r1, b1, 1.f);
-                  finish_pair(fmaf(r0 * ac, q0, neg_m), fmaf(r1 * ac, q1, neg_m), c, i,
-                              apply_mask);
+                  const float t0 = tanh_approx(__uint_as_float(sr[c][i]) * p.a);
+                  const float t1 = tanh_approx(__uint_as_float(sr[c][i + 1]) * p.a);
+                  finish_pair(fmaf(t0, p.c2, neg_m), fmaf(t1, p.c2, neg_m), c, i, apply_mask);
                 }
             };
             if (masked) body(true); else body(false);
           } else {
-            const float b2 = a2 * a2 * (2.f / 15.f);
-            const float b3 = a2 * a2 * a2 * (-17.f / 315.f);
             auto body = [&](bool apply_mask) {
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                  const float r0 = __uint_as_float(sr[c][i]), r1 = __uint_as_float(sr[c][i + 1]);
-                  const float y0 = r0 * r0, y1 = r1 * r1;
-                  const float q0 = fmaf(fmaf(fmaf(y0, b3, b2), y0, b1), y0, 1.f);
-                  const float q1 = fmaf(fmaf(fmaf(y1, b3, b2), y1, b1), y1, 1.f);
-                  finish_pair(fmaf(r0 * ac, q0, neg_m), fmaf(r1 * ac, q1, neg_m), c, i,
-                              apply_mask);
-                }
+                for (int i = 0; i < 32; i += 2)
+                  finish_pair(fmaf(__uint_as_float(sr[c][i]), p.c2, neg_m),
+                              fmaf(__uint_as_float(sr[c][i + 1]), p.c2, neg_m), c, i, apply_mask);
             };
             if (masked) body(true); else body(false);
           }
-        } else if constexpr (MODE == kModeSoftcap) {
-          auto body = [&](bool apply_mask) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                const float t0 = tanh_approx(__uint_as_float(sr[c][i]) * p.a);
-                const float t1 = tanh_approx(__uint_as_float(sr[c][i + 1]) * p.a);
-                finish_pair(fmaf(t0, p.c2, neg_m), fmaf(t1, p.c2, neg_m), c, i, apply_mask);
-              }
-          };
-          if (masked) body(true); else body(false);
-        } else {
-          auto body = [&](bool apply_mask) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; i += 2)
-                finish_pair(fmaf(__uint_as_float(sr[c][i]), p.c2, neg_m),
-                            fmaf(__uint_as_float(sr[c][i + 1]), p.c2, neg_m), c, i, apply_mask);
-          };
-          if (masked) body(true); else body(false);
+          const float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
+          l_run = l_run * alpha + psum;
+          tmem_st_32x32b_x32(s_addr, pk);
+          publish_p(buf);
         }
-        const float psum = (ps[0] + ps[1]) + (ps[2] + ps[3]);
-        l_run = l_run * alpha + psum;
-        tmem_st_32x32b_x32(s_addr, pk);
-        publish_p(buf);
       }
 
       // Epilogue: O_t / l -> bf16 -> global (one row per thread).
