@@ -934,78 +934,83 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           }
         }
 
-        // Plain and biased scores. P is taken against the reference that the row has, without looking for
-        // the block's maximum first: P may then exceed 1, which bf16 and fp32 hold as exactly as any other
-        // magnitude. Only when a row has no reference yet, or a row sum passes kFastRowSum, the block's own
-        // maximum is found and the reference moves. Looking for the maximum was a sixth of the pass's
-        // instructions, and the vote on the rescale stood in front of the exp2 (causal B=1 Hq=32 Hkv=8
-        // S=8192 D=128 559 -> 528 us, B=2 Hq=32 S=4096 D=64 294 -> 267 us). The row sum is taken over the
-        // bf16-rounded values that the PV product sees, so that numerator and denominator carry the same
-        // rounding; against fp64 that is no worse than fp32 P: 1.98e-3 against 2.02e-3 (causal 2 x 4 x 512).
-        // One copy of each part, and masks in a pass of their own: what the warps of an SM run over and
+        // Plain and biased scores, fast pass: where every row of the warp has a reference and sees the whole
+        // block, P is taken against that reference without looking for the block's maximum first. P may then
+        // exceed 1, which bf16 and fp32 hold as exactly as any other magnitude. The row sum of such a block
+        // is taken over the bf16-rounded values that the PV product sees, so that numerator and denominator
+        // carry the same rounding; against fp64 that is no worse than fp32 P.
+        // Own-maximum pass, for the other blocks (a row's first, masked ones, and those whose fast row sum
+        // passed kFastRowSum): masks set scores to -inf, the reference moves if the block's maximum asks for
+        // it, and the row sum is taken over P in fp32.
+        // Each pass exists once, and masks are a pass over the scores: what the warps of an SM run over and
         // over has to fit its instruction caches.
         if constexpr (MODE == kModeNone || MODE == kModeBias) {
-          if (__any_sync(0xffffffffu, masked)) {
+          uint32_t pk[32];
+          bool own_max = __any_sync(0xffffffffu, masked || m_used == -INFINITY);
+          if (!own_max) {
+            float fs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (c * 32 + i < rel_lo || c * 32 + i > rel_hi) sr[c][i] = 0xff800000u;  // -inf
+              for (int i = 0; i < 32; i += 2) {
+                const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c][i]), p.c2, -m_used));
+                const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c][i + 1]), p.c2, -m_used));
+                const uint32_t pkv = pack_bf16x2(p0, p1);
+                pk[c * 16 + (i >> 1)] = pkv;
+                if ((i >> 1) & 1) add_bf16x2_to_f32(fs[2], fs[3], pkv);
+                else add_bf16x2_to_f32(fs[0], fs[1], pkv);
+              }
+            const float sum = (fs[0] + fs[1]) + (fs[2] + fs[3]);
+            own_max = __any_sync(0xffffffffu, !(sum <= kFastRowSum));
+            if (!own_max) l_run += sum;
           }
-          uint32_t pk[32];
-          float sum;
-          bool move = __any_sync(0xffffffffu, m_used == -INFINITY), moved = false;
-#pragma unroll 1
-          for (;;) {
-            if (move) {
-              float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          if (own_max) {
+            if (__any_sync(0xffffffffu, masked)) {
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                  mx[2 * c] = max3(mx[2 * c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
-                  mx[2 * c + 1] = max3(mx[2 * c + 1], __uint_as_float(sr[c][i + 2]),
-                                       __uint_as_float(sr[c][i + 3]));
-                }
-              const float m_new =
-                  fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.c2);
-              // Lazy rescale: move the reference only when it grew by more than 2^8.
-              float alpha = 1.f;
-              if (m_new > -INFINITY && (m_used == -INFINITY || m_new - m_used > kRescaleThreshold)) {
-                alpha = ex2_approx(m_used - m_new);  // 0 when m_used is -inf
-                m_used = m_new;
+                for (int i = 0; i < 32; ++i)
+                  if (c * 32 + i < rel_lo || c * 32 + i > rel_hi) sr[c][i] = 0xff800000u;  // -inf
+            }
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                mx[2 * c] = max3(mx[2 * c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
+                mx[2 * c + 1] = max3(mx[2 * c + 1], __uint_as_float(sr[c][i + 2]),
+                                     __uint_as_float(sr[c][i + 3]));
               }
-              if (k > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                if (!pvs_before_complete(k)) {
-                  ok = false;
-                  break;
-                }
+            const float m_new =
+                fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.c2);
+            // Lazy rescale: move the reference only when it grew by more than 2^8.
+            float alpha = 1.f;
+            if (m_new > -INFINITY && (m_used == -INFINITY || m_new - m_used > kRescaleThreshold)) {
+              alpha = ex2_approx(m_used - m_new);  // 0 when m_used is -inf
+              m_used = m_new;
+            }
+            if (k > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+              if (!pvs_before_complete(k)) {
+                ok = false;
+                break;
+              }
 #pragma unroll 1
-                for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
-              }
-              l_run *= alpha;
-              moved = true;
+              for (int c = 0; c < D / 32; ++c) rescale_o(c, alpha);
             }
             const float neg_m = m_used == -INFINITY ? 0.f : -m_used;
-            float fs[4] = {0.f, 0.f, 0.f, 0.f};
+            float ps[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
                 const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c][i]), p.c2, neg_m));
                 const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c][i + 1]), p.c2, neg_m));
-                const uint32_t pkv = pack_bf16x2(p0, p1);
-                pk[c * 16 + (i >> 1)] = pkv;
-                if ((i >> 1) & 1) add_bf16x2_to_f32(fs[2], fs[3], pkv);
-                else add_bf16x2_to_f32(fs[0], fs[1], pkv);
+                ps[(c * 2 + (i >> 1)) & 3] += p0;
+                ps[(c * 2 + (i >> 1) + 2) & 3] += p1;
+                pk[c * 16 + (i >> 1)] = pack_bf16x2(p0, p1);
               }
-            sum = (fs[0] + fs[1]) + (fs[2] + fs[3]);
-            if (moved) break;
-            move = __any_sync(0xffffffffu, !(sum <= kFastRowSum));
-            if (!move) break;
+            l_run = fmaf(l_run, alpha, (ps[0] + ps[1]) + (ps[2] + ps[3]));
           }
-          if (!ok) break;
-          l_run += sum;
           if constexpr (MODE == kModeBias) request_bias(k + 1);
           tmem_st_32x32b_x32(s_addr, pk);
           publish_p(buf);

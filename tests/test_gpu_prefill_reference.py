@@ -121,3 +121,28 @@ def test_large_values_behind_a_low_reference_do_not_overflow(B, H, Sq, D, biased
     out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), score_bias=bias)
     want = v[:, :, Skv // 2:].double().mean(2, keepdim=True).expand(B, H, Sq, D)
     assert (out.double().cpu() - want).abs().max().item() <= 2.0 ** -8 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("biased", [False, True])
+def test_row_sums_of_masked_and_first_blocks_hold_fp32_probabilities(biased):
+    """All keys but the first score x1 < 0, so every P but one is exp(x1), which bf16 rounds by nearly half
+    a step, and with the identity as V column 0 of a row is the reciprocal of its row sum. In 192 rows of
+    one head every block is a row's first one or a masked one; their sums are taken over P in fp32 (error
+    below 1e-6), so the reciprocal rounds to the bf16 nearest to the exact value. Rows where that value
+    lies within 2e-5 of a rounding boundary are left out."""
+    n, D = 192, 64
+    x1 = -torch.arange(1, 200, dtype=torch.float64) / 128          # exact in bf16
+    P = torch.exp(x1)
+    off = ((P.bfloat16().double() - P) / P).abs()
+    x1 = x1[off.argmax()].item()
+    q, k, v = torch.zeros(1, 1, n, D), torch.zeros(1, 1, n, D), torch.zeros(1, 1, n, D)
+    q[..., 0] = 1.0
+    k[..., 1:, 0] = x1
+    v[0, 0, 0, 0] = 1.0
+    q, k, v = (t.bfloat16().cuda() for t in (q, k, v))
+    bias = torch.zeros(1, 1, n, n, dtype=torch.bfloat16, device="cuda") if biased else None
+    got = F.prefill_attention(q, k, v, mask_kind=S.MASK_CAUSAL, score_bias=bias)[0, 0, :, 0].cpu()
+    want = 1 / (1 + torch.arange(n, dtype=torch.float64) * torch.exp(torch.tensor(x1).double()))
+    clear = (want * (1 - 2e-5)).bfloat16() == (want * (1 + 2e-5)).bfloat16()
+    assert clear.sum() > n - 8
+    assert torch.equal(got[clear], want.bfloat16()[clear])
