@@ -37,6 +37,7 @@
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <float.h>
 #include <math.h>
 
 #include <atomic>
@@ -1761,7 +1762,9 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
       if (pre > 0.f) {
         mode = kModeNone;
         p.a = 1.f;
-        p.c2 = pre * kLog2eF;
+        // (Subnormal factors are flushed on the device, and a masked score of -inf times 0 is NaN. The
+        // smallest normal number is as near to such a factor as 0 is.)
+        p.c2 = fmaxf(pre * kLog2eF, FLT_MIN);
       }
     } else if (a->mod_op[i] == LF_MOD_TANH) {
       int j = i + 1;

@@ -146,3 +146,18 @@ def test_row_sums_of_masked_and_first_blocks_hold_fp32_probabilities(biased):
     clear = (want * (1 - 2e-5)).bfloat16() == (want * (1 + 2e-5)).bfloat16()
     assert clear.sum() > n - 8
     assert torch.equal(got[clear], want.bfloat16()[clear])
+
+
+@pytest.mark.parametrize("D,D_pe", [(64, 0), (128, 0), (64, 8)])
+@pytest.mark.parametrize("scale", [1e-38, 1e-40, 1e-45])
+def test_masked_scores_with_a_scale_below_the_normal_numbers(scale, D, D_pe):
+    """Scores that vanish next to 1: each row is the mean of the values that it sees. The P are 1 and
+    sums of 200 values err by less than 1e-5, so half a bf16 step of the result remains."""
+    g = torch.Generator().manual_seed(6)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    n = 200
+    q, k, v = mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D)
+    pe = dict(q_pe=mk(1, 2, n, D_pe).cuda(), k_pe=mk(1, 2, n, D_pe).cuda()) if D_pe else {}
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=scale, mask_kind=S.MASK_CAUSAL, **pe)
+    want = v.double().cumsum(2) / torch.arange(1, n + 1, dtype=torch.float64).view(1, 1, n, 1)
+    assert ((out.double().cpu() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
