@@ -795,21 +795,23 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // device instead of 28.9, and two more launches and allocations on the host.)
         if (p.q_bias) {
           constexpr int kPieces = D / 8;
+          // (Rows past Sq keep their zeros: they vote on the warp's passes too.)
+          const bool real = grow < p.Sq;
           const __nv_bfloat16* qb = p.q_bias + b * p.qb_stride[0] + h * p.qb_stride[1] +
-                                    static_cast<int64_t>(min(grow, p.Sq - 1)) * p.qb_stride[2];
+                                    static_cast<int64_t>(grow) * p.qb_stride[2];
           const int first_piece = split ? t * (kPieces / 2) : 0;
           const int n_pieces = split ? kPieces / 2 : kPieces;
           uint4 add[kPieces];
 #pragma unroll
           for (int i = 0; i < kPieces; ++i)
-            if (i < n_pieces) add[i] = ldg_stream_16(qb + (first_piece + i) * 8);
+            if (real && i < n_pieces) add[i] = ldg_stream_16(qb + (first_piece + i) * 8);
           if (!mbar_wait(&bars->q_full[tq], 0)) {
             report_timeout(p.status, 16 + t);
             ok = false;
           }
 #pragma unroll
           for (int i = 0; i < kPieces; ++i)
-            if (i < n_pieces) {
+            if (real && i < n_pieces) {
               const int c = first_piece + i;
               uint4* piece = reinterpret_cast<uint4*>(sQ + tq * kQTileBytes + (c >> 3) * kQBlockBytes +
                                                       row * 128 + (((c & 7) ^ (row & 7)) << 4));

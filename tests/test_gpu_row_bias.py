@@ -39,3 +39,25 @@ def test_same_bits_as_separate_adds(B, H, n, D):
     odd = mk(B, H, n, D + 4)[..., :D]                                 # rows that are not 16-byte aligned
     with pytest.raises(Exception):
         fn(q, k, v, odd, args[4], one_row)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_rows_past_the_last_one_get_no_query_bias(D):
+    """Rows past Sq share a warp with the last ones, and a warp repeats a block with its own maximum when any
+    row's sum leaves its range. Here only those rows could ask for it, by the query bias of the last row
+    (which that row's Q cancels), in a block where valid rows score 2^10 above their reference."""
+    n = 200
+    g = torch.Generator(device="cuda").manual_seed(D)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16() * 0.2
+    q, k, v, q_bias, score_bias, out_bias = mk(1, 1, n, D), mk(1, 1, n, D), mk(1, 1, n, D), \
+        mk(1, 1, n, D), mk(1, 1, n, n), mk(1, 1, n, D)
+    up = D ** 0.5 / 3.5 / 1.4427       # q . k that moves a score by 1 in the log2 domain
+    for t in (q, k, q_bias):
+        t[..., :2] = 0
+    q_bias[..., n - 1, 0], q[..., n - 1, 0] = 16.0, -16.0
+    k[..., 128:192, 0] = 24 * up / 16
+    q[..., 192:n - 1, 1] = 8.0
+    k[..., 150, 1] = 11 * up / 8
+    args = (q, k, v, q_bias, score_bias, out_bias)
+    fn = torch.compile(_biased, backend=loopfuse_backend, dynamic=True)
+    assert torch.equal(fn(*args), _separate(*args))
