@@ -670,37 +670,41 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       };
 
       // Prologue: scores of the first two KV tiles (one stage).
-      if (ok) {
-        const int stage = wait_stage(3);
+      {
+        const int stage = ok ? wait_stage(3) : -1;
         if (stage >= 0) {
           tc_fence_after();
           if (active(lo)) issue_qk(stage, 0, lo);
           if (lo + 1 < hi && active(lo + 1)) issue_qk(stage, 1, lo + 1);
-          tc_commit_if(elected, &bars->kv_empty[stage]);
         }
+        __syncwarp();  // (as below)
+        tc_commit_if(elected && ok, &bars->kv_empty[0]);
       }
       const int nblk_t = split ? (hi - lo + 1 - t) >> 1 : has_work(t) ? hi_t(t) - lo_t(t) : 0;
-      for (int j = lo; j < hi && ok; ++j) {
+      for (int j = lo; j < hi; ++j) {
         const int st = wait_stage(4);  // {V(j), K(j+2)}
-        if (st < 0) break;
         tc_fence_after();
         // (Split: K(j+2) is this slot's next block, not the one after it; its scores are made
         // while the softmax of block j runs. Its buffer was read by the slot's last PV.)
-        if (split && j + 2 < hi && active(j)) issue_qk(st, 1, j + 2);
-        if (active(j)) {
+        if (split && st >= 0 && j + 2 < hi && active(j)) issue_qk(st, 1, j + 2);
+        if (st >= 0 && active(j)) {
           const int kt = block_of(j);
-          if (!mbar_wait(&bars->p_full[t][kt & 1], (kt >> 1) & 1)) {
+          if (mbar_wait(&bars->p_full[t][kt & 1], (kt >> 1) & 1)) {
+            tc_fence_after();
+            issue_pv(st, kt);
+            // Completion points the softmax warps may wait on: the second-to-last PV (for a
+            // rescale in the last block) and the last PV (for the epilogue).
+            tc_commit_if(elected && kt == nblk_t - 2, &bars->pv_done[t]);
+            tc_commit_if(elected && kt == nblk_t - 1, &bars->o_final[t]);
+          } else {
             report_timeout(p.status, 6 + t);
             ok = false;
-            break;
           }
-          tc_fence_after();
-          issue_pv(st, kt);
-          // Completion points the softmax warps may wait on: the second-to-last PV (for a
-          // rescale in the last block) and the last PV (for the epilogue).
-          tc_commit_if(elected && kt == nblk_t - 2, &bars->pv_done[t]);
-          tc_commit_if(elected && kt == nblk_t - 1, &bars->o_final[t]);
         }
+        // The lanes meet once per step, before anything is issued that lets a barrier that they wait on in
+        // this step complete its next phase (a lane left behind would then wait on a parity that has
+        // flipped), and they leave together when a wait ran out.
+        if (!__all_sync(0xffffffffu, ok)) break;
         if (!split && j + 2 < hi && active(j + 2)) issue_qk(st, 1, j + 2);
         tc_commit_if(elected, &bars->kv_empty[st]);
       }
