@@ -234,40 +234,20 @@ class CompiledAttention:
             self._check(status, plan)
             return (out,)
         # Prefill. K and V may be paged independently, as in the reference's own paged-attention
-        # tests (tests/test_accuracy.py:253-311: K through paged_load, V dense); the gather of a
-        # paged operand is fused into the kernel's tile loads.
-        if spec.k.paged or spec.v.paged:
-            out = F.prefill_attention(
-                q, args[spec.k.placeholder], args[spec.v.placeholder], scale=plan.scale,
-                mods=plan.mods, mask_kind=spec.mask_kind, window=plan.window, status=status,
-                k_block_table=args[spec.k.block_table] if spec.k.paged else None,
-                v_block_table=args[spec.v.block_table] if spec.v.paged else None)
-        elif spec.q_pe is not None:
-            # Two-matmul (MLA-style) scores, tests/test_attention.py:126-151 of the reference.
-            out = F.prefill_attention(
-                q, args[spec.k.placeholder], args[spec.v.placeholder], scale=plan.scale,
-                mods=plan.mods, mask_kind=spec.mask_kind, window=plan.window, status=status,
-                q_pe=args[spec.q_pe], k_pe=args[spec.k_pe])
-            if spec.out_bias is not None:
-                F.add_bf16(out, args[spec.out_bias], out=out)
-        elif spec.q_bias is not None or spec.out_bias is not None or spec.score_bias is not None:
-            # Modified attention of the reference's tests (tests/test_accuracy.py:176-194): the
-            # query bias is added first (one bf16 rounding, as in the eager graph), the score
-            # bias is read inside the attention kernel, the output bias is added in place.
-            k, v = args[spec.k.placeholder], args[spec.v.placeholder]
-            if spec.q_bias is not None:
-                q = F.add_bf16(q, args[spec.q_bias])
-            out = F.prefill_attention(
-                q, k, v, scale=plan.scale, mods=plan.mods, mask_kind=spec.mask_kind,
-                window=plan.window, status=status,
-                score_bias=args[spec.score_bias] if spec.score_bias is not None else None,
-                bias_pos=self._bias_pos(plan))
-            if spec.out_bias is not None:
-                F.add_bf16(out, args[spec.out_bias], out=out)
-        else:
-            out = F.prefill_attention(
-                q, args[spec.k.placeholder], args[spec.v.placeholder], scale=plan.scale,
-                mods=plan.mods, mask_kind=plan.mask_kind, window=plan.window, status=status)
+        # tests (tests/test_accuracy.py:253-311: K through paged_load, V dense); a second score
+        # product is the MLA form of tests/test_attention.py:126-151, the biases are those of
+        # tests/test_accuracy.py:176-194.
+        def at(i: Optional[int]) -> Optional[torch.Tensor]:
+            return None if i is None else args[i]
+
+        out = F.prefill_attention(
+            q, args[spec.k.placeholder], args[spec.v.placeholder], scale=plan.scale,
+            mods=plan.mods, mask_kind=plan.mask_kind, window=plan.window, status=status,
+            k_block_table=at(spec.k.block_table), v_block_table=at(spec.v.block_table),
+            score_bias=at(spec.score_bias),
+            bias_pos=self._bias_pos(plan) if spec.score_bias is not None else None,
+            q_pe=at(spec.q_pe), k_pe=at(spec.k_pe), q_bias=at(spec.q_bias),
+            out_bias=at(spec.out_bias))
         self._check(status, plan)
         return (out,)
 

@@ -423,6 +423,37 @@ Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
   return out;
 }
 
+// A prefill with a query and / or output bias. In one launch where the library can (a score bias in front
+// of the mask); otherwise the query bias is added first and the output bias in place, by kernels of their
+// own. The same bits: each is one bf16 rounding, as in the eager graph.
+// (Out of line: its argument records would be part of every call's frame.)
+[[gnu::noinline]] Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o,
+                                        const Tensor* q_bias, const Tensor* out_bias, Tensor out) {
+  if (q_bias) check_add(*p.q, p.q->sizes(), *q_bias);
+  if (out_bias) check_add(*p.q, p.q->sizes(), *out_bias);
+  if (p.score_bias) {
+    LfPrefillArgs a;
+    LfRowBias rows;
+    Tensor result = out;
+    std::vector<Tensor> keep;
+    fill_prefill(a, p, o, result, keep);
+    std::memset(&rows, 0, sizeof(rows));
+    if (q_bias) rows.q_bias = q_bias->data_ptr(), strides3(rows.q_bias_stride, *q_bias);
+    if (out_bias) rows.out_bias = out_bias->data_ptr(), strides3(rows.out_bias_stride, *out_bias);
+    const int rc =
+        launch(p.q->device(), [&](void* st) { return lib.prefill_row_bias(&a, &rows, st); });
+    if (rc != LF_ERR_UNSUPPORTED && rc != LF_ERR_ALIGNMENT) {
+      check_rc(rc, "lf_prefill_row_bias_bf16");
+      return result;
+    }
+  }
+  const Tensor biased = q_bias ? run_add(*p.q, *q_bias, Tensor()) : Tensor();
+  if (q_bias) p.q = &biased;
+  out = run_prefill(p, o, std::move(out));
+  if (out_bias) run_add(out, *out_bias, out);
+  return out;
+}
+
 void run_kv_append(const Tensor& kn, const Tensor& vn, const Tensor& k_pool, const Tensor& v_pool,
                    const Tensor& table, const Tensor* table_v, const Tensor* seq_pos,
                    int64_t start_pos, const Tensor* status) {
@@ -652,11 +683,15 @@ void parse_prefill(PyObject* const* a, PrefillTensors& t, PrefillOptions& o, Ten
 
 PyObject* py_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&] {
-    want_args(n, kPrefillArgCount);
+    want_args(n, kPrefillArgCount + 2);
     PrefillTensors t;
     PrefillOptions o;
     Tensor out;
     parse_prefill(a, t, o, out);
+    const Tensor* q_bias = optional_tensor(a[kPrefillArgCount], "q_bias");
+    const Tensor* out_bias = optional_tensor(a[kPrefillArgCount + 1], "out_bias");
+    if (q_bias || out_bias)
+      return THPVariable_Wrap(run_row_biased(t, o, q_bias, out_bias, std::move(out)));
     return THPVariable_Wrap(run_prefill(t, o, std::move(out)));
   });
 }
@@ -812,37 +847,6 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
   });
 }
 
-// A prefill with a query and / or output bias. In one launch where the library can (a score bias in front
-// of the mask); otherwise the query bias is added first and the output bias in place, by kernels of their
-// own. The same bits: each is one bf16 rounding, as in the eager graph.
-// (Out of line: its argument records would be part of every call's frame.)
-[[gnu::noinline]] Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o,
-                                        const Tensor* q_bias, const Tensor* out_bias) {
-  if (q_bias) check_add(*p.q, p.q->sizes(), *q_bias);
-  if (out_bias) check_add(*p.q, p.q->sizes(), *out_bias);
-  if (p.score_bias) {
-    LfPrefillArgs a;
-    LfRowBias rows;
-    Tensor out;
-    std::vector<Tensor> keep;
-    fill_prefill(a, p, o, out, keep);
-    std::memset(&rows, 0, sizeof(rows));
-    if (q_bias) rows.q_bias = q_bias->data_ptr(), strides3(rows.q_bias_stride, *q_bias);
-    if (out_bias) rows.out_bias = out_bias->data_ptr(), strides3(rows.out_bias_stride, *out_bias);
-    const int rc =
-        launch(p.q->device(), [&](void* st) { return lib.prefill_row_bias(&a, &rows, st); });
-    if (rc != LF_ERR_UNSUPPORTED && rc != LF_ERR_ALIGNMENT) {
-      check_rc(rc, "lf_prefill_row_bias_bf16");
-      return out;
-    }
-  }
-  const Tensor biased = q_bias ? run_add(*p.q, *q_bias, Tensor()) : Tensor();
-  if (q_bias) p.q = &biased;
-  Tensor out = run_prefill(p, o, Tensor());
-  if (out_bias) run_add(out, *out_bias, out);
-  return out;
-}
-
 // One pass of the graph on its arguments; returns the output tensor.
 Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
   const Tensor* t[kOperands];
@@ -861,7 +865,7 @@ Tensor run_call(const Call& c, PyObject* const* args, Py_ssize_t n) {
     p.q_pe = t[kQPe];
     p.k_pe = t[kKPe];
     if (t[kQBias] || t[kOutBias])
-      return run_row_biased(p, c.prefill, t[kQBias], t[kOutBias]);
+      return run_row_biased(p, c.prefill, t[kQBias], t[kOutBias], Tensor());
     return run_prefill(p, c.prefill, Tensor());
   }
   const Tensor &q = *t[kQ], &k = *t[kK], &v = *t[kV];

@@ -72,7 +72,9 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scal
                       score_bias: Optional[torch.Tensor] = None,
                       bias_pos: Optional[int] = None,
                       q_pe: Optional[torch.Tensor] = None,
-                      k_pe: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      k_pe: Optional[torch.Tensor] = None,
+                      q_bias: Optional[torch.Tensor] = None,
+                      out_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """softmax(mask(mods(scale * q k^T))) v for q [B,Hq,Sq,D], k/v [B,Hkv,Skv,D] (bf16).
 
     ``score_bias`` (bf16 ``[B, Hq, Sq, Skv]``) is added to the scores after the first
@@ -82,6 +84,10 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scal
     ``q_pe`` ``[B, Hq, Sq, D_pe]`` and ``k_pe`` ``[B, Hkv, Skv, D_pe]`` (bf16, D_pe a multiple of
     8 up to 64) add a second product to the scores: ``scale * (q k^T + q_pe k_pe^T)``, the
     two-matmul (MLA-style) form; ``mods`` may then hold constant multipliers only.
+
+    ``q_bias`` and ``out_bias`` (bf16, the shape of ``q``) are added to ``q`` before the scores and to
+    the output, each with one rounding to bf16: in the same launch where a ``score_bias`` with only
+    multipliers in front of it is given, else by ``add_bf16`` (the same bits).
 
     With ``k_block_table`` (``v_block_table``), ``k`` (``v``) is a paged pool
     ``[pages, page_size, Hkv, D]`` (or ``[pages, Hkv, D]``, one token per page) read through that
@@ -93,7 +99,8 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scal
     that runs at the same time on another stream)."""
     return _native.host().prefill(q, k, v, out, status, dbg_ranges, k_block_table, v_block_table,
                                   score_bias, q_pe, k_pe, scale, mods, mask_kind, window,
-                                  causal_offset, kv_tile, sm_margin, seq_len, bias_pos)
+                                  causal_offset, kv_tile, sm_margin, seq_len, bias_pos, q_bias,
+                                  out_bias)
 
 
 def add_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

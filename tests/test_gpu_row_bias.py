@@ -61,3 +61,33 @@ def test_rows_past_the_last_one_get_no_query_bias(D):
     args = (q, k, v, q_bias, score_bias, out_bias)
     fn = torch.compile(_biased, backend=loopfuse_backend, dynamic=True)
     assert torch.equal(fn(*args), _separate(*args))
+
+
+def _allocations(call):
+    """Device allocations of one call (its inputs' and the compiler's are behind it)."""
+    call()
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    call()
+    return torch.cuda.memory_stats()["allocation.all.allocated"] - before
+
+
+def test_status_checking_calls_run_the_fused_kernel(monkeypatch):
+    """A call with a status word takes the same single launch: the output is all it allocates (adds of
+    their own would also allocate a Q), and the word stays clean."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    n, D = 136, 64
+    args = (mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, n),
+            mk(1, 2, n, D))
+    want = _separate(*args)
+    monkeypatch.setenv("LF_CHECK_STATUS", "1")
+    fn = torch.compile(_biased, backend=loopfuse_backend, dynamic=True)
+    assert torch.equal(fn(*args), want)
+    assert _allocations(lambda: fn(*args)) == 1
+    q, k, v, q_bias, score_bias, out_bias = args
+    st = F.new_status("cuda")
+    out = F.prefill_attention(q, k, v, scale=D ** -0.5, mods=[S.ScoreMod(S.MOD_MUL, 3.5)],
+                              mask_kind=S.MASK_CAUSAL, score_bias=score_bias, q_bias=q_bias,
+                              out_bias=out_bias, status=st)
+    F.check_status(st)
+    assert torch.equal(out, want)
