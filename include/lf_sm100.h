@@ -238,8 +238,9 @@ const char* lf_last_cuda_error(void);
 int lf_prefill_bf16(const LfPrefillArgs* args, void* stream);
 /* lf_prefill_bf16 with row biases, in the same launch. Only where a score bias with nothing but
  * multipliers in front of it goes through the biased kernel; LF_ERR_UNSUPPORTED otherwise, and
- * LF_ERR_ALIGNMENT where a row bias is not 16-byte aligned (nothing is launched: add them with
- * lf_add_bf16). */
+ * LF_ERR_ALIGNMENT where q (an expanded one, say) or a row bias is not laid out for it. Nothing is
+ * launched then, and the biases can be added with lf_add_bf16, which takes any q whose rows are 16-byte
+ * aligned. Row biases that are not 16-byte aligned are refused by both. */
 int lf_prefill_row_bias_bf16(const LfPrefillArgs* args, const LfRowBias* rows, void* stream);
 
 /* KV tile size (64 or 128 keys) of the kernel lf_prefill_bf16 would run for these arguments, or

@@ -429,8 +429,14 @@ Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
 // (Out of line: its argument records would be part of every call's frame.)
 [[gnu::noinline]] Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o,
                                         const Tensor* q_bias, const Tensor* out_bias, Tensor out) {
-  if (q_bias) check_add(*p.q, p.q->sizes(), *q_bias);
-  if (out_bias) check_add(*p.q, p.q->sizes(), *out_bias);
+  // (What neither way takes is refused before anything is launched.)
+  for (const Tensor* bias : {q_bias, out_bias}) {
+    if (!bias) continue;
+    check_add(*p.q, p.q->sizes(), *bias);
+    bool aligned = reinterpret_cast<uintptr_t>(bias->data_ptr()) % 16 == 0;
+    for (int i = 0; i < 3; ++i) aligned = aligned && bias->stride(i) % 8 == 0;
+    if (!aligned) check_rc(LF_ERR_ALIGNMENT, "lf_add_bf16");
+  }
   if (p.score_bias) {
     LfPrefillArgs a;
     LfRowBias rows;

@@ -5,7 +5,7 @@ repeat along a dimension, and operands that the fused form cannot take."""
 import pytest
 import torch
 
-from loopfuse_b200 import functional as F, loopfuse_backend, spec as S
+from loopfuse_b200 import _native, functional as F, loopfuse_backend, spec as S
 import loopfuse_b200.ops  # noqa: F401  (registers loopfuse::causal_mask)
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +91,23 @@ def test_status_checking_calls_run_the_fused_kernel(monkeypatch):
                               out_bias=out_bias, status=st)
     F.check_status(st)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("which", ["q_bias", "out_bias"])
+@pytest.mark.parametrize("fits", [True, False])
+def test_misaligned_row_biases_are_refused_before_any_launch(which, fits):
+    """Whether the graph could take the biases in one launch or not (a tanh in front of the score bias)."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    n, D = 136, 64
+    q, k, v, sb, good = mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, n), mk(1, 2, n, D)
+    odd = mk(1, 2, n, D + 4)[..., :D]
+    mods = [S.ScoreMod(S.MOD_MUL, 3.5)] if fits else [S.ScoreMod(S.MOD_TANH)]
+    rows = dict(q_bias=good, out_bias=good)
+    call = lambda: F.prefill_attention(q, k, v, mods=mods, score_bias=sb, **rows)
+    call()
+    rows[which] = odd
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    with pytest.raises(_native.LfError, match="lf_add_bf16 failed.*align"):
+        call()
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
