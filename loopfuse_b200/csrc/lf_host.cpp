@@ -427,7 +427,7 @@ Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
 // of the mask); otherwise the query bias is added first and the output bias in place, by kernels of their
 // own. The same bits: each is one bf16 rounding, as in the eager graph.
 // (Out of line: its argument records would be part of every call's frame.)
-[[gnu::noinline]] Tensor run_row_biased(PrefillTensors p, const PrefillOptions& o,
+[[gnu::noinline]] Tensor run_row_biased(const PrefillTensors& p, const PrefillOptions& o,
                                         const Tensor* q_bias, const Tensor* out_bias, Tensor out) {
   // (What neither way takes is refused before anything is launched.)
   for (const Tensor* bias : {q_bias, out_bias}) {
@@ -437,25 +437,28 @@ Tensor run_add(const Tensor& x, const Tensor& y, Tensor out) {
     for (int i = 0; i < 3; ++i) aligned = aligned && bias->stride(i) % 8 == 0;
     if (!aligned) check_rc(LF_ERR_ALIGNMENT, "lf_add_bf16");
   }
+  LfPrefillArgs a;
+  std::vector<Tensor> keep;
+  fill_prefill(a, p, o, out, keep);
+  const c10::Device dev = p.q->device();
   if (p.score_bias) {
-    LfPrefillArgs a;
     LfRowBias rows;
-    Tensor result = out;
-    std::vector<Tensor> keep;
-    fill_prefill(a, p, o, result, keep);
     std::memset(&rows, 0, sizeof(rows));
     if (q_bias) rows.q_bias = q_bias->data_ptr(), strides3(rows.q_bias_stride, *q_bias);
     if (out_bias) rows.out_bias = out_bias->data_ptr(), strides3(rows.out_bias_stride, *out_bias);
-    const int rc =
-        launch(p.q->device(), [&](void* st) { return lib.prefill_row_bias(&a, &rows, st); });
+    const int rc = launch(dev, [&](void* st) { return lib.prefill_row_bias(&a, &rows, st); });
     if (rc != LF_ERR_UNSUPPORTED && rc != LF_ERR_ALIGNMENT) {
       check_rc(rc, "lf_prefill_row_bias_bf16");
-      return result;
+      return out;
     }
   }
-  const Tensor biased = q_bias ? run_add(*p.q, *q_bias, Tensor()) : Tensor();
-  if (q_bias) p.q = &biased;
-  out = run_prefill(p, o, std::move(out));
+  Tensor biased;
+  if (q_bias) {
+    biased = run_add(*p.q, *q_bias, Tensor());
+    a.q = biased.data_ptr();
+    strides3(a.q_stride, biased);
+  }
+  check_rc(launch(dev, [&](void* st) { return lib.prefill(&a, st); }), "lf_prefill_bf16");
   if (out_bias) run_add(out, *out_bias, out);
   return out;
 }

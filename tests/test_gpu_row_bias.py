@@ -111,3 +111,18 @@ def test_misaligned_row_biases_are_refused_before_any_launch(which, fits):
     with pytest.raises(_native.LfError, match="lf_add_bf16 failed.*align"):
         call()
     assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+
+
+def test_biases_that_are_added_by_passes_of_their_own_cost_one_buffer():
+    """A tanh in front of the score bias: the biased Q and the output are all that a call allocates."""
+    def attention(q, k, v, q_bias, score_bias, out_bias):
+        s = (q + q_bias) @ k.transpose(-2, -1) * (q.shape[-1] ** -0.5)
+        return torch.softmax(torch.tanh(s) + score_bias, dim=-1) @ v + out_bias
+
+    g = torch.Generator(device="cuda").manual_seed(10)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    n, D = 136, 64
+    args = (mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, n),
+            mk(1, 2, n, D))
+    fn = torch.compile(attention, backend=loopfuse_backend, dynamic=True)
+    assert _allocations(lambda: fn(*args)) == 2
