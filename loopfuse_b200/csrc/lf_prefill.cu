@@ -800,7 +800,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         if (p.q_bias) {
           constexpr int kPieces = D / 8;
           // (Rows past Sq keep their zeros: they vote on the warp's passes too.)
-          const bool real = grow < p.Sq;
+          const bool real = grow < p.Sq &&
+                            LF_BOUNDS(grow >= 0 && b * p.Hq + h < p.n_heads, p.status, 62);
           const __nv_bfloat16* qb = p.q_bias + b * p.qb_stride[0] + h * p.qb_stride[1] +
                                     static_cast<int64_t>(grow) * p.qb_stride[2];
           const int first_piece = split ? t * (kPieces / 2) : 0;
@@ -1225,7 +1226,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           // (The output bias of the four pieces that this thread stores, requested before they are made.)
           [[maybe_unused]] uint4 bias4[4];
           if constexpr (MODE == kModeBias) {
-            if (ob) {
+            if (ob && LF_BOUNDS(row0 >= 0 && b * p.Hq + h < p.n_heads && c * 32 + 32 <= D, p.status, 63)) {
 #pragma unroll
               for (int rr = 0; rr < 4; ++rr)
                 bias4[rr] = ldg_stream_16(

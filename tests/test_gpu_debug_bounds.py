@@ -64,6 +64,17 @@ CHILD = textwrap.dedent("""
         s = O.causal_mask_general(q.float() @ k.float().transpose(-2, -1) * 0.125 + sb.float())
         want = torch.softmax(s, dim=-1) @ v.float()
         assert (out.float().cpu() - want).abs().max().item() <= TOL, S
+        for rows in (("q_bias",), ("out_bias",), ("q_bias", "out_bias")):
+            b = {n: mk(1, 2, S, 64) for n in rows}
+            out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=0.125,
+                                      mask_kind=SP.MASK_CAUSAL, score_bias=sb_full.cuda()[..., :S],
+                                      status=st, **{n: t.cuda() for n, t in b.items()})
+            qq = q + b["q_bias"] if "q_bias" in b else q
+            s = O.causal_mask_general(qq.float() @ k.float().transpose(-2, -1) * 0.125 + sb.float())
+            want = torch.softmax(s, dim=-1) @ v.float()
+            if "out_bias" in b: want = want + b["out_bias"].float()
+            # (the sum with the output bias is rounded once more: half a bf16 step)
+            assert ((out.float().cpu() - want).abs() <= TOL + want.abs() / 256).all(), (S, rows)
     torch.cuda.synchronize()
     assert int(st.item()) == 0, hex(int(st.item()))
     print("debug-bounds cases ok")
