@@ -975,10 +975,18 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
           if (own_max) {
             if (__any_sync(0xffffffffu, masked)) {
 #pragma unroll
-              for (int c = 0; c < 2; ++c)
+              for (int c = 0; c < 2; ++c) {
+                // Bit i: column c * 32 + i is visible (shifts by 32 and more give 0). Comparing each column
+                // with both bounds took three instructions per score: causal 2 x 4 x 512 D=64 7.24 ->
+                // 6.99 us, 8 x 32 x 512 D=128 42.4 -> 40.8, biased 4 x 8 x 1024 29.3 -> 28.9.
+                uint32_t seen, upto;
+                asm("shl.b32 %0, 0xffffffff, %1;" : "=r"(seen) : "r"(max(rel_lo - c * 32, 0)));
+                asm("shl.b32 %0, 0xfffffffe, %1;" : "=r"(upto) : "r"(max(rel_hi - c * 32, 0)));
+                seen = rel_hi < c * 32 ? 0u : seen & ~upto;
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                  if (c * 32 + i < rel_lo || c * 32 + i > rel_hi) sr[c][i] = 0xff800000u;  // -inf
+                  if (!(seen & (1u << i))) sr[c][i] = 0xff800000u;  // -inf
+              }
             }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll

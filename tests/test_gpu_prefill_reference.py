@@ -161,3 +161,21 @@ def test_masked_scores_with_a_scale_below_the_normal_numbers(scale, D, D_pe):
     out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=scale, mask_kind=S.MASK_CAUSAL, **pe)
     want = v.double().cumsum(2) / torch.arange(1, n + 1, dtype=torch.float64).view(1, 1, n, 1)
     assert ((out.double().cpu() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window", [1, 31, 32, 33, 64, 65])
+def test_windows_around_the_words_of_a_block(window, D):
+    """The visible columns of a row in a block are two words of 32 bits; every first and last column of a
+    row occurs. A window of one key returns the values themselves."""
+    g = torch.Generator().manual_seed(window)
+    mk = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    n = 200
+    q, k, v = mk(1, 2, n, D), mk(1, 2, n, D), mk(1, 2, n, D)
+    out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
+                              mask_kind=S.MASK_CAUSAL_WINDOW, window=window).cpu()
+    s = O.sliding_mask_ref(q.double() @ k.double().transpose(-2, -1) * D ** -0.5, window)
+    want = torch.softmax(s, dim=-1) @ v.double()
+    assert (out.double() - want).abs().max().item() <= TOL
+    if window == 1:
+        assert torch.equal(out, v)
