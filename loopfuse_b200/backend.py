@@ -174,8 +174,8 @@ class CompiledAttention:
     # -- launch --------------------------------------------------------------------------
     def dispatcher(self):
         """The native callable of the graph: finds the bound call for the arguments' sizes (the
-        first time through ``bind``) and launches it. ``__call__`` is the same in Python, for the
-        runs that print or check something around the launch."""
+        first time through ``bind``) and launches it. ``__call__`` makes the same launches from
+        Python, for the runs that print or check something around them."""
         return _native.host().Dispatcher(self.bind)
 
     def _status_for(self, device) -> Optional[torch.Tensor]:

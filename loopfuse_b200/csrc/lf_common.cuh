@@ -437,8 +437,8 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       : "memory");
 }
 
-// The same, issued where `issue` holds (the elected lane): predicated instructions in a warp that stays
-// converged. Behind a branch every group of MMAs is a divergent region of its own, and the descriptors
+// The same, issued where `issue` holds (the elected lane): predicated instructions for a warp whose lanes
+// run together (the caller brings them back together once per step). Behind a branch every group of MMAs is a divergent region of its own, and the descriptors
 // have to be moved into uniform registers inside it.
 __device__ __forceinline__ void mma_ss_if(bool issue, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                           uint32_t idesc, uint32_t accumulate) {
