@@ -563,24 +563,33 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
           tmem_wait_ld();
           float psum[4] = {0.f, 0.f, 0.f, 0.f};
           float ymax0 = 0.f, ymax1 = 0.f;
-          // Plain fp32 instructions: this loop is bound by instruction issue (12 per pair), and
-          // the packed f32x2 forms, although fewer, take longer in their pipe (measured 1116
-          // against 763 clocks per 32 x 128 scores of a scheduler).
+          // What limits this loop is the issue slots of the scheduler, which the warps that issue MMAs
+          // share: next to scalar fp32 at one instruction per clock a tcgen05.mma goes out every 122
+          // to 180 clocks instead of every 65 (two to four arithmetic warps per scheduler), next to
+          // the packed forms, which take two clocks of their pipe each, every 65. The short polynomial
+          // is therefore packed (9 instructions per pair instead of 12; the same roundings): causal
+          // 8 x 32 x 2048 D = 128 525 -> 513 thousand clocks, 345 -> 341 us under the power cap; window
+          // 256, four heads per kv head, 205 -> 197 thousand, 124.7 -> 122.4 us.
           auto body = [&](auto path_tag, bool apply_mask) {
             constexpr int kPath = decltype(path_tag)::value;
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
               const float r0 = __uint_as_float(sr[i]), r1 = __uint_as_float(sr[i + 1]);
-              const float y0 = r0 * r0, y1 = r1 * r1;
-              if ((i >> 1) & 1) ymax1 = max3(ymax1, y0, y1); else ymax0 = max3(ymax0, y0, y1);
-              float z0, z1;
+              float y0, y1, z0, z1;
               if constexpr (kPath == 0) {
-                z0 = r0 * fmaf(y0, p.qc[1], p.qc[0]);
-                z1 = r1 * fmaf(y1, p.qc[1], p.qc[0]);
-              } else if constexpr (kPath == 1) {
+                const uint64_t rr = pack2(r0, r1), yy = mul2(rr, rr);
+                const uint64_t q = fma2(yy, pack2(p.qc[1], p.qc[1]), pack2(p.qc[0], p.qc[0]));
+                unpack2(yy, y0, y1);
+                unpack2(mul2(rr, q), z0, z1);
+              } else {
+                y0 = r0 * r0;
+                y1 = r1 * r1;
+              }
+              if ((i >> 1) & 1) ymax1 = max3(ymax1, y0, y1); else ymax0 = max3(ymax0, y0, y1);
+              if constexpr (kPath == 1) {
                 z0 = r0 * fmaf(fmaf(fmaf(y0, p.qc[3], p.qc[2]), y0, p.qc[1]), y0, p.qc[0]);
                 z1 = r1 * fmaf(fmaf(fmaf(y1, p.qc[3], p.qc[2]), y1, p.qc[1]), y1, p.qc[0]);
-              } else {
+              } else if constexpr (kPath == 2) {
                 z0 = tanh_approx(r0 * p.a) * p.c2;
                 z1 = tanh_approx(r1 * p.a) * p.c2;
               }
