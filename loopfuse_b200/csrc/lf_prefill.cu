@@ -184,14 +184,30 @@ struct PrefillStages {
   static constexpr int value = PE ? (D == 64 ? 4 : 2) : StagesFor<D>::value;
 };
 
-template <int D, int MODE, bool PE>
-__global__ void __launch_bounds__(kPrefillThreads, 1)
+// `NARROW`: one query tile per CTA and one slot, with half of an SM's registers, shared and tensor
+// memory, so that two CTAs share an SM and the start and end of one lie under the blocks of the other.
+template <int D, bool PE, bool NARROW>
+struct PrefillShape {
+  static constexpr int kSlots = NARROW ? 1 : 2;
+  static constexpr int kThreads = NARROW ? 8 * 32 : kPrefillThreads;
+  static constexpr int kStages = NARROW ? (D == 64 ? 4 : 2) : PrefillStages<D, PE>::value;
+  // Output staging of the softmax warps (2 KB each), and row numbers of the gather warps behind it.
+  static constexpr uint32_t kStaging = NARROW ? 4 * 2048 + 4096 : kStageBytesTotal;
+  static constexpr uint32_t kTmemColumns = NARROW ? 256 : 512;
+  static constexpr size_t kSmem = 1024 /*align slack*/ + 1024 /*barriers*/ + kStaging +
+                                  static_cast<size_t>(kSlots) * kTileQ * (D + (PE ? 64 : 0)) * 2 +
+                                  static_cast<size_t>(kStages) * 2 * kTileK * (D + (PE ? 64 : 0)) * 2;
+};
+
+template <int D, int MODE, bool PE, bool NARROW>
+__global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW ? 2 : 1)
     prefill_kernel(const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v,
                    const __grid_constant__ CUtensorMap tmap_qpe,
                    const __grid_constant__ CUtensorMap tmap_kpe, const PrefillParams p) {
-  constexpr int kStages = PrefillStages<D, PE>::value;
+  using Shape = PrefillShape<D, PE, NARROW>;
+  constexpr int kStages = Shape::kStages;
   constexpr int kBlocksD = D / 64;                    // 64-column swizzle blocks per tile row
   constexpr int kBlocksQK = kBlocksD + (PE ? 1 : 0);  // ... of a Q or K tile
   constexpr uint32_t kQBlockBytes = kTileQ * 128;     // one [128][64] bf16 block of Q
@@ -202,8 +218,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   constexpr uint32_t kKVTileBytes = kKTileBytes;      // size of a ring slot (two per stage)
   constexpr uint32_t kIdescQK = make_idesc_bf16(128, kTileK, 0);
   constexpr uint32_t kIdescPV = make_idesc_bf16(128, D, 1);
-  constexpr uint32_t kColO = 256;
-  constexpr int kSoftmaxWarps = 8;
+  constexpr uint32_t kColO = Shape::kSlots * 128;
+  constexpr int kSoftmaxWarps = Shape::kSlots * 4;
   constexpr int kProducerWarp = kSoftmaxWarps;
   constexpr int kMmaWarp0 = kSoftmaxWarps + 1;
   constexpr int kGatherWarp = kSoftmaxWarps + 3;
@@ -213,9 +229,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
   PrefillBarriers* bars = reinterpret_cast<PrefillBarriers*>(smem);
-  unsigned char* sStage = smem + 1024;  // 8 x 2 KB: output staging of the softmax warps
-  unsigned char* sQ = sStage + kStageBytesTotal;
-  unsigned char* sKV = sQ + 2 * kQTileBytes;
+  unsigned char* sStage = smem + 1024;  // 2 KB per softmax warp: output staging
+  unsigned char* sQ = sStage + Shape::kStaging;
+  unsigned char* sKV = sQ + Shape::kSlots * kQTileBytes;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -236,8 +252,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   const int hkv = static_cast<int>(p.div_group.div(h));
   // (`single`: one query tile per CTA. Its key blocks alternate between the two slots, which have a
   // softmax warp group, S buffers and an O each and are merged at the end; chosen by the host.)
-  const bool split = p.single;
-  const int iq0 = split ? pair : pair * 2;
+  const bool split = !NARROW && p.single;
+  const int iq0 = NARROW || split ? pair : pair * 2;
 
   // (Scalars and selects: an array indexed with the warp's slot lies in local memory, and with nearly all of
   // the SM's memory taken as shared memory such a read goes to L2.)
@@ -245,7 +261,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0, &lo0, &hi0);
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq0 + 1, &lo1,
              &hi1);
-  const bool valid0 = iq0 * kTileQ < p.Sq, valid1 = !split && (iq0 + 1) * kTileQ < p.Sq;
+  const bool valid0 = iq0 * kTileQ < p.Sq, valid1 = !NARROW && !split && (iq0 + 1) * kTileQ < p.Sq;
   const bool work0 = valid0 && hi0 > lo0, work1 = valid1 && hi1 > lo1;
   auto lo_t = [&](int t) { return t ? lo1 : lo0; };
   auto hi_t = [&](int t) { return t ? hi1 : hi0; };
@@ -280,7 +296,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
         // (paged operands: one arrival of either gather warp, or one for the TMA part and one for the
         // warp's own copies)
         mbar_init(&bars->kv_full[s], p.paged ? 2 : 1);
-        mbar_init(&bars->kv_empty[s], 2);
+        mbar_init(&bars->kv_empty[s], Shape::kSlots);
       }
       for (int t = 0; t < 2; ++t) {
         for (int bf = 0; bf < 2; ++bf) {
@@ -325,7 +341,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     __syncwarp();
   }
   if (warp == 0) {
-    tmem_alloc(&bars->tmem_base, 512);
+    tmem_alloc(&bars->tmem_base, Shape::kTmemColumns);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -334,7 +350,14 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   const uint32_t tmem_base = bars->tmem_base;
   pdl_wait();  // (so far only the producer warp, which waited itself, has touched global memory)
 
+  // (Two CTAs of 256 threads have 128 registers per thread: 184 for the softmax warps, 72 for the others; 4 x 184
+  // + 4 x 72 = 8 x 128.)
+  auto few_registers = [] {
+    if constexpr (NARROW) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  };
+
   if ((warp == kProducerWarp || warp == kGatherWarp) && p.gather) {
+    few_registers();
     // ---------------- producer with a paged K and / or V, by TMA row gather ----------------
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table entries,
     // then gather the rows) as tile::gather4 loads of four rows x 64 columns, straight into the
@@ -352,7 +375,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     const int n_rows = p.n_pages * p.page_size;
     constexpr int kWindow = 8;  // tiles
     // [K or V][tile of the window][32 tokens] of this warp, in the output staging of warps 4..7: their
-    // tile is the last to finish, after the last gather.
+    // tile is the last to finish, after the last gather. (`NARROW`: behind the staging.)
     int* const row_ids = reinterpret_cast<int*>(sStage + 4 * 2048) + part * (2 * kWindow * 32);
     static_assert(2 * 2 * kWindow * 32 * 4 <= 4 * 2048, "row numbers in the staging of four warps");
     auto page_of = [&](int t) { return p.page_shift >= 0 ? (t >> p.page_shift) : (t / p.page_size); };
@@ -446,6 +469,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       for (int j = lo; j < hi; ++j) load_pair(true, j, second(j + 2));
     }
   } else if (warp == kProducerWarp && p.paged) {
+    few_registers();
     // ---------------- producer with a paged K and / or V ----------------
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table
     // entries, then gather the rows) fused into the tile load: a dense operand still arrives by
@@ -554,6 +578,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
     cp_async_wait<0>();
     publish_up_to(n);
   } else if (warp == kProducerWarp) {
+    few_registers();
     // ---------------- TMA producer ----------------
     // The whole warp runs the loop and waits; the elected lane issues the copies (a warp that
     // has diverged into a single-lane branch gets few issue slots next to the softmax warps).
@@ -595,7 +620,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       };
       for (int j = lo; j < hi; ++j) load_pair(j, j + 2 < hi ? j + 2 : -1);
     }
-  } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
+  } else if (warp >= kMmaWarp0 && warp < kMmaWarp0 + Shape::kSlots) {
+    few_registers();
     // ---------------- MMA issuers: one warp per query tile ----------
     // Two issuing threads halve the per-instruction issue overhead; the tensor pipe serialises
     // the two independent streams. Both walk the same K/V ring and both release every stage
@@ -710,6 +736,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
       }
     }
   } else if (warp < kSoftmaxWarps) {
+    if constexpr (NARROW) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
     // ---------------- softmax warps ----------------
     const int t = warp >> 2;                 // slot of this warp group
     const int tq = split ? 0 : t;            // and its query tile
@@ -1305,6 +1332,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
 #pragma unroll
       for (int c = 0; c < D; c += 8) *reinterpret_cast<uint4*>(orow + c) = nan4;
     }
+  } else {
+    few_registers();
   }
 
   // ---------------- teardown ----------------
@@ -1312,7 +1341,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, Shape::kTmemColumns);
   }
 }
 
@@ -1460,21 +1489,71 @@ static int make_tile_map(CUtensorMap* map, const void* base, int B, int H, int S
   return LF_OK;
 }
 
-template <int D, int MODE, bool PE = false>
+static int device_sm_count(int dev) {
+  static thread_local int sm_count = 0;
+  if (sm_count == 0) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+  return sm_count;
+}
+
+// How prefill_kernel deals the query tiles out.
+enum class PrefillForm {
+  kPairs,   // two tiles of a head per CTA, one CTA per SM
+  kSplit,   // one tile per CTA, its key blocks split over the CTA's two slots
+  kNarrow,  // one tile per CTA, two CTAs per SM
+};
+
+// One query tile per CTA, its key blocks split over the two slots:
+//   - where all the tiles are resident at once, one per SM: half the steps of the longest tile (8
+//     heads, 1024 queries, 8192 keys, D = 64: 111 -> 59 us);
+//   - up to two tiles per SM, where the others would leave the short ones' SMs idle while the longest
+//     runs: a pair of tiles takes as many steps as its longer tile has blocks; split tiles,
+//     longest first, the mean load, half of the shortest tile, and about five steps for the start
+//     and end of the second CTA of an SM (causal, 16 heads, 2048 keys, D = 64: pairs 34.9 us, narrow 27.9,
+//     split 21.3; 7 tiles x 32 heads that see 3.4 to 4.1 thousand keys each, D = 128: pairs 64, split 75). With a
+//     paged operand a step of split tiles gathers twice the rows: 1.4 steps.
+// Two CTAs per SM (`can_narrow`: the kernel has that form): the start and end of a CTA, some 13 thousand clocks
+// that pairs leave bare, lie under the other one's blocks, no slot is empty where a head has an odd number of
+// tiles, and the issuing warps of two tiles no longer wait for one ring. Back to back for half a second (causal;
+// pairs -> narrow):
+//   D = 64, any length: 8 x 32 x 512 34.1 -> 29.7 us, 4 x 16 x 2048 68.4 -> 62.5, 1 x 16 x 8192 209.8 -> 194.5; paged
+//   8 x 32 x 1024 100.4 -> 91.2, biased 8 x 16 x 512 38.2 -> 34.0; one tile a head (two slots -> narrow), 8 x 32 x 64,
+//   8.3 -> 4.4.
+//   D = 128 up to 24 blocks a tile: 8 x 64 x 100 22.0 -> 13.6, 8 x 32 x 640 59.1 -> 51.9, 8 x 32 x 1024 105.7 -> 101.8,
+//   4 x 32 x 1536 103.8 -> 101.7, biased 4 x 16 x 1024 69.4 -> 64.3. Further on the chip runs at its power limit and
+//   K and V read once for both tiles count for more: chunks of 1024 with 4000 keys before them 158.8 -> 160.9,
+//   1 x 32 x 8192 444.6 -> 453.7; but for three tiles a head, of whose four slots one is empty (300 rows and 4000
+//   keys, 4 x 64 heads, 235.8 -> 219.4).
+// Up to two tiles per SM narrow takes the place of pairs at D = 64 and with paged operands (777 rows and 3319 keys
+// before them, 32 heads, D = 64 58.0 -> 54.6, paged 4 x 8 x 1024 19.6 -> 18.8; D = 128, dense 65.0 -> 65.4).
+static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_count, bool can_narrow) {
+  const int64_t n_tiles = static_cast<int64_t>(p.n_qtiles) * p.Hq * B;
+  if (n_tiles <= sm_count) return PrefillForm::kSplit;
+  int lo, hi;
+  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, 0, &lo, &hi);
+  const int shortest = hi - lo;
+  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1, &lo, &hi);
+  const int longest = hi - lo;
+  if (p.n_qtiles == 1) return can_narrow ? PrefillForm::kNarrow : PrefillForm::kSplit;
+  if (n_tiles <= 2ll * sm_count) {
+    const double split = 0.25 * (shortest + longest) * static_cast<double>(n_tiles) / sm_count + 0.5 * shortest;
+    if (split * (p.paged ? 1.4 : 1.0) + 5.0 < longest) return PrefillForm::kSplit;
+    return can_narrow && (D == 64 || p.paged) ? PrefillForm::kNarrow : PrefillForm::kPairs;
+  }
+  return can_narrow && (D == 64 || longest <= 24 || p.n_qtiles == 3) ? PrefillForm::kNarrow : PrefillForm::kPairs;
+}
+
+template <int D, int MODE, bool PE = false, bool NARROW = false>
 static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                          const PrefillParams& p, int B, cudaStream_t st,
+                          const PrefillParams& p, int B, cudaStream_t st, PrefillForm form,
                           const CUtensorMap* mqpe = nullptr, const CUtensorMap* mkpe = nullptr) {
-  constexpr size_t kQTileBytes = static_cast<size_t>(kTileQ) * (D + (PE ? 64 : 0)) * 2;
-  constexpr size_t kKVTileBytes = static_cast<size_t>(kTileK) * (D + (PE ? 64 : 0)) * 2;
-  constexpr size_t smem = 1024 /*align slack*/ + 1024 /*barriers*/ + kStageBytesTotal +
-                          2 * kQTileBytes +
-                          PrefillStages<D, PE>::value * 2 * kKVTileBytes;
-  static_assert(smem <= 232448, "shared memory of a CTA");
+  using Shape = PrefillShape<D, PE, NARROW>;
+  constexpr size_t smem = Shape::kSmem;
+  static_assert(smem <= 232448 && (!NARROW || 2 * (smem + 1024) <= 233472), "shared memory of a CTA");
   static thread_local int configured_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_dev != dev) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_kernel<D, MODE, PE>,
+    cudaError_t e = cudaFuncSetAttribute(prefill_kernel<D, MODE, PE, NARROW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) {
@@ -1484,33 +1563,8 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
     configured_dev = dev;
   }
   const int pairs = (p.n_qtiles + 1) / 2;
-  static thread_local int sm_count = 0;
-  if (sm_count == 0) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   PrefillParams pp = p;
-  // One query tile per CTA, its key blocks split over the two slots:
-  //   - where all the tiles are resident at once, one per SM: half the steps of the longest tile (8
-  //     heads, 1024 queries, 8192 keys, D = 64: 111 -> 59 us);
-  //   - where one tile is all a head has;
-  //   - up to two tiles per SM, where pairs would leave the short ones' SMs idle while the longest
-  //     pair runs: a pair of tiles takes as many steps as its longer tile has blocks; single tiles,
-  //     longest first, the mean load, half of the shortest tile, and about five steps for the start
-  //     and end of the second CTA of an SM (causal, 16 heads, 2048 keys, D = 64: 34.9 -> 25.4 us;
-  //     7 tiles x 32 heads that see 3.4 to 4.1 thousand keys each: pairs 71 us, singles 75). With a
-  //     paged operand a step of singles gathers twice the rows: 1.4 steps.
-  // Above that pairs are the better: a K/V tile in shared memory serves two query tiles.
-  const int64_t n_tiles = static_cast<int64_t>(p.n_qtiles) * p.Hq * B;
-  pp.single = p.n_qtiles == 1 || n_tiles <= sm_count;
-  if (!pp.single && n_tiles <= 2ll * sm_count) {
-    int lo, hi;
-    skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, 0, &lo, &hi);
-    const int shortest = hi - lo;
-    skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1,
-               &lo, &hi);
-    const int longest = hi - lo;
-    const double singles = 0.25 * (shortest + longest) * static_cast<double>(n_tiles) / sm_count +
-                           0.5 * shortest;
-    pp.single = singles * (p.paged ? 1.4 : 1.0) + 5.0 < longest;
-  }
+  pp.single = form != PrefillForm::kPairs;
   // Order of the CTAs: the heaviest tiles of a group of heads, then the next lighter ones, ..., then
   // the next group. With a head's tiles next to each other the last head's longest tile started
   // when the rest was nearly done (single launches of B=1 Hq=32 Hkv=8
@@ -1530,9 +1584,24 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   pp.div_group = FastDiv::make(p.group);
   const unsigned grid = static_cast<unsigned>(per_group * groups * tiles);
   // (without a second score product the two extra maps are never read)
-  launch_pdl(prefill_kernel<D, MODE, PE>, dim3(grid), kPrefillThreads, smem, st, mq, mk, mv,
+  launch_pdl(prefill_kernel<D, MODE, PE, NARROW>, dim3(grid), Shape::kThreads, smem, st, mq, mk, mv,
              mqpe ? *mqpe : mq, mkpe ? *mkpe : mk, pp);
   return check_launch("prefill_kernel");
+}
+
+template <int D, int MODE>
+static int launch_prefill_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                               const PrefillParams& p, int B, cudaStream_t st) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  // Plain and biased scores have the narrow form. (Rows that the producer warp copies itself need three ring
+  // stages, which it has at D = 64.)
+  constexpr bool kHasNarrow = MODE == kModeNone || MODE == kModeBias;
+  const PrefillForm form =
+      choose_form(p, D, B, device_sm_count(dev), kHasNarrow && (!p.paged || p.gather || D == 64));
+  if constexpr (kHasNarrow)
+    if (form == PrefillForm::kNarrow) return launch_prefill<D, MODE, false, true>(mq, mk, mv, p, B, st, form);
+  return launch_prefill<D, MODE>(mq, mk, mv, p, B, st, form);
 }
 
 // Ticket counters of the persistent kernel: a small ring in the library image, so that launching
@@ -1892,30 +1961,33 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
     if (rc != LF_OK) return rc;
     rc = make_tile_map(&mkpe, a->k_pe, a->B, a->Hkv, a->Skv, a->D_pe, a->kpe_stride, kTileK);
     if (rc != LF_OK) return rc;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const PrefillForm form = choose_form(p, a->D, a->B, device_sm_count(dev), false);
     if (a->D == 128)
-      return launch_prefill<128, kModeNone, true>(mq, mk, mv, p, a->B, st, &mqpe, &mkpe);
-    return launch_prefill<64, kModeNone, true>(mq, mk, mv, p, a->B, st, &mqpe, &mkpe);
+      return launch_prefill<128, kModeNone, true>(mq, mk, mv, p, a->B, st, form, &mqpe, &mkpe);
+    return launch_prefill<64, kModeNone, true>(mq, mk, mv, p, a->B, st, form, &mqpe, &mkpe);
   }
   if (a->D == 128) {
-    if (mode == kModeNone) return launch_prefill<128, kModeNone>(mq, mk, mv, p, a->B, st);
-    if (mode == kModeSoftcap) return launch_prefill<128, kModeSoftcap>(mq, mk, mv, p, a->B, st);
+    if (mode == kModeNone) return launch_prefill_form<128, kModeNone>(mq, mk, mv, p, a->B, st);
+    if (mode == kModeSoftcap) return launch_prefill_form<128, kModeSoftcap>(mq, mk, mv, p, a->B, st);
     if (mode == kModeBounded)
       return kv_tile == kWideK ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st)
              : pack == 4       ? launch_prefill_bounded<128, 4>(mq, mk, mv, mo, p, a->B, st)
              : pack == 2       ? launch_prefill_bounded<128, 2>(mq, mk, mv, mo, p, a->B, st)
                                : launch_prefill_bounded<128>(mq, mk, mv, mo, p, a->B, st);
-    if (mode == kModeBias) return launch_prefill<128, kModeBias>(mq, mk, mv, p, a->B, st);
-    return launch_prefill<128, kModeGeneric>(mq, mk, mv, p, a->B, st);
+    if (mode == kModeBias) return launch_prefill_form<128, kModeBias>(mq, mk, mv, p, a->B, st);
+    return launch_prefill_form<128, kModeGeneric>(mq, mk, mv, p, a->B, st);
   }
-  if (mode == kModeNone) return launch_prefill<64, kModeNone>(mq, mk, mv, p, a->B, st);
-  if (mode == kModeSoftcap) return launch_prefill<64, kModeSoftcap>(mq, mk, mv, p, a->B, st);
+  if (mode == kModeNone) return launch_prefill_form<64, kModeNone>(mq, mk, mv, p, a->B, st);
+  if (mode == kModeSoftcap) return launch_prefill_form<64, kModeSoftcap>(mq, mk, mv, p, a->B, st);
   if (mode == kModeBounded)
     return kv_tile == kWideK ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st)
            : pack == 4       ? launch_prefill_bounded<64, 4>(mq, mk, mv, mo, p, a->B, st)
            : pack == 2       ? launch_prefill_bounded<64, 2>(mq, mk, mv, mo, p, a->B, st)
                              : launch_prefill_bounded<64>(mq, mk, mv, mo, p, a->B, st);
-  if (mode == kModeBias) return launch_prefill<64, kModeBias>(mq, mk, mv, p, a->B, st);
-  return launch_prefill<64, kModeGeneric>(mq, mk, mv, p, a->B, st);
+  if (mode == kModeBias) return launch_prefill_form<64, kModeBias>(mq, mk, mv, p, a->B, st);
+  return launch_prefill_form<64, kModeGeneric>(mq, mk, mv, p, a->B, st);
 }
 
 }  // namespace lf
