@@ -1611,24 +1611,43 @@ constexpr int kTicketSlots = 256;
 static __device__ unsigned int g_prefill_tickets[kTicketSlots];
 static std::atomic<unsigned int> g_next_ticket_slot{0};
 
-template <int D, int PACK = 1>
+// Whether the fixed-reference kernel runs as two CTAs of one tile slot per SM (narrow) instead of one of two. The slots
+// then no longer share a ring and an item's end, and a tile that has an SM to itself has all of it; but every tile
+// fetches its own K and V. Both back to back for half a second, softcap 50 (two slots -> narrow):
+//   D = 64, always: 8 x 32 x 1024 79.7 -> 76.7 us, 2 x 16 x 4096 142.6 -> 129.4, 2 x 4 x 512 14.3 -> 12.3, window 256,
+//   four heads per kv head, 8 x 32 x 2048 87.7 -> 87.2, 1 x 8 x 2048 12.3 -> 10.3;
+//   D = 128, no more tiles than SMs: 1 x 8 x 2048 38.5 -> 30.6, 2 x 8 x 1024 24.4 -> 19.7; up to 10 blocks a tile:
+//   8 x 64 x 256 30.7 -> 28.7, 8 x 32 x 512 41.7 -> 40.1, 8 x 16 x 600 32.8 -> 30.8; up to 16 and four tiles per SM:
+//   2 x 32 x 700 26.9 -> 24.6, 4 x 16 x 1024 36.3 -> 35.1; beyond, the chip's power limit decides and K and V read
+//   once for two tiles win (8 x 32 x 1024 107.4 -> 108.5, 8 x 32 x 2048 338.7 -> 346.6, 1 x 8 x 8192 175.1 -> 180.0);
+//   D = 128 packed, up to four chunks per SM (1 x 8 x 2048, window 256 14.4 -> 12.3; 2 x 16 x 2048, window 1000
+//   45.2 -> 42.8; 8 x 32 x 2048, window 256 121.3 -> 124.3).
+static bool bounded_is_narrow(const PrefillParams& p, int D, int pack, int B, int sm_count) {
+  if (p.sm_margin > 0) return false;  // (two CTAs per SM would spread over the SMs to be left free)
+  if (D == 64) return true;
+  const int rows = kTileQ / pack;
+  const int64_t n_tiles = static_cast<int64_t>((p.Sq + rows - 1) / rows) * (p.Hq / pack) * B;
+  const bool few = n_tiles <= 4ll * sm_count;
+  if (pack > 1) return few;
+  int lo, hi;
+  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1, &lo, &hi);
+  return n_tiles <= sm_count || hi - lo <= (few ? 16 : 10);
+}
+
+template <int D, int PACK = 1, bool NARROW = false>
 static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
                                   const CUtensorMap& mv, const CUtensorMap& mo, PrefillParams p,
                                   int B, cudaStream_t st) {
-  constexpr size_t kQTileBytes = static_cast<size_t>(kTileQ) * D * 2;
-  constexpr size_t kKVTileBytes = static_cast<size_t>(kTileK) * D * 2;
-  constexpr bool kBig = PACK > 1 && D == 128;
-  constexpr size_t smem = 1024 /*align slack*/ + 1024 /*barriers*/ +
-                          (kBig ? 16 * 4096 : kBoundedStageBytes) + 2 * kQTileBytes +
-                          (kBig ? 3 : StagesFor<D>::value) * 2 * kKVTileBytes;
-  static_assert(smem <= 232448, "smem");
+  using Shape = BoundedShape<D, PACK, NARROW>;
+  constexpr size_t smem = Shape::kSmem;
+  static_assert(smem <= 232448 && (!NARROW || 2 * (smem + 1024) <= 233472), "shared memory of a CTA");
   static thread_local int configured_dev = -1;
   static thread_local unsigned int* tickets = nullptr;
   static thread_local int sm_count = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_dev != dev) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_bounded_kernel<D, PACK>,
+    cudaError_t e = cudaFuncSetAttribute(prefill_bounded_kernel<D, PACK, NARROW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e == cudaSuccess)
@@ -1644,7 +1663,7 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
   // item is a pair of chunks of one kv head, for all of its query heads at once.
   const int heads = PACK > 1 ? p.Hq / p.group : p.Hq;
   if (PACK > 1) p.n_qtiles = (p.Sq + kTileQ / PACK - 1) / (kTileQ / PACK);
-  p.n_pairs = (p.n_qtiles + 1) / 2;
+  p.n_pairs = NARROW ? p.n_qtiles : (p.n_qtiles + 1) / 2;
   p.n_deferred = (p.mask_kind == LF_MASK_CAUSAL && p.Sq == p.Skv) ? p.n_pairs / 4 : 0;
   p.main_items = static_cast<int32_t>(static_cast<int64_t>(p.n_pairs - p.n_deferred) * heads * B);
   p.div_main = FastDiv::make(p.n_pairs - p.n_deferred);
@@ -1661,9 +1680,24 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
     return LF_ERR_CUDA;
   }
   const int ctas = sm_count - p.sm_margin > 0 ? sm_count - p.sm_margin : 1;
-  const int grid = static_cast<int>(n_items < ctas ? n_items : ctas);
-  prefill_bounded_kernel<D, PACK><<<grid, kBoundedThreads, smem, st>>>(mq, mk, mv, mo, p);
+  const int64_t slots = static_cast<int64_t>(ctas) * (NARROW ? 2 : 1);
+  const int grid = static_cast<int>(n_items < slots ? n_items : slots);
+  prefill_bounded_kernel<D, PACK, NARROW><<<grid, Shape::kThreads, smem, st>>>(mq, mk, mv, mo, p);
   return check_launch("prefill_bounded_kernel");
+}
+
+template <int D>
+static int launch_prefill_bounded_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                                       const CUtensorMap& mo, const PrefillParams& p, int B, cudaStream_t st,
+                                       int pack, bool narrow) {
+  if (pack == 4)
+    return narrow ? launch_prefill_bounded<D, 4, true>(mq, mk, mv, mo, p, B, st)
+                  : launch_prefill_bounded<D, 4>(mq, mk, mv, mo, p, B, st);
+  if (pack == 2)
+    return narrow ? launch_prefill_bounded<D, 2, true>(mq, mk, mv, mo, p, B, st)
+                  : launch_prefill_bounded<D, 2>(mq, mk, mv, mo, p, B, st);
+  return narrow ? launch_prefill_bounded<D, 1, true>(mq, mk, mv, mo, p, B, st)
+                : launch_prefill_bounded<D>(mq, mk, mv, mo, p, B, st);
 }
 
 template <int D>
@@ -1947,9 +1981,13 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   }
 
   CUtensorMap mo;  // output store boxes of the persistent kernels: 32 rows x 32 columns
+  bool narrow = false;
   if (mode == kModeBounded) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    narrow = kv_tile != kWideK && bounded_is_narrow(p, a->D, pack, a->B, device_sm_count(dev));
     rc = make_tile_map(&mo, a->out, a->B, a->Hq, a->Sq, a->D, a->o_stride, 32,
-                       (pack > 1 && a->D == 128) ? 64 : 32);
+                       (pack > 1 && a->D == 128 && !narrow) ? 64 : 32);
     if (rc != LF_OK) return rc;
   }
 
@@ -1972,20 +2010,18 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
     if (mode == kModeNone) return launch_prefill_form<128, kModeNone>(mq, mk, mv, p, a->B, st);
     if (mode == kModeSoftcap) return launch_prefill_form<128, kModeSoftcap>(mq, mk, mv, p, a->B, st);
     if (mode == kModeBounded)
-      return kv_tile == kWideK ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st)
-             : pack == 4       ? launch_prefill_bounded<128, 4>(mq, mk, mv, mo, p, a->B, st)
-             : pack == 2       ? launch_prefill_bounded<128, 2>(mq, mk, mv, mo, p, a->B, st)
-                               : launch_prefill_bounded<128>(mq, mk, mv, mo, p, a->B, st);
+      return kv_tile == kWideK
+               ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st)
+               : launch_prefill_bounded_form<128>(mq, mk, mv, mo, p, a->B, st, pack, narrow);
     if (mode == kModeBias) return launch_prefill_form<128, kModeBias>(mq, mk, mv, p, a->B, st);
     return launch_prefill_form<128, kModeGeneric>(mq, mk, mv, p, a->B, st);
   }
   if (mode == kModeNone) return launch_prefill_form<64, kModeNone>(mq, mk, mv, p, a->B, st);
   if (mode == kModeSoftcap) return launch_prefill_form<64, kModeSoftcap>(mq, mk, mv, p, a->B, st);
   if (mode == kModeBounded)
-    return kv_tile == kWideK ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st)
-           : pack == 4       ? launch_prefill_bounded<64, 4>(mq, mk, mv, mo, p, a->B, st)
-           : pack == 2       ? launch_prefill_bounded<64, 2>(mq, mk, mv, mo, p, a->B, st)
-                             : launch_prefill_bounded<64>(mq, mk, mv, mo, p, a->B, st);
+    return kv_tile == kWideK
+               ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st)
+               : launch_prefill_bounded_form<64>(mq, mk, mv, mo, p, a->B, st, pack, narrow);
   if (mode == kModeBias) return launch_prefill_form<64, kModeBias>(mq, mk, mv, p, a->B, st);
   return launch_prefill_form<64, kModeGeneric>(mq, mk, mv, p, a->B, st);
 }

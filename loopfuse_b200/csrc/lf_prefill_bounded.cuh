@@ -72,7 +72,8 @@ struct ItemGeom {
 // slot holds 32 rows of each of the four query heads of one kv head (then `h` is the first of
 // the four, the items run over kv heads, and iq0 counts 32-row chunks).
 __device__ __forceinline__ ItemGeom decode_item(const PrefillParams& p, int it,
-                                                int tile_k = kTileK, int rows_q = kTileQ) {
+                                                int tile_k = kTileK, int rows_q = kTileQ,
+                                                bool one_tile = false) {
   ItemGeom g;
   g.it = it;
   // Heaviest query tiles of a head first. With a causal mask the lightest quarter of the pairs
@@ -96,12 +97,12 @@ __device__ __forceinline__ ItemGeom decode_item(const PrefillParams& p, int it,
     g.hkv = hb - g.b * static_cast<int>(p.div_hq.d);
     g.h = g.hkv * p.group;
   }
-  g.iq0 = pair * 2;
+  g.iq0 = one_tile ? pair : pair * 2;
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, rows_q, tile_k, g.iq0, &g.lo0,
              &g.hi0);
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, rows_q, tile_k, g.iq0 + 1,
              &g.lo1, &g.hi1);
-  const bool v0 = g.iq0 * rows_q < p.Sq, v1 = (g.iq0 + 1) * rows_q < p.Sq;
+  const bool v0 = g.iq0 * rows_q < p.Sq, v1 = !one_tile && (g.iq0 + 1) * rows_q < p.Sq;
   const bool w0 = v0 && g.hi0 > g.lo0, w1 = v1 && g.hi1 > g.lo1;
   g.flags = (v0 ? 1 : 0) | (v1 ? 2 : 0) | (w0 ? 4 : 0) | (w1 ? 8 : 0);
   g.lo = 0;
@@ -126,8 +127,25 @@ __device__ __forceinline__ ItemGeom decode_item(const PrefillParams& p, int it,
 // instead of six, and six ring stages per item instead of eight), and the heads share every K/V
 // tile in shared memory, not just in L2. Tensor-memory lane quadrant q (32 rows) belongs to
 // head h0 + q * PACK / 4 and holds rows (q % (4 / PACK)) * 32 .. + 32 of the slot's chunk.
-template <int D, int PACK>
-__global__ void __launch_bounds__(kBoundedThreads, 1)
+//
+// NARROW: one tile slot, half of an SM's registers, shared and tensor memory, two CTAs per SM (12 warps: 8 softmax,
+// the producer, the PV and the QK^T issuer, one idle). The two never wait for one another: the end of an item of
+// one lies under the blocks of the other. (At D = 128 two CTAs fill the SM's shared memory to the byte, so the
+// array is declared with the alignment of the swizzled tiles and has no slack in front.)
+template <int D, int PACK, bool NARROW>
+struct BoundedShape {
+  static constexpr int kSlots = NARROW ? 1 : 2;
+  static constexpr int kThreads = NARROW ? 12 * 32 : kBoundedThreads;
+  static constexpr bool kBig = PACK > 1 && D == 128 && !NARROW;
+  static constexpr int kStages = NARROW ? (D == 64 ? 4 : 2) : kBig ? 3 : StagesFor<D>::value;
+  static constexpr uint32_t kWarpStage = kBig ? 4096 : 2048;
+  static constexpr uint32_t kTmemColumns = NARROW ? 256 : 512;
+  static constexpr size_t kSmem = 1024 /*barriers*/ + kSlots * (8 * kWarpStage + static_cast<size_t>(kTileQ) * D * 2) +
+                                  static_cast<size_t>(kStages) * 2 * kTileK * D * 2 + (NARROW ? 0 : 1024 /*align slack*/);
+};
+
+template <int D, int PACK, bool NARROW>
+__global__ void __launch_bounds__(BoundedShape<D, PACK, NARROW>::kThreads, NARROW ? 2 : 1)
     prefill_bounded_kernel(const __grid_constant__ CUtensorMap tmap_q,
                            const __grid_constant__ CUtensorMap tmap_k,
                            const __grid_constant__ CUtensorMap tmap_v,
@@ -137,9 +155,12 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
   // bulk store of full 128-byte row segments and nobody waits for the store engine inside the
   // epilogue; the room comes from a K/V ring of three stages instead of four (an item has six
   // stages there). Measured on the same box: 574 -> 591 TFLOP/s on window_gqa_softcap.
-  constexpr bool kBig = PACK > 1 && D == 128;
-  constexpr int kStages = kBig ? 3 : StagesFor<D>::value;
-  constexpr uint32_t kWarpStage = kBig ? 4096 : 2048;
+  using Shape = BoundedShape<D, PACK, NARROW>;
+  constexpr bool kBig = Shape::kBig;
+  constexpr int kStages = Shape::kStages;
+  constexpr uint32_t kWarpStage = Shape::kWarpStage;
+  constexpr int kSlots = Shape::kSlots;
+  constexpr int kSoftmaxWarps = kSlots * 8;
   constexpr int kBlocksD = D / 64;
   static_assert(PACK == 1 || PACK == 2 || PACK == 4, "heads per tile");
   constexpr bool PACKED = PACK > 1;
@@ -150,21 +171,21 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
   constexpr uint32_t kKVTileBytes = kKVBlockBytes * kBlocksD;
   constexpr uint32_t kIdescQK = make_idesc_bf16(128, kTileK, 0);
   constexpr uint32_t kIdescPV = make_idesc_bf16(128, D, 1);
-  constexpr uint32_t kColO = 256;
-  constexpr int kProducerWarp = 16;
-  constexpr int kMmaWarp0 = 17;
+  constexpr uint32_t kColO = kSlots * 128;
+  constexpr int kProducerWarp = kSoftmaxWarps;
+  constexpr int kMmaWarp0 = kSoftmaxWarps + 1;
 
-  extern __shared__ unsigned char smem_unaligned[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
+  extern __shared__ __align__(1024) unsigned char smem_aligned[];
+  unsigned char* smem = NARROW ? smem_aligned : reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_aligned) + 1023) & ~static_cast<uintptr_t>(1023));
   BoundedBarriers* bars = reinterpret_cast<BoundedBarriers*>(smem);
   static_assert(sizeof(BoundedBarriers) + 16 + kItemSlots * sizeof(ItemGeom) <= 1024, "barrier page");
   static_assert(sizeof(ItemGeom) == 48, "three 16-byte pieces");
   ItemGeom* item_slots =
       reinterpret_cast<ItemGeom*>(smem + ((sizeof(BoundedBarriers) + 15) & ~size_t(15)));
   unsigned char* sStage = smem + 1024;  // 16 x 2 KB output staging (one buffer per softmax warp)
-  unsigned char* sQ = sStage + 16 * kWarpStage;
-  unsigned char* sKV = sQ + 2 * kQTileBytes;
+  unsigned char* sQ = sStage + kSoftmaxWarps * kWarpStage;
+  unsigned char* sKV = sQ + kSlots * kQTileBytes;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -185,11 +206,11 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
     }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->kv_empty[s], 4);  // every MMA thread releases every stage
+      mbar_init(&bars->kv_empty[s], 2 * kSlots);  // every MMA thread releases every stage
     }
     for (int s = 0; s < kItemSlots; ++s) {
       mbar_init(&bars->item_full[s], 1);
-      mbar_init(&bars->item_empty[s], 20);
+      mbar_init(&bars->item_empty[s], 10 * kSlots);
     }
     mbar_fence_init();
   }
@@ -200,7 +221,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
     tma_prefetch_desc(&tmap_o);
   }
   if (warp == 0) {
-    tmem_alloc(&bars->tmem_base, 512);
+    tmem_alloc(&bars->tmem_base, Shape::kTmemColumns);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -277,7 +298,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
           break;
         }
         ItemGeom g;
-        if (it >= 0) g = decode_item(p, it, kTileK, kRowsQ);
+        if (it >= 0) g = decode_item(p, it, kTileK, kRowsQ, NARROW);
         else g.it = -1, g.b = g.h = g.hkv = g.iq0 = g.lo0 = g.hi0 = g.lo1 = g.hi1 = g.flags = g.lo = g.hi = 0;
         if (elected) {
           item_slots[slot] = g;
@@ -285,7 +306,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
         }
         __syncwarp();
         if (it < 0) break;
-        for (int t = 0; t < 2 && ok; ++t) {
+        for (int t = 0; t < kSlots && ok; ++t) {
           if (!g.work(t)) continue;
           // Q_t is free once the last QK^T of the previous item with work for this tile is done.
           if (qseq[t] > 0 && !mbar_wait(&bars->q_free[t], (qseq[t] - 1) & 1)) {
@@ -320,7 +341,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
         }
       }
     }
-  } else if (warp >= kMmaWarp0 && warp < kMmaWarp0 + 4) {
+  } else if (warp >= kMmaWarp0 && warp < kMmaWarp0 + 2 * kSlots) {
     // ---------------- MMA issuers: a PV thread and a QK^T thread per query tile ----------
     // All four threads walk every ring stage and each releases it (kv_empty counts four
     // arrivals) once the MMAs it issued from the stage, if any, are complete. A thread must see
@@ -329,8 +350,8 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
     // issues MMAs and commits. A warp that has diverged into a single-lane branch gets far fewer
     // issue slots next to the busy softmax warps (measured: one MMA per ~150 clocks, not 64).
     {
-      const int t = (warp - kMmaWarp0) & 1;
-      const bool is_qk = warp - kMmaWarp0 >= 2;
+      const int t = NARROW ? 0 : (warp - kMmaWarp0) & 1;
+      const bool is_qk = warp - kMmaWarp0 >= kSlots;
       const bool elected = elect_one_sync();
       bool ok = true;
       constexpr uint32_t kStageUnits = (2 * kKVTileBytes) >> 4;  // a stage is a pair of tiles
@@ -465,7 +486,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
         if (work) gblk += hi_tt - lo_tt;
       }
     }
-  } else {
+  } else if (warp < kSoftmaxWarps) {
     // ---------------- softmax warps ----------------
     // Query tile t = warpgroup / 2; inside a tile, warpgroup `half` takes columns
     // [32*half, 32*half + 32) of every 64-key block, one thread per (row, half). With the fixed
@@ -757,7 +778,7 @@ __global__ void __launch_bounds__(kBoundedThreads, 1)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, Shape::kTmemColumns);
   }
 }
 

@@ -1,7 +1,7 @@
-"""The running-max prefill kernel deals query tiles out in three forms, by their number: split over the
-two slots of a CTA (no more tiles than SMs), pairs, or two CTAs per SM. Every kind of call on the two-CTA
-side of the rule, at the edges of tiles and of the rule itself, against the same rows computed a few heads
-at a time in the split form, and against fp32."""
+"""The prefill kernels deal query tiles out in several forms, by their number and length: pairs of tiles per
+CTA, one tile split over the two slots of a CTA (running-max kernel, no more tiles than SMs), or two CTAs
+per SM. Every kind of call on the two-CTA side of the rules, at the edges of tiles, against another form of
+the same call and against fp32."""
 import pytest
 import torch
 
@@ -105,3 +105,40 @@ def test_two_ctas_per_sm_paged(P, heads_first, D):
     F.check_status(st)
     k = pool[table.long()].reshape(B, blocks * P, Hkv, D)[:, :Skv].transpose(1, 2)
     _close(out, _fp32(q, k, v, S.MASK_CAUSAL, 0))
+
+
+SOFTCAP = [S.ScoreMod(S.MOD_DIV, 30.0), S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_MUL, 30.0)]
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,mask,off,window,gain", [
+    (1, 2, 2, 1, 1, S.MASK_CAUSAL, 0, 0, 1.0),
+    (2, 3, 1, 129, 129, S.MASK_CAUSAL, 0, 0, 1.0),
+    (1, 4, 4, 130, 1000, S.MASK_NONE, 0, 0, 30.0),             # the stronger forms of tanh
+    (2, 40, 40, 600, 600, S.MASK_CAUSAL, 0, 0, 1.0),           # more items than CTAs
+    (1, 2, 1, 700, 300, S.MASK_CAUSAL, -200, 0, 1.0),          # tiles and rows without a key
+    (3, 8, 8, 515, 515, S.MASK_CAUSAL_WINDOW, 0, 100, 1.0),
+    (2, 8, 4, 515, 515, S.MASK_CAUSAL_WINDOW, 0, 65, 1.0),     # packed: two heads a tile,
+    (1, 16, 4, 515, 515, S.MASK_CAUSAL_WINDOW, 0, 64, 10.0),   # four
+    (4, 32, 8, 300, 300, S.MASK_CAUSAL_WINDOW, 0, 1, 1.0),     # one key a row
+    (1, 4, 1, 33, 400, S.MASK_CAUSAL_WINDOW, 367, 256, 1.0),
+])
+def test_softcap_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, gain, D):
+    """Against the form of one CTA per SM, which a margin of one SM asks for."""
+    torch.manual_seed(4)
+    q = (torch.randn(B, Sq, Hq, D, device="cuda") * gain).bfloat16().transpose(1, 2)
+    k, v = (torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16() for _ in range(2))
+    st = F.new_status("cuda")
+    kw = dict(scale=D ** -0.5, mods=SOFTCAP, mask_kind=mask, window=window, causal_offset=off, status=st)
+    out = F.prefill_attention(q, k, v, **kw)
+    _close(out, F.prefill_attention(q, k, v, sm_margin=1, **kw))
+    F.check_status(st)
+    group = Hq // Hkv
+    s = q.float() @ k.float().repeat_interleave(group, 1).transpose(-2, -1) * D ** -0.5
+    s = torch.tanh(s / 30.0) * 30.0
+    i, j = torch.arange(Sq, device="cuda")[:, None] + off, torch.arange(Skv, device="cuda")[None]
+    if mask != S.MASK_NONE:
+        s = s.masked_fill(j > i, float("-inf"))
+    if mask == S.MASK_CAUSAL_WINDOW:
+        s = s.masked_fill(j <= i - window, float("-inf"))
+    _close(out, torch.softmax(s, -1) @ v.float().repeat_interleave(group, 1))
