@@ -53,8 +53,8 @@ METRIC = "prefill TFLOP/s (causal-adjusted FLOPs) per job; decode HBM GB/s under
 # workload's dominant kernel, from ncu captures of a smaller batch scaled by the batch ratio (the
 # traffic is proportional to the batch).
 NCU_TRAFFIC_BYTES = {
-    "causal_softcap": 4 * (108.67e6 + 14.64e6),
-    "window_gqa_softcap": 2 * (100.74e6 + 30.84e6),
+    "causal_softcap": 4 * (108.53e6 + 13.97e6),
+    "window_gqa_softcap": 2 * (100.73e6 + 29.55e6),
     "decode": 8 * (268.56e6 + 3.22e6),
     "paged_decode_gqa": 2 * (268.78e6 + 4.01e6),
 }

@@ -122,7 +122,8 @@ typedef struct {
   int32_t n_pages;
   int32_t sm_margin;    /* persistent kernels only: leave this many SMs without a CTA, for
                            kernels that must run at the same time (a collective on another
-                           stream cannot start while one CTA per SM is resident); 0 = use all */
+                           stream cannot start while one CTA per SM is resident); 0 = use all.
+                           A margin also keeps these kernels at one CTA per SM */
   /* Additive score bias (NULL = none): bf16 [B, Hq, Sq, Skv], innermost stride 1, 16-byte
    * aligned rows; bias_stride = element strides of (b, h, row). It is added to the score after
    * the first `bias_pos` ops of the mod chain (0 <= bias_pos <= n_mod) and before the mask:

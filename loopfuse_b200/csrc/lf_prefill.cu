@@ -3,13 +3,13 @@
 // and tensor-memory layouts and the host code of this file:
 //
 //   prefill_kernel<D, MODE> (this file): the running-max modes - plain scores, generic score
-//       mods, softcap with a large cap. One CTA per pair of query tiles.
+//       mods, softcap with a large cap. One CTA per pair of query tiles, or two of one tile per SM.
 //   prefill_bounded_kernel<D> (lf_prefill_bounded.cuh): softcap whose output range needs no
-//       running max (the benchmark configurations). Persistent, one CTA per SM.
+//       running max (the benchmark configurations). Persistent, one CTA per SM, or two of one tile slot.
 //
 // prefill_kernel: one CTA owns two consecutive 128-row query tiles of one (batch, q head) and
 // walks the 64-key KV tiles that the skip range leaves (fully masked tiles are never loaded or
-// multiplied). 384 threads:
+// multiplied). 384 threads (the narrow form, for one tile, has half of each role: see PrefillShape):
 //   warps 0-3   softmax for query tile 0 (one thread per score row)
 //   warps 4-7   softmax for query tile 1
 //   warp  8     TMA producer: Q tiles once, then pairs of K/V tiles into a ring, in the order
@@ -1129,10 +1129,10 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
           }
           const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
 
-          // Pass 2: p = exp2(score * c2 - m). Plain fp32 instructions and every exp2 on MUFU: the
-          // loop is bound by instruction issue, and the packed f32x2 forms (fewer instructions,
-          // but slower in their pipe) and an FMA-pipe emulation of part of the exp2 both measured
-          // slower than this in the fixed-reference kernel, which runs the same arithmetic.
+          // Pass 2: p = exp2(score * c2 - m). Plain fp32 instructions and every exp2 on MUFU: a packed
+          // f32x2 multiply-add in front of exp2 made the plain pass slower (1 x 32 x 8192, D = 128, 853 ->
+          // 896 thousand clocks; the long polynomials of the fixed-reference kernel gain by it), and so did
+          // an FMA-pipe emulation of part of the exp2.
           const float neg_m = -m_safe;
           float ps[4] = {0.f, 0.f, 0.f, 0.f};
           uint32_t pk[32];
