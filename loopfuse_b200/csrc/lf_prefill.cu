@@ -620,7 +620,9 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
       };
       for (int j = lo; j < hi; ++j) load_pair(j, j + 2 < hi ? j + 2 : -1);
     }
-  } else if (warp >= kMmaWarp0 && warp < kMmaWarp0 + Shape::kSlots) {
+  } else if (warp == kMmaWarp0 || (!NARROW && warp == kMmaWarp0 + 1)) {
+    // (Two comparisons: as a range the two-slot form came out 0.1 us a launch slower, causal 4 x 8 x 593 D = 64
+    // 9.01 -> 9.10 us.)
     few_registers();
     // ---------------- MMA issuers: one warp per query tile ----------
     // Two issuing threads halve the per-instruction issue overhead; the tensor pipe serialises

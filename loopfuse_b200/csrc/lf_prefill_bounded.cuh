@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(BoundedShape<D, PACK, NARROW>::kThreads, NARRO
         if (work) gblk += hi_tt - lo_tt;
       }
     }
-  } else if (warp < kSoftmaxWarps) {
+  } else if (!NARROW || warp < kSoftmaxWarps) {
     // ---------------- softmax warps ----------------
     // Query tile t = warpgroup / 2; inside a tile, warpgroup `half` takes columns
     // [32*half, 32*half + 32) of every 64-key block, one thread per (row, half). With the fixed
