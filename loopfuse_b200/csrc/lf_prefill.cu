@@ -350,14 +350,14 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
   const uint32_t tmem_base = bars->tmem_base;
   pdl_wait();  // (so far only the producer warp, which waited itself, has touched global memory)
 
-  // (Two CTAs of 256 threads have 128 registers per thread: 184 for the softmax warps, 72 for the others; 4 x 184
-  // + 4 x 72 = 8 x 128.)
-  auto few_registers = [] {
-    if constexpr (NARROW) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  };
+  // Two CTAs of 256 threads have 128 registers per thread: 184 for the softmax warps (below), 72 for the others; 4 x 184 +
+  // 4 x 72 = 8 x 128. setmaxnreg has to be one instruction for all warps of a warpgroup, so it stands in front of the
+  // dispatch of roles, on a condition that is the same in all four.
+  if constexpr (NARROW) {
+    if (warp >= kSoftmaxWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  }
 
   if ((warp == kProducerWarp || warp == kGatherWarp) && p.gather) {
-    few_registers();
     // ---------------- producer with a paged K and / or V, by TMA row gather ----------------
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table entries,
     // then gather the rows) as tile::gather4 loads of four rows x 64 columns, straight into the
@@ -469,7 +469,6 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
       for (int j = lo; j < hi; ++j) load_pair(true, j, second(j + 2));
     }
   } else if (warp == kProducerWarp && p.paged) {
-    few_registers();
     // ---------------- producer with a paged K and / or V ----------------
     // The two-level load of the reference (loopfuse/codegen.py:738-872: read tile_K table
     // entries, then gather the rows) fused into the tile load: a dense operand still arrives by
@@ -578,7 +577,6 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
     cp_async_wait<0>();
     publish_up_to(n);
   } else if (warp == kProducerWarp) {
-    few_registers();
     // ---------------- TMA producer ----------------
     // The whole warp runs the loop and waits; the elected lane issues the copies (a warp that
     // has diverged into a single-lane branch gets few issue slots next to the softmax warps).
@@ -623,7 +621,6 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
   } else if (warp == kMmaWarp0 || (!NARROW && warp == kMmaWarp0 + 1)) {
     // (Two comparisons: as a range the two-slot form came out 0.1 us a launch slower, causal 4 x 8 x 593 D = 64
     // 9.01 -> 9.10 us.)
-    few_registers();
     // ---------------- MMA issuers: one warp per query tile ----------
     // Two issuing threads halve the per-instruction issue overhead; the tensor pipe serialises
     // the two independent streams. Both walk the same K/V ring and both release every stage
@@ -1334,8 +1331,6 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
 #pragma unroll
       for (int c = 0; c < D; c += 8) *reinterpret_cast<uint4*>(orow + c) = nan4;
     }
-  } else {
-    few_registers();
   }
 
   // ---------------- teardown ----------------
