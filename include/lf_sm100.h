@@ -254,6 +254,15 @@ int lf_prefill_kv_tile(const LfPrefillArgs* args);
  * one (lo, hi) per (batch, query head, chunk of that many rows): int32 [B * Hq * ceil(Sq /
  * q_tile) * 2]. Negative LfStatus on error; launches nothing. */
 int lf_prefill_q_tile(const LfPrefillArgs* args);
+/* How that kernel deals the query tiles out on a device of `sm_count` SMs (0 = the current
+ * device), by their number and length: LF_FORM_PAIRS (a CTA of two tiles per SM), LF_FORM_SPLIT
+ * (the key blocks of one tile split over a CTA's two slots) or LF_FORM_NARROW (two CTAs of one
+ * tile per SM). Negative LfStatus on error; launches nothing, and needs no device when
+ * `sm_count` is given. */
+#define LF_FORM_PAIRS 0
+#define LF_FORM_SPLIT 1
+#define LF_FORM_NARROW 2
+int lf_prefill_form(const LfPrefillArgs* args, int32_t sm_count);
 /* Hit / miss counters of the library's cache of encoded tensor maps (keyed by address, shape,
  * strides and box; the per-call host work the reference's launcher repeats on every call,
  * loopfuse/codegen.py:215-298). Either pointer may be NULL. */

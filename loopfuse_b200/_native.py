@@ -19,7 +19,7 @@ EXPORTS = [
     "lf_decode_workspace_bytes", "lf_decode_launches", "lf_combine_f32", "lf_paged_gather_bf16",
     "lf_decode_bf16_static", "lf_prefill_kv_tile", "lf_prefill_q_tile", "lf_tile_map_cache_stats",
     "lf_kv_append_bf16", "lf_selftest_wait_timeout", "lf_add_bf16", "lf_debug_bounds",
-    "lf_prefill_row_bias_bf16",
+    "lf_prefill_row_bias_bf16", "lf_prefill_form",
 ]
 
 LF_STATIC_SCRATCH_BYTES = 8 << 20
@@ -114,6 +114,8 @@ def load() -> C.CDLL:
     lib.lf_prefill_q_tile.restype = C.c_int
     lib.lf_prefill_kv_tile.argtypes = [C.POINTER(LfPrefillArgs)]
     lib.lf_prefill_kv_tile.restype = C.c_int
+    lib.lf_prefill_form.argtypes = [C.POINTER(LfPrefillArgs), C.c_int32]
+    lib.lf_prefill_form.restype = C.c_int
     lib.lf_tile_map_cache_stats.argtypes = [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]
     lib.lf_tile_map_cache_stats.restype = None
     lib.lf_kv_append_bf16.argtypes = [C.POINTER(LfKvAppendArgs), C.c_void_p]

@@ -1492,11 +1492,11 @@ static int device_sm_count(int dev) {
   return sm_count;
 }
 
-// How prefill_kernel deals the query tiles out.
+// How the prefill kernels deal the query tiles out.
 enum class PrefillForm {
-  kPairs,   // two tiles of a head per CTA, one CTA per SM
-  kSplit,   // one tile per CTA, its key blocks split over the CTA's two slots
-  kNarrow,  // one tile per CTA, two CTAs per SM
+  kPairs = LF_FORM_PAIRS,    // two tiles of a head per CTA, one CTA per SM
+  kSplit = LF_FORM_SPLIT,    // one tile per CTA, its key blocks split over the CTA's two slots
+  kNarrow = LF_FORM_NARROW,  // one tile per CTA, two CTAs per SM
 };
 
 // One query tile per CTA, its key blocks split over the two slots:
@@ -1588,15 +1588,8 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
 
 template <int D, int MODE>
 static int launch_prefill_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                               const PrefillParams& p, int B, cudaStream_t st) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  // Plain and biased scores have the narrow form. (Rows that the producer warp copies itself need three ring
-  // stages, which it has at D = 64.)
-  constexpr bool kHasNarrow = MODE == kModeNone || MODE == kModeBias;
-  const PrefillForm form =
-      choose_form(p, D, B, device_sm_count(dev), kHasNarrow && (!p.paged || p.gather || D == 64));
-  if constexpr (kHasNarrow)
+                               const PrefillParams& p, int B, cudaStream_t st, PrefillForm form) {
+  if constexpr (MODE == kModeNone || MODE == kModeBias)  // (form_of)
     if (form == PrefillForm::kNarrow) return launch_prefill<D, MODE, false, true>(mq, mk, mv, p, B, st, form);
   return launch_prefill<D, MODE>(mq, mk, mv, p, B, st, form);
 }
@@ -1629,6 +1622,17 @@ static bool bounded_is_narrow(const PrefillParams& p, int D, int pack, int B, in
   int lo, hi;
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1, &lo, &hi);
   return n_tiles <= sm_count || hi - lo <= (few ? 16 : 10);
+}
+
+// The form of a call's kernel. Plain and biased scores have the narrow form of prefill_kernel. (Rows that the
+// producer warp copies itself need three ring stages, which it has at D = 64.)
+static PrefillForm form_of(const PrefillParams& p, int mode, bool has_pe, int D, int pack, int kv_tile, int B,
+                           int sm_count) {
+  if (mode == kModeBounded)
+    return kv_tile != kWideK && bounded_is_narrow(p, D, pack, B, sm_count) ? PrefillForm::kNarrow
+                                                                           : PrefillForm::kPairs;
+  const bool can_narrow = (mode == kModeNone || mode == kModeBias) && !has_pe && (!p.paged || p.gather || D == 64);
+  return choose_form(p, D, B, sm_count, can_narrow);
 }
 
 template <int D, int PACK = 1, bool NARROW = false>
@@ -1686,7 +1690,8 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
 template <int D>
 static int launch_prefill_bounded_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                        const CUtensorMap& mo, const PrefillParams& p, int B, cudaStream_t st,
-                                       int pack, bool narrow) {
+                                       int pack, PrefillForm form) {
+  const bool narrow = form == PrefillForm::kNarrow;
   if (pack == 4)
     return narrow ? launch_prefill_bounded<D, 4, true>(mq, mk, mv, mo, p, B, st)
                   : launch_prefill_bounded<D, 4>(mq, mk, mv, mo, p, B, st);
@@ -1755,8 +1760,15 @@ static int choose_kv_tile(const LfPrefillArgs* a, int mode) {
   return a->kv_tile != 0 ? a->kv_tile : kTileK;
 }
 
+// What a call runs, for the queries.
+struct PrefillChoice {
+  int q_tile = 0;
+  int sm_count = 0;  // in: of the device that is asked about; 0 = the current one, -1 = the form is not asked for
+  int form = 0;
+};
+
 // `launch` == nullptr: only resolve the kernel choice and return its KV tile size.
-static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile = nullptr,
+static int prefill_impl(const LfPrefillArgs* a, void* const* launch, PrefillChoice* choice = nullptr,
                         const LfRowBias* rows = nullptr) {
   if (!a || !a->q || !a->k || !a->v || !a->out) return LF_ERR_INVALID_ARG;
   if (a->B <= 0 || a->Hq <= 0 || a->Hkv <= 0 || a->Sq <= 0 || a->Skv <= 0)
@@ -1948,8 +1960,27 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   // fixed-reference kernel (128 / group query rows of each of the heads per tile slot).
   const int pack = (mode == kModeBounded && kv_tile != kWideK && (p.group == 2 || p.group == 4) &&
                     a->mask_kind == LF_MASK_CAUSAL_WINDOW) ? p.group : 1;
-  if (q_tile) *q_tile = kTileQ / pack;
-  if (launch == nullptr) return kv_tile;  // query only
+  const int64_t k_row = p.paged & 1 ? gather_row_stride(a->k_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
+  const int64_t v_row = p.paged & 2 ? gather_row_stride(a->v_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
+  p.gather = p.paged && k_row && v_row;
+  auto form_on = [&](int sm_count) {
+    return form_of(p, mode, has_pe, a->D, pack, kv_tile, a->B, sm_count);
+  };
+  int dev = 0;
+  if (launch == nullptr) {  // query only
+    if (choice) {
+      choice->q_tile = kTileQ / pack;
+      if (choice->sm_count == 0) {
+        cudaGetDevice(&dev);
+        choice->sm_count = device_sm_count(dev);
+        if (choice->sm_count <= 0) return LF_ERR_CUDA;
+      }
+      if (choice->sm_count > 0) choice->form = static_cast<int>(form_on(choice->sm_count));
+    }
+    return kv_tile;
+  }
+  cudaGetDevice(&dev);
+  const PrefillForm form = form_on(device_sm_count(dev));
 
   CUtensorMap mq, mk, mv;
   int rc = make_tile_map(&mq, a->q, a->B, a->Hq, a->Sq, a->D, a->q_stride, kTileQ / pack);
@@ -1959,9 +1990,6 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
     return make_tile_map(m, pool, 0, 0, a->n_pages * a->page_size,
                          static_cast<int>((a->Hkv - 1) * head_stride + a->D), st, 1);
   };
-  const int64_t k_row = p.paged & 1 ? gather_row_stride(a->k_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
-  const int64_t v_row = p.paged & 2 ? gather_row_stride(a->v_stride, a->n_pages, a->page_size, a->Hkv, a->D) : 1;
-  p.gather = p.paged && k_row && v_row;
   if (p.paged & 1) {
     mk = mq;  // (not used when the producer warp copies the rows of K itself)
     if (p.gather && (rc = pool_map(&mk, a->k, k_row, a->k_stride[2])) != LF_OK) return rc;
@@ -1978,13 +2006,9 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
   }
 
   CUtensorMap mo;  // output store boxes of the persistent kernels: 32 rows x 32 columns
-  bool narrow = false;
   if (mode == kModeBounded) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    narrow = kv_tile != kWideK && bounded_is_narrow(p, a->D, pack, a->B, device_sm_count(dev));
     rc = make_tile_map(&mo, a->out, a->B, a->Hq, a->Sq, a->D, a->o_stride, 32,
-                       (pack > 1 && a->D == 128 && !narrow) ? 64 : 32);
+                       (pack > 1 && a->D == 128 && form != PrefillForm::kNarrow) ? 64 : 32);
     if (rc != LF_OK) return rc;
   }
 
@@ -1996,31 +2020,28 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, int* q_tile
     if (rc != LF_OK) return rc;
     rc = make_tile_map(&mkpe, a->k_pe, a->B, a->Hkv, a->Skv, a->D_pe, a->kpe_stride, kTileK);
     if (rc != LF_OK) return rc;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const PrefillForm form = choose_form(p, a->D, a->B, device_sm_count(dev), false);
     if (a->D == 128)
       return launch_prefill<128, kModeNone, true>(mq, mk, mv, p, a->B, st, form, &mqpe, &mkpe);
     return launch_prefill<64, kModeNone, true>(mq, mk, mv, p, a->B, st, form, &mqpe, &mkpe);
   }
   if (a->D == 128) {
-    if (mode == kModeNone) return launch_prefill_form<128, kModeNone>(mq, mk, mv, p, a->B, st);
-    if (mode == kModeSoftcap) return launch_prefill_form<128, kModeSoftcap>(mq, mk, mv, p, a->B, st);
+    if (mode == kModeNone) return launch_prefill_form<128, kModeNone>(mq, mk, mv, p, a->B, st, form);
+    if (mode == kModeSoftcap) return launch_prefill_form<128, kModeSoftcap>(mq, mk, mv, p, a->B, st, form);
     if (mode == kModeBounded)
       return kv_tile == kWideK
                ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st)
-               : launch_prefill_bounded_form<128>(mq, mk, mv, mo, p, a->B, st, pack, narrow);
-    if (mode == kModeBias) return launch_prefill_form<128, kModeBias>(mq, mk, mv, p, a->B, st);
-    return launch_prefill_form<128, kModeGeneric>(mq, mk, mv, p, a->B, st);
+               : launch_prefill_bounded_form<128>(mq, mk, mv, mo, p, a->B, st, pack, form);
+    if (mode == kModeBias) return launch_prefill_form<128, kModeBias>(mq, mk, mv, p, a->B, st, form);
+    return launch_prefill_form<128, kModeGeneric>(mq, mk, mv, p, a->B, st, form);
   }
-  if (mode == kModeNone) return launch_prefill_form<64, kModeNone>(mq, mk, mv, p, a->B, st);
-  if (mode == kModeSoftcap) return launch_prefill_form<64, kModeSoftcap>(mq, mk, mv, p, a->B, st);
+  if (mode == kModeNone) return launch_prefill_form<64, kModeNone>(mq, mk, mv, p, a->B, st, form);
+  if (mode == kModeSoftcap) return launch_prefill_form<64, kModeSoftcap>(mq, mk, mv, p, a->B, st, form);
   if (mode == kModeBounded)
     return kv_tile == kWideK
                ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st)
-               : launch_prefill_bounded_form<64>(mq, mk, mv, mo, p, a->B, st, pack, narrow);
-  if (mode == kModeBias) return launch_prefill_form<64, kModeBias>(mq, mk, mv, p, a->B, st);
-  return launch_prefill_form<64, kModeGeneric>(mq, mk, mv, p, a->B, st);
+               : launch_prefill_bounded_form<64>(mq, mk, mv, mo, p, a->B, st, pack, form);
+  if (mode == kModeBias) return launch_prefill_form<64, kModeBias>(mq, mk, mv, p, a->B, st, form);
+  return launch_prefill_form<64, kModeGeneric>(mq, mk, mv, p, a->B, st, form);
 }
 
 }  // namespace lf
@@ -2039,9 +2060,18 @@ int lf_prefill_row_bias_bf16(const LfPrefillArgs* args, const LfRowBias* rows, v
 int lf_prefill_kv_tile(const LfPrefillArgs* args) { return lf::prefill_impl(args, nullptr); }
 
 int lf_prefill_q_tile(const LfPrefillArgs* args) {
-  int q_tile = 0;
-  const int rc = lf::prefill_impl(args, nullptr, &q_tile);
-  return rc < 0 ? rc : q_tile;
+  lf::PrefillChoice choice;
+  choice.sm_count = -1;
+  const int rc = lf::prefill_impl(args, nullptr, &choice);
+  return rc < 0 ? rc : choice.q_tile;
+}
+
+int lf_prefill_form(const LfPrefillArgs* args, int32_t sm_count) {
+  if (sm_count < 0) return LF_ERR_INVALID_ARG;
+  lf::PrefillChoice choice;
+  choice.sm_count = sm_count;
+  const int rc = lf::prefill_impl(args, nullptr, &choice);
+  return rc < 0 ? rc : choice.form;
 }
 
 void lf_tile_map_cache_stats(uint64_t* hits, uint64_t* misses) {

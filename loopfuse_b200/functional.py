@@ -173,6 +173,30 @@ def prefill_q_tile(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: 
     return rc
 
 
+PREFILL_FORMS = ("pairs", "split", "narrow")
+
+
+def prefill_form(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: float = 1.0,
+                 mods: Sequence[ScoreMod] = (), mask_kind: int = MASK_NONE, window: int = 0,
+                 causal_offset: int = 0, kv_tile: int = 0, sm_margin: int = 0,
+                 k_block_table: Optional[torch.Tensor] = None,
+                 v_block_table: Optional[torch.Tensor] = None, seq_len: Optional[int] = None,
+                 score_bias: Optional[torch.Tensor] = None, bias_pos: Optional[int] = None,
+                 q_pe: Optional[torch.Tensor] = None,
+                 k_pe: Optional[torch.Tensor] = None) -> str:
+    """How the kernel that ``prefill_attention`` runs for these arguments deals the query tiles
+    out: ``"pairs"`` (a CTA of two tiles per SM), ``"split"`` (one tile on a CTA's two slots) or
+    ``"narrow"`` (two CTAs of one tile per SM). (Row biases do not change it.)"""
+    rec, _, _ = _native.host().prefill_record(
+        q, k, v, q, None, None, k_block_table, v_block_table, score_bias, q_pe, k_pe, scale, mods,
+        mask_kind, window, causal_offset, kv_tile, sm_margin, seq_len, bias_pos)
+    a = _native.LfPrefillArgs.from_buffer_copy(rec)
+    rc = _native.load().lf_prefill_form(C.byref(a), 0)
+    if rc < 0:
+        _native.check(rc, "lf_prefill_form")
+    return PREFILL_FORMS[rc]
+
+
 def _prefill_record(q, k, v, scale, mods, mask_kind, window, causal_offset, out, status, kv_tile,
                     sm_margin):
     """(LfPrefillArgs, out) of a dense prefill, checked and filled but not launched."""

@@ -75,6 +75,33 @@ CHILD = textwrap.dedent("""
             if "out_bias" in b: want = want + b["out_bias"].float()
             # (the sum with the output bias is rounded once more: half a bf16 step)
             assert ((out.float().cpu() - want).abs() <= TOL + want.abs() / 256).all(), (S, rows)
+    # Forms that only larger grids take: two CTAs per SM, plain, biased (with row biases) and paged; pairs.
+    for D in (64, 128):
+        B, H, S = 2, 100, 213
+        q, k, v = (torch.randn(B, H, S, D, device="cuda").bfloat16() for _ in range(3))
+        qb, ob = (torch.randn(B, H, S, D, device="cuda").bfloat16() for _ in range(2))
+        sb = torch.randn(B, H, S, 216, device="cuda").bfloat16()[..., :S]
+        blocks = -(-S // 16)
+        pool = torch.randn(B * blocks + 1, 16, H, D, device="cuda").bfloat16()
+        table = torch.randperm(B * blocks + 1, device="cuda")[:B * blocks].view(B, blocks).int()
+        kk = pool[table.long()].reshape(B, blocks * 16, H, D)[:, :S].transpose(1, 2)
+        kw = dict(scale=D ** -0.5, mask_kind=SP.MASK_CAUSAL)
+        for h, form in ((H, "narrow"), (40, "pairs")):   # (all heads, and a few)
+            cut = lambda t: t[:, :h]
+            if D == 64 and form == "pairs": continue
+            for name, key, extra in (("plain", k, {}), ("biased", k, dict(score_bias=cut(sb))),
+                                     ("paged", kk, dict(k_block_table=table, seq_len=S))):
+                args = (cut(q), pool[:, :, :h] if name == "paged" else cut(key), cut(v))
+                if name != "paged": assert F.prefill_form(*args, **extra, **kw) == form, (D, h, name)
+                more = dict(q_bias=cut(qb), out_bias=cut(ob)) if name == "biased" else {}
+                out = F.prefill_attention(*args, status=st, **extra, **more, **kw)
+                qq = cut(q + qb) if more else cut(q)
+                s = qq.float() @ cut(key).float().transpose(-2, -1) * D ** -0.5
+                s = s + cut(sb).float() if name == "biased" else s
+                s = s.masked_fill(torch.ones_like(s).triu(1) > 0, float("-inf"))
+                want = torch.softmax(s, dim=-1) @ cut(v).float()
+                want = want + cut(ob).float() if more else want
+                assert ((out.float() - want).abs() <= TOL + want.abs() / 256).all(), (D, h, name)
     torch.cuda.synchronize()
     assert int(st.item()) == 0, hex(int(st.item()))
     print("debug-bounds cases ok")

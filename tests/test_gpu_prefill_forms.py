@@ -32,9 +32,11 @@ def _by_heads(fn, q, *per_head, chunk):
     return torch.cat(parts, dim=1)
 
 
-def _fp32(q, k, v, mask, off, window=0):
+def _fp32(q, k, v, mask, off, window=0, scale=None, bias=None):
     k, v = (t.float().repeat_interleave(q.shape[1] // k.shape[1], dim=1) for t in (k, v))
-    s = q.float() @ k.transpose(-2, -1) * q.shape[-1] ** -0.5
+    s = q.float() @ k.transpose(-2, -1) * (scale or q.shape[-1] ** -0.5)
+    if bias is not None:
+        s = s + bias.float()
     i = torch.arange(q.shape[2], device="cuda")[:, None] + off
     j = torch.arange(k.shape[2], device="cuda")[None]
     if mask != S.MASK_NONE:
@@ -49,26 +51,42 @@ def _fp32(q, k, v, mask, off, window=0):
     (2, 152, 38, 1, 1, S.MASK_CAUSAL, 0, 0),          # one tile per head, one row
     (3, 104, 52, 128, 65, S.MASK_NONE, 0, 0),
     (5, 60, 20, 129, 129, S.MASK_CAUSAL, 0, 0),       # a last tile of one row
-    (2, 52, 13, 300, 1100, S.MASK_CAUSAL, 800, 0),    # three tiles a head, a chunk
+    (3, 52, 13, 300, 1100, S.MASK_CAUSAL, 800, 0),    # three tiles a head, a chunk
+    (1, 304, 38, 100, 2100, S.MASK_CAUSAL, 2000, 0),  # one tile a head, long rows
     (3, 52, 26, 257, 200, S.MASK_CAUSAL, -60, 0),     # rows without a key
     (2, 76, 19, 250, 250, S.MASK_CAUSAL_WINDOW, 0, 70),
     (2, 40, 10, 520, 520, S.MASK_CAUSAL, 0, 0),
 ])
 def test_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, D):
-    assert -(-Sq // 128) * Hq * B > 2 * torch.cuda.get_device_properties(0).multi_processor_count
     torch.manual_seed(1)
     # Heads inside the rows, and K and V in one tensor: strides of a packed projection.
     q = torch.randn(B, Sq, Hq, D, device="cuda").bfloat16().transpose(1, 2)
     kv = torch.randn(B, Skv, 2 * Hkv, D, device="cuda").bfloat16().transpose(1, 2)
     k, v = kv[:, :Hkv], kv[:, Hkv:]
     st = F.new_status("cuda")
-    call = lambda q, k, v: F.prefill_attention(q, k, v, scale=D ** -0.5, mask_kind=mask, window=window,
-                                               causal_offset=off, status=st)
+    kw = dict(scale=D ** -0.5, mask_kind=mask, window=window, causal_offset=off)
+    assert F.prefill_form(q, k, v, **kw) == "narrow"
+    call = lambda q, k, v: F.prefill_attention(q, k, v, status=st, **kw)
     out = call(q, k, v)
     F.check_status(st)
     _close(out, _fp32(q, k, v, mask, off, window))
     _close(out, _by_heads(call, q, k, v, chunk=Hq // Hkv))
     assert torch.equal(out.nan_to_num(), call(q, k, v).nan_to_num())
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv", [(1, 80, 10, 520, 520), (1, 64, 8, 700, 1400)])
+def test_pairs_and_two_ctas_per_sm_give_the_same_bits(B, Hq, Hkv, Sq, Skv):
+    """Half of the heads run as pairs, all of them as two CTAs per SM: the same steps for every tile."""
+    torch.manual_seed(5)
+    q = torch.randn(B, Hq, Sq, 128, device="cuda").bfloat16()
+    k, v = (torch.randn(B, Hkv, Skv, 128, device="cuda").bfloat16() for _ in range(2))
+    kw = dict(scale=128 ** -0.5, mask_kind=S.MASK_CAUSAL, causal_offset=Skv - Sq)
+    assert F.prefill_form(q, k, v, **kw) == "narrow"
+    out = F.prefill_attention(q, k, v, **kw)
+    for i in range(2):
+        half = (q[:, i * Hq // 2:(i + 1) * Hq // 2], *(t[:, i * Hkv // 2:(i + 1) * Hkv // 2] for t in (k, v)))
+        assert F.prefill_form(*half, **kw) == "pairs"
+        assert torch.equal(out[:, i * Hq // 2:(i + 1) * Hq // 2], F.prefill_attention(*half, **kw))
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -78,33 +96,45 @@ def test_two_ctas_per_sm_with_biases(B, H, Sq, Skv, pad, D):
     mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()
     q, k, v, qb, ob = mk(B, H, Sq, D), mk(B, H, Skv, D), mk(B, H, Skv, D), mk(B, H, Sq, D), mk(B, H, Sq, D)
     bias = mk(B, H, Sq, (Skv + 7) // 8 * 8 + pad)[..., :Skv]
-    call = lambda q, k, v, bias, qb, ob: F.prefill_attention(
-        q, k, v, scale=D ** -0.5, mods=[S.ScoreMod(S.MOD_MUL, 2.0)], mask_kind=S.MASK_CAUSAL, score_bias=bias,
-        q_bias=qb, out_bias=ob)
+    kw = dict(scale=D ** -0.5, mods=[S.ScoreMod(S.MOD_MUL, 2.0)], mask_kind=S.MASK_CAUSAL)
+    assert F.prefill_form(q, k, v, score_bias=bias, **kw) == "narrow"
+    call = lambda q, k, v, bias, qb, ob: F.prefill_attention(q, k, v, score_bias=bias, q_bias=qb, out_bias=ob, **kw)
     out = call(q, k, v, bias, qb, ob)
     few = _by_heads(call, q, k, v, bias, qb, ob, chunk=2)
     _close(out.float() - ob.float(), few.float() - ob.float())
+    # (the sum with the output bias is rounded once more: half a bf16 step of it)
+    want = _fp32(q + qb, k, v, S.MASK_CAUSAL, 0, scale=2 * D ** -0.5, bias=bias)
+    assert ((out.float() - (want + ob.float())).abs() <= MAX_ABS + (want + ob.float()).abs() / 256).all()
 
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("P,heads_first", [(1, False), (16, False), (16, True)])
-def test_two_ctas_per_sm_paged(P, heads_first, D):
-    """Row gathers, and pools whose rows the producer warp copies itself."""
+@pytest.mark.parametrize("which,Sq,Skv", [("k", 330, 330), ("v", 330, 330), ("kv", 250, 700)])
+def test_two_ctas_per_sm_paged(which, Sq, Skv, P, heads_first, D):
+    """Row gathers (more than one window of eight tiles among them), and pools whose rows the producer warp
+    copies itself, which has the two-CTA form at D = 64 only."""
     torch.manual_seed(3)
-    B, Hkv, G, Sq, Skv = 4, 8, 4, 330, 330
+    B, Hkv, G = 4, 8, 4
     blocks = -(-Skv // P)
     shape = (B * blocks + 2, Hkv, P, D) if heads_first else (B * blocks + 2, P, Hkv, D)
-    pool = torch.randn(*shape, device="cuda").bfloat16()
-    pool = pool.transpose(1, 2) if heads_first else pool
     table = torch.randperm(B * blocks + 2, device="cuda")[:B * blocks].view(B, blocks).int()
     q = torch.randn(B, Hkv * G, Sq, D, device="cuda").bfloat16()
-    v = torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16()
+    given, dense, kw = [], [], dict(scale=D ** -0.5, mask_kind=S.MASK_CAUSAL, causal_offset=Skv - Sq, seq_len=Skv)
+    for n in "kv":
+        if n in which:
+            pool = torch.randn(*shape, device="cuda").bfloat16()
+            pool = pool.transpose(1, 2) if heads_first else pool
+            given.append(pool)
+            dense.append(pool[table.long()].reshape(B, blocks * P, Hkv, D)[:, :Skv].transpose(1, 2))
+            kw[n + "_block_table"] = table
+        else:
+            given.append(torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16())
+            dense.append(given[-1])
+    assert F.prefill_form(q, *given, **kw) == ("pairs" if heads_first and D == 128 else "narrow")
     st = F.new_status("cuda")
-    out = F.prefill_attention(q, pool, v, scale=D ** -0.5, mask_kind=S.MASK_CAUSAL, k_block_table=table,
-                              seq_len=Skv, status=st)
+    out = F.prefill_attention(q, *given, status=st, **kw)
     F.check_status(st)
-    k = pool[table.long()].reshape(B, blocks * P, Hkv, D)[:, :Skv].transpose(1, 2)
-    _close(out, _fp32(q, k, v, S.MASK_CAUSAL, 0))
+    _close(out, _fp32(q, *dense, S.MASK_CAUSAL, Skv - Sq))
 
 
 SOFTCAP = [S.ScoreMod(S.MOD_DIV, 30.0), S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_MUL, 30.0)]
@@ -129,9 +159,11 @@ def test_softcap_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, gain, D
     q = (torch.randn(B, Sq, Hq, D, device="cuda") * gain).bfloat16().transpose(1, 2)
     k, v = (torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16() for _ in range(2))
     st = F.new_status("cuda")
-    kw = dict(scale=D ** -0.5, mods=SOFTCAP, mask_kind=mask, window=window, causal_offset=off, status=st)
-    out = F.prefill_attention(q, k, v, **kw)
-    _close(out, F.prefill_attention(q, k, v, sm_margin=1, **kw))
+    kw = dict(scale=D ** -0.5, mods=SOFTCAP, mask_kind=mask, window=window, causal_offset=off)
+    assert F.prefill_form(q, k, v, **kw) == "narrow"
+    assert F.prefill_form(q, k, v, sm_margin=1, **kw) == "pairs"
+    out = F.prefill_attention(q, k, v, status=st, **kw)
+    _close(out, F.prefill_attention(q, k, v, sm_margin=1, status=st, **kw))
     F.check_status(st)
     group = Hq // Hkv
     s = q.float() @ k.float().repeat_interleave(group, 1).transpose(-2, -1) * D ** -0.5
@@ -142,3 +174,37 @@ def test_softcap_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, gain, D
     if mask == S.MASK_CAUSAL_WINDOW:
         s = s.masked_fill(j <= i - window, float("-inf"))
     _close(out, torch.softmax(s, -1) @ v.float().repeat_interleave(group, 1))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,mask,window", [
+    (2, 38, 38, 1100, S.MASK_CAUSAL, 0),               # nine tiles a head: the last one without a partner
+    (3, 32, 16, 700, S.MASK_CAUSAL_WINDOW, 200),       # packed: two heads a tile, an odd number of chunks
+    (3, 32, 16, 705, S.MASK_CAUSAL_WINDOW, 200),       # ... an even one
+    (3, 40, 10, 1000, S.MASK_CAUSAL_WINDOW, 257),      # four heads a tile, even
+    (3, 40, 10, 990, S.MASK_CAUSAL_WINDOW, 700),       # odd
+    (3, 40, 10, 950, S.MASK_CAUSAL_WINDOW, 1),
+])
+def test_softcap_both_forms_with_many_items(B, Hq, Hkv, Sq, mask, window, D):
+    """Both forms of the persistent kernel with more items than CTAs and several blocks an item: the hand-over
+    between items, tiles without a partner, and the key blocks that each tile visits."""
+    torch.manual_seed(6)
+    q = (torch.randn(B, Hq, Sq, D, device="cuda") * 2).bfloat16()
+    k, v = (torch.randn(B, Hkv, Sq, D, device="cuda").bfloat16() for _ in range(2))
+    kw = dict(scale=D ** -0.5, mods=SOFTCAP, mask_kind=mask, window=window)
+    rows = F.prefill_q_tile(q, k, v, **kw)
+    n = -(-Sq // rows)
+    s = q.float() @ k.float().repeat_interleave(Hq // Hkv, 1).transpose(-2, -1) * D ** -0.5
+    s = torch.tanh(s / 30.0) * 30.0
+    i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Sq, device="cuda")[None]
+    s = s.masked_fill((j > i) | ((j <= i - window) if window else (j > i)), float("-inf"))
+    want = torch.softmax(s, -1) @ v.float().repeat_interleave(Hq // Hkv, 1)
+    table = torch.tensor(S.skip_table(mask, window, 0, Sq, Sq, tile_q=rows))
+    for margin in (0, 1, 100):
+        dbg = torch.full((B * Hq * n * 2,), -1, dtype=torch.int32, device="cuda")
+        st = F.new_status("cuda")
+        out = F.prefill_attention(q, k, v, sm_margin=margin, dbg_ranges=dbg, status=st, **kw)
+        F.check_status(st)
+        _close(out, want)
+        assert (dbg.view(B * Hq, n, 2).cpu() == table).all()
+    assert F.prefill_form(q, k, v, sm_margin=1, **kw) == "pairs"

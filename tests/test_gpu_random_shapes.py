@@ -39,13 +39,14 @@ def test_random_prefill_shapes():
         softcap = rnd.random() < 0.7
         q, k, v = mk(B, Hkv * G, Sq, D), mk(B, Hkv, Skv, D), mk(B, Hkv, Skv, D)
         kind = {"window": S.MASK_CAUSAL_WINDOW, "causal": S.MASK_CAUSAL, "none": S.MASK_NONE}[mask]
-        out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
-                                  mods=SOFTCAP if softcap else [], mask_kind=kind, window=W,
-                                  causal_offset=Skv - Sq, status=st)
         want = O.attention_ref(q, k, v, mods=O.softcap_mods(50.0) if softcap else [], mask=mask,
                                window=W, offset=Skv - Sq, batch_chunk=B)
-        assert _close_with_nan(out, want), dict(D=D, G=G, Hkv=Hkv, B=B, Sq=Sq, Skv=Skv, W=W,
-                                                mask=mask, softcap=softcap)
+        for margin in (0, 1):  # (both forms of the persistent kernel)
+            out = F.prefill_attention(q.cuda(), k.cuda(), v.cuda(), scale=D ** -0.5,
+                                      mods=SOFTCAP if softcap else [], mask_kind=kind, window=W,
+                                      causal_offset=Skv - Sq, status=st, sm_margin=margin)
+            assert _close_with_nan(out, want), dict(D=D, G=G, Hkv=Hkv, B=B, Sq=Sq, Skv=Skv, W=W,
+                                                    mask=mask, softcap=softcap, margin=margin)
     F.check_status(st)
 
 

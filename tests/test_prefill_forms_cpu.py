@@ -1,9 +1,10 @@
 """The forms of the prefill kernels, as far as they can be checked without a GPU."""
+import ctypes as C
 import re
 
 import pytest
 
-from loopfuse_b200 import build as B
+from loopfuse_b200 import _native, build as B, spec as S
 
 
 def test_registers_change_hands_once_per_warpgroup():
@@ -29,3 +30,64 @@ def test_registers_change_hands_once_per_warpgroup():
         assert len(forms) == 4
         for spill, regs in forms:
             assert 4 * few + 4 * many <= 8 * int(regs) and int(regs) * 512 <= 65536
+
+
+PAIRS, SPLIT, NARROW = range(3)
+SOFTCAP = [(S.MOD_DIV, 50.0), (S.MOD_TANH, 0.0), (S.MOD_MUL, 50.0)]
+
+
+def call(B, Hq, Hkv, Sq, Skv, D, *, mask=S.MASK_CAUSAL, window=0, off=None, softcap=False, bias=False, page=0,
+         margin=0, kv_tile=0):
+    """The arguments of a prefill on made-up addresses, for what only looks at them."""
+    a = _native.LfPrefillArgs()
+    a.q = a.k = a.v = a.out = 0x1000
+    a.B, a.Hq, a.Hkv, a.Sq, a.Skv, a.D = B, Hq, Hkv, Sq, Skv, D
+    for i, (s, t) in enumerate(((Hq * Sq * D, Hkv * Skv * D), (Sq * D, Skv * D), (D, D))):
+        a.q_stride[i] = a.o_stride[i] = s
+        a.k_stride[i] = a.v_stride[i] = t
+    a.scale, a.mask_kind, a.window = D ** -0.5, mask, window
+    a.causal_offset = Skv - Sq if off is None else off
+    a.sm_margin, a.kv_tile = margin, kv_tile
+    if softcap:
+        a.n_mod = len(SOFTCAP)
+        for i, (op, arg) in enumerate(SOFTCAP):
+            a.mod_op[i], a.mod_arg[i] = op, arg
+    if bias:
+        a.score_bias = 0x1000
+        row = (Skv + 7) // 8 * 8
+        for i, s in enumerate((Hq * Sq * row, Sq * row, row)):
+            a.bias_stride[i] = s
+    if page:
+        a.k_block_table = 0x1000
+        a.page_size, a.n_pages, a.bt_stride = page, B * -(-Skv // page), -(-Skv // page)
+        for i, s in enumerate((page * Hkv * D, Hkv * D, D)):
+            a.k_stride[i] = s
+    return a
+
+
+def form(lib, *args, sms=148, **kw):
+    return lib.lf_prefill_form(C.byref(call(*args, **kw)), sms)
+
+
+def test_form_query(native_lib):
+    """The query answers for any number of SMs without a device, by the same rules as a call."""
+    ask = lambda *a, **kw: form(native_lib, *a, **kw)
+    assert ask(4, 8, 8, 593, 593, 64) == ask(4, 8, 8, 593, 593, 128) == SPLIT      # 160 tiles
+    assert ask(1, 8, 8, 512, 512, 64) == SPLIT                                     # fewer than SMs
+    assert ask(8, 32, 32, 2048, 2048, 64) == NARROW
+    assert ask(8, 32, 32, 2048, 2048, 128) == PAIRS
+    assert ask(8, 32, 8, 512, 512, 128) == NARROW
+    assert ask(8, 32, 8, 512, 512, 128, sms=4000) == SPLIT
+    assert ask(8, 32, 8, 512, 512, 128, page=16) == NARROW
+    assert ask(8, 16, 16, 512, 512, 128, bias=True) == NARROW
+    assert ask(8, 32, 32, 2048, 2048, 128, softcap=True) == PAIRS
+    assert ask(8, 32, 32, 2048, 2048, 64, softcap=True) == NARROW
+    assert ask(8, 32, 32, 2048, 2048, 64, softcap=True, margin=1) == PAIRS
+    assert ask(8, 32, 32, 2048, 2048, 64, softcap=True, kv_tile=128) == PAIRS
+    assert ask(8, 32, 8, 2048, 2048, 128, softcap=True, mask=S.MASK_CAUSAL_WINDOW, window=256) == PAIRS
+    assert ask(1, 32, 8, 1024, 1024, 128, softcap=True, mask=S.MASK_CAUSAL_WINDOW, window=256) == NARROW
+    a = call(8, 32, 32, 2048, 2048, 128)
+    assert native_lib.lf_prefill_form(C.byref(a), -1) == -1
+    assert native_lib.lf_prefill_q_tile(C.byref(a)) == 128
+    a.D = 96
+    assert native_lib.lf_prefill_form(C.byref(a), 148) == -2
