@@ -1486,10 +1486,22 @@ static int make_tile_map(CUtensorMap* map, const void* base, int B, int H, int S
   return LF_OK;
 }
 
-static int device_sm_count(int dev) {
-  static thread_local int sm_count = 0;
-  if (sm_count == 0) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  return sm_count;
+// SMs of the current device (asked once per device); 0 after an error, which is recorded.
+static int current_sm_count() {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> counts[kMaxDevices];
+  int dev = 0, n = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev < kMaxDevices) n = counts[dev].load(std::memory_order_relaxed);
+  if (e == cudaSuccess && n == 0) {
+    e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && dev < kMaxDevices) counts[dev].store(n, std::memory_order_relaxed);
+  }
+  if (e != cudaSuccess) {
+    set_cuda_error(e, "number of SMs");
+    return 0;
+  }
+  return n;
 }
 
 // How the prefill kernels deal the query tiles out.
@@ -1638,13 +1650,12 @@ static PrefillForm form_of(const PrefillParams& p, int mode, bool has_pe, int D,
 template <int D, int PACK = 1, bool NARROW = false>
 static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
                                   const CUtensorMap& mv, const CUtensorMap& mo, PrefillParams p,
-                                  int B, cudaStream_t st) {
+                                  int B, cudaStream_t st, int sm_count) {
   using Shape = BoundedShape<D, PACK, NARROW>;
   constexpr size_t smem = Shape::kSmem;
   static_assert(smem <= 232448 && (!NARROW || 2 * (smem + 1024) <= 233472), "shared memory of a CTA");
   static thread_local int configured_dev = -1;
   static thread_local unsigned int* tickets = nullptr;
-  static thread_local int sm_count = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_dev != dev) {
@@ -1653,7 +1664,6 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
                                          static_cast<int>(smem));
     if (e == cudaSuccess)
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&tickets), g_prefill_tickets);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
       set_cuda_error(e, "prefill_bounded_kernel setup");
       return LF_ERR_CUDA;
@@ -1690,29 +1700,28 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
 template <int D>
 static int launch_prefill_bounded_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                        const CUtensorMap& mo, const PrefillParams& p, int B, cudaStream_t st,
-                                       int pack, PrefillForm form) {
+                                       int pack, PrefillForm form, int sm_count) {
   const bool narrow = form == PrefillForm::kNarrow;
   if (pack == 4)
-    return narrow ? launch_prefill_bounded<D, 4, true>(mq, mk, mv, mo, p, B, st)
-                  : launch_prefill_bounded<D, 4>(mq, mk, mv, mo, p, B, st);
+    return narrow ? launch_prefill_bounded<D, 4, true>(mq, mk, mv, mo, p, B, st, sm_count)
+                  : launch_prefill_bounded<D, 4>(mq, mk, mv, mo, p, B, st, sm_count);
   if (pack == 2)
-    return narrow ? launch_prefill_bounded<D, 2, true>(mq, mk, mv, mo, p, B, st)
-                  : launch_prefill_bounded<D, 2>(mq, mk, mv, mo, p, B, st);
-  return narrow ? launch_prefill_bounded<D, 1, true>(mq, mk, mv, mo, p, B, st)
-                : launch_prefill_bounded<D>(mq, mk, mv, mo, p, B, st);
+    return narrow ? launch_prefill_bounded<D, 2, true>(mq, mk, mv, mo, p, B, st, sm_count)
+                  : launch_prefill_bounded<D, 2>(mq, mk, mv, mo, p, B, st, sm_count);
+  return narrow ? launch_prefill_bounded<D, 1, true>(mq, mk, mv, mo, p, B, st, sm_count)
+                : launch_prefill_bounded<D>(mq, mk, mv, mo, p, B, st, sm_count);
 }
 
 template <int D>
 static int launch_prefill_wide(const CUtensorMap& mq, const CUtensorMap& mk,
                                const CUtensorMap& mv, const CUtensorMap& mo, PrefillParams p,
-                               int B, cudaStream_t st) {
+                               int B, cudaStream_t st, int sm_count) {
   constexpr size_t kQTileBytes = static_cast<size_t>(kTileQ) * D * 2;
   constexpr size_t kKVTileBytes = static_cast<size_t>(kWideK) * D * 2;
   constexpr size_t smem = 1024 /*align slack*/ + 1024 /*barriers*/ + kBoundedStageBytes +
                           2 * kQTileBytes + WideRingFor<D>::value * kKVTileBytes;
   static thread_local int configured_dev = -1;
   static thread_local unsigned int* tickets = nullptr;
-  static thread_local int sm_count = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_dev != dev) {
@@ -1721,7 +1730,6 @@ static int launch_prefill_wide(const CUtensorMap& mq, const CUtensorMap& mk,
                                          static_cast<int>(smem));
     if (e == cudaSuccess)
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&tickets), g_prefill_tickets);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
       set_cuda_error(e, "prefill_wide_kernel setup");
       return LF_ERR_CUDA;
@@ -1966,21 +1974,17 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, PrefillChoi
   auto form_on = [&](int sm_count) {
     return form_of(p, mode, has_pe, a->D, pack, kv_tile, a->B, sm_count);
   };
-  int dev = 0;
   if (launch == nullptr) {  // query only
     if (choice) {
       choice->q_tile = kTileQ / pack;
-      if (choice->sm_count == 0) {
-        cudaGetDevice(&dev);
-        choice->sm_count = device_sm_count(dev);
-        if (choice->sm_count <= 0) return LF_ERR_CUDA;
-      }
+      if (choice->sm_count == 0 && (choice->sm_count = current_sm_count()) == 0) return LF_ERR_CUDA;
       if (choice->sm_count > 0) choice->form = static_cast<int>(form_on(choice->sm_count));
     }
     return kv_tile;
   }
-  cudaGetDevice(&dev);
-  const PrefillForm form = form_on(device_sm_count(dev));
+  const int sm_count = current_sm_count();
+  if (sm_count == 0) return LF_ERR_CUDA;
+  const PrefillForm form = form_on(sm_count);
 
   CUtensorMap mq, mk, mv;
   int rc = make_tile_map(&mq, a->q, a->B, a->Hq, a->Sq, a->D, a->q_stride, kTileQ / pack);
@@ -2029,8 +2033,8 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, PrefillChoi
     if (mode == kModeSoftcap) return launch_prefill_form<128, kModeSoftcap>(mq, mk, mv, p, a->B, st, form);
     if (mode == kModeBounded)
       return kv_tile == kWideK
-               ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st)
-               : launch_prefill_bounded_form<128>(mq, mk, mv, mo, p, a->B, st, pack, form);
+               ? launch_prefill_wide<128>(mq, mk, mv, mo, p, a->B, st, sm_count)
+               : launch_prefill_bounded_form<128>(mq, mk, mv, mo, p, a->B, st, pack, form, sm_count);
     if (mode == kModeBias) return launch_prefill_form<128, kModeBias>(mq, mk, mv, p, a->B, st, form);
     return launch_prefill_form<128, kModeGeneric>(mq, mk, mv, p, a->B, st, form);
   }
@@ -2038,8 +2042,8 @@ static int prefill_impl(const LfPrefillArgs* a, void* const* launch, PrefillChoi
   if (mode == kModeSoftcap) return launch_prefill_form<64, kModeSoftcap>(mq, mk, mv, p, a->B, st, form);
   if (mode == kModeBounded)
     return kv_tile == kWideK
-               ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st)
-               : launch_prefill_bounded_form<64>(mq, mk, mv, mo, p, a->B, st, pack, form);
+               ? launch_prefill_wide<64>(mq, mk, mv, mo, p, a->B, st, sm_count)
+               : launch_prefill_bounded_form<64>(mq, mk, mv, mo, p, a->B, st, pack, form, sm_count);
   if (mode == kModeBias) return launch_prefill_form<64, kModeBias>(mq, mk, mv, p, a->B, st, form);
   return launch_prefill_form<64, kModeGeneric>(mq, mk, mv, p, a->B, st, form);
 }

@@ -1,6 +1,9 @@
 """The forms of the prefill kernels, as far as they can be checked without a GPU."""
 import ctypes as C
+import os
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -91,3 +94,35 @@ def test_form_query(native_lib):
     assert native_lib.lf_prefill_q_tile(C.byref(a)) == 128
     a.D = 96
     assert native_lib.lf_prefill_form(C.byref(a), 148) == -2
+
+
+FAKE_RUNTIME = r"""
+static int current, asked;
+extern "C" {
+void fake_set(int dev) { current = dev; }
+int fake_asked() { return asked; }
+int cudaGetDevice(int* dev) { *dev = current; return 0; }
+int cudaDeviceGetAttribute(int* value, int attribute, int dev) { ++asked; *value = dev == 0 ? 148 : 4000; return 0; }
+}
+"""
+ASK = """
+import ctypes as C, sys
+fake, lib = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL), C.CDLL(sys.argv[2])
+args = C.create_string_buffer(bytes.fromhex(sys.argv[3]))
+for dev in (0, 1, 0, 1):
+    fake.fake_set(dev)
+    print(lib.lf_prefill_form(args, 0))
+print(fake.fake_asked())
+"""
+
+
+def test_number_of_sms_is_the_current_devices(native_lib, tmp_path):
+    """Two devices of different size behind a stand-in for the CUDA runtime's two queries: each is asked once,
+    and a thread that changes device gets the form for the one it is on."""
+    shim = tmp_path / "fake.so"
+    (tmp_path / "fake.cpp").write_text(FAKE_RUNTIME)
+    subprocess.run(["g++", "-shared", "-fPIC", str(tmp_path / "fake.cpp"), "-o", str(shim)], check=True)
+    args = bytes(call(8, 32, 8, 512, 512, 128)).hex()
+    out = subprocess.run([sys.executable, "-c", ASK, str(shim), str(_native.LIB_PATH), args], check=True, text=True,
+                         capture_output=True, env=dict(os.environ, LD_PRELOAD=str(shim)))
+    assert [int(x) for x in out.stdout.split()] == [NARROW, SPLIT, NARROW, SPLIT, 2]
