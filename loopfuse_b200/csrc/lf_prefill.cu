@@ -1525,13 +1525,17 @@ enum class PrefillForm {
 // tiles, and the issuing warps of two tiles no longer wait for one ring. Back to back for half a second (causal;
 // pairs -> narrow):
 //   D = 64, any length: 8 x 32 x 512 34.1 -> 29.7 us, 4 x 16 x 2048 68.4 -> 62.5, 1 x 16 x 8192 209.8 -> 194.5; paged
-//   8 x 32 x 1024 100.4 -> 91.2, biased 8 x 16 x 512 38.2 -> 34.0; one tile a head (two slots -> narrow), 8 x 32 x 64,
-//   8.3 -> 4.4.
+//   8 x 32 x 1024 100.4 -> 91.2, biased 8 x 16 x 512 38.2 -> 34.0.
 //   D = 128 up to 24 blocks a tile: 8 x 64 x 100 22.0 -> 13.6, 8 x 32 x 640 59.1 -> 51.9, 8 x 32 x 1024 105.7 -> 101.8,
 //   4 x 32 x 1536 103.8 -> 101.7, biased 4 x 16 x 1024 69.4 -> 64.3. Further on the chip runs at its power limit and
 //   K and V read once for both tiles count for more: chunks of 1024 with 4000 keys before them 158.8 -> 160.9,
 //   1 x 32 x 8192 444.6 -> 453.7; but for three tiles a head, of whose four slots one is empty (300 rows and 4000
 //   keys, 4 x 64 heads, 235.8 -> 219.4).
+// One tile a head (split -> narrow; 128 rows): 240 tiles of 64 keys 8.5 -> 4.4, of 4096 63.2 -> 57.5; D = 128 10.2 ->
+// 5.8 and 94 -> 71; 592 tiles of 1024 keys 45.5 -> 34.4 and 67 -> 46. Between two and three tiles per SM split tiles
+// take three rounds of half the steps against two of all, which is as good for plain scores (440 tiles, D = 128: 2048
+// keys 76.9 -> 74.5, 4096 139.8 -> 142.8) and the better for biased ones, whose steps wait for their bias (320 tiles of 512
+// keys the same, 1024 56.9 -> 59.3, 2048 98.5 -> 107.0; D = 128 65.3 -> 69.6 and 112.7 -> 125.4).
 // Up to two tiles per SM narrow takes the place of pairs at D = 64 and with paged operands (777 rows and 3319 keys
 // before them, 32 heads, D = 64 58.0 -> 54.6, paged 4 x 8 x 1024 19.6 -> 18.8; D = 128, dense 65.0 -> 65.4).
 static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_count, bool can_narrow) {
@@ -1542,7 +1546,11 @@ static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_coun
   const int shortest = hi - lo;
   skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1, &lo, &hi);
   const int longest = hi - lo;
-  if (p.n_qtiles == 1) return can_narrow ? PrefillForm::kNarrow : PrefillForm::kSplit;
+  if (p.n_qtiles == 1) {
+    const bool three_rounds = n_tiles > 2ll * sm_count && n_tiles <= 3ll * sm_count;
+    const bool split = !can_narrow || (p.bias && three_rounds && longest >= 12);
+    return split ? PrefillForm::kSplit : PrefillForm::kNarrow;
+  }
   if (n_tiles <= 2ll * sm_count) {
     const double split = 0.25 * (shortest + longest) * static_cast<double>(n_tiles) / sm_count + 0.5 * shortest;
     if (split * (p.paged ? 1.4 : 1.0) + 5.0 < longest) return PrefillForm::kSplit;

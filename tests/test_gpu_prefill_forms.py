@@ -90,20 +90,24 @@ def test_pairs_and_two_ctas_per_sm_give_the_same_bits(B, Hq, Hkv, Sq, Skv):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("B,H,Sq,Skv,pad", [(3, 52, 200, 200, 0), (2, 40, 513, 260, 8), (2, 150, 40, 72, 0)])
-def test_two_ctas_per_sm_with_biases(B, H, Sq, Skv, pad, D):
+@pytest.mark.parametrize("B,H,Sq,Skv,pad,form", [
+    (3, 52, 200, 200, 0, "narrow"), (2, 40, 513, 260, 8, "narrow"), (2, 150, 40, 72, 0, "narrow"),
+    (1, 320, 60, 1000, 8, "split"),  # split tiles, more of them than SMs
+])
+def test_two_ctas_per_sm_with_biases(B, H, Sq, Skv, pad, form, D):
     torch.manual_seed(2)
     mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()
     q, k, v, qb, ob = mk(B, H, Sq, D), mk(B, H, Skv, D), mk(B, H, Skv, D), mk(B, H, Sq, D), mk(B, H, Sq, D)
     bias = mk(B, H, Sq, (Skv + 7) // 8 * 8 + pad)[..., :Skv]
-    kw = dict(scale=D ** -0.5, mods=[S.ScoreMod(S.MOD_MUL, 2.0)], mask_kind=S.MASK_CAUSAL)
-    assert F.prefill_form(q, k, v, score_bias=bias, **kw) == "narrow"
+    off = Skv - Sq if form == "split" else 0
+    kw = dict(scale=D ** -0.5, mods=[S.ScoreMod(S.MOD_MUL, 2.0)], mask_kind=S.MASK_CAUSAL, causal_offset=off)
+    assert F.prefill_form(q, k, v, score_bias=bias, **kw) == form
     call = lambda q, k, v, bias, qb, ob: F.prefill_attention(q, k, v, score_bias=bias, q_bias=qb, out_bias=ob, **kw)
     out = call(q, k, v, bias, qb, ob)
     few = _by_heads(call, q, k, v, bias, qb, ob, chunk=2)
     _close(out.float() - ob.float(), few.float() - ob.float())
     # (the sum with the output bias is rounded once more: half a bf16 step of it)
-    want = _fp32(q + qb, k, v, S.MASK_CAUSAL, 0, scale=2 * D ** -0.5, bias=bias)
+    want = _fp32(q + qb, k, v, S.MASK_CAUSAL, off, scale=2 * D ** -0.5, bias=bias)
     assert ((out.float() - (want + ob.float())).abs() <= MAX_ABS + (want + ob.float()).abs() / 256).all()
 
 

@@ -96,6 +96,18 @@ def test_form_query(native_lib):
     assert native_lib.lf_prefill_form(C.byref(a), 148) == -2
 
 
+def test_one_tile_a_head(native_lib):
+    """Narrow, but for long biased rows where split tiles take three rounds of half the steps against two."""
+    ask = lambda heads, keys, D=64, **kw: form(native_lib, 1, heads, heads, 128, keys, D, **kw)
+    for D in (64, 128):
+        assert [ask(n, 2048, D, bias=True) for n in (149, 296, 297, 444, 445, 900)] == [
+            NARROW, NARROW, SPLIT, SPLIT, NARROW, NARROW]
+        assert [ask(320, keys, D, bias=True) for keys in (64, 700, 704, 705, 8192)] == [
+            NARROW, NARROW, NARROW, SPLIT, SPLIT]
+        assert [ask(n, 2048, D) for n in (149, 320, 444, 900)] == [NARROW] * 4
+        assert ask(148, 2048, D) == SPLIT
+
+
 FAKE_RUNTIME = r"""
 static int current, asked;
 extern "C" {
