@@ -1529,8 +1529,11 @@ enum class PrefillForm {
 //   D = 128 up to 24 blocks a tile: 8 x 64 x 100 22.0 -> 13.6, 8 x 32 x 640 59.1 -> 51.9, 8 x 32 x 1024 105.7 -> 101.8,
 //   4 x 32 x 1536 103.8 -> 101.7, biased 4 x 16 x 1024 69.4 -> 64.3. Further on the chip runs at its power limit and
 //   K and V read once for both tiles count for more: chunks of 1024 with 4000 keys before them 158.8 -> 160.9,
-//   1 x 32 x 8192 444.6 -> 453.7; but for three tiles a head, of whose four slots one is empty (300 rows and 4000
-//   keys, 4 x 64 heads, 235.8 -> 219.4).
+//   1 x 32 x 8192 444.6 -> 453.7; but for heads of which pairs leave a good part of the slots empty. Three tiles a head
+//   (a quarter empty): 456 tiles of 2500 / 4200 / 8200 keys 112 -> 99, 181 -> 161, 350 -> 305, 2592 of them 0.91 to 0.92 of
+//   pairs, 444 0.90 to 1.00, but 384 of 1800 / 2500 / 4300 keys 51.8 -> 53.2, 68.4 -> 72.0, 114 -> 126 (paged, 2000:
+//   65.0 -> 69.0; of 1200 and 8300 keys 0.95 to 1.01, biased 0.93 to 0.98). Five (a sixth): 680 tiles 1.02 to 1.06 of pairs, 1280 0.91 to
+//   0.99, 2600 0.92 to 0.94. Seven: 0.95 to 1.05, nine 0.95 to 1.03, four 0.95 to 1.02.
 // One tile a head (split -> narrow; 128 rows): 240 tiles of 64 keys 8.5 -> 4.4, of 4096 63.2 -> 57.5; D = 128 10.2 ->
 // 5.8 and 94 -> 71; 592 tiles of 1024 keys 45.5 -> 34.4 and 67 -> 46. Between two and three tiles per SM split tiles
 // take three rounds of half the steps against two of all, which is as good for plain scores (440 tiles, D = 128: 2048
@@ -1556,7 +1559,13 @@ static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_coun
     if (split * (p.paged ? 1.4 : 1.0) + 5.0 < longest) return PrefillForm::kSplit;
     return can_narrow && (D == 64 || p.paged) ? PrefillForm::kNarrow : PrefillForm::kPairs;
   }
-  return can_narrow && (D == 64 || longest <= 24 || p.n_qtiles == 3) ? PrefillForm::kNarrow : PrefillForm::kPairs;
+  if (!can_narrow) return PrefillForm::kPairs;
+  if (D == 64) return PrefillForm::kNarrow;
+  // (2.2 to 3 tiles per SM: a second round of narrow CTAs that leaves most SMs half empty or empty)
+  const bool half_round = n_tiles * 10 >= sm_count * 22ll && n_tiles < 3ll * sm_count;
+  if (p.n_qtiles == 3 && half_round && longest > 20 && longest < 100 && !p.bias) return PrefillForm::kPairs;
+  const bool empty_slots = p.n_qtiles == 3 || (p.n_qtiles == 5 && n_tiles > 6ll * sm_count);
+  return longest <= 24 || empty_slots ? PrefillForm::kNarrow : PrefillForm::kPairs;
 }
 
 template <int D, int MODE, bool PE = false, bool NARROW = false>

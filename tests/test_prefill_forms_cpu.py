@@ -108,6 +108,20 @@ def test_one_tile_a_head(native_lib):
         assert ask(148, 2048, D) == SPLIT
 
 
+def test_empty_slots_of_pairs(native_lib):
+    """D = 128, past two tiles per SM: long rows take narrow only where a head has three tiles, or five and there are
+    many of them; three plain tiles a head keep pairs in between where narrow needs half a round more."""
+    ask = lambda heads, rows, keys, **kw: form(native_lib, 1, heads, heads, rows, keys, 128, **kw)
+    for kw in ({}, dict(page=16)):
+        assert [ask(h, 300, 4300, **kw) for h in (99, 108, 109, 128, 147, 148, 900)] == [NARROW] * 2 + [PAIRS] * 3 + [NARROW] * 2
+        assert [ask(128, 300, keys, **kw) for keys in (1280, 1281, 6336, 6337)] == [NARROW, PAIRS, PAIRS, NARROW]
+        assert [ask(148, 300, keys, **kw) for keys in (1280, 1281, 6336)] == [NARROW] * 3
+        assert [ask(h, 600, 4300, **kw) for h in (60, 128, 177, 178, 500)] == [PAIRS] * 3 + [NARROW] * 2
+        assert [ask(h, rows, 4300, **kw) for h in (160, 900) for rows in (200, 500, 900, 1100)] == [PAIRS] * 8
+        assert [ask(h, rows, 1500, **kw) for h in (160, 900) for rows in (200, 500, 600, 900, 1100)] == [NARROW] * 10
+    assert [ask(h, 300, 4300, bias=True) for h in (99, 128, 148)] == [NARROW] * 3
+
+
 FAKE_RUNTIME = r"""
 static int current, asked;
 extern "C" {
