@@ -1511,6 +1511,15 @@ enum class PrefillForm {
   kNarrow = LF_FORM_NARROW,  // one tile per CTA, two CTAs per SM
 };
 
+// Between one and two tiles per SM, with an SM for every pair: whether two CTAs per SM would place enough beside the
+// longest tiles to be the slower form. A pair leaves the longest tile of an odd number alone on its SM; two tiles a
+// head are no better off apart at D = 128. (From 1.2 tiles per SM on, and from 1.35 with five tiles a head or more, of
+// which the first to share an SM are very light.)
+static bool longest_tile_alone(int tiles, int64_t n_tiles, int D, int sm_count) {
+  if (tiles == 2 ? D == 64 : tiles % 2 == 0) return false;
+  return n_tiles * 20 >= sm_count * (tiles <= 3 ? 24ll : 27ll);
+}
+
 // One query tile per CTA, its key blocks split over the two slots:
 //   - where all the tiles are resident at once, one per SM: half the steps of the longest tile (8
 //     heads, 1024 queries, 8192 keys, D = 64: 111 -> 59 us);
@@ -1539,8 +1548,14 @@ enum class PrefillForm {
 // take three rounds of half the steps against two of all, which is as good for plain scores (440 tiles, D = 128: 2048
 // keys 76.9 -> 74.5, 4096 139.8 -> 142.8) and the better for biased ones, whose steps wait for their bias (320 tiles of 512
 // keys the same, 1024 56.9 -> 59.3, 2048 98.5 -> 107.0; D = 128 65.3 -> 69.6 and 112.7 -> 125.4).
-// Up to two tiles per SM narrow takes the place of pairs at D = 64 and with paged operands (777 rows and 3319 keys
-// before them, 32 heads, D = 64 58.0 -> 54.6, paged 4 x 8 x 1024 19.6 -> 18.8; D = 128, dense 65.0 -> 65.4).
+// Up to two tiles per SM (ratios are narrow / pairs):
+//   - where pairs need a second round (three tiles of 384 rows x 96 heads, D = 128 15.4 -> 10.6 us, 2000 keys 57 -> 35;
+//     D = 64 0.60 to 0.68) narrow;
+//   - D = 64 and paged operands, otherwise: narrow (777 rows and 3319 keys before them, 32 heads, 58.0 -> 54.6, paged
+//     4 x 8 x 1024 19.6 -> 18.8; 2 to 16 tiles a head 0.80 to 1.00), but for an odd number of short tiles a head: the
+//     longest has an SM to itself as a pair, where narrow has to place others beside it (180 to 216 tiles, three a head, 6 blocks 1.04 to 1.08, 15 blocks 1.04 to 1.07, 53 blocks 1.00; five a head,
+//     10 blocks 1.04; paged 1.00 to 1.07); two short paged tiles a head at D = 128 are no better (1.00 to 1.04);
+//   - D = 128, dense: pairs (777 rows and 3319 keys 65.0 -> 65.4; two tiles a head 1.01 to 1.08, three 1.02 to 1.16).
 static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_count, bool can_narrow) {
   const int64_t n_tiles = static_cast<int64_t>(p.n_qtiles) * p.Hq * B;
   if (n_tiles <= sm_count) return PrefillForm::kSplit;
@@ -1557,7 +1572,11 @@ static PrefillForm choose_form(const PrefillParams& p, int D, int B, int sm_coun
   if (n_tiles <= 2ll * sm_count) {
     const double split = 0.25 * (shortest + longest) * static_cast<double>(n_tiles) / sm_count + 0.5 * shortest;
     if (split * (p.paged ? 1.4 : 1.0) + 5.0 < longest) return PrefillForm::kSplit;
-    return can_narrow && (D == 64 || p.paged) ? PrefillForm::kNarrow : PrefillForm::kPairs;
+    if (!can_narrow) return PrefillForm::kPairs;
+    if ((p.n_qtiles + 1ll) / 2 * p.Hq * B > sm_count) return PrefillForm::kNarrow;
+    if (D == 128 && !p.paged) return PrefillForm::kPairs;
+    const bool alone = longest_tile_alone(p.n_qtiles, n_tiles, D, sm_count);
+    return alone && longest <= 20 ? PrefillForm::kPairs : PrefillForm::kNarrow;
   }
   if (!can_narrow) return PrefillForm::kPairs;
   if (D == 64) return PrefillForm::kNarrow;
@@ -1639,18 +1658,33 @@ static std::atomic<unsigned int> g_next_ticket_slot{0};
 //   8 x 64 x 256 30.7 -> 28.7, 8 x 32 x 512 41.7 -> 40.1, 8 x 16 x 600 32.8 -> 30.8; up to 16 and four tiles per SM:
 //   2 x 32 x 700 26.9 -> 24.6, 4 x 16 x 1024 36.3 -> 35.1; beyond, the chip's power limit decides and K and V read
 //   once for two tiles win (8 x 32 x 1024 107.4 -> 108.5, 8 x 32 x 2048 338.7 -> 346.6, 1 x 8 x 8192 175.1 -> 180.0);
+//   between one and two tiles per SM as in prefill_kernel: narrow where pairs need a second round (three tiles a head,
+//   294 in all, D = 128 0.78, D = 64 3000 keys 0.63), two slots where an odd number of tiles leaves the longest one alone
+//   (180 to 240 tiles, three a head 1.00 to 1.16; 200 to 240, five 1.00 to 1.12, seven 1.00 to 1.10), for seven causal tiles a head also
+//   past 148 pairs, the light ones of which then take two turns under the longest (1.03), and for two tiles a head at
+//   D = 128 (256 rows x 128 heads 12.4 against 13.1 us; 1.00 to 1.08);
 //   D = 128 packed, up to four chunks per SM (1 x 8 x 2048, window 256 14.4 -> 12.3; 2 x 16 x 2048, window 1000
 //   45.2 -> 42.8; 8 x 32 x 2048, window 256 121.3 -> 124.3).
 static bool bounded_is_narrow(const PrefillParams& p, int D, int pack, int B, int sm_count) {
   if (p.sm_margin > 0) return false;  // (two CTAs per SM would spread over the SMs to be left free)
-  if (D == 64) return true;
+  if (D == 64 && pack > 1) return true;
   const int rows = kTileQ / pack;
-  const int64_t n_tiles = static_cast<int64_t>((p.Sq + rows - 1) / rows) * (p.Hq / pack) * B;
+  const int64_t heads = static_cast<int64_t>(p.Hq / pack) * B, n_tiles = (p.Sq + rows - 1) / rows * heads;
   const bool few = n_tiles <= 4ll * sm_count;
   if (pack > 1) return few;
-  int lo, hi;
-  skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, p.n_qtiles - 1, &lo, &hi);
-  return n_tiles <= sm_count || hi - lo <= (few ? 16 : 10);
+  auto blocks = [&](int iq) {
+    int lo, hi;
+    skip_range(p.mask_kind, p.window, p.causal_offset, p.Sq, p.Skv, kTileQ, kTileK, iq, &lo, &hi);
+    return hi - lo;
+  };
+  const int longest = blocks(p.n_qtiles - 1);
+  if (p.n_qtiles > 1 && n_tiles > sm_count && n_tiles <= 2ll * sm_count) {
+    const bool light = 2 * (blocks(1) + 5) <= longest + 5;  // (a CTA's start and end count as five blocks)
+    if ((p.n_qtiles + 1ll) / 2 * heads > sm_count && !light) return true;
+    if (longest_tile_alone(p.n_qtiles, n_tiles, D, sm_count)) return false;
+  }
+  if (D == 64) return true;
+  return n_tiles <= sm_count || longest <= (few ? 16 : 10);
 }
 
 // The form of a call's kernel. Plain and biased scores have the narrow form of prefill_kernel. (Rows that the

@@ -74,13 +74,14 @@ def test_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, D):
     assert torch.equal(out.nan_to_num(), call(q, k, v).nan_to_num())
 
 
-@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv", [(1, 80, 10, 520, 520), (1, 64, 8, 700, 1400)])
-def test_pairs_and_two_ctas_per_sm_give_the_same_bits(B, Hq, Hkv, Sq, Skv):
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D", [
+    (1, 80, 10, 520, 520, 128), (1, 64, 8, 700, 1400, 128), (1, 80, 10, 520, 520, 64), (1, 136, 34, 300, 620, 64)])
+def test_pairs_and_two_ctas_per_sm_give_the_same_bits(B, Hq, Hkv, Sq, Skv, D):
     """Half of the heads run as pairs, all of them as two CTAs per SM: the same steps for every tile."""
     torch.manual_seed(5)
-    q = torch.randn(B, Hq, Sq, 128, device="cuda").bfloat16()
-    k, v = (torch.randn(B, Hkv, Skv, 128, device="cuda").bfloat16() for _ in range(2))
-    kw = dict(scale=128 ** -0.5, mask_kind=S.MASK_CAUSAL, causal_offset=Skv - Sq)
+    q = torch.randn(B, Hq, Sq, D, device="cuda").bfloat16()
+    k, v = (torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16() for _ in range(2))
+    kw = dict(scale=D ** -0.5, mask_kind=S.MASK_CAUSAL, causal_offset=Skv - Sq)
     assert F.prefill_form(q, k, v, **kw) == "narrow"
     out = F.prefill_attention(q, k, v, **kw)
     for i in range(2):
@@ -113,7 +114,7 @@ def test_two_ctas_per_sm_with_biases(B, H, Sq, Skv, pad, form, D):
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("P,heads_first", [(1, False), (16, False), (16, True)])
-@pytest.mark.parametrize("which,Sq,Skv", [("k", 330, 330), ("v", 330, 330), ("kv", 250, 700)])
+@pytest.mark.parametrize("which,Sq,Skv", [("k", 330, 330), ("v", 330, 330), ("kv", 380, 700)])
 def test_two_ctas_per_sm_paged(which, Sq, Skv, P, heads_first, D):
     """Row gathers (more than one window of eight tiles among them), and pools whose rows the producer warp
     copies itself, which has the two-CTA form at D = 64 only."""

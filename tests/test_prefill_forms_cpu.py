@@ -122,6 +122,31 @@ def test_empty_slots_of_pairs(native_lib):
     assert [ask(h, 300, 4300, bias=True) for h in (99, 128, 148)] == [NARROW] * 3
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_one_to_two_tiles_per_sm(native_lib, D):
+    """Pairs that all find an SM stay where the longest tile would lose its own; pairs that need a second round
+    do not, unless the light ones make it."""
+    ask = lambda heads, rows, keys, **kw: form(native_lib, 1, heads, heads, rows, keys, D, **kw)
+    narrow_64 = NARROW if D == 64 else PAIRS
+    # three tiles a head: 74 heads fill 148 SMs with pairs
+    assert [ask(h, 384, 384) for h in (50, 59, 60, 74, 75, 98)] == [narrow_64] * 2 + [PAIRS] * 2 + [NARROW] * 2
+    assert [ask(h, 384, 2000) for h in (50, 60, 74, 75, 98)] == [narrow_64] * 3 + [NARROW] * 2
+    assert [ask(h, 384, 1200, page=16) for h in (50, 60, 74, 75, 98)] == [NARROW, PAIRS, PAIRS, NARROW, NARROW]
+    # two, four: an SM for every pair always
+    assert [ask(h, 256, 256) for h in (75, 90, 148)] == [narrow_64] * 3
+    assert [ask(h, 256, 256, page=16) for h in (75, 90, 148)] == [NARROW] + [narrow_64] * 2
+    assert [ask(h, 512, 512, page=16) for h in (45, 74)] == [NARROW] * 2
+    assert [ask(h, 896, 1496) for h in (36, 40)] == [PAIRS if D == 128 else NARROW, NARROW]
+    # the persistent kernel
+    soft = lambda heads, rows, keys: ask(heads, rows, keys, softcap=True)
+    assert [soft(h, 384, 384) for h in (50, 59, 60, 74, 75, 98)] == [NARROW] * 2 + [PAIRS] * 2 + [NARROW] * 2
+    assert [soft(h, 384, 3384) for h in (60, 74, 75, 98)] == [PAIRS] * 2 + [NARROW] * 2
+    assert [soft(h, 256, 256) for h in (75, 90, 148)] == [NARROW] + [narrow_64] * 2
+    assert [soft(h, 512, 512) for h in (45, 74)] == [NARROW] * 2
+    # (seven, causal: the light pairs of 40 heads fit behind the long ones, with more keys in front they do not)
+    assert [soft(40, 896, 896 + more) for more in (0, 600)] == [PAIRS, NARROW]
+
+
 FAKE_RUNTIME = r"""
 static int current, asked;
 extern "C" {
