@@ -1658,6 +1658,9 @@ static std::atomic<unsigned int> g_next_ticket_slot{0};
 //   8 x 64 x 256 30.7 -> 28.7, 8 x 32 x 512 41.7 -> 40.1, 8 x 16 x 600 32.8 -> 30.8; up to 16 and four tiles per SM:
 //   2 x 32 x 700 26.9 -> 24.6, 4 x 16 x 1024 36.3 -> 35.1; beyond, the chip's power limit decides and K and V read
 //   once for two tiles win (8 x 32 x 1024 107.4 -> 108.5, 8 x 32 x 2048 338.7 -> 346.6, 1 x 8 x 8192 175.1 -> 180.0);
+//   ... unless a head has one tile: it then has an SM to itself in either form, and the deeper ring of the two-slot
+//   form holds its keys' latency better (8 to 148 tiles of 1000 keys 18.5 -> 19.3 to 22.6 -> 24.7, of 4000 52 -> 63, 148 of
+//   8000 117 -> 146);
 //   between one and two tiles per SM as in prefill_kernel: narrow where pairs need a second round (three tiles a head,
 //   294 in all, D = 128 0.78, D = 64 3000 keys 0.63), two slots where an odd number of tiles leaves the longest one alone
 //   (180 to 240 tiles, three a head 1.00 to 1.16; 200 to 240, five 1.00 to 1.12, seven 1.00 to 1.10), for seven causal tiles a head also
@@ -1684,6 +1687,7 @@ static bool bounded_is_narrow(const PrefillParams& p, int D, int pack, int B, in
     if (longest_tile_alone(p.n_qtiles, n_tiles, D, sm_count)) return false;
   }
   if (D == 64) return true;
+  if (p.n_qtiles == 1 && n_tiles <= sm_count) return false;
   return n_tiles <= sm_count || longest <= (few ? 16 : 10);
 }
 

@@ -165,7 +165,8 @@ def test_softcap_two_ctas_per_sm(B, Hq, Hkv, Sq, Skv, mask, off, window, gain, D
     k, v = (torch.randn(B, Hkv, Skv, D, device="cuda").bfloat16() for _ in range(2))
     st = F.new_status("cuda")
     kw = dict(scale=D ** -0.5, mods=SOFTCAP, mask_kind=mask, window=window, causal_offset=off)
-    assert F.prefill_form(q, k, v, **kw) == "narrow"
+    lone = D == 128 and Sq == 1  # (one tile a head and an SM for each)
+    assert F.prefill_form(q, k, v, **kw) == ("pairs" if lone else "narrow")
     assert F.prefill_form(q, k, v, sm_margin=1, **kw) == "pairs"
     out = F.prefill_attention(q, k, v, status=st, **kw)
     _close(out, F.prefill_attention(q, k, v, sm_margin=1, status=st, **kw))

@@ -147,6 +147,15 @@ def test_one_to_two_tiles_per_sm(native_lib, D):
     assert [soft(40, 896, 896 + more) for more in (0, 600)] == [PAIRS, NARROW]
 
 
+def test_softcap_tiles_with_an_sm_each(native_lib):
+    """Where a head has one tile, both forms give it an SM: the one with the deeper ring."""
+    ask = lambda heads, rows, keys, D: form(native_lib, 1, heads, heads, rows, keys, D, softcap=True)
+    assert [ask(h, 100, keys, 128) for h in (1, 148) for keys in (100, 1000, 8000)] == [PAIRS] * 6
+    assert [ask(149, 100, keys, 128) for keys in (100, 600)] == [NARROW] * 2
+    assert [ask(h, 100, 1000, 64) for h in (1, 148, 149)] == [NARROW] * 3
+    assert [ask(h, 256, 1000, 128) for h in (1, 74)] == [NARROW] * 2
+
+
 FAKE_RUNTIME = r"""
 static int current, asked;
 extern "C" {
