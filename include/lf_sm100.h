@@ -235,7 +235,9 @@ const char* lf_last_cuda_error(void);
  * persistent kernel on one stream (or ordered), or every 256th eager launch could share the
  * replay's counter and lose work items. The first call of each kernel variant (head dim,
  * score-function mode) on a host thread sets kernel attributes and looks up symbol addresses:
- * make it outside stream capture, from the thread that will capture. */
+ * make it outside stream capture, from the thread that will capture. (The forms of
+ * lf_prefill_form are variants too, and a call of another size can be the first of its form:
+ * such a first call has worked inside captures, CUDA 12.9.) */
 int lf_prefill_bf16(const LfPrefillArgs* args, void* stream);
 /* lf_prefill_bf16 with row biases, in the same launch. Only where a score bias with nothing but
  * multipliers in front of it goes through the biased kernel; LF_ERR_UNSUPPORTED otherwise, and

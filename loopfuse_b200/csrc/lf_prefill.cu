@@ -53,8 +53,9 @@ constexpr int kPrefillThreads = 12 * 32;  // 8 softmax, 1 producer, 2 MMA-issuer
 constexpr int kMaxStages = 16;
 constexpr uint32_t kStageBytesTotal = 8 * 2048;
 // K/V ring depth in stages of two 64-key tiles: 4 x 32 KB at D=128, 8 x 16 KB at D=64 (which
-// also keeps the CTA above half of the shared memory, so two CTAs never compete for the 512
-// tensor-memory columns).
+// also keeps the CTA above half of the shared memory, so that two CTAs never compete for the 512
+// tensor-memory columns). The narrow forms take 256 columns and less than half of the shared memory, but more
+// than a third: two of them fit an SM, a third does not, nor one of them beside a CTA of the other forms.
 template <int D>
 struct StagesFor {
   static constexpr int value = D == 64 ? 8 : 4;
@@ -171,6 +172,11 @@ struct __align__(8) PrefillBarriers {
 
 __device__ __forceinline__ void report_timeout(int32_t* status, int where) {
   if (status) atomicCAS(status, LF_DEV_OK, LF_DEV_TIMEOUT | (where << 8));
+}
+
+// An SM's 512 columns, by shared memory: never three narrow CTAs, nor one (of 96256 bytes at least) beside another form's.
+constexpr bool keeps_tensor_memory(size_t smem, bool narrow) {
+  return narrow ? smem >= 96256 && 3 * (smem + 1024) > 233472 : smem + 1024 + 96256 + 1024 > 233472;
 }
 
 // `PE`: scores are the sum of two products, Q K^T + Q_pe K_pe^T (the two-matmul form of the
@@ -1130,8 +1136,8 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
 
           // Pass 2: p = exp2(score * c2 - m). Plain fp32 instructions and every exp2 on MUFU: a packed
           // f32x2 multiply-add in front of exp2 made the plain pass slower (1 x 32 x 8192, D = 128, 853 ->
-          // 896 thousand clocks; the long polynomials of the fixed-reference kernel gain by it), and so did
-          // an FMA-pipe emulation of part of the exp2.
+          // 896 thousand clocks; the short polynomial of the fixed-reference kernel, three of them per pair, gains by
+          // it), and so did an FMA-pipe emulation of part of the exp2.
           const float neg_m = -m_safe;
           float ps[4] = {0.f, 0.f, 0.f, 0.f};
           uint32_t pk[32];
@@ -1531,12 +1537,13 @@ static bool longest_tile_alone(int tiles, int64_t n_tiles, int D, int sm_count) 
 //     paged operand a step of split tiles gathers twice the rows: 1.4 steps.
 // Two CTAs per SM (`can_narrow`: the kernel has that form): the start and end of a CTA, some 13 thousand clocks
 // that pairs leave bare, lie under the other one's blocks, no slot is empty where a head has an odd number of
-// tiles, and the issuing warps of two tiles no longer wait for one ring. Back to back for half a second (causal;
-// pairs -> narrow):
-//   D = 64, any length: 8 x 32 x 512 34.1 -> 29.7 us, 4 x 16 x 2048 68.4 -> 62.5, 1 x 16 x 8192 209.8 -> 194.5; paged
-//   8 x 32 x 1024 100.4 -> 91.2, biased 8 x 16 x 512 38.2 -> 34.0.
-//   D = 128 up to 24 blocks a tile: 8 x 64 x 100 22.0 -> 13.6, 8 x 32 x 640 59.1 -> 51.9, 8 x 32 x 1024 105.7 -> 101.8,
-//   4 x 32 x 1536 103.8 -> 101.7, biased 4 x 16 x 1024 69.4 -> 64.3. Further on the chip runs at its power limit and
+// tiles, and the issuing warps of two tiles no longer wait for one ring. Past two tiles per SM, back to back for half
+// a second (causal; pairs -> narrow):
+//   D = 64, any length: 8 x 32 x 512 34.0 -> 29.7 us, 8 x 32 x 1024 84.1 -> 76.5, 4 x 16 x 2048 68.4 -> 62.5, 1 x 16 x
+//   8192 210 -> 194; paged 8 x 32 x 1024 100.4 -> 91.2, biased 8 x 16 x 512 38.1 -> 33.9.
+//   D = 128 up to 24 blocks a tile: 8 x 64 x 100 23.1 -> 13.3, 8 x 32 x 640 59.0 -> 51.6, 8 x 32 x 1024 105.4 -> 101.7,
+//   4 x 32 x 1536 103.5 -> 101.7, biased 4 x 16 x 1024 69.5 -> 64.4; windows of 64 to 1300 0.85 to 0.97 of pairs (also where
+//   the last tile sees no key: the rule looks at that one alone). Further on the chip runs at its power limit and
 //   K and V read once for both tiles count for more: chunks of 1024 with 4000 keys before them 158.8 -> 160.9,
 //   1 x 32 x 8192 444.6 -> 453.7; but for heads of which pairs leave a good part of the slots empty. Three tiles a head
 //   (a quarter empty): 456 tiles of 2500 / 4200 / 8200 keys 112 -> 99, 181 -> 161, 350 -> 305, 2592 of them 0.91 to 0.92 of
@@ -1594,6 +1601,7 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
   using Shape = PrefillShape<D, PE, NARROW>;
   constexpr size_t smem = Shape::kSmem;
   static_assert(smem <= 232448 && (!NARROW || 2 * (smem + 1024) <= 233472), "shared memory of a CTA");
+  static_assert(keeps_tensor_memory(smem, NARROW), "tensor memory of an SM");
   static thread_local int configured_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1652,22 +1660,22 @@ static std::atomic<unsigned int> g_next_ticket_slot{0};
 // Whether the fixed-reference kernel runs as two CTAs of one tile slot per SM (narrow) instead of one of two. The slots
 // then no longer share a ring and an item's end, and a tile that has an SM to itself has all of it; but every tile
 // fetches its own K and V. Both back to back for half a second, softcap 50 (two slots -> narrow):
-//   D = 64, always: 8 x 32 x 1024 79.7 -> 76.7 us, 2 x 16 x 4096 142.6 -> 129.4, 2 x 4 x 512 14.3 -> 12.3, window 256,
-//   four heads per kv head, 8 x 32 x 2048 87.7 -> 87.2, 1 x 8 x 2048 12.3 -> 10.3;
-//   D = 128, no more tiles than SMs: 1 x 8 x 2048 38.5 -> 30.6, 2 x 8 x 1024 24.4 -> 19.7; up to 10 blocks a tile:
-//   8 x 64 x 256 30.7 -> 28.7, 8 x 32 x 512 41.7 -> 40.1, 8 x 16 x 600 32.8 -> 30.8; up to 16 and four tiles per SM:
-//   2 x 32 x 700 26.9 -> 24.6, 4 x 16 x 1024 36.3 -> 35.1; beyond, the chip's power limit decides and K and V read
-//   once for two tiles win (8 x 32 x 1024 107.4 -> 108.5, 8 x 32 x 2048 338.7 -> 346.6, 1 x 8 x 8192 175.1 -> 180.0);
-//   ... unless a head has one tile: it then has an SM to itself in either form, and the deeper ring of the two-slot
-//   form holds its keys' latency better (8 to 148 tiles of 1000 keys 18.5 -> 19.3 to 22.6 -> 24.7, of 4000 52 -> 63, 148 of
-//   8000 117 -> 146);
-//   between one and two tiles per SM as in prefill_kernel: narrow where pairs need a second round (three tiles a head,
-//   294 in all, D = 128 0.78, D = 64 3000 keys 0.63), two slots where an odd number of tiles leaves the longest one alone
-//   (180 to 240 tiles, three a head 1.00 to 1.16; 200 to 240, five 1.00 to 1.12, seven 1.00 to 1.10), for seven causal tiles a head also
-//   past 148 pairs, the light ones of which then take two turns under the longest (1.03), and for two tiles a head at
-//   D = 128 (256 rows x 128 heads 12.4 against 13.1 us; 1.00 to 1.08);
+//   D = 64: 8 x 32 x 1024 78.9 -> 76.9 us, 2 x 16 x 4096 142.0 -> 129.6, 2 x 4 x 512 14.5 -> 12.3, window 256, four heads
+//   per kv head, 8 x 32 x 2048 87.7 -> 87.2, 1 x 8 x 2048 12.3 -> 10.3;
+//   D = 128, no more tiles than SMs: 1 x 8 x 2048 38.4 -> 30.7, 2 x 8 x 1024 23.9 -> 19.1; unless a head has one tile, which
+//   has an SM to itself in either form, where the deeper ring of the two-slot form holds its keys' latency better (8 to
+//   148 tiles of 1000 keys 18.5 -> 19.3 to 22.6 -> 24.7, of 4000 52 -> 63, 148 of 8000 117 -> 146);
+//   up to 10 blocks a tile: 8 x 64 x 256 30.7 -> 28.9, 8 x 32 x 512 41.9 -> 40.3, 8 x 16 x 600 32.7 -> 31.0; up to 16 and
+//   four tiles per SM: 2 x 32 x 700 26.7 -> 24.5, 4 x 16 x 1024 35.8 -> 35.2; beyond, the chip's power limit decides and K
+//   and V read once for two tiles win (8 x 32 x 1024 108.1 -> 109.1, 8 x 32 x 2048 338.7 -> 346.6, 1 x 8 x 8192 175.1 ->
+//   180.0);
+//   between one and two tiles per SM, at either head size: narrow where pairs need a second round (three tiles a head,
+//   294 in all, D = 128 0.78, D = 64 over 3000 keys 0.63), two slots where an odd number of tiles leaves the longest one
+//   alone (180 to 240 tiles, three a head 1.00 to 1.16; 200 to 240, five 1.00 to 1.12, seven 1.00 to 1.10), for seven causal
+//   tiles a head also past 148 pairs, the light ones of which then take two turns under the longest (1.03), and for two
+//   tiles a head at D = 128 (256 rows x 128 heads 12.4 against 13.1 us; 1.00 to 1.08);
 //   D = 128 packed, up to four chunks per SM (1 x 8 x 2048, window 256 14.4 -> 12.3; 2 x 16 x 2048, window 1000
-//   45.2 -> 42.8; 8 x 32 x 2048, window 256 121.3 -> 124.3).
+//   45.1 -> 43.2; 8 x 32 x 2048, window 256 121.3 -> 124.3).
 static bool bounded_is_narrow(const PrefillParams& p, int D, int pack, int B, int sm_count) {
   if (p.sm_margin > 0) return false;  // (two CTAs per SM would spread over the SMs to be left free)
   if (D == 64 && pack > 1) return true;
@@ -1709,6 +1717,7 @@ static int launch_prefill_bounded(const CUtensorMap& mq, const CUtensorMap& mk,
   using Shape = BoundedShape<D, PACK, NARROW>;
   constexpr size_t smem = Shape::kSmem;
   static_assert(smem <= 232448 && (!NARROW || 2 * (smem + 1024) <= 233472), "shared memory of a CTA");
+  static_assert(keeps_tensor_memory(smem, NARROW), "tensor memory of an SM");
   static thread_local int configured_dev = -1;
   static thread_local unsigned int* tickets = nullptr;
   int dev = 0;

@@ -4,7 +4,8 @@
 // Softcap gives logit2 = c2 * tanh(a * raw) with |logit2| <= c2; when c2 <= 80, exp2(logit2) can
 // be taken against the fixed reference 0 instead of a running row max. Then the blocks of a row
 // are independent, O is never rescaled, and a row can be split between two threads with nothing
-// to exchange but the final row sum. 672 threads:
+// to exchange but the final row sum. 672 threads (the narrow form, of one tile slot and two CTAs per SM, has half of
+// each role, one producer and a warp to spare: 384):
 //   warps 0-7   softmax for query tile 0: two threads per score row, 32 columns of a block each
 //   warps 8-15  softmax for query tile 1
 //   warp  16    TMA producer and item dispatcher
@@ -16,7 +17,7 @@
 // each 32-column half of its S buffer (each thread stores over its own scores).
 //
 // One CTA per SM walks a queue of work items (one item = two consecutive query tiles of one
-// (batch, head)), taken from a ticket counter in the launch order of the non-persistent grid
+// (batch, head); narrow: two CTAs, one tile), taken from a ticket counter in the launch order of the non-persistent grid
 // (the query-tile pairs of one head next to each other, heaviest first, so that they run at the
 // same time on different SMs and share K/V through L2). Nothing drains between items:
 //   - the K/V ring just continues with the next item's tiles;
@@ -49,7 +50,7 @@ struct __align__(8) BoundedBarriers {
   uint64_t o_free[2];      // [tile] epilogue has read O_t (one arrival per warp)
   uint64_t l_ready[2];     // [tile] both halves of every row sum are published
   uint64_t item_full[kItemSlots];   // producer -> everybody: item published
-  uint64_t item_empty[kItemSlots];  // 4 MMA threads + 16 softmax warps have read it
+  uint64_t item_empty[kItemSlots];  // the MMA threads and softmax warps (4 + 16; narrow: 2 + 8) have read it
   uint32_t tmem_base;
   uint32_t pad;
 };
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(BoundedShape<D, PACK, NARROW>::kThreads, NARRO
   static_assert(sizeof(ItemGeom) == 48, "three 16-byte pieces");
   ItemGeom* item_slots =
       reinterpret_cast<ItemGeom*>(smem + ((sizeof(BoundedBarriers) + 15) & ~size_t(15)));
-  unsigned char* sStage = smem + 1024;  // 16 x 2 KB output staging (one buffer per softmax warp)
+  unsigned char* sStage = smem + 1024;  // output staging, a buffer per softmax warp (kWarpStage)
   unsigned char* sQ = sStage + kSoftmaxWarps * kWarpStage;
   unsigned char* sKV = sQ + kSlots * kQTileBytes;
 
@@ -343,8 +344,8 @@ __global__ void __launch_bounds__(BoundedShape<D, PACK, NARROW>::kThreads, NARRO
     }
   } else if (warp >= kMmaWarp0 && warp < kMmaWarp0 + 2 * kSlots) {
     // ---------------- MMA issuers: a PV thread and a QK^T thread per query tile ----------
-    // All four threads walk every ring stage and each releases it (kv_empty counts four
-    // arrivals) once the MMAs it issued from the stage, if any, are complete. A thread must see
+    // All of them walk every ring stage and each releases it (kv_empty counts two arrivals per
+    // tile slot) once the MMAs it issued from the stage, if any, are complete. A thread must see
     // a stage full before it releases it: that keeps its arrivals one per phase.
     // The whole warp runs the loop (every lane waits on the barriers); the elected lane alone
     // issues MMAs and commits. A warp that has diverged into a single-lane branch gets far fewer
@@ -588,9 +589,12 @@ __global__ void __launch_bounds__(BoundedShape<D, PACK, NARROW>::kThreads, NARRO
           // share: next to scalar fp32 at one instruction per clock a tcgen05.mma goes out every 122
           // to 180 clocks instead of every 65 (two to four arithmetic warps per scheduler), next to
           // the packed forms, which take two clocks of their pipe each, every 65. The short polynomial
-          // is therefore packed (9 instructions per pair instead of 12; the same roundings): causal
-          // 8 x 32 x 2048 D = 128 525 -> 513 thousand clocks, 345 -> 341 us under the power cap; window
-          // 256, four heads per kv head, 205 -> 197 thousand, 124.7 -> 122.4 us.
+          // is therefore packed (9 instructions per pair instead of 12; the same roundings, but that the packed
+          // forms keep subnormal numbers, which the scalar ones flush): causal 8 x 32 x 2048 D = 128 529 ->
+          // 512 thousand clocks, 343.4 -> 339.0 us under the power cap; window 256, four heads per kv head,
+          // 204 -> 196 thousand, 123.9 -> 121.6 us. (In the two-slot forms at D = 128 a warp has no register
+          // left: 20 bytes spilled, 12 and 8 packed, instead of 8, 0 and 0. 64-bit coefficients in the
+          // parameters instead of pack2 change nothing.)
           auto body = [&](auto path_tag, bool apply_mask) {
             constexpr int kPath = decltype(path_tag)::value;
 #pragma unroll

@@ -2,6 +2,10 @@
 CTA, one tile split over the two slots of a CTA (running-max kernel, no more tiles than SMs), or two CTAs
 per SM. Every kind of call on the two-CTA side of the rules, at the edges of tiles, against another form of
 the same call and against fp32."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -140,6 +144,37 @@ def test_two_ctas_per_sm_paged(which, Sq, Skv, P, heads_first, D):
     out = F.prefill_attention(q, *given, status=st, **kw)
     F.check_status(st)
     _close(out, _fp32(q, *dense, S.MASK_CAUSAL, Skv - Sq))
+
+
+FIRST_IN_CAPTURE = """
+import torch
+from loopfuse_b200 import functional as F, spec as S
+cap = [S.ScoreMod(S.MOD_DIV, 50.0), S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_MUL, 50.0)]
+mk = lambda h, n: [torch.randn(1, h, n, 128, device="cuda").bfloat16() for _ in range(3)]
+bias = lambda h, n: dict(score_bias=torch.randn(1, h, n, n, device="cuda").bfloat16())
+for mods, with_bias, first, second in (([], False, (8, 512), (128, 512)), ([], True, (8, 512), (128, 512)),
+                                       (cap, False, (40, 2048), (8, 512))):
+    calls = []
+    for h, n in (first, second):
+        kw = dict(scale=128 ** -0.5, mask_kind=S.MASK_CAUSAL, mods=mods, **(bias(h, n) if with_bias else {}))
+        calls.append((mk(h, n), kw))
+    (a, kwa), (b, kwb) = calls
+    assert F.prefill_form(*a, **kwa) != "narrow" and F.prefill_form(*b, **kwb) == "narrow"
+    F.prefill_attention(*a, **kwa)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = F.prefill_attention(*b, **kwb)
+    g.replay()
+    assert torch.equal(out, F.prefill_attention(*b, **kwb))
+"""
+
+
+def test_a_form_can_be_first_used_inside_a_capture():
+    """A program that has called a kernel once, and then captures a call of another size."""
+    root = str(Path(__file__).resolve().parents[1])
+    r = subprocess.run([sys.executable, "-c", FIRST_IN_CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 SOFTCAP = [S.ScoreMod(S.MOD_DIV, 30.0), S.ScoreMod(S.MOD_TANH), S.ScoreMod(S.MOD_MUL, 30.0)]
