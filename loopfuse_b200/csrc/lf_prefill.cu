@@ -356,9 +356,10 @@ __global__ void __launch_bounds__(PrefillShape<D, PE, NARROW>::kThreads, NARROW 
   const uint32_t tmem_base = bars->tmem_base;
   pdl_wait();  // (so far only the producer warp, which waited itself, has touched global memory)
 
-  // Two CTAs of 256 threads have 128 registers per thread: 184 for the softmax warps (below), 72 for the others; 4 x 184 +
-  // 4 x 72 = 8 x 128. setmaxnreg has to be one instruction for all warps of a warpgroup, so it stands in front of the
-  // dispatch of roles, on a condition that is the same in all four.
+  // Two CTAs of 256 threads have 128 registers per thread: 184 for the softmax warps, 72 for the others; 4 x 184 +
+  // 4 x 72 = 8 x 128. setmaxnreg has to be one instruction for all warps of a warpgroup, so this one stands in front
+  // of the dispatch of roles, on a condition that is the same in all four; the other is the first of the softmax
+  // branch, which is that warpgroup's alone. (With both in front the compiler gives every warp 72: up to 1 KB spilled.)
   if constexpr (NARROW) {
     if (warp >= kSoftmaxWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   }
